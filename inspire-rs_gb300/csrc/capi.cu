@@ -116,15 +116,15 @@ struct HostChaCha {
 
 namespace {
 
-// Build the client key table into m from y_body or y_all.  From y_body at
-// gamma = 16 the table holds NTT(y_body) only (48 KiB, the Respond kernel
-// forms each rotation in registers); from an explicit y_all, or at smaller
-// gamma, all (gamma-1)*ELL rotated polys.  sync: wait for the build here
-// (otherwise the launches that use the table follow on the same stream).
+// Build the client key table into m from y_body or y_all.  From y_body the
+// table holds NTT(y_body) only (48 KiB, the Respond kernels form each
+// rotation as they read); from an explicit y_all all (gamma-1)*ELL rotated
+// polys.  sync: wait for the build here (otherwise the launches that use the
+// table follow on the same stream).
 int build_key_table(inspire_ctx* c, const uint64_t* y_body, const uint64_t* y_all, DevMem& m, bool& body_form,
                     bool sync) {
   const int gamma = c->gamma;
-  body_form = !y_all && gamma == MAX_GAMMA;
+  body_form = !y_all && gamma > 1;
   const size_t tbl_words = (size_t)std::max(1, body_form ? ELL : (gamma - 1) * ELL) * poly_words();
   if (m.ensure(tbl_words * sizeof(uint32_t)) != cudaSuccess)
     return fail(INSPIRE_ERR_OUT_OF_MEMORY, alloc_failure(c, "client key table allocation"));
@@ -140,11 +140,9 @@ int build_key_table(inspire_ctx* c, const uint64_t* y_body, const uint64_t* y_al
     memcpy(c->h_keys.p, y_all ? y_all : y_body, in_bytes);
     CUDA_TRY(cudaMemcpyAsync(c->d_keys.p, c->h_keys.p, in_bytes, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaEventRecord(c->keys_ev, c->stream));
-    CUDA_TRY(y_all ? launch_client_from_yall(c->P, c->d_keys.as<uint64_t>(), m.as<uint32_t>(), c->stream)
-                   : launch_client_from_ybody(c->P, c->d_keys.as<uint64_t>(), m.as<uint32_t>(),
-                                              body_form ? 1 : gamma - 1, c->stream));
+    CUDA_TRY(launch_client_keys_ntt(c->P, c->d_keys.as<uint64_t>(), (int)in_polys, m.as<uint32_t>(), c->stream));
     // the Respond kernel multiplies the third key by R_{i+1} instead of NTT(d2)
-    CUDA_TRY(launch_fold_third_digit(c->P, m.as<uint32_t>(), body_form ? 1 : gamma - 1, c->stream));
+    CUDA_TRY(launch_fold_third_digit(c->P, m.as<uint32_t>(), m.as<uint32_t>(), (int)in_polys / ELL, false, c->stream));
     if (sync) CUDA_TRY(cudaStreamSynchronize(c->stream));
   }
   return INSPIRE_OK;
@@ -726,8 +724,7 @@ int inspire_crs_load(inspire_ctx* c, const uint8_t w_seed[32], uint32_t num_colu
   CUDA_TRY(c->what.ensure(sizeof(uint32_t) * (size_t)std::max(1, (gamma - 1) * ELL) * 2 * N));
   CUDA_TRY(launch_crs_what(c->P, c->wmask.as<uint32_t>(), c->what.as<uint32_t>(), c->stream));
   CUDA_TRY(c->what3.ensure(c->what.bytes));
-  CUDA_TRY(cudaMemcpyAsync(c->what3.p, c->what.p, c->what.bytes, cudaMemcpyDeviceToDevice, c->stream));
-  CUDA_TRY(launch_fold_third_digit(c->P, c->what3.as<uint32_t>(), gamma - 1, c->stream));
+  CUDA_TRY(launch_fold_third_digit(c->P, c->what.as<uint32_t>(), c->what3.as<uint32_t>(), gamma - 1, true, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   // key tables of registered clients were built for the previous gamma
   for (size_t i = 0; i < c->clients.size(); i++) release_keys(c, (int32_t)i);

@@ -49,13 +49,13 @@ struct RespondArgs {
   const uint64_t* brows;         // [nq][ELL][2][N] b-polys of rows ELL..2ELL-1
   const int32_t* client;         // [nq] client id
   // [nclients] -> client key table: [(gamma-1)][ELL][2][N] rotated keys,
-  // or, when the pointer's bit 0 is set (gamma = 16 only), the body table
-  // [ELL][2][N] whose rotations the kernel forms; third digit folded in
+  // or, when the pointer's bit 0 is set, the body table [ELL][2][N] whose
+  // rotations the kernel forms; rows [h][x], third digit folded in
   const uint32_t* const* yhat_table;
   int nclients, nshards;
-  const uint32_t* E;             // [nshards][2][gamma][ELL][N] contracted database, by recursion step
+  const uint32_t* E;             // [nshards][2][gamma][ELL][N] contracted database, by recursion step, quads
   const uint16_t* H;             // [nshards][gamma][N] raw 16-bit columns
-  const uint32_t* what;          // [(gamma-1)][ELL][2][N] rotated w_mask (CRS), third digit folded in
+  const uint32_t* what;          // [(gamma-1)][ELL][2][N] rotated w_mask (CRS), quads, third digit folded in
   uint64_t* out;                 // [nq][2][2][N] response (a_hat, b) residues
   int* status;                   // [nq]
   // Serving loop: per-query descriptors in device memory (override shard,
@@ -176,7 +176,7 @@ cudaError_t launch_client_keys(const KeyGenArgs& a, int n, cudaStream_t st);
 size_t nopacking_smem_bytes();
 cudaError_t launch_nopacking(const NoPackingArgs& a, bool seeded, cudaStream_t st);
 
-size_t respond_smem_bytes(int mode, bool qdb);
+size_t respond_smem_bytes(int mode);
 // max_ctas > 0 caps the grid: each CTA then answers several queries in turn.
 // Otherwise batches of at most pair_max queries run on the two-CTA cluster
 // kernel (respond_pair.cu), larger ones on the one-CTA kernel.
@@ -192,16 +192,16 @@ cudaError_t launch_encode_E(const DevParams& P, const uint16_t* H, int nshards, 
                             cudaStream_t st);
 cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t* what,
                             cudaStream_t st);
-// Fold the third gadget digit into ngroups key triples [g][k<3][2][N] in
-// place (k0 - z^-2 k2, k1 - z^-1 k2, n z^-2 k2): the Respond kernel then
-// multiplies the third key by R_{i+1} instead of by NTT(d2).
-cudaError_t launch_fold_third_digit(const DevParams& P, uint32_t* tbl, int ngroups, cudaStream_t st);
-// The first nrot rotations y_all[0..nrot) of the client key table (nrot =
-// gamma - 1: the full table; 1: the body table the Respond kernel rotates).
-cudaError_t launch_client_from_ybody(const DevParams& P, const uint64_t* ybody, uint32_t* yhat, int nrot,
-                                     cudaStream_t st);
-cudaError_t launch_client_from_yall(const DevParams& P, const uint64_t* yall, uint32_t* yhat,
+// Fold the third gadget digit into ngroups key triples [g][k<3][2][N]
+// (k0 - z^-2 k2, k1 - z^-1 k2, n z^-2 k2): the Respond kernel then multiplies
+// the third key by R_{i+1} instead of by NTT(d2).  In place, or (quads) from
+// slot order into the order that the Respond kernels read the CRS keys in.
+cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, bool quads,
                                     cudaStream_t st);
+// NTT of a client's key polys [npolys][2][N] (y_body: ELL polys, whose
+// rotations the Respond kernels form; or an explicit y_all).
+cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, uint32_t* yhat,
+                                   cudaStream_t st);
 
 // kernel-level operations
 // decrypt + extract_inspiring of n responses ct[n][2][2][N] (u64) with the

@@ -1,4 +1,5 @@
-// respond.cu -- fused InsPIRe^2 Respond kernel: one CTA per query.
+// respond.cu -- fused InsPIRe^2 Respond kernel: one CTA of 256 threads per
+// query, two CTAs per SM.
 //
 // Computes, for one seeded query against one resident shard, exactly what
 // respond_seeded_inspiring / respond_inspiring (src/pir/respond.rs:284-398)
@@ -11,192 +12,386 @@
 //    every digit of its zero a-part is 0 (rgsw/external_product.rs:122-147).
 //  * b-part of each column product, coefficient 0 only
 //    (rlwe/enc.rs:195-208): b0_c = sum_t sum_i d_{c,t}[i] * b'_t[i] with
-//    d = base-2^20 digits of Delta*h and b'_t the negacyclic reversal of row
+//    d = base-2^20 digits of Delta*h_c and b'_t the negacyclic reversal of row
 //    ELL+t's b, accumulated exactly in 64 bits.
 //  * a-part + the first stage of packing_offline (inspiring2.rs:948-982): the
 //    per-slot 16x16 monomial inner products, the 1/gamma scaling and the 16
 //    NTT-domain automorphisms reduce to a length-gamma DFT per NTT slot, which
 //    is folded into the resident database ("E", built in setup.cu); per slot
-//    only sum_t E[k,t][u] * A_t[u] remains.
+//    only sum_t E[i,t][s] * A_t[tau_i(s)] remains.
 //  * the backward recursion (inspiring2.rs:984-1008) and packing_online run
 //    interleaved: each T[i][k] NTT is multiplied into R[i] with the CRS key
-//    w_all and into the b accumulator with the client key y_all.
+//    w_all and into the b accumulator with the client key y_all, the third
+//    gadget digit folded into the keys (fold_third_digit_kernel, setup.cu).
 //
-// Layout: 768 threads = six groups of 128, group g = 3 r + k owns CRT residue
-// r and gadget digit k.  Per recursion step, groups (r,0) run the inverse NTT
-// while groups (r,1),(r,2) scatter the query-only term R_i; then the three
-// digit NTTs of each residue run concurrently.  All intermediate state lives
-// in shared memory and registers, and no global scratch is used: device-row
-// launches take the b side from bside_kernel, which parks it in the last
-// 128 bytes of each query's response slot.
+// Layout.  Group r of 128 threads owns CRT residue r, thread x of it the 16
+// NTT slots 16x .. 16x+15 of every polynomial.  The automorphisms tau_{g^i}
+// (g = 2N/gamma + 1) permute slots only inside such runs (rot_rows,
+// respond_common.cuh), so a recursion step is private to its thread in the
+// NTT domain: R_{i+1} and the b accumulator stay in registers, the row
+// transforms (AH) in words of shared memory that no other thread reads, and
+// the nine products of a slot share two Montgomery reductions.  Threads meet
+// only in the transforms' exchanges and, warp to warp, where the composite
+// coefficient needs both residues:
+//   [A] INTT(R_{i+1}) in registers;
+//   [B] the residues swapped through shared memory, digits d0, d1 of the
+//       composite coefficients computed by both groups (64-thread barrier);
+//   [C] NTT(d0), NTT(d1) together (one set of twiddle loads);
+//   [D] R_i = sum_t E A_t + NTT(d0) w'0 + NTT(d1) w'1 + R_{i+1} w'2,
+//       b += NTT(d0) y'0 + NTT(d1) y'1 + R_{i+1} y'2.
+// Three barriers a step, each over one group or one pair of warps.
+//
+// What bounds it: the integer multiply-add pipe (64 lane-operations per
+// cycle and SM, a high or wide product costs two) and, with 16 warps per SM,
+// the latency between dependent operations: IPC 2.15.  One call of 2048
+// queries takes 1507 us; the six-group kernel this one replaced (768 threads,
+// one CTA per SM, four CTA-wide barriers a step, its 24 warps in step with
+// one another, the b side in a launch of its own) took 2290 us, and 174
+// against 154 us for 128 queries (fewer queries than SMs).  Two CTAs of
+// different queries share the SM without waiting for each other, and 128
+// registers a thread let each warp keep 16 independent butterflies in flight.
 #include "expand.cuh"
 #include "kernels.h"
+#include "ntt_joint.cuh"
 #include "respond_common.cuh"
 
 namespace ig {
 
 namespace {
 
-// b0_c for every column c and residue (see file comment).  rows holds the
-// query's rows ELL..2ELL-1 (b polys, u64; device memory or staged in shared
-// memory); bp (6N words) is scratch; bpoly[r * 16 + c] receives the result.
-// Warp c handles column c:
-// lane l takes the coefficient pairs i = 2 (l + 32 m) + {0, 1}, reading the
-// raw column as u32 pairs and the staged rows as 64-bit words, so every
-// shared-memory read of a warp covers 256 contiguous bytes (no bank
-// conflicts).  Each lane issues its column loads 16 at a time, so the column
-// costs two memory latencies.
-template <int NT>
-__device__ void column_b0(const DevParams& P, const uint16_t* __restrict__ H, const uint64_t* rows, uint32_t* bp,
-                          uint32_t* bpoly) {
-  const int tid = threadIdx.x, gamma = P.gamma;
-  const int lane = tid & 31, c = tid >> 5;
-#pragma unroll 8
-  for (int idx = tid; idx < ELL * 2 * N; idx += NT) {
-    const int i = idx & (N - 1), tr = idx >> LOGN, r = tr & 1;
-    uint32_t v = (uint32_t)rows[(size_t)tr * N + (i == 0 ? 0 : N - i)];
-    if (i != 0 && v != 0) v = P.r[r].q - v;
-    bp[idx] = v;
-  }
-  __syncthreads();
-  if (c < gamma) {
-    const uint32_t* h2 = reinterpret_cast<const uint32_t*>(H + (size_t)c * N);
-    const uint2* b2 = reinterpret_cast<const uint2*>(bp);
-    uint64_t acc0 = 0, acc1 = 0;
-#pragma unroll 1
-    for (int m0 = 0; m0 < N / 64; m0 += 16) {
-      uint32_t hw[16];
-#pragma unroll
-      for (int m = 0; m < 16; m++) hw[m] = __ldg(h2 + lane + 32 * (m0 + m));
-#pragma unroll
-      for (int m = 0; m < 16; m++) {
-        const int j = lane + 32 * (m0 + m);  // pair index: coefficients 2j, 2j + 1
-        const uint2 b00 = b2[0 * (N / 2) + j], b01 = b2[1 * (N / 2) + j];  // digit 0: residue 0, 1
-        const uint2 b10 = b2[2 * (N / 2) + j], b11 = b2[3 * (N / 2) + j];  // digit 1
-        const uint2 b20 = b2[4 * (N / 2) + j], b21 = b2[5 * (N / 2) + j];  // digit 2
-#pragma unroll
-        for (int e = 0; e < 2; e++) {
-          const uint64_t xv = P.delta * (uint64_t)((hw[m] >> (16 * e)) & 0xFFFFu);
-          const uint32_t d0 = (uint32_t)xv & 0xFFFFFu, d1 = (uint32_t)(xv >> 20) & 0xFFFFFu,
-                         d2 = (uint32_t)(xv >> 40);
-          acc0 += (uint64_t)d0 * (e ? b00.y : b00.x) + (uint64_t)d1 * (e ? b10.y : b10.x) +
-                  (uint64_t)d2 * (e ? b20.y : b20.x);
-          acc1 += (uint64_t)d0 * (e ? b01.y : b01.x) + (uint64_t)d1 * (e ? b11.y : b11.x) +
-                  (uint64_t)d2 * (e ? b21.y : b21.x);
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      acc0 += __shfl_down_sync(0xffffffffu, acc0, o);
-      acc1 += __shfl_down_sync(0xffffffffu, acc1, o);
-    }
-    if (lane == 0) {
-      bpoly[c] = (uint32_t)(acc0 % P.r[0].q);
-      bpoly[16 + c] = (uint32_t)(acc1 % P.r[1].q);
-    }
-  }
-  __syncthreads();
-}
+constexpr int QT = 256;  // threads per query
 
-// Device-row launches compute the b side in a launch of their own
-// (bside_kernel, 512 threads and 48 KiB of shared memory per query, so many
-// queries' loads are in flight per SM) and park each query's 32 b0 values in
-// the last 128 bytes of its response, which the Respond kernel reads at its
-// start and overwrites with the response at its end.
-constexpr int BSIDE_THREADS = 512;
-__device__ __forceinline__ uint32_t* b_parking(uint64_t* out, int qi) {
-  return reinterpret_cast<uint32_t*>(out + (size_t)qi * 4 * N + 4 * N - 16);
-}
-
-__global__ void __launch_bounds__(BSIDE_THREADS) bside_kernel(const __grid_constant__ RespondArgs A) {
-  extern __shared__ __align__(16) uint32_t sm[];  // [ELL][2][N] staged rows, then bpoly[32]
-  const int qi = blockIdx.x;
-  const uint32_t shard = A.shard[qi];
-  if (shard >= (uint32_t)A.nshards) return;  // the Respond kernel reports it
-  uint32_t* bpoly = sm + ELL * 2 * N;
-  if (threadIdx.x < 32) bpoly[threadIdx.x] = 0;  // columns past gamma
-  column_b0<BSIDE_THREADS>(A.P, A.H + (size_t)shard * A.P.gamma * N, A.brows + (size_t)qi * ELL * 2 * N, sm, bpoly);
-  if (threadIdx.x < 32) b_parking(A.out, qi)[threadIdx.x] = bpoly[threadIdx.x];
-}
-
-// Shared-memory layout in u32 words (NR = residues of the a side).  With the
-// 1 KiB every CTA reserves, the device-row variant (163 KiB) fills the SM's
-// 164 KiB configuration and the serving variant (195 KiB) its 196 KiB one,
-// so the SM keeps 92 or 60 KiB of L1, which holds the transforms' twiddle
-// tables.  Each residue's b accumulator is the scratch of its group (r,2),
-// which runs no transform during the recursion (words [0, N)); words
-// N..N+15 of it keep the residue's b side (bpoly) until the outputs.
-template <int NR, bool QDB>
+// Shared memory in u32 words (NR = residues of the a side).  80 KiB and a
+// little: two CTAs fit the SM's 164 KiB configuration, which leaves it 92 KiB
+// of L1 for the twiddles and the client keys.
+template <int NR>
 struct Smem {
-  static constexpr int AHAT = 0;                    // [ELL][NR][N] row transforms
-  static constexpr int SC = AHAT + ELL * NR * N;    // [RG][NTT_SCRATCH] per-group exchange scratch
-  static constexpr int T = SC + RG * NTT_SCRATCH;   // [2][N] R_{i+1} (slots) -> its inverse (coefficients) -> digits d0, d1
-  static constexpr int PB1 = T + 2 * N;             // [2][N] NTT(d1) w'[i][1]
-  static constexpr int SCAT = PB1 + 2 * N;          // [2 steps][2][N] query-only term of R_i (slots), then partial R_i
-  // T..T+6N also hold the unseeded rows' a parts and SCAT+2N.. the
-  // expansion's workspace ws[3][20] (device rows).  The serving variant
-  // stages the query's raw b rows (u64, 12N words) from T on until the b
-  // side, and keeps ws[3][20], the staged seeds (96 B) and the rows'
-  // mbarrier in MISC, the words of SC past the expansion's candidates (6N
-  // words), until the row transforms reuse them
-  static constexpr int MISC = QDB ? SC + 6 * N : SCAT + 4 * N;
-  static constexpr int TOTAL = QDB ? T + 12 * N : SCAT + 4 * N;
-  static_assert(!QDB || MISC + 128 <= SC + 5 * NTT_SCRATCH + N, "MISC stays clear of the b side's words");
+  static constexpr int AH = 0;                 // [ELL][NR][16 rows h][128] row transforms
+  static constexpr int XC = AH + ELL * NR * N; // [4][N] exchange buffers: 2 shared by turns, 1 per residue
+  static constexpr int WS = XC + 4 * N;        // [2][8] scan totals, [3] expansion totals, flags
+  static constexpr int BP = WS + 32;           // [2][16] the b side
+  static constexpr int SEED = BP + 32;         // [ELL * 8] staged seeds (serving loop)
+  static constexpr int BAR = SEED + 24;        // the staged rows' mbarrier
+  static constexpr int TOTAL = BAR + 8;
 };
 
-// Slots of the next step's query-only term computed by group (r,2) in [A];
-// the rest follow in [C].
-constexpr int SCATTER_SPLIT = N / 8;
+// Serving loop: the query's b rows (u64) are staged in four chunks, one after
+// the other in the exchange buffers.  Chunk m covers coefficients i in
+// [512 m, 512 m + 512) of the reversed rows, i.e. row words N - i: words
+// 512 (3 - m) .. and one pair more (for m = 0 that pair is words 0, 1).
+constexpr int CH = 512;
+constexpr int CHW = CH + 2;  // u64 words of one polynomial's chunk
+static_assert(2 * ELL * CHW * 8 <= 4 * N * 4, "a chunk fits the exchange buffers");
+
+__device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows, int m, uint64_t* bar) {
+  mbar_expect_tx(bar, 2 * ELL * CHW * 8);
+  const int k0 = N - CH * (m + 1);
+#pragma unroll 1
+  for (int p = 0; p < 2 * ELL; p++) {
+    uint64_t* d = dst + p * CHW;
+    const uint64_t* s = brows + (size_t)p * N;
+    if (m == 0) {
+      bulk_g2s(d, s + k0, CH * 8, bar);
+      bulk_g2s(d + CH, s, 16, bar);
+    } else {
+      bulk_g2s(d, s + k0, CHW * 8, bar);
+    }
+  }
+}
+
+// Exclusive rank of this thread's `cnt` over the CTA, total of all threads.
+// ws: 8 ints of this call's own (reused two calls later at the earliest).
+__device__ __forceinline__ int scan_cta(int cnt, int* ws, int& total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) ws[warp] = incl;
+  __syncthreads();
+  int base = 0;
+  total = 0;
+#pragma unroll
+  for (int w = 0; w < QT / 32; w++) {
+    const int t = ws[w];
+    if (w < warp) base += t;
+    total += t;
+  }
+  return base + incl - cnt;
+}
+
+__device__ __forceinline__ int scan_warp(int cnt, int& total) {
+  const int lane = threadIdx.x & 31;
+  int incl = cnt;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  total = __shfl_sync(0xffffffffu, incl, 31);
+  return incl - cnt;
+}
+
+__device__ __forceinline__ void load_key(const uint8_t* seed, uint32_t key[8]) {
+  const uint32_t* s = reinterpret_cast<const uint32_t*>(seed);
+  if ((reinterpret_cast<uintptr_t>(seed) & 3) == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; i++) key[i] = s[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      key[i] = (uint32_t)seed[4 * i] | ((uint32_t)seed[4 * i + 1] << 8) | ((uint32_t)seed[4 * i + 2] << 16) |
+               ((uint32_t)seed[4 * i + 3] << 24);
+  }
+}
+
+// The eight draws of one keystream block under gen_range(0..q): bit k of the
+// mask is set if draw k is accepted, val[k] its value.  zone = (q << lz) - 1
+// has 32 low ones (q < 2^32), so lo64(v q) <= zone is decided by the high
+// words.
+__device__ __forceinline__ unsigned draw8(const uint32_t w[16], uint32_t q, uint32_t zone_hi, uint32_t val[8]) {
+  unsigned mask = 0;
+#pragma unroll
+  for (int k = 0; k < 8; k++) {
+    const uint64_t hi = (uint64_t)w[2 * k + 1] * q + __umulhi(w[2 * k], q);
+    val[k] = (uint32_t)(hi >> 32);
+    mask |= ((uint32_t)hi <= zone_hi ? 1u : 0u) << k;
+  }
+  return mask;
+}
+
+__device__ __forceinline__ void put_draws(uint32_t* dst, int p, unsigned mask, const uint32_t val[8]) {
+#pragma unroll
+  for (int k = 0; k < 8; k++)
+    if ((mask >> k) & 1u) {
+      if (p < N) dst[p] = val[k];
+      p++;
+    }
+}
+
+// One row by the general routine (256-thread sub-block), for streams that
+// reject more draws than the fast path allows for.
+template <int NR>
+__device__ __noinline__ bool expand_row_general(const DevParams& P, const uint8_t* seed, uint64_t* cand, uint32_t* a0,
+                                                int* ws) {
+  return expand_seeded_row<NR>(P, seed, cand, a0, a0 + N, ws, 3, threadIdx.x);
+}
+
+// Poly::from_seed_moduli (poly.rs:251-281) of the ELL rows by the whole CTA.
+// Draws 0 .. 2047 (blocks 0-255, a thread each) go to residue 0, whose few
+// missing values (rejections: 2^28 - q of 2^28 draws) come from the start of
+// the next 256 blocks, found by warp 0; residue 1 follows there, and one warp
+// per row draws the last ~155 values.  Seven rounds of ChaCha20 for the three
+// rows together (one row after the other needs nine, three of them tails of
+// one warp).  A row whose stream rejects more than that leaves 0 in
+// ok[row]: a general pass redoes it.
+template <int NR>
+__device__ __forceinline__ void expand_rows(const DevParams& P, const uint8_t* seeds, uint32_t* AH, int* ws) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t q0 = P.r[0].q, z0 = (uint32_t)(P.r[0].zone >> 32);
+  const uint32_t q1 = P.r[1].q, z1 = (uint32_t)(P.r[1].zone >> 32);
+  int* tot = ws + 16;   // [ELL] values drawn so far: residue 0, then residue 1
+  int* ok = ws + 20;    // [ELL]
+#pragma unroll 1
+  for (int t = 0; t < ELL; t++) {
+    uint32_t key[8], w[16], val[8];
+    load_key(seeds + 32 * t, key);
+    chacha20_block(key, tid, P.one, w);
+    const unsigned mask = draw8(w, q0, z0, val);
+    int total;
+    const int p = scan_cta(__popc(mask), ws + 8 * (t & 1), total);
+    put_draws(AH + t * NR * N, p, mask, val);
+    if (tid == 0) tot[t] = total;
+  }
+  __syncthreads();
+  if (NR == 2) {
+#pragma unroll 1
+    for (int t = 0; t < ELL; t++) {
+      uint32_t key[8], w[16], val[8];
+      load_key(seeds + 32 * t, key);
+      chacha20_block(key, QT + tid, P.one, w);
+      uint32_t* a0 = AH + t * NR * N;
+      int start = 0;  // warp 0: draws before it belong to residue 0
+      if (warp == 0) {
+        const int have = tot[t];
+        if (have < N) {  // uniform over the warp
+          const unsigned m0 = draw8(w, q0, z0, val);
+          int all;
+          const int p = have + scan_warp(__popc(m0), all);
+          put_draws(a0, p, m0, val);
+          // the lane that holds value N - 1 knows where residue 1 starts
+          int end = 0, pp = p;
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            if ((m0 >> k) & 1u) {
+              if (pp == N - 1) end = 8 * lane + k + 1;
+              pp++;
+            }
+          start = __reduce_max_sync(0xffffffffu, end);
+          if (lane == 0) ok[t] = start != 0;
+        } else if (lane == 0) {
+          ok[t] = 1;
+        }
+      }
+      unsigned mask = draw8(w, q1, z1, val);
+      if (warp == 0) {
+        const int skip = start - 8 * lane;  // leading draws of this lane to skip
+        if (skip > 0) mask &= skip >= 8 ? 0u : ~((1u << skip) - 1u);
+      }
+      int total;
+      const int p = scan_cta(__popc(mask), ws + 8 * ((t + 1) & 1), total);
+      put_draws(a0 + N, p, mask, val);
+      if (tid == 0) tot[t] = total;
+    }
+    __syncthreads();
+  }
+  if (warp < ELL) {  // the tails, one warp per row
+    const int t = warp;
+    uint32_t key[8], w[16], val[8];
+    load_key(seeds + 32 * t, key);
+    chacha20_block(key, (NR == 2 ? 2 * QT : QT) + lane, P.one, w);
+    const unsigned mask = NR == 2 ? draw8(w, q1, z1, val) : draw8(w, q0, z0, val);
+    int all;
+    const int have = tot[t];
+    const int p = have + scan_warp(__popc(mask), all);
+    put_draws(AH + (t * NR + NR - 1) * N, p, mask, val);
+    if (lane == 0) ok[t] = (NR == 1 || ok[t]) && have + all >= N;
+  }
+}
+
+// The b side (see the file comment): b0_c = -sum_i d_{c}[i] v[i] with v[0] =
+// q - b[0], v[i] = b[N - i].  Thread tid takes the coefficient pairs j = tid +
+// 256 m, m < 4, of every column, so each row word is read once, straight
+// from its buffer (QDB: from the staged chunks), and every column word once;
+// 32 sums (column, residue) per thread, exact in 64 bits (6144 products below
+// 2^48), are then transposed and added over the warp by shuffles, five
+// halving exchanges, and over the warps in shared memory.  Measured against
+// the separate launch it replaces: 14.3 us per 128 queries there.
+// Returns -1, or (QDB) the chunk that did not arrive.
+template <bool QDB>
+__device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __restrict__ H, const uint64_t* brows,
+                                          uint64_t* stage, uint64_t* bar, uint32_t wait_iters, uint64_t* red,
+                                          uint32_t* bpoly) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gamma = P.gamma;
+  const uint32_t* h2 = reinterpret_cast<const uint32_t*>(H) + tid;
+  uint64_t acc[32];  // [column][residue]
+#pragma unroll
+  for (int k = 0; k < 32; k++) acc[k] = 0;
+#pragma unroll 1
+  for (int m = 0; m < 4; m++) {
+    uint32_t hw[MAX_GAMMA];
+#pragma unroll
+    for (int c = 0; c < MAX_GAMMA; c++) hw[c] = c < gamma ? __ldg(h2 + (size_t)c * (N / 2) + QT * m) : 0u;
+    uint32_t bv[2][2 * ELL];
+    const int i0 = 2 * (tid + QT * m);
+    if (QDB) {
+      const bool arrived = mbar_wait(bar, m & 1, wait_iters);
+      if (__syncthreads_or(!arrived)) return m;
+      const uint32_t* s = reinterpret_cast<const uint32_t*>(stage);
+#pragma unroll
+      for (int p = 0; p < 2 * ELL; p++) {
+        bv[0][p] = s[2 * (p * CHW + CH - 2 * tid)];
+        bv[1][p] = s[2 * (p * CHW + CH - 2 * tid - 1)];
+      }
+      if (m < 3) {
+        __syncthreads();
+        if (tid == 0) {
+          // the next chunk's copies (async proxy) follow these reads
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          stage_chunk(stage, brows, m + 1, bar);
+        }
+      }
+    } else {
+      const uint32_t* s = reinterpret_cast<const uint32_t*>(brows);
+      const int k0 = i0 ? N - i0 : 0, k1 = N - i0 - 1;
+#pragma unroll
+      for (int p = 0; p < 2 * ELL; p++) {
+        bv[0][p] = __ldg(s + 2 * (p * N + k0));
+        bv[1][p] = __ldg(s + 2 * (p * N + k1));
+      }
+    }
+    if (i0 == 0) {
+#pragma unroll
+      for (int p = 0; p < 2 * ELL; p++) bv[0][p] = P.r[p & 1].q - bv[0][p];
+    }
+#pragma unroll
+    for (int c = 0; c < MAX_GAMMA; c++) {
+      if (c >= gamma) continue;
+#pragma unroll
+      for (int e = 0; e < 2; e++) {
+        const uint64_t xv = P.delta * (uint64_t)((hw[c] >> (16 * e)) & 0xFFFFu);
+        const uint32_t d0 = (uint32_t)xv & 0xFFFFFu, d1 = (uint32_t)(xv >> 20) & 0xFFFFFu, d2 = (uint32_t)(xv >> 40);
+        acc[2 * c] += (uint64_t)d0 * bv[e][0] + (uint64_t)d1 * bv[e][2] + (uint64_t)d2 * bv[e][4];
+        acc[2 * c + 1] += (uint64_t)d0 * bv[e][1] + (uint64_t)d1 * bv[e][3] + (uint64_t)d2 * bv[e][5];
+      }
+    }
+  }
+  // lane l ends with the warp's sum of value l
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int k = 0; k < o; k++) {
+      const uint64_t send = up ? acc[k] : acc[k + o], keep = up ? acc[k + o] : acc[k];
+      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  if (QDB) __syncthreads();  // the last chunk has been read
+  red[warp * 32 + lane] = acc[0];
+  __syncthreads();
+  if (tid < 32) {
+    uint64_t s = 0;
+#pragma unroll
+    for (int w = 0; w < QT / 32; w++) s += red[w * 32 + tid];
+    const uint32_t q = P.r[tid & 1].q;
+    const uint32_t v = (uint32_t)(s % q);
+    bpoly[(tid & 1) * 16 + (tid >> 1)] = v ? q - v : 0;
+  }
+  __syncthreads();
+  return -1;
+}
+
+// Streaming loads of the contracted shard and the CRS keys: read once per
+// query, kept out of L1 (which holds the twiddles and the client's keys).
+__device__ __forceinline__ uint4 ld_stream(const uint32_t* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
+// REDC of T < 2^64 - q 2^32: T 2^-32 mod q, below T / 2^32 + q.
+__device__ __forceinline__ uint32_t redc_wide(uint64_t T, uint32_t q, uint32_t qinv) {
+  const uint32_t m = (uint32_t)T * qinv;
+  return (uint32_t)((T + (uint64_t)m * q) >> 32);
+}
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
-//
-// The recursion step of packing_offline (inspiring2.rs:984-1008) with
-// packing_online interleaved needs, per residue, sum_k NTT(d_k) w[i][k] for
-// R_i and sum_k NTT(d_k) y[i][k] for b, over the three gadget digits d_k of
-// INTT(R_{i+1}).  The key tables here have the third digit folded in
-// (fold_third_digit_kernel, setup.cu): with keys k' the sums are
-// k'0 NTT(d0) + k'1 NTT(d1) + k'2 R_{i+1}, so d2 is never formed and only two
-// digit transforms run per residue and step.  Per step i (gamma-2 .. 0),
-// residue r's three groups:
-//  [A] (r,0)+(r,1) as one 256-thread team: inverse NTT of R_{i+1} (T[r]),
-//      written back to T[r] once (r,2) has read it (named barrier 9 + r);
-//      (r,2): SCAT[r] += R_{i+1} w'2 and the b accumulator += R_{i+1} y'2,
-//      then the first part of the next step's query-only term R_{i-1}
-//      (into the other SCAT buffer);
-//  [B] all threads: CRT compose + digits d0, d1 into T;
-//  [C] (r,0): NTT(d0); SCAT[r] += NTT(d0) w'0 (in place), the b
-//      accumulator += NTT(d0) y'0;
-//      (r,1): NTT(d1); PB1 = NTT(d1) w'1, NTT(d1) y'1 kept in registers;
-//      (r,2): the rest of R_{i-1};
-//  [D] (r,0): R_i = SCAT[r] + PB1 -> T[r] (slots) for the next step;
-//      (r,1): the b accumulator += NTT(d1) y'1.
 template <int MODE, bool SEEDED, bool QDB>
 __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) {
   constexpr int NR = MODE == MODE_COMPAT ? 1 : 2;
-  using L = Smem<NR, QDB>;
+  using L = Smem<NR>;
   extern __shared__ __align__(16) uint32_t smem[];
-  uint32_t* Ahat = smem + L::AHAT;
-  uint32_t* SC = smem + L::SC;
-  uint32_t* T = smem + L::T;
-  uint32_t* PB1 = smem + L::PB1;
-  uint32_t* SCAT = smem + L::SCAT;
-  uint32_t* bpoly = QDB ? SC + 5 * NTT_SCRATCH + N : nullptr;  // serving: the b side, both residues, until the recursion
-  int* wsb = reinterpret_cast<int*>(QDB ? smem + L::MISC + 32 : SCAT + 2 * N);
+  uint32_t* AH = smem + L::AH;
+  uint32_t* XC = smem + L::XC;
+  int* ws = reinterpret_cast<int*>(smem + L::WS);
+  uint32_t* bpoly = smem + L::BP;
 
   const DevParams& P = A.P;
-  const int tid = threadIdx.x, g = tid >> 7, x = tid & 127;
-  const int r = g / 3, kd = g - 3 * r;  // residue, role of this group
+  const int tid = threadIdx.x, r = tid >> 7, x = tid & 127;
   const int gamma = P.gamma;
   // QDB (serving loop): this query's fields come from its descriptor in
   // device memory, its rows and response from / to pinned host memory;
   // otherwise from the launch's arrays.  Descriptor fields are re-read where
-  // used (reload_*) rather than held in registers.
+  // used (reload_ptr) rather than held in registers.
   const QueryDesc* D = QDB ? A.qdesc + qi : nullptr;
   const uint32_t shard = QDB ? D->shard : A.shard[qi];
   const int32_t cid = QDB ? D->client : A.client[qi];
   const uint32_t* Ebase = QDB ? D->db.E : A.E;
-  const uint16_t* Hbase = QDB ? D->db.H : A.H;
+  const uint16_t* H = (QDB ? D->db.H : A.H) + (size_t)shard * gamma * N;
   const int nshards = QDB ? D->db.nshards : A.nshards;
   auto status_ptr = [&]() -> int32_t* {
     return QDB ? reload_ptr(&D->status) : A.status + qi;
@@ -205,316 +400,224 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     if (tid == 0) *status_ptr() = ERR_INDEX;
     return;  // uniform over the CTA
   }
-  const uint32_t* E = Ebase + (size_t)shard * 2 * ELL * gamma * N;
-  const uint16_t* H = Hbase + (size_t)shard * gamma * N;
+  // the a side's residue: this group's, or residue 0 for both in compat mode
+  const int sres = MODE == MODE_CRT_FIXED ? r : 0;
+  const uint32_t* E = Ebase + ((size_t)shard * 2 + sres) * ELL * gamma * N;
   // The client's key table: a body table (tag bit 0 set: NTT(y_body[k]),
-  // ELL polys, 48 KiB) whose rotations are formed in registers, or the full
-  // table of (gamma-1)*ELL rotated polys (explicit y_all).
+  // ELL polys, 48 KiB) whose rotations are formed by the rows read, or the
+  // full table of (gamma-1)*ELL rotated polys (explicit y_all).
   const uintptr_t ytag = reinterpret_cast<uintptr_t>(A.yhat_table[cid]);
   const bool ybody = (ytag & 1) != 0;
   const uint32_t* Y = reinterpret_cast<const uint32_t*>(ytag & ~(uintptr_t)1);
   const ResidueConsts& C = P.r[r];
-  const uint32_t q = C.q, qinv = C.qinv, q2 = 2 * q;
+  const uint32_t q = C.q, qinv = C.qinv;
   const uint64_t* brows = QDB ? D->brows : A.brows + (size_t)qi * ELL * 2 * N;
+  uint64_t* rbar = reinterpret_cast<uint64_t*>(smem + L::BAR);
+  uint64_t* stage = reinterpret_cast<uint64_t*>(XC);
 
-  // Serving loop (rows in host memory): the query's b rows (96 KiB) are
-  // bulk-copied (TMA) into shared memory (T..T+12N) while the rows are
-  // expanded, so the host link's latency stays off the critical path, and the
-  // b side follows the row NTTs.  Rows in device memory: bside_kernel has
-  // already computed the b side and parked it in the response slot; the
-  // contracted shard and client keys are streamed into L2 from the start.
-  uint64_t* raw = reinterpret_cast<uint64_t*>(T);                      // 16-byte aligned
-  uint64_t* rbar = reinterpret_cast<uint64_t*>(smem + L::MISC + 120);  // the rows' mbarrier
-  if (QDB && tid == 0) {
-    mbar_init(rbar);
-    wsb[18] = 0;  // set when the rows do not arrive
-  }
-  if (QDB && tid == 0) prefetch_l2(H, sizeof(uint16_t) * (size_t)gamma * N);
-  // the seeds, inline in the query's descriptor: staged into shared memory
-  // (ordered before the expansion by the barrier below)
-  uint8_t* seed_sm = reinterpret_cast<uint8_t*>(smem + L::MISC + 96);
-  if (QDB && tid < ELL * 32) seed_sm[tid] = D->seeds[tid];
   if (tid == 0) {
-    // the contracted shard's blocks of the first three steps (the rest are
-    // prefetched two steps ahead of their use in the recursion)
+    if (QDB) mbar_init(rbar);
+    // the contracted shard's blocks of the first steps (the rest are
+    // prefetched two steps ahead of their use), the raw columns, the keys
+    prefetch_l2(H, sizeof(uint16_t) * (size_t)gamma * N);
     const int i0 = gamma >= 3 ? gamma - 3 : 0;
     for (int rr = 0; rr < NR; rr++)
-      prefetch_l2(E + ((size_t)rr * gamma + i0) * ELL * N, sizeof(uint32_t) * (size_t)(gamma - i0) * ELL * N);
+      prefetch_l2(Ebase + (((size_t)shard * 2 + rr) * gamma + i0) * ELL * N,
+                  sizeof(uint32_t) * (size_t)(gamma - i0) * ELL * N);
     if (gamma > 1) prefetch_l2(Y, sizeof(uint32_t) * (size_t)(ybody ? 1 : gamma - 1) * ELL * 2 * N);
   }
+  const uint8_t* seeds = nullptr;
+  if (SEEDED) seeds = QDB ? reinterpret_cast<const uint8_t*>(smem + L::SEED) : A.seeds + (size_t)qi * ELL * 32;
   if (QDB) {
+    // the seeds, inline in the query's descriptor
+    if (SEEDED && tid < ELL * 32) reinterpret_cast<uint8_t*>(smem + L::SEED)[tid] = D->seeds[tid];
     __syncthreads();  // the mbarrier is initialised, the seeds staged
-    if (tid == 0) {
-      mbar_expect_tx(rbar, (uint32_t)(sizeof(uint64_t) * ELL * 2 * N));
-#pragma unroll
-      for (int p = 0; p < 2 * ELL; p++) bulk_g2s(raw + (size_t)p * N, brows + (size_t)p * N, sizeof(uint64_t) * N, rbar);
+    if (tid == 0) stage_chunk(stage, brows, 0, rbar);
+  }
+
+  // ---- rows ELL..2ELL-1, coefficients, into AH [t][NR][N] ----
+  if (SEEDED) {
+    expand_rows<NR>(P, seeds, AH, ws);
+  } else {
+    const uint64_t* ar = A.arows + (size_t)qi * ELL * 2 * N;
+#pragma unroll 4
+    for (int j = tid; j < ELL * NR * N; j += QT) {
+      const int t = j / (NR * N);
+      AH[j] = (uint32_t)__ldg(ar + (size_t)t * 2 * N + (j - t * NR * N));
     }
   }
 
-  // ---- rows ELL..2ELL-1: expand (one sub-block per row), forward NTT ----
-  {
-    const int t = tid >> 8, lt = tid & 255;
-    uint64_t* cand = reinterpret_cast<uint64_t*>(SC) + t * N;  // 3 x 16 KiB within SC
-    // serving loop: in place of the row's transforms (T..T+12N hold the
-    // staged rows); otherwise within T..PB1
-    uint32_t* a0 = QDB ? Ahat + t * NR * N : T + t * 2 * N;
-    uint32_t* a1 = a0 + N;
-    if (SEEDED) {
-      const uint8_t* seed = QDB ? seed_sm + 32 * t : A.seeds + ((size_t)qi * ELL + t) * 32;
-      const bool ok = expand_seeded_row<NR>(P, seed, cand, a0, a1, wsb + 20 * t, 7 + t, lt);
-      if (lt == 0) wsb[20 * t + 17] = ok;
-    } else {
-      const uint64_t* ar = A.arows + ((size_t)qi * ELL + t) * 2 * N;
-      for (int j = lt; j < NR * N; j += SUB) a0[j] = (uint32_t)ar[j];  // a1 follows a0
-    }
-  }
-  if (QDB) {
-    // rows that do not arrive within A.stage_wait_iters end the query with
-    // a status, after a second bounded wait for the copies still in flight
-    const bool arrived = mbar_wait(rbar, 0, A.stage_wait_iters);
-    if (!arrived) wsb[18] = 1;
-  }
-  __syncthreads();
-  const bool exp_ok = !SEEDED || (wsb[17] && wsb[37] && wsb[57]);
-  if (QDB && wsb[18]) {
+  // ---- the b side ----
+  const int missing = column_b0<QDB>(P, H, brows, stage, rbar, A.stage_wait_iters, reinterpret_cast<uint64_t*>(XC), bpoly);
+  if (QDB && missing >= 0) {
     // The CTA must not exit while its bulk copies can still write into its
-    // shared memory (the next CTA on this SM would own it).  If even the
-    // drain wait runs out, ERR_STAGE_LOST tells the host to drop every
-    // result of this launch.
-    const int lost = __syncthreads_or(!mbar_wait(rbar, 0, STAGE_DRAIN_ITERS));
+    // shared memory (the next CTA on this SM would own it): a second bounded
+    // wait, for the chunk in flight.  If even that runs out, ERR_STAGE_LOST
+    // tells the host to drop every result of this launch.
+    const int lost = __syncthreads_or(!mbar_wait(rbar, missing & 1, STAGE_DRAIN_ITERS));
     if (tid == 0) *status_ptr() = lost ? ERR_STAGE_LOST : ERR_STAGE;
     return;  // uniform over the CTA
   }
-  if (QDB) {
-    // the row transforms reuse the words of the workspace, seeds and mbarrier
-    if (tid == 0) mbar_inval(rbar);
-    __syncthreads();
-  }
-  // the query's status is written once, by one thread
-  if (tid == 0) *status_ptr() = exp_ok ? 0 : ERR_EXPAND;
-  if (r < NR) {  // group (r, t=kd) transforms row kd, residue r
-    uint32_t v[16];
-    const uint32_t* src = QDB ? Ahat + (kd * NR + r) * N : T + kd * 2 * N + r * N;
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = src[x + 128 * j];
-    ntt_fwd(v, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = canon16(v[j], q);
-    store16(Ahat + (kd * NR + r) * N, x, v);
-  }
-  __syncthreads();
-
-  // ---- serving loop: b part of the column products (bp in SC, rows staged) ----
-  if (QDB) column_b0<RBLOCK>(P, H, raw, SC, bpoly);
-
-  // Eg: the scatter's residue of the contracted shard; with per-query
-  // databases it is re-derived at each use from the query's view
-  const uint32_t* Eg_fixed = QDB ? nullptr : E;
-  auto Eg_at = [&](int sres) -> const uint32_t* {
-    if (!QDB) return Eg_fixed + (size_t)sres * ELL * gamma * N;
-    const uint32_t sh = *reinterpret_cast<const volatile uint32_t*>(&D->shard);
-    return reload_ptr(&D->db.E) + ((size_t)sh * 2 * ELL + (size_t)sres * ELL) * gamma * N;
-  };
-
-  // ---- R_{gamma-1} into T, R_{gamma-2} into SCAT[(gamma-2) & 1], by all
-  //      groups (fixed: each residue's 384 threads; compat: residue 0 by all) ----
-  {
-    const int sres = MODE == MODE_CRT_FIXED ? r : 0;
-    const int sp = MODE == MODE_CRT_FIXED ? kd * NTT_GT + x : tid;
-    const int snthr = MODE == MODE_CRT_FIXED ? 3 * NTT_GT : RBLOCK;
-    const uint32_t sq = P.r[sres].q, sqinv = P.r[sres].qinv;
-    const uint32_t* Ag = Ahat + sres * N;
-    scatter_r(P, gamma - 1, Eg_at(sres), Ag, NR * N, T + sres * N, sp, snthr, sq, sqinv,
-              MODE == MODE_COMPAT ? T + N : nullptr);
-    if (gamma > 1) {
-      uint32_t* sc2 = SCAT + ((gamma - 2) & 1) * 2 * N;
-      scatter_r(P, gamma - 2, Eg_at(sres), Ag, NR * N, sc2 + sres * N, sp, snthr, sq, sqinv,
-                MODE == MODE_COMPAT ? sc2 + N : nullptr);
-    }
-    for (int j = tid; j < 2 * N; j += RBLOCK) SC[(3 * (j >> LOGN) + 2) * NTT_SCRATCH + (j & (N - 1))] = 0;
-    // the b side (serving: computed above; device rows: parked by
-    // bside_kernel), residue r's beside its accumulator
-    if (tid < 32) {
-      const uint32_t bv = QDB ? bpoly[tid] : b_parking(A.out, qi)[tid];
-      __syncwarp();
-      SC[(3 * (tid >> 4) + 2) * NTT_SCRATCH + N + (tid & 15)] = bv;
-    }
-  }
-  __syncthreads();
-
-  const int team_t = tid - 384 * r;  // thread of residue r's (r,0)+(r,1) team, valid for kd < 2
-  uint32_t* team_sc = SC + 3 * r * NTT_SCRATCH;  // the team's exchange scratch (two groups' worth)
-  // the next step's query-only term by the (r,2) groups, in two parts ([A] and [C])
-  auto scatter_next = [&](int i, int u0, int u1) {
-    const int sres = MODE == MODE_CRT_FIXED ? r : 0;
-    const int sp = MODE == MODE_CRT_FIXED ? x : r * NTT_GT + x;
-    const int snthr = MODE == MODE_CRT_FIXED ? NTT_GT : 2 * NTT_GT;
-    uint32_t* sc2 = SCAT + ((i - 1) & 1) * 2 * N;
-    scatter_r(P, i - 1, Eg_at(sres), Ahat + sres * N, NR * N, sc2 + sres * N, sp, snthr, P.r[sres].q, P.r[sres].qinv,
-              MODE == MODE_COMPAT ? sc2 + N : nullptr, u0, u1);
-  };
-  const int f = (x >> 1) & 3;  // chunk swizzle of this thread's 16-slot run (store16 / load16)
-  for (int i = gamma - 2; i >= 0; i--) {
-    const size_t yoff = ybody ? (size_t)i * ELL * 2 * N : 0;  // body tables: the key slices of i = 0, rotated
-    if (tid == 0 && i >= 2)  // the block the next step's scatter reads (R_{i-2})
-      for (int rr = 0; rr < NR; rr++) prefetch_l2(Eg_at(rr) + (size_t)(i - 2) * ELL * N, sizeof(uint32_t) * ELL * N);
-    // [A] inverse NTT of R_{i+1} by residue r's team; the products of
-    //     R_{i+1} with the third key slices by group (r,2)
-    if (kd < 2) {
-      uint32_t v[8];
-      const int s0 = 8 * team_t;
-      const uint4 lo = *reinterpret_cast<const uint4*>(T + r * N + swz(s0));
-      const uint4 hi = *reinterpret_cast<const uint4*>(T + r * N + swz(s0 + 4));
-      v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
-      v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-      ntt_inv_noscale8(v, team_sc, inv_tw(C), q, team_t, 7 + r);
-      named_sync(9 + r, 3 * NTT_GT);  // group (r,2) has read R_{i+1}
-#pragma unroll
-      for (int j = 0; j < 8; j++) T[r * N + team_t + 256 * j] = canon2(v[j], q);
-    } else {
-      uint32_t rs[16];
-      load16(T + r * N, x, rs);
-      named_arrive(9 + r, 3 * NTT_GT);
-      const size_t off2 = ((size_t)(i * ELL + 2) * 2 + r) * N + 16 * x;
-      uint4 wv[4], yv[4];
-      key_run(A.what + off2, wv);
-      key_run(Y + off2 - yoff, yv);
-      if (ybody) rotate_key_run(yv, i, x);
-      uint32_t* accb = SC + g * NTT_SCRATCH;  // the residue's b accumulator
-      uint32_t* part = SCAT + (i & 1) * 2 * N + r * N;
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        const int o = 16 * x + 4 * (r4 ^ f);
-        uint4* ap = reinterpret_cast<uint4*>(accb + o);
-        uint4* hp = reinterpret_cast<uint4*>(part + o);
-        const uint4 a4 = *ap, h4 = *hp;
-        uint32_t ab[4], pr[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int j = 4 * r4 + e;
-          ab[e] = acc_2q(u4e(a4, e), redc_lazy((uint64_t)rs[j] * u4e(yv[r4], e), q, qinv), q2);
-          pr[e] = u4e(h4, e) + redc_lazy((uint64_t)rs[j] * u4e(wv[r4], e), q, qinv);  // [0, 3q)
-        }
-        *ap = make_uint4(ab[0], ab[1], ab[2], ab[3]);
-        *hp = make_uint4(pr[0], pr[1], pr[2], pr[3]);
+  // ---- rows that the fast expansion left to the general one ----
+  if (SEEDED) {
+    bool good = true;
+#pragma unroll 1
+    for (int t = 0; t < ELL; t++)
+      if (!ws[20 + t]) {  // uniform; ordered by the b side's barriers
+        good &= expand_row_general<NR>(P, seeds + 32 * t, reinterpret_cast<uint64_t*>(XC), AH + t * NR * N, ws);
+        __syncthreads();
       }
-      if (i >= 1) scatter_next(i, 0, SCATTER_SPLIT);
-    }
-    __syncthreads();
-    // [B] gadget_decompose of the composite coefficients (rgsw/external_product.rs:16-37):
-    //     digits 0 and 1 (the third is folded into the keys)
-    for (int j = tid; j < N; j += RBLOCK) {
-      const uint64_t c = crt_compose(P, T[j], T[N + j]);
-      T[j] = (uint32_t)c & 0xFFFFFu;
-      T[N + j] = (uint32_t)(c >> 20) & 0xFFFFFu;
-    }
-    __syncthreads();
-    // [C]
-    uint32_t* accb = SC + (3 * r + 2) * NTT_SCRATCH;  // the residue's b accumulator
-    uint32_t py[16];  // group (r,1): NTT(d1) y'1, added to the b accumulator in [D]
-    if (kd < 2) {
-      const size_t off = ((size_t)(i * ELL + kd) * 2 + r) * N + 16 * x;
-      uint4 wv[4], yv[4];
-      key_run(A.what + off, wv);  // this step's key slices, fetched before the transform
-      key_run(Y + off - yoff, yv);
-      uint32_t v[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) v[j] = T[kd * N + x + 128 * j];
-      ntt_fwd(v, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);  // slots 16x.., [0, 14q)
-      if (ybody) rotate_key_run(yv, i, x);
-      // group (r,0): the b accumulator and the partial R_i in place of the
-      // query-only term; group (r,1): PB1
-      uint32_t* pdst = kd == 0 ? SCAT + (i & 1) * 2 * N + r * N : PB1 + r * N;
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        const int o = 16 * x + 4 * (r4 ^ f);
-        uint4* hp = reinterpret_cast<uint4*>(pdst + o);
-        const uint4 h4 = kd == 0 ? *hp : make_uint4(0, 0, 0, 0);
-        uint32_t pr[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-          pr[e] = redc_lazy((uint64_t)v[4 * r4 + e] * u4e(wv[r4], e), q, qinv) + u4e(h4, e);  // [0, 5q)
-        *hp = make_uint4(pr[0], pr[1], pr[2], pr[3]);
-#pragma unroll
-        for (int e = 0; e < 4; e++) py[4 * r4 + e] = redc_lazy((uint64_t)v[4 * r4 + e] * u4e(yv[r4], e), q, qinv);
-        if (kd == 0) {
-          uint4* ap = reinterpret_cast<uint4*>(accb + o);
-          const uint4 a4 = *ap;
-          *ap = make_uint4(acc_2q(a4.x, py[4 * r4], q2), acc_2q(a4.y, py[4 * r4 + 1], q2),
-                           acc_2q(a4.z, py[4 * r4 + 2], q2), acc_2q(a4.w, py[4 * r4 + 3], q2));
-        }
-      }
-    } else if (i >= 1) {
-      scatter_next(i, SCATTER_SPLIT, N);
-    }
-    __syncthreads();
-    // [D] R_i (group (r,0)); b += NTT(d1) y'1 (group (r,1))
-    if (kd == 1) {
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        uint4* ap = reinterpret_cast<uint4*>(accb + 16 * x + 4 * (r4 ^ f));
-        const uint4 a4 = *ap;
-        *ap = make_uint4(acc_2q(a4.x, py[4 * r4], q2), acc_2q(a4.y, py[4 * r4 + 1], q2),
-                         acc_2q(a4.z, py[4 * r4 + 2], q2), acc_2q(a4.w, py[4 * r4 + 3], q2));
-      }
-    } else if (kd == 0) {
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        const int o = r * N + 16 * x + 4 * (r4 ^ f);
-        const uint4 pa = *reinterpret_cast<const uint4*>(SCAT + (i & 1) * 2 * N + o);
-        const uint4 p1 = *reinterpret_cast<const uint4*>(PB1 + o);
-        uint32_t outv[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          uint32_t sum = u4e(pa, e) + u4e(p1, e);  // < 7q < 2^31
-          sum = min(sum, sum - 4 * q);
-          sum = min(sum, sum - 2 * q);
-          outv[e] = min(sum, sum - q);
-        }
-        *reinterpret_cast<uint4*>(T + o) = make_uint4(outv[0], outv[1], outv[2], outv[3]);  // R_i for the next step
-      }
-    }
-    __syncthreads();
-  }
-
-  // ---- outputs: a_hat = INTT(R_0) (inspiring2.rs:1027-1029) by each
-  //      residue's team, b = b_poly + INTT(sum y_all * bold_t)
-  //      (inspiring2.rs:1217-1221) by group (r,2) ----
-  uint64_t* out = QDB ? reload_ptr(&D->out) : A.out + (size_t)qi * 4 * N;
-  if (kd < 2) {
-    uint32_t v[8];
-    const int s0 = 8 * team_t;
-    const uint4 lo = *reinterpret_cast<const uint4*>(T + r * N + swz(s0));
-    const uint4 hi = *reinterpret_cast<const uint4*>(T + r * N + swz(s0 + 4));
-    v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
-    v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
-    ntt_inv_noscale8(v, team_sc, inv_tw(C), q, team_t, 7 + r);
-#pragma unroll
-    for (int j = 0; j < 8; j++) out[r * N + team_t + 256 * j] = canon2(v[j], q);
+    if (tid == 0) *status_ptr() = good ? 0 : ERR_EXPAND;
   } else {
-    uint32_t b0[16];
-    load16(SC + g * NTT_SCRATCH, x, b0);  // the b accumulator, [0, 2q)
-    const uint32_t bp = x < gamma ? SC[g * NTT_SCRATCH + N + x] : 0;
-    ntt_inv_noscale(b0, SC + g * NTT_SCRATCH, inv_tw(C), q, x, 1 + g);  // first exchange after a group barrier
+    if (tid == 0) *status_ptr() = 0;
+  }
+
+  // ---- row transforms, into rows h of AH (a slot's words are its thread's).
+  //      Consecutive transforms use two exchange buffers by turns: one ends
+  //      with reads that another warp's next first writes could overtake ----
+  {
+    const ResidueConsts& Cs = P.r[sres];
+#pragma unroll 1
+    for (int t = NR == 2 ? 0 : r, turn = 0; t < ELL; t += NR == 2 ? 1 : 2, turn ^= 1) {
+      uint32_t* row = AH + (t * NR + sres) * N;
+      uint32_t v[1][16];
+      uint32_t* const sc[1] = {XC + (turn ? r : 2 + r) * N};
 #pragma unroll
-    for (int j = 0; j < 16; j++) b0[j] = canon2(b0[j], q);
-    if (x < gamma) b0[0] = add_mod(b0[0], bp, q);
+      for (int j = 0; j < 16; j++) v[0][j] = row[x + 128 * j];
+      jntt_fwd<1, true>(v, sc, fwd_tw(Cs), Cs.q, x, 1 + r);
 #pragma unroll
-    for (int j = 0; j < 16; j++) out[2 * N + r * N + x + 128 * j] = b0[j];
+      for (int j = 0; j < 16; j++) row[128 * h_of(j) + x] = canon16(v[0][j], Cs.q);
+    }
+    if (NR == 1) __syncthreads();  // both groups read the rows of residue 0
+  }
+
+  const uint32_t* Ax = AH + sres * N + x;  // row h of row transform t: Ax[t * NR * N + 128 * h]
+  const uint32_t* Ex = E + 4 * x;
+  const uint32_t* Wx = A.what + r * N + 4 * x;
+  const uint32_t* Yx = Y + r * N + x;
+  // sum_t E[i,t][s] A_t[tau_i(s)] for the four slots h = 4 a + j of this thread
+  auto query_only = [&](int i, int a, uint32_t rot, uint64_t T[4]) {
+    const uint32_t* e = Ex + (size_t)i * ELL * N + 512 * a;
+    const uint4 e0 = ld_stream(e), e1 = ld_stream(e + N), e2 = ld_stream(e + 2 * N);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const uint32_t* ar = Ax + 128 * ((4 * a + j + rot) & 15);
+      T[j] = (uint64_t)u4e(e0, j) * ar[0] + (uint64_t)u4e(e1, j) * ar[NR * N] + (uint64_t)u4e(e2, j) * ar[2 * NR * N];
+    }
+  };
+  // compat mode, residue 1: rebuilt from the residue-0 value as the crate's
+  // apply_automorphism_ntt does
+  const bool conv1 = MODE == MODE_COMPAT && r == 1;
+  auto converted = [&](uint64_t T) -> uint32_t {
+    return compat_residue1_ninv(P, redc(T, P.r[0].q, P.r[0].qinv));
+  };
+
+  uint32_t R[16], acc[16];  // R_{i+1} and the b accumulator, slot layout
+  {
+    const uint32_t rot = rot_rows(gamma, gamma - 1, x);
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      uint64_t T[4];
+      query_only(gamma - 1, a, rot, T);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int l = h_of(4 * a + j);
+        R[l] = conv1 ? converted(T[j]) : redc_wide(T[j], q, qinv);
+        acc[l] = 0;
+      }
+    }
+  }
+
+#pragma unroll 1
+  for (int i = gamma - 2; i >= 0; i--) {
+    if (tid == 0 && i >= 2)  // the block that step i - 2 reads
+      for (int rr = 0; rr < NR; rr++)
+        prefetch_l2(Ebase + (((size_t)shard * 2 + rr) * gamma + (i - 2)) * ELL * N, sizeof(uint32_t) * ELL * N);
+    // [A] inverse NTT of R_{i+1} ([0, 3.2 q))
+    uint32_t* const own = XC + (2 + r) * N;
+    uint32_t* const mine = XC + (r ^ (i & 1)) * N;
+    uint32_t* const other = XC + (r ^ 1 ^ (i & 1)) * N;
+    uint32_t v[2][16];
+    {
+      uint32_t c[1][16], o[1][16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) c[0][j] = R[j];
+      uint32_t* const sc[1] = {own};
+      jntt_inv<1>(c, sc, fwd_tw(C), q, x, 1 + r);
+      // [B] the residues trade coefficients, thread for thread: each writes
+      // its own to the buffer it has been using, reads the other group's,
+      // and goes on with that buffer.  Digits 0 and 1 of the composite
+      // coefficients (gadget_decompose, rgsw/external_product.rs:16-37).
+      uint32_t* const sm1[1] = {mine};
+      uint32_t* const so1[1] = {other};
+      jx_store_co<1>(c, sm1, x);
+      named_sync(3 + (x >> 5), 64);
+      jx_load_co<1>(o, so1, x);
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        const uint64_t cc = crt_compose(P, r ? o[0][j] : c[0][j], r ? c[0][j] : o[0][j]);
+        v[0][j] = (uint32_t)cc & 0xFFFFFu;
+        v[1][j] = (uint32_t)(cc >> 20) & 0xFFFFFu;
+      }
+    }
+    // [C]
+    uint32_t* const sc2[2] = {other, own};
+    jntt_fwd<2, false>(v, sc2, fwd_tw(C), q, x, 1 + r);  // [0, 14 q)
+    // [D] the nine products of each slot under two reductions.  With R < 3.2 q,
+    // NTT(d) < 14 q and the rest canonical, R's sum is below 34.3 q^2 (q <
+    // 2^28: < 2.2 q 2^32), so R_i < 3.2 q again; b enters its own sum times
+    // 2^32 (b 2^32 + 31.2 q^2 < 11 q 2^32) and is brought below 8 q.
+    const uint32_t rot = rot_rows(gamma, i, x);
+    const uint32_t yrot = ybody ? rot : 0;
+    const uint32_t* yi = ybody ? Yx : Yx + (size_t)i * ELL * 2 * N;
+    const uint32_t* wi = Wx + (size_t)i * ELL * 2 * N;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+      uint64_t T[4];
+      const uint4 w0 = ld_stream(wi + 512 * a), w1 = ld_stream(wi + 2 * N + 512 * a),
+                  w2 = ld_stream(wi + 4 * N + 512 * a);
+      query_only(i, a, rot, T);
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int l = h_of(4 * a + j);
+        const uint32_t* y = yi + 128 * ((4 * a + j + yrot) & 15);
+        uint64_t S = conv1 ? (uint64_t)converted(T[j]) << 32 : T[j];
+        S += (uint64_t)v[0][l] * u4e(w0, j) + (uint64_t)v[1][l] * u4e(w1, j) + (uint64_t)R[l] * u4e(w2, j);
+        const uint64_t B = ((uint64_t)acc[l] << 32) + (uint64_t)v[0][l] * __ldg(y) +
+                           (uint64_t)v[1][l] * __ldg(y + 2 * N) + (uint64_t)R[l] * __ldg(y + 4 * N);
+        R[l] = redc_wide(S, q, qinv);
+        acc[l] = csub(redc_wide(B, q, qinv), 8 * q);
+      }
+    }
+  }
+
+  // ---- outputs: a_hat = INTT(R_0) (inspiring2.rs:1027-1029), b = b_poly +
+  //      INTT(sum y_all * bold_t) (inspiring2.rs:1217-1221) ----
+  uint64_t* out = QDB ? reload_ptr(&D->out) : A.out + (size_t)qi * 4 * N;
+#pragma unroll 1
+  for (int part = 0; part < 2; part++) {
+    uint32_t o[1][16];
+    uint32_t* const sc[1] = {XC + (part ? r ^ 1 : 2 + r) * N};
+#pragma unroll
+    for (int j = 0; j < 16; j++) o[0][j] = part ? csub(acc[j], 4 * q) : R[j];
+    jntt_inv<1>(o, sc, fwd_tw(C), q, x, 1 + r);
+    if (part && x < gamma) o[0][0] = add_mod(o[0][0], bpoly[16 * r + x], q);
+#pragma unroll
+    for (int j = 0; j < 16; j++) out[part * 2 * N + r * N + x + 128 * j] = o[0][j];
   }
 }
 
 // One query per CTA.
 template <int MODE, bool SEEDED, bool QDB>
-__global__ void __launch_bounds__(RBLOCK, 1) respond_kernel(const __grid_constant__ RespondArgs A) {
+__global__ void __launch_bounds__(QT, 2) respond_kernel(const __grid_constant__ RespondArgs A) {
   respond_one<MODE, SEEDED, QDB>(A, blockIdx.x);
 }
 
 // Capped grid (device-resident rows): CTA b answers queries b, b + gridDim.x,
-// ... in turn, so a grid of one CTA per SM keeps every SM busy to the end of
-// a large batch.
+// ... in turn.
 template <int MODE, bool SEEDED>
-__global__ void __launch_bounds__(RBLOCK, 1) respond_kernel_loop(const __grid_constant__ RespondArgs A) {
+__global__ void __launch_bounds__(QT, 2) respond_kernel_loop(const __grid_constant__ RespondArgs A) {
+#pragma unroll 1
   for (int qi = blockIdx.x; qi < A.nq; qi += gridDim.x) {
     if (qi != (int)blockIdx.x) __syncthreads();  // the previous query's shared memory is no longer read
     respond_one<MODE, SEEDED, false>(A, qi);
@@ -523,38 +626,29 @@ __global__ void __launch_bounds__(RBLOCK, 1) respond_kernel_loop(const __grid_co
 
 }  // namespace
 
-size_t respond_smem_bytes(int mode, bool qdb) {
-  const int words = mode == MODE_COMPAT ? (qdb ? Smem<1, true>::TOTAL : Smem<1, false>::TOTAL)
-                                        : (qdb ? Smem<2, true>::TOTAL : Smem<2, false>::TOTAL);
-  return sizeof(uint32_t) * words;
+size_t respond_smem_bytes(int mode) {
+  return sizeof(uint32_t) * (mode == MODE_COMPAT ? Smem<1>::TOTAL : Smem<2>::TOTAL);
 }
 
 template <int MODE, bool SEEDED, bool QDB>
 static cudaError_t set_smem_attr() {
   cudaError_t e = cudaFuncSetAttribute(respond_kernel<MODE, SEEDED, QDB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)respond_smem_bytes(MODE, QDB));
+                                       (int)respond_smem_bytes(MODE));
   if (e == cudaSuccess && !QDB)
     e = cudaFuncSetAttribute(respond_kernel_loop<MODE, SEEDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)respond_smem_bytes(MODE, false));
+                             (int)respond_smem_bytes(MODE));
   return e;
 }
 
 // Launches issue no configuration call (so they can be captured in a CUDA
 // graph): the shared-memory attribute of every variant is set once per
 // device by prepare_respond_kernels.
-size_t bside_smem_bytes() { return sizeof(uint32_t) * ((size_t)ELL * 2 * N + 32); }
-
 template <int MODE, bool SEEDED, bool QDB>
 static cudaError_t launch_one(const RespondArgs& a, int ctas, cudaStream_t st) {
-  if (!QDB) {
-    bside_kernel<<<a.nq, BSIDE_THREADS, bside_smem_bytes(), st>>>(a);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
   if (!QDB && ctas < a.nq)
-    respond_kernel_loop<MODE, SEEDED><<<ctas, RBLOCK, respond_smem_bytes(MODE, false), st>>>(a);
+    respond_kernel_loop<MODE, SEEDED><<<ctas, QT, respond_smem_bytes(MODE), st>>>(a);
   else
-    respond_kernel<MODE, SEEDED, QDB><<<a.nq, RBLOCK, respond_smem_bytes(MODE, QDB), st>>>(a);
+    respond_kernel<MODE, SEEDED, QDB><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
   return cudaGetLastError();
 }
 
@@ -566,7 +660,7 @@ cudaError_t prepare_respond_kernels() {
       set_smem_attr<MODE_CRT_FIXED, false, true>(),  set_smem_attr<MODE_CRT_FIXED, true, true>()};
   for (cudaError_t e : es)
     if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(bside_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bside_smem_bytes());
+  return cudaSuccess;
 }
 
 template <int MODE>

@@ -69,81 +69,77 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   return false;
 }
 
-// R_i (NTT domain, scaled by n^-1) of packing_offline step 1 for one residue,
-// scattered to dst[slot]: source slot u contributes to slot s with
-// 2brv(s)+1 = h_i (2brv(u)+1) mod 2n, where h_i = g^-i
-// (inspiring2.rs:952-981 with the tables of :208-263).  Eg is this residue's
-// contracted shard [gamma][ELL][N], stored by step (encode_E_kernel): the
-// three rows' DFT outputs for slot u of step i sit at [i][t][u], so the loads
-// of consecutive slots are contiguous.  Threads p in [0, nthr) handle
-// u = p + nthr * v.
+// ---- slot order of the resident tables ----
+// tau_{g^i} in the NTT domain is the slot permutation s -> u with 2brv(u)+1 =
+// g^i (2brv(s)+1) mod 2N (inspiring2.rs:208-263).  With g = 2N/gamma + 1 and
+// gamma <= 16 a power of two, g^i = 1 + (2N/gamma) i mod 2N, so brv(u) =
+// brv(s) + (N/gamma) (i (2brv(s)+1) mod gamma) mod N: only the top four bits
+// of brv(s) move, i.e. only the low four bits of s, by an amount that depends
+// on s >> 4 alone.  With s = 16 x + l and h = brv4(l), the top four bits of
+// brv(s), u is (x, h + rot_rows(gamma, i, x) mod 16).
+//
+// Tables are therefore stored by (h, x):
+//   quads  [h >> 2][x][h & 3]: thread x reads its 16 slots with four coalesced
+//          128-bit loads (contracted shard, CRS keys);
+//   rows   [h][x]: row h + rot of 128 threads, the rotation uniform over 16
+//          threads, so that a warp's load of a rotated slot touches two
+//          half lines (client keys, row transforms).
+__device__ __forceinline__ uint32_t rot_rows(int gamma, int i, int x) {
+  const uint32_t c = 2u * (__brev((uint32_t)x) >> 25) + 1u;  // 2 brv(s) + 1 mod 16
+  return (((uint32_t)i * c) & (uint32_t)(gamma - 1)) * (uint32_t)(MAX_GAMMA / gamma);
+}
+__host__ __device__ constexpr int h_of(int l) { return ((l & 1) << 3) | ((l & 2) << 1) | ((l & 4) >> 1) | ((l & 8) >> 3); }
+__host__ __device__ constexpr int quad_word(int h, int x) { return (h >> 2) * 512 + 4 * x + (h & 3); }
+__host__ __device__ constexpr int row_word(int h, int x) { return h * 128 + x; }
+
+// R_i (NTT domain, scaled by n^-1) of packing_offline step 1 for one residue
+// (inspiring2.rs:952-981 with the tables of :208-263): slot s takes sum_t
+// E[i][t][s] A_t[u], u = tau_i(s).  Eg is this residue's contracted shard
+// [gamma][ELL][N] in quads by destination slot (encode_E_kernel); Ag the row
+// transforms in (swizzled) slot order.  Threads p in [0, nthr) handle table
+// words w = w0 + p + nthr * v < w1.
 // In compat mode `dst1`, if not null, receives residue 1 rebuilt from each
 // residue-0 value as the crate's apply_automorphism_ntt does (`dst` may then
 // be null: only residue 1 is written).
 __device__ __forceinline__ void scatter_r(const DevParams& P, int i, const uint32_t* __restrict__ Eg, const uint32_t* Ag,
                                           int astride, uint32_t* dst, int p, int nthr, uint32_t q, uint32_t qinv,
-                                          uint32_t* dst1 = nullptr, int u0 = 0, int u1 = N) {
-  const int gamma = P.gamma;
-  const uint32_t mi = (uint32_t)(gamma - i) & (uint32_t)(gamma - 1);
-  const uint32_t hi = (1u + (uint32_t)(2 * N / gamma) * mi) & (2 * N - 1);
+                                          uint32_t* dst1 = nullptr, int w0 = 0, int w1 = N) {
   const uint32_t* Ei = Eg + (size_t)i * ELL * N;
 #pragma unroll 4
-  for (int u = u0 + p; u < u1; u += nthr) {
-    const uint32_t e = 2 * brv11(u) + 1;
-    const int us = swz(u);
-    const uint64_t T = (uint64_t)__ldg(Ei + u) * Ag[us] + (uint64_t)__ldg(Ei + N + u) * Ag[astride + us] +
-                       (uint64_t)__ldg(Ei + 2 * N + u) * Ag[2 * astride + us];
-    const uint32_t s = brv11(((hi * e) & (2 * N - 1)) >> 1);
+  for (int w = w0 + p; w < w1; w += nthr) {
+    const int x = (w >> 2) & 127, h = ((w >> 9) << 2) | (w & 3);
+    const int us = swz(16 * x + h_of((h + (int)rot_rows(P.gamma, i, x)) & 15));
+    const uint64_t T = (uint64_t)__ldg(Ei + w) * Ag[us] + (uint64_t)__ldg(Ei + N + w) * Ag[astride + us] +
+                       (uint64_t)__ldg(Ei + 2 * N + w) * Ag[2 * astride + us];
+    const int s = swz(16 * x + h_of(h));
     const uint32_t val = redc(T, q, qinv);
-    if (dst) dst[swz(s)] = val;
-    if (dst1) dst1[swz(s)] = compat_residue1_ninv(P, val);
+    if (dst) dst[s] = val;
+    if (dst1) dst1[s] = compat_residue1_ninv(P, val);
   }
 }
 
-// y_all[i][k] from NTT(y_body[k]) in registers (gamma = 16).  In the NTT
-// domain tau_{g^i} (generate_rotations, inspiring2.rs:1309-1323) is the slot
-// permutation s -> u with 2brv(u)+1 = g^i (2brv(s)+1) mod 2n.  With
-// g = 2n/16 + 1, g^i = 1 + 256 i mod 2n, so brv(u) = brv(s) + 128 delta mod
-// 2n with delta = i (2brv(s)+1) mod 16: only the top four bits of brv(s)
-// move, i.e. only the low four bits of s, and delta depends on s only
-// through s >> 4.  Each thread's run of slots 16x..16x+15 is therefore a
-// rotation by delta of itself, indexed by brv4 of the slot's low bits:
-// out[brv4(h)] = in[brv4((h + delta) mod 16)].  Done as a four-stage barrel
-// shift of register selects.
-__device__ __forceinline__ void rotate_key_run(uint4 (&y)[4], int i, int x) {
-  uint32_t z[16];  // z[h] = in[brv4(h)]
-#pragma unroll
-  for (int h = 0; h < 16; h++) {
-    const int j = ((h & 1) << 3) | ((h & 2) << 1) | ((h & 4) >> 1) | ((h & 8) >> 3);
-    const uint4& c = y[j >> 2];
-    z[h] = (j & 3) == 0 ? c.x : (j & 3) == 1 ? c.y : (j & 3) == 2 ? c.z : c.w;
-  }
-  const uint32_t delta = ((uint32_t)i * (2u * brv11(16u * (uint32_t)x) + 1u)) & 15u;
-#pragma unroll
-  for (int b = 0; b < 4; b++) {
-    const bool on = (delta >> b) & 1u;
-    uint32_t t[16];
-#pragma unroll
-    for (int h = 0; h < 16; h++) t[h] = on ? z[(h + (1 << b)) & 15] : z[h];
-#pragma unroll
-    for (int h = 0; h < 16; h++) z[h] = t[h];
-  }
+// A thread's 16 slots (slot order, as four uint4) of one key polynomial of
+// the CRS table (quads) or of a client table (rows; rot: rot_rows for a body
+// table, 0 for a table of rotated polynomials).
+__device__ __forceinline__ void key_quads(const uint32_t* poly, int x, uint4 (&k)[4]) {
   uint32_t o[16];
 #pragma unroll
-  for (int h = 0; h < 16; h++) {
-    const int j = ((h & 1) << 3) | ((h & 2) << 1) | ((h & 4) >> 1) | ((h & 8) >> 3);
-    o[j] = z[h];
+  for (int a = 0; a < 4; a++) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(poly + 512 * a + 4 * x));
+    o[h_of(4 * a)] = v.x;
+    o[h_of(4 * a + 1)] = v.y;
+    o[h_of(4 * a + 2)] = v.z;
+    o[h_of(4 * a + 3)] = v.w;
   }
 #pragma unroll
-  for (int r4 = 0; r4 < 4; r4++) y[r4] = make_uint4(o[4 * r4], o[4 * r4 + 1], o[4 * r4 + 2], o[4 * r4 + 3]);
+  for (int r4 = 0; r4 < 4; r4++) k[r4] = make_uint4(o[4 * r4], o[4 * r4 + 1], o[4 * r4 + 2], o[4 * r4 + 3]);
 }
-
-// Load a 16-slot run of a key slice (uint4 x 4; y: rotated from the body
-// table when `ybody`).
-__device__ __forceinline__ void key_run(const uint32_t* p, uint4 (&k)[4]) {
-  const uint4* k4 = reinterpret_cast<const uint4*>(p);
+__device__ __forceinline__ void key_rows(const uint32_t* poly, int x, uint32_t rot, uint4 (&k)[4]) {
+  uint32_t o[16];
 #pragma unroll
-  for (int r4 = 0; r4 < 4; r4++) k[r4] = __ldg(k4 + r4);
+  for (int h = 0; h < 16; h++) o[h_of(h)] = __ldg(poly + row_word((h + rot) & 15, x));
+#pragma unroll
+  for (int r4 = 0; r4 < 4; r4++) k[r4] = make_uint4(o[4 * r4], o[4 * r4 + 1], o[4 * r4 + 2], o[4 * r4 + 3]);
 }
 
 __device__ __forceinline__ uint32_t u4e(const uint4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }

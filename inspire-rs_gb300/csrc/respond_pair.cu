@@ -317,6 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RBLOCK, 1)
     const int p = i & 1;
     uint32_t* TC = smem + L::TC + p * 2 * N;
     const size_t yoff = ybody ? (size_t)i * ELL * 2 * N : 0;  // body tables: the key slices of i = 0, rotated
+    const uint32_t yrot = ybody ? rot_rows(gamma, i, x) : 0;
     if (tid == 0 && i >= 2) prefetch_l2(Eg_at() + (size_t)(i - 2) * ELL * N, sizeof(uint32_t) * ELL * N);
     // [A]
     if (tid < 2 * NTT_GT) {
@@ -349,15 +350,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RBLOCK, 1)
     // [C]
     if (g < 2) {
       const int kd = g;
-      const size_t off = ((size_t)(i * ELL + kd) * 2 + r) * N + 16 * x;
+      const size_t off = ((size_t)(i * ELL + kd) * 2 + r) * N;
       uint4 wv[4], yv[4];
-      key_run(A.what + off, wv);  // this step's key slices, fetched before the transform
-      key_run(Y + off - yoff, yv);
+      key_quads(A.what + off, x, wv);  // this step's key slices, fetched before the transform
+      key_rows(Y + off - yoff, x, yrot, yv);
       uint32_t v[16];
 #pragma unroll
       for (int j = 0; j < 16; j++) v[j] = TC[kd * N + x + 128 * j];
       ntt_fwd(v, SC + kd * NTT_SCRATCH, fwd_tw(C), q, x, 2 + kd);  // slots 16x.., [0, 14q)
-      if (ybody) rotate_key_run(yv, i, x);
       uint32_t* accb = ACC + kd * N;
       uint32_t* pdst = kd == 0 ? SCAT + p * N : PB1;
 #pragma unroll
@@ -399,7 +399,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RBLOCK, 1)
     } else if (g == 2) {
       // PB2 = R_{i+1} w'2
       uint4 wv[4];
-      key_run(A.what + ((size_t)(i * ELL + 2) * 2 + r) * N + 16 * x, wv);
+      key_quads(A.what + ((size_t)(i * ELL + 2) * 2 + r) * N, x, wv);
       uint32_t rs[16], pr[16];
       load16(RN, x, rs);
 #pragma unroll
@@ -409,8 +409,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RBLOCK, 1)
     } else if (g == 3) {
       // b += R_{i+1} y'2
       uint4 k2[4];
-      key_run(Y + ((size_t)(i * ELL + 2) * 2 + r) * N + 16 * x - yoff, k2);
-      if (ybody) rotate_key_run(k2, i, x);
+      key_rows(Y + ((size_t)(i * ELL + 2) * 2 + r) * N - yoff, x, yrot, k2);
       uint32_t* accb = ACC + 2 * N;
 #pragma unroll
       for (int r4 = 0; r4 < 4; r4++) {

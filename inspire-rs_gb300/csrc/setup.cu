@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "respond_common.cuh"
 
 namespace ig {
 
@@ -64,11 +65,12 @@ __global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, cons
     for (int rr = 0; rr < 4; rr++) dst[rr] = make_uint4(v[4 * rr], v[4 * rr + 1], v[4 * rr + 2], v[4 * rr + 3]);
   }
   __syncthreads();
-  // Stored by recursion step: the scatter of R_i reads, at source slot u, the
-  // DFT output k = (2brv(u)+1) m_i mod gamma with m_i = (gamma - i) mod gamma
-  // (scatter_r), so entry [i][t][u] holds output k of (t, u) and a warp's
-  // loads at consecutive slots are contiguous.  For odd 2brv(u)+1 the map
-  // i -> k is a bijection: the table is a permutation of the outputs.
+  // Stored by recursion step i and, within it, by the slot s that R_i takes
+  // the value at: source slot u contributes the DFT output k = (2brv(u)+1) m_i
+  // mod gamma, m_i = (gamma - i) mod gamma, to s = tau_i^-1(u), i.e. (rot_rows)
+  // to row h - rot of the same 16-slot run.  For odd 2brv(u)+1 the map i -> k
+  // is a bijection: the table is a permutation of the outputs.  A warp's 32
+  // source slots are two runs, whose words of each quad plane are 32 bytes.
   uint32_t* Eo = E + (((size_t)s * 2 + r) * gamma * ELL + t) * N;
   for (int v = 0; v < N / BLOCK; v++) {
     const int u = tid + BLOCK * v;
@@ -77,6 +79,7 @@ __global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, cons
 #pragma unroll
     for (int j = 0; j < MAX_GAMMA; j++)
       if (j < gamma) c[j] = mont_mul(Dh[j * N + u], __ldg(C.psi_pow + ((e * j) & (2 * N - 1))), q, qinv);
+    const int ux = u >> 4, uh = h_of(u & 15);
     for (int i = 0; i < gamma; i++) {
       const int k = (int)((e * ((uint32_t)(gamma - i) & (uint32_t)(gamma - 1))) & (uint32_t)(gamma - 1));
       uint64_t T = 0;
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, cons
         if (j < gamma) T += (uint64_t)zp[(k * j) & (gamma - 1)] * c[j];
       // the two REDCs divided by 2^64; e_scale = gamma^-1 n^-1 2^96 leaves
       // the factor 2^32 gamma^-1 n^-1
-      Eo[(size_t)i * ELL * N + u] = mul_shoup(redc(T, q, qinv), C.e_scale, C.e_scale_p, q);
+      Eo[(size_t)i * ELL * N + quad_word((uh - (int)rot_rows(gamma, i, ux)) & 15, ux)] = mul_shoup(redc(T, q, qinv), C.e_scale, C.e_scale_p, q);
     }
   }
 }
@@ -125,42 +128,13 @@ __global__ void __launch_bounds__(BLOCK) crs_what_kernel(const DevParams P, cons
   }
 }
 
-// Client key table from y_body: generate_rotations (inspiring2.rs:1309-1323)
-// followed by the forward NTT of packing_online (:1199-1213).  tau in the
-// coefficient domain is the slot permutation in the NTT domain on both
-// residues.  Stored times n^-1 2^32.  The first nrot rotations are written
-// (nrot = 1: the body table NTT(y_body[k]), rotated by the Respond kernel).
-__global__ void __launch_bounds__(BLOCK) client_ybody_kernel(const DevParams P, const uint64_t* __restrict__ yb,
-                                                             uint32_t* __restrict__ yhat, int nrot) {
-  __shared__ __align__(16) uint32_t W[2][N];
-  __shared__ uint32_t SC[2][NTT_SCRATCH];
-  const int k = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
-  const int gamma = P.gamma;
-  const ResidueConsts& C = P.r[g];
-  {
-    uint32_t v[16];
-#pragma unroll
-    for (int rr = 0; rr < 16; rr++) v[rr] = (uint32_t)yb[((size_t)k * 2 + g) * N + x + 128 * rr];
-    ntt_fwd(v, SC[g], fwd_tw(C), C.q, x, 1 + g);
-#pragma unroll
-    for (int rr = 0; rr < 16; rr++) W[g][16 * x + rr] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
-  }
-  __syncthreads();
-  for (int i = 0; i + 1 < gamma && i < nrot; i++) {
-    const uint32_t tg = gen_pow(gamma, i);
-    for (int v = 0; v < N / BLOCK; v++) {
-      const int s = tid + BLOCK * v;
-      const uint32_t es = 2 * brv11(s) + 1;
-      const int u = brv11(((tg * es) & (2 * N - 1)) >> 1);
-      yhat[(((size_t)i * ELL + k) * 2 + 0) * N + s] = W[0][u];
-      yhat[(((size_t)i * ELL + k) * 2 + 1) * N + s] = W[1][u];
-    }
-  }
-}
-
-// Client key table from an explicit y_all ((gamma-1)*ELL coefficient polys).
-__global__ void __launch_bounds__(BLOCK) client_yall_kernel(const DevParams P, const uint64_t* __restrict__ ya,
-                                                            uint32_t* __restrict__ yhat) {
+// Client key table from y_body: the forward NTT of packing_online
+// (inspiring2.rs:1199-1213) of y_body[k], in rows [h][x] and times n^-1 2^32.
+// generate_rotations (:1309-1323) is a rotation of the rows (rot_rows), which
+// the Respond kernels apply as they read.  An explicit y_all
+// ((gamma-1)*ELL coefficient polys) goes through the same kernel.
+__global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams P, const uint64_t* __restrict__ ya,
+                                                                uint32_t* __restrict__ yhat) {
   __shared__ uint32_t SC[2][NTT_SCRATCH];
   const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
   const ResidueConsts& C = P.r[g];
@@ -170,7 +144,7 @@ __global__ void __launch_bounds__(BLOCK) client_yall_kernel(const DevParams P, c
   ntt_fwd(v, SC[g], fwd_tw(C), C.q, x, 1 + g);
 #pragma unroll
   for (int rr = 0; rr < 16; rr++)
-    yhat[((size_t)p * 2 + g) * N + 16 * x + rr] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
+    yhat[((size_t)p * 2 + g) * N + row_word(h_of(rr), x)] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
 }
 
 // Key tables with the third gadget digit folded in.  In the NTT domain of
@@ -179,18 +153,22 @@ __global__ void __launch_bounds__(BLOCK) client_yall_kernel(const DevParams P, c
 // (k0, k1, k2):  k0 NTT(d0) + k1 NTT(d1) + k2 NTT(d2)
 //   = (k0 - z^-2 k2) NTT(d0) + (k1 - z^-1 k2) NTT(d1) + (z^-2 k2) R.
 // With R kept as n^-1 R (the Respond kernel's R_{i+1}), the third key is
-// n z^-2 k2.  `tbl` holds ngroups triples [g][k<3][2][N] (any constant
-// scaling, applied alike to the three keys), rewritten in place.
-__global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams P, uint32_t* __restrict__ tbl,
-                                                                 int ngroups) {
+// n z^-2 k2.  src and dst hold ngroups triples [g][k<3][2][N] (any constant
+// scaling, applied alike to the three keys).  In place, or with `quads` from
+// slot order into quads [h >> 2][x][h & 3].
+__global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams P, const uint32_t* src, uint32_t* dst,
+                                                                 int ngroups, bool quads) {
   const size_t per = (size_t)2 * N;
   const size_t total = (size_t)ngroups * per;
   for (size_t idx = (size_t)blockIdx.x * BLOCK + threadIdx.x; idx < total; idx += (size_t)gridDim.x * BLOCK) {
     const size_t g = idx / per, rs = idx - g * per;
     const int r = (int)(rs >> LOGN);
     const ResidueConsts& C = P.r[r];
-    uint32_t* t = tbl + g * 3 * per + rs;
-    const uint32_t k0 = t[0], k1 = t[per], k2 = t[2 * per];
+    const int w = (int)(rs & (N - 1));
+    const int x = (w >> 2) & 127, h = ((w >> 9) << 2) | (w & 3);
+    const uint32_t* f = src + g * 3 * per + (quads ? (size_t)r * N + 16 * x + h_of(h) : rs);
+    uint32_t* t = dst + g * 3 * per + rs;
+    const uint32_t k0 = f[0], k1 = f[per], k2 = f[2 * per];
     t[0] = sub_mod(k0, mul_shoup(k2, C.d2_z2, C.d2_z2_p, C.q), C.q);
     t[per] = sub_mod(k1, mul_shoup(k2, C.d2_z1, C.d2_z1_p, C.q), C.q);
     t[2 * per] = mul_shoup(k2, C.d2_nz2, C.d2_nz2_p, C.q);
@@ -199,11 +177,12 @@ __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams
 
 }  // namespace
 
-cudaError_t launch_fold_third_digit(const DevParams& P, uint32_t* tbl, int ngroups, cudaStream_t st) {
+cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, bool quads,
+                                    cudaStream_t st) {
   if (ngroups <= 0) return cudaSuccess;
   const size_t total = (size_t)ngroups * 2 * N;
   const unsigned blocks = (unsigned)std::min<size_t>((total + BLOCK - 1) / BLOCK, 4096);
-  fold_third_digit_kernel<<<blocks, BLOCK, 0, st>>>(P, tbl, ngroups);
+  fold_third_digit_kernel<<<blocks, BLOCK, 0, st>>>(P, src, dst, ngroups, quads);
   return cudaGetLastError();
 }
 
@@ -234,16 +213,10 @@ cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t*
   return cudaGetLastError();
 }
 
-cudaError_t launch_client_from_ybody(const DevParams& P, const uint64_t* ybody, uint32_t* yhat, int nrot,
-                                     cudaStream_t st) {
-  if (P.gamma < 2) return cudaSuccess;
-  client_ybody_kernel<<<ELL, BLOCK, 0, st>>>(P, ybody, yhat, nrot);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_client_from_yall(const DevParams& P, const uint64_t* yall, uint32_t* yhat, cudaStream_t st) {
-  if (P.gamma < 2) return cudaSuccess;
-  client_yall_kernel<<<(P.gamma - 1) * ELL, BLOCK, 0, st>>>(P, yall, yhat);
+cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, uint32_t* yhat,
+                                   cudaStream_t st) {
+  if (npolys <= 0) return cudaSuccess;
+  client_keys_ntt_kernel<<<npolys, BLOCK, 0, st>>>(P, polys, yhat);
   return cudaGetLastError();
 }
 
