@@ -140,7 +140,8 @@ int build_key_table(inspire_ctx* c, const uint64_t* y_body, const uint64_t* y_al
     memcpy(c->h_keys.p, y_all ? y_all : y_body, in_bytes);
     CUDA_TRY(cudaMemcpyAsync(c->d_keys.p, c->h_keys.p, in_bytes, cudaMemcpyHostToDevice, c->stream));
     CUDA_TRY(cudaEventRecord(c->keys_ev, c->stream));
-    CUDA_TRY(launch_client_keys_ntt(c->P, c->d_keys.as<uint64_t>(), (int)in_polys, m.as<uint32_t>(), c->stream));
+    CUDA_TRY(launch_client_keys_ntt(c->P, c->d_keys.as<uint64_t>(), (int)in_polys, y_all != nullptr, m.as<uint32_t>(),
+                                    c->stream));
     // the Respond kernel multiplies the third key by R_{i+1} instead of NTT(d2)
     CUDA_TRY(launch_fold_third_digit(c->P, m.as<uint32_t>(), m.as<uint32_t>(), (int)in_polys / ELL, false, c->stream));
     if (sync) CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -590,8 +591,8 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
     return fail(INSPIRE_ERR_CUDA, "cannot read the SM count");
   }
   c->pair_max.store(c->sm_count / 2);
-  // tables per residue: fwd pairs (2N words), inv pairs (2N words), psi_pow (2N)
-  const size_t per = 6 * (size_t)N;
+  // tables per residue: fwd pairs (2N words), inv pairs (2N words), psi_pow (2N), centred fwd pairs (2N)
+  const size_t per = 8 * (size_t)N;
   std::vector<uint32_t> host(2 * per);
   DevParams& P = c->P;
   memset(&P, 0, sizeof(P));
@@ -605,6 +606,11 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
       t[2 * k + 1] = shoup(w, qm);
       t[2 * N + 2 * k] = (uint32_t)wi;
       t[2 * N + 2 * k + 1] = shoup(wi, qm);
+      // w in (-q/2, q/2), companion round(w 2^32 / q) (below 2^31 in absolute value)
+      const bool neg = w > qm / 2;
+      const uint64_t mag = neg ? qm - w : w, mp = ((mag << 33) + qm) / (2 * qm);
+      t[6 * N + 2 * k] = neg ? 0u - (uint32_t)mag : (uint32_t)mag;
+      t[6 * N + 2 * k + 1] = neg ? 0u - (uint32_t)mp : (uint32_t)mp;
     }
     uint64_t pw = 1;
     for (int k = 0; k < 2 * N; k++) {
@@ -642,6 +648,12 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
   }
   P.q0inv_q1 = (uint32_t)inv_prime(q0, q1);
   P.q0inv_q1_p = shoup(P.q0inv_q1, q1);
+  for (int r = 0; r < 2; r++) {
+    const uint64_t mine = r ? q1 : q0, other = r ? q0 : q1;
+    P.r[r].crt_inv = (uint32_t)inv_prime(mine, other);
+    P.r[r].crt_inv_p = shoup(P.r[r].crt_inv, other);
+    P.r[r].crt_off = (uint32_t)((mine + other - 1) / other * other);
+  }
   {
     const uint64_t r64_0 = (uint64_t)(((u128)1 << 64) % q0), r64_1 = (uint64_t)(((u128)1 << 64) % q1);
     const uint64_t a = (uint64_t)((u128)N * r64_0 % q0);
@@ -670,6 +682,7 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
     P.r[r].fwd = reinterpret_cast<const uint2*>(base);
     P.r[r].inv = reinterpret_cast<const uint2*>(base + 2 * N);
     P.r[r].psi_pow = base + 4 * N;
+    P.r[r].sfwd = reinterpret_cast<const uint2*>(base + 6 * N);
   }
   e = prepare_respond_kernels();
   if (e == cudaSuccess) e = prepare_respond_pair_kernels();

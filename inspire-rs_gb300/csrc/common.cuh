@@ -25,6 +25,9 @@ struct ResidueConsts {
   const uint2* fwd;                  // {psi^brv(k), Shoup companion}, k in [1, n)
   const uint2* inv;                  // {psi^-brv(k), Shoup companion}
   const uint32_t* psi_pow;           // psi^e, e in [0, 2n)
+  const uint2* sfwd;                 // fwd with w in (-q/2, q/2) and round(w 2^32 / q) (ntt_joint.cuh)
+  uint32_t crt_inv, crt_inv_p;       // q^-1 mod the other modulus (crt_compose_from)
+  uint32_t crt_off;                  // the other modulus's first multiple from q on
   uint32_t r64, r64_p;               // 2^64 mod q: reference Montgomery factor
   uint32_t ref_inv_scale, ref_inv_scale_p;  // n^-1 * 2^-64 mod q
   uint32_t ninv_mont, ninv_mont_p;   // n^-1 * 2^32 mod q
@@ -50,6 +53,7 @@ struct DevParams {
 };
 
 __device__ __forceinline__ TwiddleRef fwd_tw(const ResidueConsts& c) { return {c.fwd}; }
+__device__ __forceinline__ TwiddleRef sfwd_tw(const ResidueConsts& c) { return {c.sfwd}; }
 __device__ __forceinline__ TwiddleRef inv_tw(const ResidueConsts& c) { return {c.inv}; }
 
 __device__ __forceinline__ uint32_t brv11(uint32_t x) { return __brev(x) >> (32 - LOGN); }
@@ -62,6 +66,16 @@ __device__ __forceinline__ uint64_t crt_compose(const DevParams& P, uint32_t a0,
   uint32_t d = sub_mod(a1, a0m, q1);
   uint32_t t = mul_shoup(d, P.q0inv_q1, P.q0inv_q1_p, q1);
   return (uint64_t)a0 + (uint64_t)q0 * t;
+}
+
+// The same composite coefficient from one residue's side: a mod q = C.q and b
+// mod the other modulus qo give a + q ((b - a) q^-1 mod qo).
+__device__ __forceinline__ uint64_t crt_compose_from(const ResidueConsts& C, uint32_t qo, uint32_t a, uint32_t b) {
+  const uint32_t t = mul_shoup(b - a + C.crt_off, C.crt_inv, C.crt_inv_p, qo);
+  const uint64_t w = (uint64_t)C.q * t;  // a is added outside the multiply-add, which would need a 64-bit copy of it
+  uint32_t lo, hi;
+  asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, %4, 0;" : "=r"(lo), "=r"(hi) : "r"((uint32_t)w), "r"(a), "r"((uint32_t)(w >> 32)));
+  return ((uint64_t)hi << 32) | lo;
 }
 
 // Residue 1 rebuilt from a residue-0 NTT value as the reference does in

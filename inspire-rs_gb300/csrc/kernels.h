@@ -199,8 +199,9 @@ cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t*
 cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, bool quads,
                                     cudaStream_t st);
 // NTT of a client's key polys [npolys][2][N] (y_body: ELL polys, whose
-// rotations the Respond kernels form; or an explicit y_all).
-cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, uint32_t* yhat,
+// rotations the Respond kernels form; or, rotated, an explicit y_all, its
+// rows turned so that the kernels read either the same way).
+cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, bool rotated, uint32_t* yhat,
                                    cudaStream_t st);
 
 // kernel-level operations

@@ -7,7 +7,17 @@
 //  * K polynomials share every twiddle load and every address, and give each
 //    warp K times the independent butterflies, so that few warps fill the
 //    integer multiply-add pipe (64 lane-operations per cycle and SM, a
-//    high product costs two).
+//    high product costs two: at most 16 butterflies per cycle).
+//  * One table of centred twiddles w in (-q/2, q/2) with companions
+//    w' = round(w 2^32 / q) and signed products: for |a| < 2^31,
+//    a w - floor(a w' / 2^32) q = a w mod q in (-|a| / 2^33 q, q + |a| / 2^33 q).
+//    The forward butterfly is then a' = (b w + a) - h q, b' = 2a - a': four
+//    instructions, none with three different added registers (measured in
+//    registers: 14.5 butterflies per cycle and SM, 12.4 as x + t, x - t + 2q
+//    on unsigned values); the inverse one takes the difference without an
+//    offset (13.9, 11.6 with it).
+//  * Values are reduced only where 32 bits would overflow: their bounds are
+//    tracked per register at compile time.
 //  * Both exchanges keep one XOR-swizzled index map, jsw, in place: a thread
 //    overwrites exactly the words it read last, so an exchange needs one
 //    barrier (between its writes and its reads) instead of two.  Elements
@@ -18,8 +28,6 @@
 //    for k in [m, 2m), m a power of two (brv(k) is 2^(10-s) (2 i' + 1), and
 //    complementing i' inside its level negates the exponent mod N), so the
 //    difference is taken the other way round.  Half the table stays in L1.
-//  * The inverse's sums are reduced only where a 32-bit overflow could
-//    follow (bounds are tracked per register at compile time).
 #pragma once
 #include <cstdint>
 
@@ -35,66 +43,85 @@ __device__ __forceinline__ int jsw(int e) { return e ^ (((e >> 5) & 3) << 2) ^ (
 
 // x in [0, b q) -> [0, max(c, b - c) q)
 __device__ __forceinline__ uint32_t csub(uint32_t x, uint32_t cq) { return min(x, x - cq); }
+// signed x in (-2 c, 2 c) -> [-c, c), c a multiple of q
+__device__ __forceinline__ uint32_t centre(uint32_t x, uint32_t c) {
+  return x - c + ((uint32_t)((int32_t)x >> 31) & (2 * c));
+}
 
-// Exchange accesses.  tr: elements 128 b + y + 8 r; ru: elements 16 x + r.
+// 2 a - b as additions: the compiler would turn 2 a - b into a multiply-add,
+// on the pipe that the transforms are bound by.
+__device__ __forceinline__ uint32_t twice_minus(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("sub.u32 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d + a;
+}
+
+// Exchange buffers are addressed by 32-bit shared-memory addresses, a
+// multiple of 128 bytes, so that a swizzled access is one XOR away from its
+// thread's base.
+__device__ __forceinline__ uint32_t jx_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t& jx_at(uint32_t a) {
+  return *reinterpret_cast<uint32_t*>(__cvta_shared_to_generic(a));
+}
+__device__ __forceinline__ uint4& jx_at4(uint32_t a) { return *reinterpret_cast<uint4*>(__cvta_shared_to_generic(a)); }
+
+// Byte offsets of this thread's first element in the three layouts.
+__device__ __forceinline__ uint32_t jx_co(int x) { return 4u * (uint32_t)(x ^ (((x >> 5) & 3) << 2)); }
+__device__ __forceinline__ uint32_t jx_tr(int x) {
+  return 4u * (uint32_t)(128 * (x >> 3) + ((x & 7) ^ (((x >> 3) & 3) << 3)));
+}
+__device__ __forceinline__ uint32_t jx_ru(int x) {
+  return 4u * (uint32_t)((16 * x) ^ (((x >> 1) & 3) << 2) ^ (((x >> 3) & 3) << 3));
+}
+// Element r's distance from it: an XOR of bits 2-6 and a multiple of 128.
+__host__ __device__ constexpr uint32_t jx_co_x(int r) { return 4u * ((r & 3) << 3); }
+__host__ __device__ constexpr uint32_t jx_co_o(int r) { return 4u * 128u * (uint32_t)r; }
+__host__ __device__ constexpr uint32_t jx_tr_x(int r) { return 4u * ((((r & 3) ^ (r >> 3)) << 3) ^ (((r >> 2) & 1) << 2)); }
+__host__ __device__ constexpr uint32_t jx_tr_o(int r) { return 4u * 32u * (uint32_t)(r >> 2); }
+
 template <int K>
-__device__ __forceinline__ void jx_store_tr(const uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = 128 * (x >> 3) + ((x & 7) ^ (((x >> 3) & 3) << 3));
+__device__ __forceinline__ void jx_store_tr(const uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const int o = (e0 ^ (((r & 3) ^ (r >> 3)) << 3) ^ (((r >> 2) & 1) << 2)) + 32 * (r >> 2);
+  for (int r = 0; r < 16; r++)
 #pragma unroll
-    for (int k = 0; k < K; k++) sc[k][o] = v[k][r];
-  }
+    for (int k = 0; k < K; k++) jx_at(((sc[k] + jx_tr(x)) ^ jx_tr_x(r)) + jx_tr_o(r)) = v[k][r];
 }
 template <int K>
-__device__ __forceinline__ void jx_load_tr(uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = 128 * (x >> 3) + ((x & 7) ^ (((x >> 3) & 3) << 3));
+__device__ __forceinline__ void jx_load_tr(uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const int o = (e0 ^ (((r & 3) ^ (r >> 3)) << 3) ^ (((r >> 2) & 1) << 2)) + 32 * (r >> 2);
+  for (int r = 0; r < 16; r++)
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k][r] = sc[k][o];
-  }
+    for (int k = 0; k < K; k++) v[k][r] = jx_at(((sc[k] + jx_tr(x)) ^ jx_tr_x(r)) + jx_tr_o(r));
 }
 template <int K>
-__device__ __forceinline__ void jx_store_co(const uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = x ^ (((x >> 5) & 3) << 2);
+__device__ __forceinline__ void jx_store_co(const uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const int o = (e0 ^ ((r & 3) << 3)) + 128 * r;
+  for (int r = 0; r < 16; r++)
 #pragma unroll
-    for (int k = 0; k < K; k++) sc[k][o] = v[k][r];
-  }
+    for (int k = 0; k < K; k++) jx_at(((sc[k] + jx_co(x)) ^ jx_co_x(r)) + jx_co_o(r)) = v[k][r];
 }
 template <int K>
-__device__ __forceinline__ void jx_load_co(uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = x ^ (((x >> 5) & 3) << 2);
+__device__ __forceinline__ void jx_load_co(uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
-  for (int r = 0; r < 16; r++) {
-    const int o = (e0 ^ ((r & 3) << 3)) + 128 * r;
+  for (int r = 0; r < 16; r++)
 #pragma unroll
-    for (int k = 0; k < K; k++) v[k][r] = sc[k][o];
-  }
+    for (int k = 0; k < K; k++) v[k][r] = jx_at(((sc[k] + jx_co(x)) ^ jx_co_x(r)) + jx_co_o(r));
 }
 template <int K>
-__device__ __forceinline__ void jx_store_ru(const uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = (16 * x) ^ (((x >> 1) & 3) << 2) ^ (((x >> 3) & 3) << 3);
+__device__ __forceinline__ void jx_store_ru(const uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
   for (int c = 0; c < 4; c++)
 #pragma unroll
     for (int k = 0; k < K; k++)
-      *reinterpret_cast<uint4*>(sc[k] + (e0 ^ (4 * c))) =
-          make_uint4(v[k][4 * c], v[k][4 * c + 1], v[k][4 * c + 2], v[k][4 * c + 3]);
+      jx_at4((sc[k] + jx_ru(x)) ^ (16u * c)) = make_uint4(v[k][4 * c], v[k][4 * c + 1], v[k][4 * c + 2], v[k][4 * c + 3]);
 }
 template <int K>
-__device__ __forceinline__ void jx_load_ru(uint32_t (&v)[K][16], uint32_t* const (&sc)[K], int x) {
-  const int e0 = (16 * x) ^ (((x >> 1) & 3) << 2) ^ (((x >> 3) & 3) << 3);
+__device__ __forceinline__ void jx_load_ru(uint32_t (&v)[K][16], const uint32_t (&sc)[K], int x) {
 #pragma unroll
   for (int c = 0; c < 4; c++)
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      const uint4 t = *reinterpret_cast<const uint4*>(sc[k] + (e0 ^ (4 * c)));
+      const uint4 t = jx_at4((sc[k] + jx_ru(x)) ^ (16u * c));
       v[k][4 * c] = t.x;
       v[k][4 * c + 1] = t.y;
       v[k][4 * c + 2] = t.z;
@@ -102,67 +129,106 @@ __device__ __forceinline__ void jx_load_ru(uint32_t (&v)[K][16], uint32_t* const
     }
 }
 
+// ---- bounds: element r is below B[r] q / 64 (in absolute value in the
+//      forward transform); 32-bit signed values allow 8 q = 512 units ----
+constexpr int JB_MAX = 512;
+
+__host__ __device__ constexpr int jb_max(const int (&B)[16]) {
+  int m = 0;
+  for (int r = 0; r < 16; r++) m = B[r] > m ? B[r] : m;
+  return m;
+}
+
 // Forward stage S (element r pairs with r + H, twiddle (1 << S) + first +
 // (r >> SHIFT)) of K polynomials.
 template <int K, int S, int SHIFT>
-__device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], TwiddleRef tw, int first, uint32_t q, uint32_t q2) {
+__device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], int (&B)[16], TwiddleRef tw, int first, uint32_t q) {
   constexpr int CNT = 16 >> SHIFT;
   constexpr int H = (S < 4) ? (8 >> S) : (S < 8 ? (8 >> (S - 4)) : (4 >> (S - 8)));
   uint2 run[CNT];
   tw_run<CNT>(tw, (1 << S) + first, run);
 #pragma unroll
   for (int r = 0; r < 16; r++)
-    if ((r & H) == 0)
+    if ((r & H) == 0) {
+      const int grow = 64 + (B[r + H] + 31) / 32;  // |b w mod q| <= q (1 + |b| / 2^33)
+      if (B[r] + grow > JB_MAX) {
 #pragma unroll
-      for (int k = 0; k < K; k++) ct_bfly(v[k][r], v[k][r + H], run[r >> SHIFT], q, q2);
+        for (int k = 0; k < K; k++) v[k][r] = centre(v[k][r], 4 * q);
+        B[r] = JB_MAX / 2;
+      }
+      const uint2 w = run[r >> SHIFT];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const uint32_t a = v[k][r], b = v[k][r + H];
+        const uint32_t h = (uint32_t)__mulhi((int)b, (int)w.y);
+        const uint32_t s = b * w.x + a;
+        v[k][r] = s - h * q;
+        v[k][r + H] = twice_minus(a, v[k][r]);
+      }
+      B[r] += grow;
+      B[r + H] = B[r];
+    }
 }
 
 // Forward transforms, coefficient layout (v[k][r] = a_k[x + 128 r]) in, slot
-// layout (v[k][r] = A_k[16 x + r], [0, 14 q)) out.  Inputs below 2^20
-// (gadget digits), or below q with FULL.  sc[k]: K exchange buffers of 2048
-// words, whose words at this thread's coefficient positions (jsw(x + 128 r))
-// must be free to this thread; bar: the group's named barrier.
+// layout (v[k][r] = A_k[16 x + r], signed, below JFWD_OUT q / 64) out.
+// Inputs below 2^20 (gadget digits), or in [0, q) with FULL.  sc[k]: K
+// exchange buffers of 2048 words, whose words at this thread's coefficient
+// positions (jsw(x + 128 r)) must be free to this thread; bar: the group's
+// named barrier.
 //
-// Bounds (q < 2^28, so 16 q < 2^32): a stage adds at most 2 q, or 1 + B / 16
-// to its sums where the twiddled operand is below B q.  Digits: below 8 q +
-// 2^20 after stages 0-3; in stages 4-7 only element 14, the one that takes
-// the difference three times, could pass 16 q, and is reduced before stage
-// 7.  One reduction below 8 q before stages 8-10, which end below 14 q.
-template <int K, bool FULL>
-__device__ __forceinline__ void jntt_fwd(uint32_t (&v)[K][16], uint32_t* const (&sc)[K], TwiddleRef tw, uint32_t q,
-                                         int x, int bar) {
-  const uint32_t q2 = 2 * q, q8 = 8 * q;
-  jfwd_stage<K, 0, 4>(v, tw, 0, q, q2);
-  jfwd_stage<K, 1, 3>(v, tw, 0, q, q2);
-  jfwd_stage<K, 2, 2>(v, tw, 0, q, q2);
-  jfwd_stage<K, 3, 1>(v, tw, 0, q, q2);
-  if (FULL) {
+// Digits count as 1/64 q: for q near 2^28 they are 1/256 q, and for smaller q
+// every bound, an absolute sum of 2^20 and multiples of q, is smaller too.
+constexpr int JFWD_OUT = 416;
+struct NoHook {
+  __device__ __forceinline__ void operator()() const {}
+};
+// `hook` runs before stages 8-10 (to issue loads that they can hide).
+template <int K, bool FULL, class Hook = NoHook>
+__device__ __forceinline__ void jntt_fwd(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef tw, uint32_t q, int x,
+                                         int bar, Hook&& hook = Hook()) {
+  int B[16];
 #pragma unroll
-    for (int k = 0; k < K; k++) reduce_8q(v[k], q);  // < 9 q -> < 8 q
-  }
+  for (int r = 0; r < 16; r++) B[r] = FULL ? 64 : 1;
+  jfwd_stage<K, 0, 4>(v, B, tw, 0, q);
+  jfwd_stage<K, 1, 3>(v, B, tw, 0, q);
+  jfwd_stage<K, 2, 2>(v, B, tw, 0, q);
+  jfwd_stage<K, 3, 1>(v, B, tw, 0, q);
   jx_store_co<K>(v, sc, x);
   group_sync(bar);
   jx_load_tr<K>(v, sc, x);
+  {
+    const int m = jb_max(B);
+#pragma unroll
+    for (int r = 0; r < 16; r++) B[r] = m;
+  }
   const int b = x >> 3;
-  jfwd_stage<K, 4, 4>(v, tw, b, q, q2);
-  jfwd_stage<K, 5, 3>(v, tw, b << 1, q, q2);
-  jfwd_stage<K, 6, 2>(v, tw, b << 2, q, q2);
-#pragma unroll
-  for (int k = 0; k < K; k++) v[k][14] = csub(v[k][14], q8);
-  jfwd_stage<K, 7, 1>(v, tw, b << 3, q, q2);
-#pragma unroll
-  for (int k = 0; k < K; k++) reduce_8q(v[k], q);  // < 16 q -> < 8 q
+  jfwd_stage<K, 4, 4>(v, B, tw, b, q);
+  jfwd_stage<K, 5, 3>(v, B, tw, b << 1, q);
+  jfwd_stage<K, 6, 2>(v, B, tw, b << 2, q);
+  jfwd_stage<K, 7, 1>(v, B, tw, b << 3, q);
   jx_store_tr<K>(v, sc, x);
   __syncwarp();
   jx_load_ru<K>(v, sc, x);
-  jfwd_stage<K, 8, 3>(v, tw, x << 1, q, q2);
-  jfwd_stage<K, 9, 2>(v, tw, x << 2, q, q2);
-  jfwd_stage<K, 10, 1>(v, tw, x << 3, q, q2);
+  hook();
+  {
+    const int m = jb_max(B);
+#pragma unroll
+    for (int r = 0; r < 16; r++) B[r] = m;
+  }
+  jfwd_stage<K, 8, 3>(v, B, tw, x << 1, q);
+  jfwd_stage<K, 9, 2>(v, B, tw, x << 2, q);
+  jfwd_stage<K, 10, 1>(v, B, tw, x << 3, q);
 }
 
-// Inverse stage S.  B[r]: bound of element r in multiples of q, known at
-// compile time (the loops unroll); sums that could pass 16 q are avoided by
-// reducing an operand above 8 q first.
+// A forward output brought to [0, q).
+__device__ __forceinline__ uint32_t jcanon_fwd(uint32_t x, uint32_t q) {
+  x = min(x, x + 8 * q);  // negative values are large as unsigned ones
+  return canon16(x, q);
+}
+
+// Inverse stage S on values in [0, B q / 64): differences signed, operands
+// below 8 q; a product of d takes q (1 + |d| / 2^33) around [0, q), plus q.
 template <int K, int S, int SHIFT>
 __device__ __forceinline__ void jinv_stage(uint32_t (&v)[K][16], int (&B)[16], TwiddleRef fwd, int first, uint32_t q) {
   constexpr int CNT = 16 >> SHIFT;
@@ -173,25 +239,26 @@ __device__ __forceinline__ void jinv_stage(uint32_t (&v)[K][16], int (&B)[16], T
 #pragma unroll
   for (int r = 0; r < 16; r++)
     if ((r & H) == 0) {
-      if (B[r] + B[r + H] > 16) {
 #pragma unroll
-        for (int e = 0; e < 2; e++) {
-          if (B[r + e * H] > 8) {
+      for (int e = 0; e < 2; e++) {
+        if (B[r + e * H] > JB_MAX) {
 #pragma unroll
-            for (int k = 0; k < K; k++) v[k][r + e * H] = csub(v[k][r + e * H], 8 * q);
-            B[r + e * H] = 8;
-          }
+          for (int k = 0; k < K; k++) v[k][r + e * H] = csub(v[k][r + e * H], 8 * q);
+          B[r + e * H] = JB_MAX;
         }
       }
-      const uint32_t bq = (uint32_t)B[r] * q;
+      const uint2 w = run[CNT - 1 - (r >> SHIFT)];
 #pragma unroll
       for (int k = 0; k < K; k++) {
-        const uint32_t a = v[k][r], b = v[k][r + H];
-        v[k][r] = a + b;
-        v[k][r + H] = mul_shoup_lazy(b - a + bq, run[CNT - 1 - (r >> SHIFT)], q);
+        const uint32_t a = v[k][r], d = v[k][r + H] - a;
+        v[k][r] = a + v[k][r + H];
+        const uint32_t h = (uint32_t)__mulhi((int)d, (int)w.y);
+        const uint32_t s = d * w.x + q;
+        v[k][r + H] = s - h * q;
       }
+      const int m = B[r] > B[r + H] ? B[r] : B[r + H];
       B[r] += B[r + H];
-      B[r + H] = 2;
+      B[r + H] = 128 + (m + 31) / 32;
     }
 }
 
@@ -202,10 +269,10 @@ __device__ __forceinline__ void jinv_reduce(uint32_t (&v)[K][16], int (&B)[16], 
   for (int r = 0; r < 16; r++) {
 #pragma unroll
     for (int c = 8; c >= C; c >>= 1) {
-      if (B[r] > c) {
+      if (B[r] > 64 * c) {
 #pragma unroll
         for (int k = 0; k < K; k++) v[k][r] = csub(v[k][r], (uint32_t)c * q);
-        B[r] = c;
+        B[r] = 64 * c;
       }
     }
   }
@@ -216,11 +283,11 @@ __device__ __forceinline__ void jinv_reduce(uint32_t (&v)[K][16], int (&B)[16], 
 // words at this thread's slot positions must be free to this thread; it
 // reads its coefficient positions last.
 template <int K>
-__device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], uint32_t* const (&sc)[K], TwiddleRef fwd, uint32_t q,
+__device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef fwd, uint32_t q,
                                          int x, int bar) {
   int B[16];
 #pragma unroll
-  for (int r = 0; r < 16; r++) B[r] = 4;
+  for (int r = 0; r < 16; r++) B[r] = 256;
   jinv_stage<K, 10, 1>(v, B, fwd, x << 3, q);
   jinv_stage<K, 9, 2>(v, B, fwd, x << 2, q);
   jinv_stage<K, 8, 3>(v, B, fwd, x << 1, q);
@@ -230,7 +297,7 @@ __device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], uint32_t* const (
   jx_load_tr<K>(v, sc, x);
   const int b = x >> 3;
 #pragma unroll
-  for (int r = 0; r < 16; r++) B[r] = 4;
+  for (int r = 0; r < 16; r++) B[r] = 256;
   jinv_stage<K, 7, 1>(v, B, fwd, b << 3, q);
   jinv_stage<K, 6, 2>(v, B, fwd, b << 2, q);
   jinv_stage<K, 5, 3>(v, B, fwd, b << 1, q);
@@ -240,7 +307,7 @@ __device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], uint32_t* const (
   group_sync(bar);
   jx_load_co<K>(v, sc, x);
 #pragma unroll
-  for (int r = 0; r < 16; r++) B[r] = 4;
+  for (int r = 0; r < 16; r++) B[r] = 256;
   jinv_stage<K, 3, 1>(v, B, fwd, 0, q);
   jinv_stage<K, 2, 2>(v, B, fwd, 0, q);
   jinv_stage<K, 1, 3>(v, B, fwd, 0, q);

@@ -42,14 +42,16 @@
 // Three barriers a step, each over one group or one pair of warps.
 //
 // What bounds it: the integer multiply-add pipe (64 lane-operations per
-// cycle and SM, a high or wide product costs two) and, with 16 warps per SM,
-// the latency between dependent operations: IPC 2.15.  One call of 2048
-// queries takes 1507 us; the six-group kernel this one replaced (768 threads,
-// one CTA per SM, four CTA-wide barriers a step, its 24 warps in step with
-// one another, the b side in a launch of its own) took 2290 us, and 174
-// against 154 us for 128 queries (fewer queries than SMs).  Two CTAs of
-// different queries share the SM without waiting for each other, and 128
-// registers a thread let each warp keep 16 independent butterflies in flight.
+// cycle and SM, a high or wide product costs two) is 73 % busy, 86 % in the
+// digit transforms; the rest waits on 16 warps' latencies.  One call of 2048
+// queries takes 1430 us (1507 us with unsigned butterflies and the step's
+// database and CRS words loaded where they are used); the six-group kernel
+// before it (768 threads, one CTA per SM, four CTA-wide barriers a step, its
+// 24 warps in step with one another, the b side in a launch of its own) took
+// 2290 us, and 174 against 142 us for 128 queries (fewer queries than SMs).
+// Two CTAs of different queries share the SM without waiting for each other,
+// and 128 registers a thread let each warp keep 16 independent butterflies in
+// flight.
 #include "expand.cuh"
 #include "kernels.h"
 #include "ntt_joint.cuh"
@@ -363,11 +365,14 @@ __device__ __forceinline__ uint4 ld_stream(const uint32_t* p) {
   return v;
 }
 
-// REDC of T < 2^64 - q 2^32: T 2^-32 mod q, below T / 2^32 + q.
+// REDC of a signed sum T: T 2^-32 mod q in [T / 2^32, T / 2^32 + q).
 __device__ __forceinline__ uint32_t redc_wide(uint64_t T, uint32_t q, uint32_t qinv) {
   const uint32_t m = (uint32_t)T * qinv;
   return (uint32_t)((T + (uint64_t)m * q) >> 32);
 }
+
+// a * b of two signed 32-bit values, as a 64-bit sum's term.
+__device__ __forceinline__ uint64_t smul(uint32_t a, uint32_t b) { return (uint64_t)((int64_t)(int32_t)a * (int32_t)b); }
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
 template <int MODE, bool SEEDED, bool QDB>
@@ -410,7 +415,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
   const bool ybody = (ytag & 1) != 0;
   const uint32_t* Y = reinterpret_cast<const uint32_t*>(ytag & ~(uintptr_t)1);
   const ResidueConsts& C = P.r[r];
-  const uint32_t q = C.q, qinv = C.qinv;
+  const uint32_t q = C.q, qinv = C.qinv, qo = P.r[r ^ 1].q;
   const uint64_t* brows = QDB ? D->brows : A.brows + (size_t)qi * ELL * 2 * N;
   uint64_t* rbar = reinterpret_cast<uint64_t*>(smem + L::BAR);
   uint64_t* stage = reinterpret_cast<uint64_t*>(XC);
@@ -472,6 +477,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     if (tid == 0) *status_ptr() = 0;
   }
 
+  const uint32_t xc = jx_addr(XC);
   // ---- row transforms, into rows h of AH (a slot's words are its thread's).
   //      Consecutive transforms use two exchange buffers by turns: one ends
   //      with reads that another warp's next first writes could overtake ----
@@ -481,28 +487,32 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     for (int t = NR == 2 ? 0 : r, turn = 0; t < ELL; t += NR == 2 ? 1 : 2, turn ^= 1) {
       uint32_t* row = AH + (t * NR + sres) * N;
       uint32_t v[1][16];
-      uint32_t* const sc[1] = {XC + (turn ? r : 2 + r) * N};
+      const uint32_t sc[1] = {xc + 4 * N * (turn ? r : 2 + r)};
 #pragma unroll
       for (int j = 0; j < 16; j++) v[0][j] = row[x + 128 * j];
-      jntt_fwd<1, true>(v, sc, fwd_tw(Cs), Cs.q, x, 1 + r);
+      jntt_fwd<1, true>(v, sc, sfwd_tw(Cs), Cs.q, x, 1 + r);
 #pragma unroll
-      for (int j = 0; j < 16; j++) row[128 * h_of(j) + x] = canon16(v[0][j], Cs.q);
+      for (int j = 0; j < 16; j++) row[128 * h_of(j) + x] = jcanon_fwd(v[0][j], Cs.q);
     }
     if (NR == 1) __syncthreads();  // both groups read the rows of residue 0
   }
 
-  const uint32_t* Ax = AH + sres * N + x;  // row h of row transform t: Ax[t * NR * N + 128 * h]
+  // Row h + rot of a table of rows, [k or t][residue][h][x], is at one byte
+  // offset in the client's keys and in AH (without the residue there in
+  // compat mode): (h + rot) << 9 in bits 9-12, the rest fixed.
+  const uint32_t ah = jx_addr(AH);
+  const uint32_t rx = 4u * (uint32_t)x + (uint32_t)r * 4u * N;
+  auto row_off = [&](uint32_t rot9, int h) -> uint32_t { return ((rot9 + 512u * (uint32_t)h) & 0x1E00u) | rx; };
+  const char* Yb = reinterpret_cast<const char*>(Y);
   const uint32_t* Ex = E + 4 * x;
   const uint32_t* Wx = A.what + r * N + 4 * x;
-  const uint32_t* Yx = Y + r * N + x;
   // sum_t E[i,t][s] A_t[tau_i(s)] for the four slots h = 4 a + j of this thread
-  auto query_only = [&](int i, int a, uint32_t rot, uint64_t T[4]) {
-    const uint32_t* e = Ex + (size_t)i * ELL * N + 512 * a;
-    const uint4 e0 = ld_stream(e), e1 = ld_stream(e + N), e2 = ld_stream(e + 2 * N);
+  auto query_only = [&](const uint4& e0, const uint4& e1, const uint4& e2, const uint32_t (&ro)[4], uint64_t T[4]) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-      const uint32_t* ar = Ax + 128 * ((4 * a + j + rot) & 15);
-      T[j] = (uint64_t)u4e(e0, j) * ar[0] + (uint64_t)u4e(e1, j) * ar[NR * N] + (uint64_t)u4e(e2, j) * ar[2 * NR * N];
+      const uint32_t ar = ah + ro[j] - (NR == 1 ? (uint32_t)r * 4u * N : 0u);
+      T[j] = (uint64_t)u4e(e0, j) * jx_at(ar) + (uint64_t)u4e(e1, j) * jx_at(ar + 4 * NR * N) +
+             (uint64_t)u4e(e2, j) * jx_at(ar + 8 * NR * N);
     }
   };
   // compat mode, residue 1: rebuilt from the residue-0 value as the crate's
@@ -514,11 +524,14 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
 
   uint32_t R[16], acc[16];  // R_{i+1} and the b accumulator, slot layout
   {
-    const uint32_t rot = rot_rows(gamma, gamma - 1, x);
+    const uint32_t rot9 = rot_rows(gamma, gamma - 1, x) << 9;
+    const uint32_t* e = Ex + (size_t)(gamma - 1) * ELL * N;
 #pragma unroll
     for (int a = 0; a < 4; a++) {
       uint64_t T[4];
-      query_only(gamma - 1, a, rot, T);
+      const uint32_t ro[4] = {row_off(rot9, 4 * a), row_off(rot9, 4 * a + 1), row_off(rot9, 4 * a + 2),
+                              row_off(rot9, 4 * a + 3)};
+      query_only(ld_stream(e + 512 * a), ld_stream(e + N + 512 * a), ld_stream(e + 2 * N + 512 * a), ro, T);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int l = h_of(4 * a + j);
@@ -528,65 +541,79 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     }
   }
 
+  const uint32_t own = xc + 4 * N * (2 + r);
+  uint32_t mine = xc + 4 * N * r, other = xc + 4 * N * (r ^ 1);
 #pragma unroll 1
   for (int i = gamma - 2; i >= 0; i--) {
     if (tid == 0 && i >= 2)  // the block that step i - 2 reads
       for (int rr = 0; rr < NR; rr++)
         prefetch_l2(Ebase + (((size_t)shard * 2 + rr) * gamma + (i - 2)) * ELL * N, sizeof(uint32_t) * ELL * N);
-    // [A] inverse NTT of R_{i+1} ([0, 3.2 q))
-    uint32_t* const own = XC + (2 + r) * N;
-    uint32_t* const mine = XC + (r ^ (i & 1)) * N;
-    uint32_t* const other = XC + (r ^ 1 ^ (i & 1)) * N;
+    // [A] inverse NTT of R_{i+1} ([0, 3.1 q))
     uint32_t v[2][16];
     {
       uint32_t c[1][16], o[1][16];
 #pragma unroll
       for (int j = 0; j < 16; j++) c[0][j] = R[j];
-      uint32_t* const sc[1] = {own};
-      jntt_inv<1>(c, sc, fwd_tw(C), q, x, 1 + r);
+      const uint32_t sc[1] = {own}, sm1[1] = {mine}, so1[1] = {other};
+      jntt_inv<1>(c, sc, sfwd_tw(C), q, x, 1 + r);
       // [B] the residues trade coefficients, thread for thread: each writes
       // its own to the buffer it has been using, reads the other group's,
       // and goes on with that buffer.  Digits 0 and 1 of the composite
       // coefficients (gadget_decompose, rgsw/external_product.rs:16-37).
-      uint32_t* const sm1[1] = {mine};
-      uint32_t* const so1[1] = {other};
       jx_store_co<1>(c, sm1, x);
       named_sync(3 + (x >> 5), 64);
       jx_load_co<1>(o, so1, x);
 #pragma unroll
       for (int j = 0; j < 16; j++) {
-        const uint64_t cc = crt_compose(P, r ? o[0][j] : c[0][j], r ? c[0][j] : o[0][j]);
+        const uint64_t cc = crt_compose_from(C, qo, c[0][j], o[0][j]);
         v[0][j] = (uint32_t)cc & 0xFFFFFu;
         v[1][j] = (uint32_t)(cc >> 20) & 0xFFFFFu;
       }
     }
-    // [C]
-    uint32_t* const sc2[2] = {other, own};
-    jntt_fwd<2, false>(v, sc2, fwd_tw(C), q, x, 1 + r);  // [0, 14 q)
-    // [D] the nine products of each slot under two reductions.  With R < 3.2 q,
-    // NTT(d) < 14 q and the rest canonical, R's sum is below 34.3 q^2 (q <
-    // 2^28: < 2.2 q 2^32), so R_i < 3.2 q again; b enters its own sum times
-    // 2^32 (b 2^32 + 31.2 q^2 < 11 q 2^32) and is brought below 8 q.
-    const uint32_t rot = rot_rows(gamma, i, x);
-    const uint32_t yrot = ybody ? rot : 0;
-    const uint32_t* yi = ybody ? Yx : Yx + (size_t)i * ELL * 2 * N;
+    // [C] with the first quad of the step's database and CRS words on its way
     const uint32_t* wi = Wx + (size_t)i * ELL * 2 * N;
+    const uint32_t* ei = Ex + (size_t)i * ELL * N;
+    uint4 nx[6];
+    auto fetch = [&](int a) {
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        nx[k] = ld_stream(ei + k * N + 512 * a);
+        nx[3 + k] = ld_stream(wi + 2 * k * N + 512 * a);
+      }
+    };
+    const uint32_t sc2[2] = {other, own};
+    jntt_fwd<2, false>(v, sc2, sfwd_tw(C), q, x, 1 + r, [&]() { fetch(0); });  // signed, below 5.25 q
+    other = mine;
+    mine = sc2[0];
+    // [D] the nine products of each slot under two reductions, in signed
+    // 64-bit sums.  With R in [0, 3.1 q), NTT(d) below 5.25 q and the rest
+    // canonical, R's sum is in (-10.5 q^2, 16.6 q^2); q < 2^28, so its
+    // reduction plus q is in (0.3 q, 3.1 q).  b's part plus q is in (0.3 q,
+    // 2.9 q), and b is kept below 8 q.
+    const uint32_t rot9 = rot_rows(gamma, i, x) << 9;
+    const char* yi = ybody ? Yb : Yb + (size_t)i * ELL * 2 * N * 4;
 #pragma unroll
     for (int a = 0; a < 4; a++) {
       uint64_t T[4];
-      const uint4 w0 = ld_stream(wi + 512 * a), w1 = ld_stream(wi + 2 * N + 512 * a),
-                  w2 = ld_stream(wi + 4 * N + 512 * a);
-      query_only(i, a, rot, T);
+      uint4 cu[6];
+#pragma unroll
+      for (int k = 0; k < 6; k++) cu[k] = nx[k];
+      if (a < 3) fetch(a + 1);
+      const uint32_t ro[4] = {row_off(rot9, 4 * a), row_off(rot9, 4 * a + 1), row_off(rot9, 4 * a + 2),
+                              row_off(rot9, 4 * a + 3)};
+      query_only(cu[0], cu[1], cu[2], ro, T);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int l = h_of(4 * a + j);
-        const uint32_t* y = yi + 128 * ((4 * a + j + yrot) & 15);
-        uint64_t S = conv1 ? (uint64_t)converted(T[j]) << 32 : T[j];
-        S += (uint64_t)v[0][l] * u4e(w0, j) + (uint64_t)v[1][l] * u4e(w1, j) + (uint64_t)R[l] * u4e(w2, j);
-        const uint64_t B = ((uint64_t)acc[l] << 32) + (uint64_t)v[0][l] * __ldg(y) +
-                           (uint64_t)v[1][l] * __ldg(y + 2 * N) + (uint64_t)R[l] * __ldg(y + 4 * N);
-        R[l] = redc_wide(S, q, qinv);
-        acc[l] = csub(redc_wide(B, q, qinv), 8 * q);
+        const uint32_t* y = reinterpret_cast<const uint32_t*>(yi + ro[j]);
+        const uint32_t y0 = __ldg(y), y1 = __ldg(y + 2 * N), y2 = __ldg(y + 4 * N);
+        uint64_t S = conv1 ? 0ull : T[j];
+        S += smul(v[0][l], u4e(cu[3], j));
+        S += smul(v[1][l], u4e(cu[4], j));
+        S += smul(R[l], u4e(cu[5], j));
+        const uint64_t B = smul(v[0][l], y0) + smul(v[1][l], y1) + smul(R[l], y2);
+        R[l] = redc_wide(S, q, qinv) + (conv1 ? converted(T[j]) : 0u) + q;
+        acc[l] = csub(acc[l] + redc_wide(B, q, qinv) + q, 8 * q);
       }
     }
   }
@@ -597,10 +624,10 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
 #pragma unroll 1
   for (int part = 0; part < 2; part++) {
     uint32_t o[1][16];
-    uint32_t* const sc[1] = {XC + (part ? r ^ 1 : 2 + r) * N};
+    const uint32_t sc[1] = {part ? mine : own};
 #pragma unroll
     for (int j = 0; j < 16; j++) o[0][j] = part ? csub(acc[j], 4 * q) : R[j];
-    jntt_inv<1>(o, sc, fwd_tw(C), q, x, 1 + r);
+    jntt_inv<1>(o, sc, sfwd_tw(C), q, x, 1 + r);
     if (part && x < gamma) o[0][0] = add_mod(o[0][0], bpoly[16 * r + x], q);
 #pragma unroll
     for (int j = 0; j < 16; j++) out[part * 2 * N + r * N + x + 128 * j] = o[0][j];

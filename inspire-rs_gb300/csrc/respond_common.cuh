@@ -119,8 +119,7 @@ __device__ __forceinline__ void scatter_r(const DevParams& P, int i, const uint3
 }
 
 // A thread's 16 slots (slot order, as four uint4) of one key polynomial of
-// the CRS table (quads) or of a client table (rows; rot: rot_rows for a body
-// table, 0 for a table of rotated polynomials).
+// the CRS table (quads) or of a client table (rows, found at h + rot).
 __device__ __forceinline__ void key_quads(const uint32_t* poly, int x, uint4 (&k)[4]) {
   uint32_t o[16];
 #pragma unroll

@@ -317,7 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(RBLOCK, 1)
     const int p = i & 1;
     uint32_t* TC = smem + L::TC + p * 2 * N;
     const size_t yoff = ybody ? (size_t)i * ELL * 2 * N : 0;  // body tables: the key slices of i = 0, rotated
-    const uint32_t yrot = ybody ? rot_rows(gamma, i, x) : 0;
+    const uint32_t yrot = rot_rows(gamma, i, x);
     if (tid == 0 && i >= 2) prefetch_l2(Eg_at() + (size_t)(i - 2) * ELL * N, sizeof(uint32_t) * ELL * N);
     // [A]
     if (tid < 2 * NTT_GT) {

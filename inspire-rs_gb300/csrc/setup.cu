@@ -131,10 +131,11 @@ __global__ void __launch_bounds__(BLOCK) crs_what_kernel(const DevParams P, cons
 // Client key table from y_body: the forward NTT of packing_online
 // (inspiring2.rs:1199-1213) of y_body[k], in rows [h][x] and times n^-1 2^32.
 // generate_rotations (:1309-1323) is a rotation of the rows (rot_rows), which
-// the Respond kernels apply as they read.  An explicit y_all
-// ((gamma-1)*ELL coefficient polys) goes through the same kernel.
+// the Respond kernels apply as they read.  An explicit y_all ((gamma-1)*ELL
+// coefficient polys, step i = p / ELL; `rotated`) is stored with slot h in row
+// h + rot, where they look for it.
 __global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams P, const uint64_t* __restrict__ ya,
-                                                                uint32_t* __restrict__ yhat) {
+                                                                bool rotated, uint32_t* __restrict__ yhat) {
   __shared__ uint32_t SC[2][NTT_SCRATCH];
   const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
   const ResidueConsts& C = P.r[g];
@@ -142,9 +143,10 @@ __global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams 
 #pragma unroll
   for (int rr = 0; rr < 16; rr++) v[rr] = (uint32_t)ya[((size_t)p * 2 + g) * N + x + 128 * rr];
   ntt_fwd(v, SC[g], fwd_tw(C), C.q, x, 1 + g);
+  const uint32_t rot = rotated ? rot_rows(P.gamma, p / ELL, x) : 0;
 #pragma unroll
   for (int rr = 0; rr < 16; rr++)
-    yhat[((size_t)p * 2 + g) * N + row_word(h_of(rr), x)] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
+    yhat[((size_t)p * 2 + g) * N + row_word((h_of(rr) + rot) & 15, x)] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
 }
 
 // Key tables with the third gadget digit folded in.  In the NTT domain of
@@ -213,10 +215,10 @@ cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t*
   return cudaGetLastError();
 }
 
-cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, uint32_t* yhat,
+cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, bool rotated, uint32_t* yhat,
                                    cudaStream_t st) {
   if (npolys <= 0) return cudaSuccess;
-  client_keys_ntt_kernel<<<npolys, BLOCK, 0, st>>>(P, polys, yhat);
+  client_keys_ntt_kernel<<<npolys, BLOCK, 0, st>>>(P, polys, rotated, yhat);
   return cudaGetLastError();
 }
 
