@@ -15,6 +15,7 @@ constexpr int ERR_STAGE = 3;   // the query's rows did not arrive in shared memo
 // the whole launch are unreliable (a later CTA on the SM may have received
 // the late copies in its shared memory)
 constexpr int ERR_STAGE_LOST = 4;
+constexpr int ERR_PEER = 5;    // the other CTA's coefficients did not come within the wait bound (two-CTA kernel)
 constexpr uint32_t STAGE_WAIT_ITERS_DEFAULT = 1u << 20;
 constexpr uint32_t STAGE_DRAIN_ITERS = 1u << 22;
 

@@ -52,10 +52,8 @@
 // Two CTAs of different queries share the SM without waiting for each other,
 // and 128 registers a thread let each warp keep 16 independent butterflies in
 // flight.
-#include "expand.cuh"
-#include "kernels.h"
 #include "ntt_joint.cuh"
-#include "respond_common.cuh"
+#include "respond_draws.cuh"
 
 namespace ig {
 
@@ -101,86 +99,6 @@ __device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows
   }
 }
 
-// Exclusive rank of this thread's `cnt` over the CTA, total of all threads.
-// ws: 8 ints of this call's own (reused two calls later at the earliest).
-__device__ __forceinline__ int scan_cta(int cnt, int* ws, int& total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) ws[warp] = incl;
-  __syncthreads();
-  int base = 0;
-  total = 0;
-#pragma unroll
-  for (int w = 0; w < QT / 32; w++) {
-    const int t = ws[w];
-    if (w < warp) base += t;
-    total += t;
-  }
-  return base + incl - cnt;
-}
-
-__device__ __forceinline__ int scan_warp(int cnt, int& total) {
-  const int lane = threadIdx.x & 31;
-  int incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  total = __shfl_sync(0xffffffffu, incl, 31);
-  return incl - cnt;
-}
-
-__device__ __forceinline__ void load_key(const uint8_t* seed, uint32_t key[8]) {
-  const uint32_t* s = reinterpret_cast<const uint32_t*>(seed);
-  if ((reinterpret_cast<uintptr_t>(seed) & 3) == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) key[i] = s[i];
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-      key[i] = (uint32_t)seed[4 * i] | ((uint32_t)seed[4 * i + 1] << 8) | ((uint32_t)seed[4 * i + 2] << 16) |
-               ((uint32_t)seed[4 * i + 3] << 24);
-  }
-}
-
-// The eight draws of one keystream block under gen_range(0..q): bit k of the
-// mask is set if draw k is accepted, val[k] its value.  zone = (q << lz) - 1
-// has 32 low ones (q < 2^32), so lo64(v q) <= zone is decided by the high
-// words.
-__device__ __forceinline__ unsigned draw8(const uint32_t w[16], uint32_t q, uint32_t zone_hi, uint32_t val[8]) {
-  unsigned mask = 0;
-#pragma unroll
-  for (int k = 0; k < 8; k++) {
-    const uint64_t hi = (uint64_t)w[2 * k + 1] * q + __umulhi(w[2 * k], q);
-    val[k] = (uint32_t)(hi >> 32);
-    mask |= ((uint32_t)hi <= zone_hi ? 1u : 0u) << k;
-  }
-  return mask;
-}
-
-__device__ __forceinline__ void put_draws(uint32_t* dst, int p, unsigned mask, const uint32_t val[8]) {
-#pragma unroll
-  for (int k = 0; k < 8; k++)
-    if ((mask >> k) & 1u) {
-      if (p < N) dst[p] = val[k];
-      p++;
-    }
-}
-
-// One row by the general routine (256-thread sub-block), for streams that
-// reject more draws than the fast path allows for.
-template <int NR>
-__device__ __noinline__ bool expand_row_general(const DevParams& P, const uint8_t* seed, uint64_t* cand, uint32_t* a0,
-                                                int* ws) {
-  return expand_seeded_row<NR>(P, seed, cand, a0, a0 + N, ws, 3, threadIdx.x);
-}
-
 // Poly::from_seed_moduli (poly.rs:251-281) of the ELL rows by the whole CTA.
 // Draws 0 .. 2047 (blocks 0-255, a thread each) go to residue 0, whose few
 // missing values (rejections: 2^28 - q of 2^28 draws) come from the start of
@@ -203,7 +121,7 @@ __device__ __forceinline__ void expand_rows(const DevParams& P, const uint8_t* s
     chacha20_block(key, tid, P.one, w);
     const unsigned mask = draw8(w, q0, z0, val);
     int total;
-    const int p = scan_cta(__popc(mask), ws + 8 * (t & 1), total);
+    const int p = scan_256(__popc(mask), ws + 8 * (t & 1), total, 0);
     put_draws(AH + t * NR * N, p, mask, val);
     if (tid == 0) tot[t] = total;
   }
@@ -243,7 +161,7 @@ __device__ __forceinline__ void expand_rows(const DevParams& P, const uint8_t* s
         if (skip > 0) mask &= skip >= 8 ? 0u : ~((1u << skip) - 1u);
       }
       int total;
-      const int p = scan_cta(__popc(mask), ws + 8 * ((t + 1) & 1), total);
+      const int p = scan_256(__popc(mask), ws + 8 * ((t + 1) & 1), total, 0);
       put_draws(a0 + N, p, mask, val);
       if (tid == 0) tot[t] = total;
     }
@@ -354,25 +272,6 @@ __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __r
   __syncthreads();
   return -1;
 }
-
-// Streaming loads of the contracted shard and the CRS keys: read once per
-// query, kept out of L1 (which holds the twiddles and the client's keys).
-__device__ __forceinline__ uint4 ld_stream(const uint32_t* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-
-// REDC of a signed sum T: T 2^-32 mod q in [T / 2^32, T / 2^32 + q).
-__device__ __forceinline__ uint32_t redc_wide(uint64_t T, uint32_t q, uint32_t qinv) {
-  const uint32_t m = (uint32_t)T * qinv;
-  return (uint32_t)((T + (uint64_t)m * q) >> 32);
-}
-
-// a * b of two signed 32-bit values, as a 64-bit sum's term.
-__device__ __forceinline__ uint64_t smul(uint32_t a, uint32_t b) { return (uint64_t)((int64_t)(int32_t)a * (int32_t)b); }
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
 template <int MODE, bool SEEDED, bool QDB>
@@ -506,7 +405,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
   const char* Yb = reinterpret_cast<const char*>(Y);
   const uint32_t* Ex = E + 4 * x;
   const uint32_t* Wx = A.what + r * N + 4 * x;
-  // sum_t E[i,t][s] A_t[tau_i(s)] for the four slots h = 4 a + j of this thread
+  // sum_t E[i,t][s] A_t[tau_i(s)] for the four slots l = 4 a + j of this thread
   auto query_only = [&](const uint4& e0, const uint4& e1, const uint4& e2, const uint32_t (&ro)[4], uint64_t T[4]) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -529,12 +428,12 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
 #pragma unroll
     for (int a = 0; a < 4; a++) {
       uint64_t T[4];
-      const uint32_t ro[4] = {row_off(rot9, 4 * a), row_off(rot9, 4 * a + 1), row_off(rot9, 4 * a + 2),
-                              row_off(rot9, 4 * a + 3)};
+      const uint32_t ro[4] = {row_off(rot9, h_of(4 * a)), row_off(rot9, h_of(4 * a + 1)),
+                              row_off(rot9, h_of(4 * a + 2)), row_off(rot9, h_of(4 * a + 3))};
       query_only(ld_stream(e + 512 * a), ld_stream(e + N + 512 * a), ld_stream(e + 2 * N + 512 * a), ro, T);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const int l = h_of(4 * a + j);
+        const int l = 4 * a + j;
         R[l] = conv1 ? converted(T[j]) : redc_wide(T[j], q, qinv);
         acc[l] = 0;
       }
@@ -599,12 +498,12 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
 #pragma unroll
       for (int k = 0; k < 6; k++) cu[k] = nx[k];
       if (a < 3) fetch(a + 1);
-      const uint32_t ro[4] = {row_off(rot9, 4 * a), row_off(rot9, 4 * a + 1), row_off(rot9, 4 * a + 2),
-                              row_off(rot9, 4 * a + 3)};
+      const uint32_t ro[4] = {row_off(rot9, h_of(4 * a)), row_off(rot9, h_of(4 * a + 1)),
+                              row_off(rot9, h_of(4 * a + 2)), row_off(rot9, h_of(4 * a + 3))};
       query_only(cu[0], cu[1], cu[2], ro, T);
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const int l = h_of(4 * a + j);
+        const int l = 4 * a + j;
         const uint32_t* y = reinterpret_cast<const uint32_t*>(yi + ro[j]);
         const uint32_t y0 = __ldg(y), y1 = __ldg(y + 2 * N), y2 = __ldg(y + 4 * N);
         uint64_t S = conv1 ? 0ull : T[j];

@@ -78,68 +78,19 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
 // on s >> 4 alone.  With s = 16 x + l and h = brv4(l), the top four bits of
 // brv(s), u is (x, h + rot_rows(gamma, i, x) mod 16).
 //
-// Tables are therefore stored by (h, x):
-//   quads  [h >> 2][x][h & 3]: thread x reads its 16 slots with four coalesced
+// Tables are therefore stored by run:
+//   quads  [l >> 2][x][l & 3]: a thread reads the slots it owns with coalesced
 //          128-bit loads (contracted shard, CRS keys);
-//   rows   [h][x]: row h + rot of 128 threads, the rotation uniform over 16
-//          threads, so that a warp's load of a rotated slot touches two
-//          half lines (client keys, row transforms).
+//   rows   [h][x]: row h + rot of 128 runs, the rotation uniform over 16 runs,
+//          so that a warp's load of a rotated slot touches two half lines
+//          (client keys, row transforms).
 __device__ __forceinline__ uint32_t rot_rows(int gamma, int i, int x) {
   const uint32_t c = 2u * (__brev((uint32_t)x) >> 25) + 1u;  // 2 brv(s) + 1 mod 16
   return (((uint32_t)i * c) & (uint32_t)(gamma - 1)) * (uint32_t)(MAX_GAMMA / gamma);
 }
 __host__ __device__ constexpr int h_of(int l) { return ((l & 1) << 3) | ((l & 2) << 1) | ((l & 4) >> 1) | ((l & 8) >> 3); }
-__host__ __device__ constexpr int quad_word(int h, int x) { return (h >> 2) * 512 + 4 * x + (h & 3); }
+__host__ __device__ constexpr int quad_word(int l, int x) { return (l >> 2) * 512 + 4 * x + (l & 3); }
 __host__ __device__ constexpr int row_word(int h, int x) { return h * 128 + x; }
-
-// R_i (NTT domain, scaled by n^-1) of packing_offline step 1 for one residue
-// (inspiring2.rs:952-981 with the tables of :208-263): slot s takes sum_t
-// E[i][t][s] A_t[u], u = tau_i(s).  Eg is this residue's contracted shard
-// [gamma][ELL][N] in quads by destination slot (encode_E_kernel); Ag the row
-// transforms in (swizzled) slot order.  Threads p in [0, nthr) handle table
-// words w = w0 + p + nthr * v < w1.
-// In compat mode `dst1`, if not null, receives residue 1 rebuilt from each
-// residue-0 value as the crate's apply_automorphism_ntt does (`dst` may then
-// be null: only residue 1 is written).
-__device__ __forceinline__ void scatter_r(const DevParams& P, int i, const uint32_t* __restrict__ Eg, const uint32_t* Ag,
-                                          int astride, uint32_t* dst, int p, int nthr, uint32_t q, uint32_t qinv,
-                                          uint32_t* dst1 = nullptr, int w0 = 0, int w1 = N) {
-  const uint32_t* Ei = Eg + (size_t)i * ELL * N;
-#pragma unroll 4
-  for (int w = w0 + p; w < w1; w += nthr) {
-    const int x = (w >> 2) & 127, h = ((w >> 9) << 2) | (w & 3);
-    const int us = swz(16 * x + h_of((h + (int)rot_rows(P.gamma, i, x)) & 15));
-    const uint64_t T = (uint64_t)__ldg(Ei + w) * Ag[us] + (uint64_t)__ldg(Ei + N + w) * Ag[astride + us] +
-                       (uint64_t)__ldg(Ei + 2 * N + w) * Ag[2 * astride + us];
-    const int s = swz(16 * x + h_of(h));
-    const uint32_t val = redc(T, q, qinv);
-    if (dst) dst[s] = val;
-    if (dst1) dst1[s] = compat_residue1_ninv(P, val);
-  }
-}
-
-// A thread's 16 slots (slot order, as four uint4) of one key polynomial of
-// the CRS table (quads) or of a client table (rows, found at h + rot).
-__device__ __forceinline__ void key_quads(const uint32_t* poly, int x, uint4 (&k)[4]) {
-  uint32_t o[16];
-#pragma unroll
-  for (int a = 0; a < 4; a++) {
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(poly + 512 * a + 4 * x));
-    o[h_of(4 * a)] = v.x;
-    o[h_of(4 * a + 1)] = v.y;
-    o[h_of(4 * a + 2)] = v.z;
-    o[h_of(4 * a + 3)] = v.w;
-  }
-#pragma unroll
-  for (int r4 = 0; r4 < 4; r4++) k[r4] = make_uint4(o[4 * r4], o[4 * r4 + 1], o[4 * r4 + 2], o[4 * r4 + 3]);
-}
-__device__ __forceinline__ void key_rows(const uint32_t* poly, int x, uint32_t rot, uint4 (&k)[4]) {
-  uint32_t o[16];
-#pragma unroll
-  for (int h = 0; h < 16; h++) o[h_of(h)] = __ldg(poly + row_word((h + rot) & 15, x));
-#pragma unroll
-  for (int r4 = 0; r4 < 4; r4++) k[r4] = make_uint4(o[4 * r4], o[4 * r4 + 1], o[4 * r4 + 2], o[4 * r4 + 3]);
-}
 
 __device__ __forceinline__ uint32_t u4e(const uint4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
 

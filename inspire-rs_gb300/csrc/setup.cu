@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, cons
   // mod gamma, m_i = (gamma - i) mod gamma, to s = tau_i^-1(u), i.e. (rot_rows)
   // to row h - rot of the same 16-slot run.  For odd 2brv(u)+1 the map i -> k
   // is a bijection: the table is a permutation of the outputs.  A warp's 32
-  // source slots are two runs, whose words of each quad plane are 32 bytes.
+  // source slots are two runs, whose words of each quad plane are 32 bytes together.
   uint32_t* Eo = E + (((size_t)s * 2 + r) * gamma * ELL + t) * N;
   for (int v = 0; v < N / BLOCK; v++) {
     const int u = tid + BLOCK * v;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, cons
         if (j < gamma) T += (uint64_t)zp[(k * j) & (gamma - 1)] * c[j];
       // the two REDCs divided by 2^64; e_scale = gamma^-1 n^-1 2^96 leaves
       // the factor 2^32 gamma^-1 n^-1
-      Eo[(size_t)i * ELL * N + quad_word((uh - (int)rot_rows(gamma, i, ux)) & 15, ux)] = mul_shoup(redc(T, q, qinv), C.e_scale, C.e_scale_p, q);
+      Eo[(size_t)i * ELL * N + quad_word(h_of((uh - (int)rot_rows(gamma, i, ux)) & 15), ux)] = mul_shoup(redc(T, q, qinv), C.e_scale, C.e_scale_p, q);
     }
   }
 }
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams 
 // With R kept as n^-1 R (the Respond kernel's R_{i+1}), the third key is
 // n z^-2 k2.  src and dst hold ngroups triples [g][k<3][2][N] (any constant
 // scaling, applied alike to the three keys).  In place, or with `quads` from
-// slot order into quads [h >> 2][x][h & 3].
+// slot order into quads [l >> 2][x][l & 3].
 __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams P, const uint32_t* src, uint32_t* dst,
                                                                  int ngroups, bool quads) {
   const size_t per = (size_t)2 * N;
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams
     const int r = (int)(rs >> LOGN);
     const ResidueConsts& C = P.r[r];
     const int w = (int)(rs & (N - 1));
-    const int x = (w >> 2) & 127, h = ((w >> 9) << 2) | (w & 3);
-    const uint32_t* f = src + g * 3 * per + (quads ? (size_t)r * N + 16 * x + h_of(h) : rs);
+    const int x = (w >> 2) & 127, l = ((w >> 9) << 2) | (w & 3);
+    const uint32_t* f = src + g * 3 * per + (quads ? (size_t)r * N + 16 * x + l : rs);
     uint32_t* t = dst + g * 3 * per + rs;
     const uint32_t k0 = f[0], k1 = f[per], k2 = f[2 * per];
     t[0] = sub_mod(k0, mul_shoup(k2, C.d2_z2, C.d2_z2_p, C.q), C.q);
