@@ -635,6 +635,14 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
     C.ninv_mont_p = shoup(nm, qm);
     C.mont = (uint32_t)r32;
     C.mont_p = shoup(r32, qm);
+    const uint64_t w1 = t[2], w1i = t[2 * N + 2];  // psi^(+-brv(1))
+    auto pair_of = [&](uint64_t a, uint64_t b) {
+      const uint64_t w = (uint64_t)((u128)a * b % qm);
+      return make_uint2((uint32_t)w, shoup(w, qm));
+    };
+    C.r64_w = pair_of(r64, w1);
+    C.ref_inv_w = pair_of(ris, w1i);
+    C.ninv_mont_w = pair_of(nm, w1i);
     const uint64_t zinv = inv_prime((1ULL << ZBITS) % qm, qm), z2inv = (uint64_t)((u128)zinv * zinv % qm);
     const uint64_t nz2 = (uint64_t)((u128)N * z2inv % qm);
     C.d2_nz2 = (uint32_t)nz2;

@@ -26,6 +26,7 @@ struct ResidueConsts {
   const uint2* inv;                  // {psi^-brv(k), Shoup companion}
   const uint32_t* psi_pow;           // psi^e, e in [0, 2n)
   const uint2* sfwd;                 // fwd with w in (-q/2, q/2) and round(w 2^32 / q) (ntt_joint.cuh)
+  uint2 r64_w, ref_inv_w, ninv_mont_w;  // r64 psi^brv(1); ref_inv_scale, ninv_mont times psi^-brv(1) (pairs)
   uint32_t crt_inv, crt_inv_p;       // q^-1 mod the other modulus (crt_compose_from)
   uint32_t crt_off;                  // the other modulus's first multiple from q on
   uint32_t r64, r64_p;               // 2^64 mod q: reference Montgomery factor

@@ -31,7 +31,7 @@
 #pragma once
 #include <cstdint>
 
-#include "ntt2048.cuh"
+#include "common.cuh"
 
 namespace ig {
 
@@ -129,6 +129,13 @@ __device__ __forceinline__ void jx_load_ru(uint32_t (&v)[K][16], const uint32_t 
     }
 }
 
+// The warp's 512 elements of a buffer as coalesced 128-bit words: chunk c of
+// lane l is elements 512 w + 128 c + 4 l .. + 3.  Between these and the slot
+// layout (jx_store_ru, jx_load_ru) only the warp's own words move.
+__device__ __forceinline__ uint32_t jx_lin(int x, int c) {
+  return 4u * (uint32_t)jsw(512 * (x >> 5) + 128 * c + 4 * (x & 31));
+}
+
 // ---- bounds: element r is below B[r] q / 64 (in absolute value in the
 //      forward transform); 32-bit signed values allow 8 q = 512 units ----
 constexpr int JB_MAX = 512;
@@ -172,25 +179,22 @@ __device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], int (&B)[16], T
 
 // Forward transforms, coefficient layout (v[k][r] = a_k[x + 128 r]) in, slot
 // layout (v[k][r] = A_k[16 x + r], signed, below JFWD_OUT q / 64) out.
-// Inputs below 2^20 (gadget digits), or in [0, q) with FULL.  sc[k]: K
-// exchange buffers of 2048 words, whose words at this thread's coefficient
-// positions (jsw(x + 128 r)) must be free to this thread; bar: the group's
-// named barrier.
+// Inputs in [0, B0 q / 64), B0 = JB_DIGIT for gadget digits.  sc[k]: K exchange
+// buffers of 2048 words, whose words at this thread's coefficient positions
+// (jsw(x + 128 r)) must be free to this thread; bar: the group's named barrier.
 //
-// Digits count as 1/64 q: for q near 2^28 they are 1/256 q, and for smaller q
-// every bound, an absolute sum of 2^20 and multiples of q, is smaller too.
+// Digits (below 2^20) count as 1/64 q: for q near 2^28 they are 1/256 q, and
+// for smaller q every bound, an absolute sum of 2^20 and multiples of q, is
+// smaller too.
+constexpr int JB_DIGIT = 1, JB_CANON = 64;
 constexpr int JFWD_OUT = 416;
 struct NoHook {
   __device__ __forceinline__ void operator()() const {}
 };
-// `hook` runs before stages 8-10 (to issue loads that they can hide).
-template <int K, bool FULL, class Hook = NoHook>
-__device__ __forceinline__ void jntt_fwd(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef tw, uint32_t q, int x,
-                                         int bar, Hook&& hook = Hook()) {
-  int B[16];
-#pragma unroll
-  for (int r = 0; r < 16; r++) B[r] = FULL ? 64 : 1;
-  jfwd_stage<K, 0, 4>(v, B, tw, 0, q);
+// Stages 1-10; `hook` runs before stages 8-10 (to issue loads that they hide).
+template <int K, class Hook = NoHook>
+__device__ __forceinline__ void jntt_fwd_from1(uint32_t (&v)[K][16], int (&B)[16], const uint32_t (&sc)[K],
+                                               TwiddleRef tw, uint32_t q, int x, int bar, Hook&& hook = Hook()) {
   jfwd_stage<K, 1, 3>(v, B, tw, 0, q);
   jfwd_stage<K, 2, 2>(v, B, tw, 0, q);
   jfwd_stage<K, 3, 1>(v, B, tw, 0, q);
@@ -219,6 +223,36 @@ __device__ __forceinline__ void jntt_fwd(uint32_t (&v)[K][16], const uint32_t (&
   jfwd_stage<K, 8, 3>(v, B, tw, x << 1, q);
   jfwd_stage<K, 9, 2>(v, B, tw, x << 2, q);
   jfwd_stage<K, 10, 1>(v, B, tw, x << 3, q);
+}
+
+template <int K, int B0, class Hook = NoHook>
+__device__ __forceinline__ void jntt_fwd(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef tw, uint32_t q, int x,
+                                         int bar, Hook&& hook = Hook()) {
+  int B[16];
+#pragma unroll
+  for (int r = 0; r < 16; r++) B[r] = B0;
+  jfwd_stage<K, 0, 4>(v, B, tw, 0, q);
+  jntt_fwd_from1<K>(v, B, sc, tw, q, x, bar, hook);
+}
+
+// The same of c times the input, any 32-bit values: stage 0 multiplies both
+// of its operands, by c and by c psi^brv(1) (Shoup pairs c, cw).
+template <int K>
+__device__ __forceinline__ void jntt_fwd_scaled(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef tw, uint2 c,
+                                                uint2 cw, uint32_t q, int x, int bar) {
+  int B[16];
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t a = mul_shoup_lazy(v[k][r], c, q), b = mul_shoup_lazy(v[k][r + 8], cw, q);
+      v[k][r] = a + b;
+      v[k][r + 8] = a - b;
+    }
+    B[r] = 256;
+    B[r + 8] = 128;
+  }
+  jntt_fwd_from1<K>(v, B, sc, tw, q, x, bar);
 }
 
 // A forward output brought to [0, q).
@@ -278,14 +312,13 @@ __device__ __forceinline__ void jinv_reduce(uint32_t (&v)[K][16], int (&B)[16], 
   }
 }
 
-// Inverse transforms without the n^-1 factor, slot layout ([0, 4 q)) in,
-// coefficient layout out, canonical.  `fwd` is the forward table.  sc[k]'s
-// words at this thread's slot positions must be free to this thread; it
-// reads its coefficient positions last.
+// Inverse stages 10-1, slot layout ([0, 4 q)) in, coefficient layout out with
+// bounds B.  `fwd` is the forward table.  sc[k]'s words at this thread's slot
+// positions must be free to this thread; it reads its coefficient positions
+// last.
 template <int K>
-__device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef fwd, uint32_t q,
-                                         int x, int bar) {
-  int B[16];
+__device__ __forceinline__ void jntt_inv_to1(uint32_t (&v)[K][16], int (&B)[16], const uint32_t (&sc)[K],
+                                             TwiddleRef fwd, uint32_t q, int x, int bar) {
 #pragma unroll
   for (int r = 0; r < 16; r++) B[r] = 256;
   jinv_stage<K, 10, 1>(v, B, fwd, x << 3, q);
@@ -311,8 +344,41 @@ __device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], const uint32_t (&
   jinv_stage<K, 3, 1>(v, B, fwd, 0, q);
   jinv_stage<K, 2, 2>(v, B, fwd, 0, q);
   jinv_stage<K, 1, 3>(v, B, fwd, 0, q);
+}
+
+// Inverse transforms without the n^-1 factor, canonical.
+template <int K>
+__device__ __forceinline__ void jntt_inv(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef fwd, uint32_t q,
+                                         int x, int bar) {
+  int B[16];
+  jntt_inv_to1<K>(v, B, sc, fwd, q, x, bar);
   jinv_stage<K, 0, 4>(v, B, fwd, 0, q);
   jinv_reduce<K, 1>(v, B, q);
+}
+
+// The same times c, canonical: stage 0 multiplies its sums by c and its
+// differences by c psi^-brv(1) (Shoup pairs c, cw), whose products need no
+// other reduction.
+template <int K>
+__device__ __forceinline__ void jntt_inv_scaled(uint32_t (&v)[K][16], const uint32_t (&sc)[K], TwiddleRef fwd, uint2 c,
+                                                uint2 cw, uint32_t q, int x, int bar) {
+  int B[16];
+  jntt_inv_to1<K>(v, B, sc, fwd, q, x, bar);
+#pragma unroll
+  for (int r = 0; r < 8; r++) {
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      if (B[r + 8 * e] > JB_MAX) {
+#pragma unroll
+        for (int k = 0; k < K; k++) v[k][r + 8 * e] = csub(v[k][r + 8 * e], 8 * q);
+      }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t a = v[k][r], b = v[k][r + 8];  // below 8 q
+      v[k][r] = reduce_2q(mul_shoup_lazy(a + b, c, q), q);
+      v[k][r + 8] = reduce_2q(mul_shoup_lazy(a - b + 8 * q, cw, q), q);
+    }
+  }
 }
 
 }  // namespace ig

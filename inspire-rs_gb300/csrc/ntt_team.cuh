@@ -110,15 +110,15 @@ __device__ __forceinline__ void jt_level(int (&B)[8]) {
   for (int r = 0; r < 8; r++) B[r] = m;
 }
 
-// Forward transform; inputs below 2^20, or in [0, q) with FULL; outputs as
-// jntt_fwd's (signed, below JFWD_OUT q / 64).  `hook` runs before the last
+// Forward transform; inputs in [0, B0 q / 64), outputs as jntt_fwd's (signed,
+// below JFWD_OUT q / 64).  `hook` runs before the last
 // two stages.
-template <bool FULL, class Hook = NoHook>
+template <int B0, class Hook = NoHook>
 __device__ __forceinline__ void jt_fwd(uint32_t (&v)[8], uint32_t sc, TwiddleRef tw, uint32_t q, int t, int bar,
                                        Hook&& hook = Hook()) {
   int B[8];
 #pragma unroll
-  for (int r = 0; r < 8; r++) B[r] = FULL ? 64 : 1;
+  for (int r = 0; r < 8; r++) B[r] = B0;
   JtRuns w;
   jt_runs(w, tw, 0, 0);
   jt_fwd_stage<4, 3, 1>(v, B, w.a, q);

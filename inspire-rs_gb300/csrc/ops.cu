@@ -3,54 +3,89 @@
 // values in Montgomery form with R = 2^64) and the general RLWE x RGSW external
 // product (src/rgsw/external_product.rs:88-150).
 #include "kernels.h"
+#include "ntt_joint.cuh"
+#include "respond_draws.cuh"
 
 namespace ig {
 
 namespace {
 
-// One polynomial (both residues) per CTA; group g transforms residue g.
+// K polynomials (both residues) per CTA; group g transforms residue g of them.
 // Layout: polys[p][r][N] u32.  Forward: coefficients -> reference NTT slots
 // (times 2^64).  Inverse: reference NTT slots -> coefficients.
-template <bool INVERSE>
-__global__ void __launch_bounds__(BLOCK) ntt_ref_kernel(const DevParams P, uint32_t* __restrict__ polys) {
-  __shared__ uint32_t SC[2][NTT_SCRATCH];
-  const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
+//
+// What bounds it: the integer multiply-add pipe in the butterflies (300 M
+// transforms/s with everything in registers and shared memory) and the
+// instructions of the loads and stores beside them.  4096 polynomials forward
+// take 41 us (47 us with one polynomial per CTA, the scale as a multiply of
+// its own and each thread storing its 64 bytes of slots directly: quarter
+// full sectors, 10 us of the stores alone), inverse 41 us (47 us).  Fetching
+// the next polynomials while these are transformed (persistent CTAs, in
+// registers or by cp.async) took 44-47 us: it only adds instructions.
+constexpr int NTT_REF_K = 2;
+template <int K, bool INVERSE>
+__global__ void __launch_bounds__(BLOCK, 3) ntt_ref_kernel(const DevParams P, uint32_t* __restrict__ polys, int npolys) {
+  __shared__ __align__(128) uint32_t SC[2][K][N];
+  const int tid = threadIdx.x, g = tid >> 7, x = tid & 127;
+  const int p0 = blockIdx.x * K;
   const ResidueConsts& C = P.r[g];
   const uint32_t q = C.q;
-  uint32_t* a = polys + ((size_t)p * 2 + g) * N;
-  uint32_t v[16];
+  uint32_t* a = polys + ((size_t)p0 * 2 + g) * N;
+  uint4* const lin = reinterpret_cast<uint4*>(a + 512 * (x >> 5)) + (x & 31);
+  uint32_t sc[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) sc[k] = jx_addr(SC[g][k]);
+  uint32_t v[K][16];
   if (!INVERSE) {
 #pragma unroll
-    for (int r = 0; r < 16; r++) v[r] = mul_shoup(a[x + 128 * r], C.r64, C.r64_p, q);
-    ntt_fwd(v, SC[g], fwd_tw(C), q, x, 1 + g);
+    for (int k = 0; k < K; k++)
 #pragma unroll
-    for (int r = 0; r < 16; r++) v[r] = canon16(v[r], q);
-    uint4* d = reinterpret_cast<uint4*>(a + 16 * x);
+      for (int r = 0; r < 16; r++)
+        v[k][r] = p0 + k < npolys ? a[(size_t)k * 2 * N + x + 128 * r] : 0u;
+    jntt_fwd_scaled<K>(v, sc, sfwd_tw(C), make_uint2(C.r64, C.r64_p), C.r64_w, q, x, 1 + g);
 #pragma unroll
-    for (int r = 0; r < 4; r++) d[r] = make_uint4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
+    for (int k = 0; k < K; k++)
+#pragma unroll
+      for (int r = 0; r < 16; r++) v[k][r] = jcanon_fwd(v[k][r], q);
+    jx_store_ru<K>(v, sc, x);
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (p0 + k < npolys)
+#pragma unroll
+        for (int c = 0; c < 4; c++) lin[(size_t)k * N / 2 + 32 * c] = jx_at4(sc[k] + jx_lin(x, c));
   } else {
-    const uint4* s = reinterpret_cast<const uint4*>(a + 16 * x);
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-      uint4 t = s[r];
-      v[4 * r] = t.x; v[4 * r + 1] = t.y; v[4 * r + 2] = t.z; v[4 * r + 3] = t.w;
-    }
-    ntt_inv_noscale(v, SC[g], inv_tw(C), q, x, 1 + g);
+    for (int k = 0; k < K; k++)
 #pragma unroll
-    for (int r = 0; r < 16; r++) a[x + 128 * r] = mul_shoup(v[r], C.ref_inv_scale, C.ref_inv_scale_p, q);
+      for (int c = 0; c < 4; c++)
+        jx_at4(sc[k] + jx_lin(x, c)) = p0 + k < npolys ? lin[(size_t)k * N / 2 + 32 * c] : make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    jx_load_ru<K>(v, sc, x);
+    jntt_inv_scaled<K>(v, sc, sfwd_tw(C), make_uint2(C.ref_inv_scale, C.ref_inv_scale_p), C.ref_inv_w, q, x, 1 + g);
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (p0 + k < npolys)
+#pragma unroll
+        for (int r = 0; r < 16; r++) a[(size_t)k * 2 * N + x + 128 * r] = v[k][r];
   }
 }
 
 // external_product(rlwe, rgsw): result = sum_i g^-1(a)_i * C[i] + g^-1(b)_i * C[ELL+i].
 // ct[p][2 (a,b)][2][N]; rgsw[p][2*ELL rows][2 (a,b)][2][N]; out[p][2][2][N].
-__global__ void __launch_bounds__(BLOCK) external_product_kernel(const DevParams P, const uint32_t* __restrict__ ct,
-                                                                 const uint32_t* __restrict__ rgsw,
-                                                                 uint32_t* __restrict__ out) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  uint32_t* dig = smem;                   // [2*ELL][N]: digits of a (rows 0..ELL-1), of b (ELL..)
-  uint32_t* SC = dig + 2 * ELL * N;       // [2][NTT_SCRATCH]
+// One pair per CTA, one residue per group; the transforms of a digit and of
+// its row's two parts share their twiddles.  1024 products take 188 us (235 us
+// one transform after the other, four CTAs per SM); 40 transforms a product
+// are 137 us at the rate above.
+constexpr int EXT_WORDS = 2 * ELL * N + 6 * N;  // digits, three exchange buffers per group
+__global__ void __launch_bounds__(BLOCK, 2) external_product_kernel(const DevParams P, const uint32_t* __restrict__ ct,
+                                                                    const uint32_t* __restrict__ rgsw,
+                                                                    uint32_t* __restrict__ out) {
+  extern __shared__ __align__(128) uint32_t smem[];
+  uint32_t* dig = smem;  // [2*ELL][N]: digits of a (rows 0..ELL-1), of b (ELL..)
   const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
   const uint32_t* c = ct + (size_t)p * 4 * N;
+#pragma unroll 4
   for (int j = tid; j < 2 * N; j += BLOCK) {
     const int part = j >> LOGN, jj = j & (N - 1);
     const uint64_t v = crt_compose(P, c[(part * 2 + 0) * N + jj], c[(part * 2 + 1) * N + jj]);
@@ -59,43 +94,44 @@ __global__ void __launch_bounds__(BLOCK) external_product_kernel(const DevParams
   }
   __syncthreads();
   const ResidueConsts& C = P.r[g];
-  const uint32_t q = C.q, qinv = C.qinv, q2 = 2 * q;
-  uint32_t accA[16], accB[16];
+  const uint32_t q = C.q, qinv = C.qinv;
+  const uint32_t xb = jx_addr(smem + 2 * ELL * N + 3 * N * g);
+  uint32_t acc[2][16];
 #pragma unroll
-  for (int r = 0; r < 16; r++) accA[r] = accB[r] = 0;
-  const uint32_t* rows = rgsw + (size_t)p * 2 * ELL * 4 * N;
+  for (int r = 0; r < 16; r++) acc[0][r] = acc[1][r] = 0;
+  const uint32_t* rows = rgsw + (size_t)p * 2 * ELL * 4 * N + (size_t)g * N + x;
+#pragma unroll 1
   for (int d = 0; d < 2 * ELL; d++) {
-    uint32_t dh[16], v[16];
+    uint32_t v[3][16];
 #pragma unroll
-    for (int r = 0; r < 16; r++) dh[r] = dig[d * N + x + 128 * r];
-    ntt_fwd(dh, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
-#pragma unroll
-    for (int r = 0; r < 16; r++) dh[r] = canon16(dh[r], q);  // keeps dh * v < 14 q^2 < q 2^32
-    // row d: (a, b) of residue g
-    for (int part = 0; part < 2; part++) {
-      const uint32_t* rp = rows + ((size_t)(d * 2 + part) * 2 + g) * N;
-#pragma unroll
-      for (int r = 0; r < 16; r++) v[r] = rp[x + 128 * r];
-      ntt_fwd(v, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
-#pragma unroll
-      for (int r = 0; r < 16; r++) {
-        const uint32_t pr = redc_lazy((uint64_t)dh[r] * v[r], q, qinv);
-        if (part == 0) accA[r] = acc_2q(accA[r], pr, q2);
-        else accB[r] = acc_2q(accB[r], pr, q2);
-      }
+    for (int r = 0; r < 16; r++) {
+      v[1][r] = csub(csub(__ldg(rows + (size_t)d * 4 * N + 128 * r), 2 * q), q);
+      v[2][r] = csub(csub(__ldg(rows + (size_t)d * 4 * N + 2 * N + 128 * r), 2 * q), q);
+      v[0][r] = dig[d * N + x + 128 * r];
     }
+    if (d) group_sync(1 + g);  // the previous transforms' last reads are done
+    const uint32_t sc[3] = {xb, xb + 4 * N, xb + 8 * N};
+    jntt_fwd<3, JB_CANON>(v, sc, sfwd_tw(C), q, x, 1 + g);
+    // |v| < 6.5 q: products below 42.3 q^2, reduced below 3.7 q and made positive
+#pragma unroll
+    for (int part = 0; part < 2; part++)
+#pragma unroll
+      for (int r = 0; r < 16; r++)
+        acc[part][r] = csub(acc[part][r] + redc_wide(smul(v[0][r], v[1 + part][r]), q, qinv) + 3 * q, 8 * q);
   }
-  uint32_t* o = out + (size_t)p * 4 * N;
+  // below 8 q each; the inverse takes values below 4 q
 #pragma unroll
-  for (int r = 0; r < 16; r++) accA[r] = reduce_2q(accA[r], q);
-  ntt_inv_noscale(accA, SC + g * NTT_SCRATCH, inv_tw(C), q, x, 1 + g);
+  for (int r = 0; r < 16; r++) {
+    acc[0][r] = csub(acc[0][r], 4 * q);
+    acc[1][r] = csub(acc[1][r], 4 * q);
+  }
+  const uint32_t sc[2] = {xb, xb + 4 * N};
+  jntt_inv_scaled<2>(acc, sc, sfwd_tw(C), make_uint2(C.ninv_mont, C.ninv_mont_p), C.ninv_mont_w, q, x, 1 + g);
+  uint32_t* o = out + (size_t)p * 4 * N + (size_t)g * N + x;
 #pragma unroll
-  for (int r = 0; r < 16; r++) o[(0 * 2 + g) * N + x + 128 * r] = mul_shoup(accA[r], C.ninv_mont, C.ninv_mont_p, q);
+  for (int part = 0; part < 2; part++)
 #pragma unroll
-  for (int r = 0; r < 16; r++) accB[r] = reduce_2q(accB[r], q);
-  ntt_inv_noscale(accB, SC + g * NTT_SCRATCH, inv_tw(C), q, x, 1 + g);
-#pragma unroll
-  for (int r = 0; r < 16; r++) o[(1 * 2 + g) * N + x + 128 * r] = mul_shoup(accB[r], C.ninv_mont, C.ninv_mont_p, q);
+    for (int r = 0; r < 16; r++) o[part * 2 * N + 128 * r] = acc[part][r];
 }
 
 // Throughput probe of the exact modular multiply the transforms are built
@@ -262,12 +298,14 @@ cudaError_t launch_mulmod_rate(const DevParams& P, int blocks, int iters, uint32
 
 cudaError_t launch_ntt_ref(const DevParams& P, uint32_t* polys, int npolys, bool inverse, cudaStream_t st) {
   if (npolys <= 0) return cudaSuccess;
-  if (inverse) ntt_ref_kernel<true><<<npolys, BLOCK, 0, st>>>(P, polys);
-  else ntt_ref_kernel<false><<<npolys, BLOCK, 0, st>>>(P, polys);
+  constexpr int K = NTT_REF_K;
+  const int grid = (npolys + K - 1) / K;
+  if (inverse) ntt_ref_kernel<K, true><<<grid, BLOCK, 0, st>>>(P, polys, npolys);
+  else ntt_ref_kernel<K, false><<<grid, BLOCK, 0, st>>>(P, polys, npolys);
   return cudaGetLastError();
 }
 
-constexpr size_t EXT_SMEM = sizeof(uint32_t) * ((size_t)2 * ELL * N + 2 * NTT_SCRATCH);
+constexpr size_t EXT_SMEM = sizeof(uint32_t) * (size_t)EXT_WORDS;
 
 cudaError_t launch_external_product(const DevParams& P, const uint32_t* ct, const uint32_t* rgsw, uint32_t* out,
                                     int npairs, cudaStream_t st) {

@@ -389,7 +389,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
       const uint32_t sc[1] = {xc + 4 * N * (turn ? r : 2 + r)};
 #pragma unroll
       for (int j = 0; j < 16; j++) v[0][j] = row[x + 128 * j];
-      jntt_fwd<1, true>(v, sc, sfwd_tw(Cs), Cs.q, x, 1 + r);
+      jntt_fwd<1, JB_CANON>(v, sc, sfwd_tw(Cs), Cs.q, x, 1 + r);
 #pragma unroll
       for (int j = 0; j < 16; j++) row[128 * h_of(j) + x] = jcanon_fwd(v[0][j], Cs.q);
     }
@@ -481,7 +481,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
       }
     };
     const uint32_t sc2[2] = {other, own};
-    jntt_fwd<2, false>(v, sc2, sfwd_tw(C), q, x, 1 + r, [&]() { fetch(0); });  // signed, below 5.25 q
+    jntt_fwd<2, JB_DIGIT>(v, sc2, sfwd_tw(C), q, x, 1 + r, [&]() { fetch(0); });  // signed, below 5.25 q
     other = mine;
     mine = sc2[0];
     // [D] the nine products of each slot under two reductions, in signed

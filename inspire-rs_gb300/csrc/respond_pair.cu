@@ -401,7 +401,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
       uint32_t v[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) v[j] = AH[k * N + t + TEAM * j];
-      jt_fwd<true>(v, k == 2 ? s1b : xb, sfwd_tw(Cs), Cs.q, t, 1 + team);
+      jt_fwd<JB_CANON>(v, k == 2 ? s1b : xb, sfwd_tw(Cs), Cs.q, t, 1 + team);
 #pragma unroll
       for (int j = 0; j < 8; j++)
         jx_at(base + 4 * (L::AH + k * N) + ah_off((h_of(j) | (uint32_t)half), x)) = jcanon_fwd(v[j], Cs.q);
@@ -499,7 +499,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
     // [C] its transform, [D] its products (bounds as in respond.cu)
     uint4 w0, w1;
     uint32_t yv[8];
-    jt_fwd<false>(v, xb, sfwd_tw(C), q, t, 1 + team, [&]() {
+    jt_fwd<JB_DIGIT>(v, xb, sfwd_tw(C), q, t, 1 + team, [&]() {
       w0 = ld_stream(wi);
       w1 = ld_stream(wi + 512);
 #pragma unroll
