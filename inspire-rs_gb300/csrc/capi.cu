@@ -419,6 +419,7 @@ int enqueue_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const ui
   a.seeds = seeded ? c->d_seeds.as<uint8_t>() : nullptr;
   a.arows = seeded ? nullptr : c->d_arows.as<uint64_t>();
   a.brows = c->d_brows.as<uint64_t>();
+  a.brow_stride = ELL * pw;
   a.nshards = db->nshards;
   a.H = db->H.as<uint16_t>();
   a.out = c->d_out.as<uint64_t>();
@@ -449,6 +450,57 @@ int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32
   if (n == 0) return INSPIRE_OK;
   const size_t pw = poly_words();
   const size_t col_words = (size_t)db->gamma * 2 * pw;
+  if (seeds && !out_columns) {
+    // Combined ciphertexts of seeded queries whose rows and responses are
+    // page-locked: the kernel reads the rows and writes the responses in
+    // place.  Small batches in other memory are gathered into page-locked
+    // memory first (as in run_batch).  Shards, seeds and status words go
+    // through page-locked memory either way.
+    const size_t out_span = sizeof(uint64_t) * n * 2 * pw;
+    const size_t rows_b = sizeof(uint64_t) * ELL * pw;
+    const uint8_t* d_rows = (uintptr_t)b_rows % 16 == 0  // (the rows are bulk-copied)
+                                ? mapped_range(b_rows, sizeof(uint64_t) * stride_polys * pw * (n - 1) + rows_b)
+                                : nullptr;
+    const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
+    const bool in_place = d_rows && d_outp;
+    if (in_place || n <= STAGE_PINNED_MAX) {
+      const size_t head = (size_t)n * (sizeof(uint32_t) + 32 * ELL);
+      const size_t rows_at = (head + 255) & ~(size_t)255;
+      CUDA_TRY(c->h_stage.ensure(rows_at + (in_place ? 0 : rows_b * n)));
+      CUDA_TRY(c->h_qstatus.ensure(sizeof(int32_t) * n));
+      if (!in_place) CUDA_TRY(c->h_out.ensure(out_span));
+      uint8_t* hb = c->h_stage.host<uint8_t>();
+      uint8_t* hseeds = hb + sizeof(uint32_t) * n;
+      int32_t* hs = c->h_qstatus.host<int32_t>();
+      memcpy(hb, shard_ids, sizeof(uint32_t) * n);
+      for (uint32_t i = 0; i < n; i++) {
+        memcpy(hseeds + (size_t)32 * ELL * i, seeds + i * seed_stride, (size_t)32 * ELL);
+        if (!in_place) memcpy(hb + rows_at + rows_b * i, b_rows + i * stride_polys * pw, rows_b);
+        hs[i] = -1;
+      }
+      const uint8_t* db_ = c->h_stage.dev<uint8_t>();
+      NoPackingArgs a{};
+      a.P = c->P;
+      a.nq = (int)n;
+      a.col_groups = 1;
+      a.shard = reinterpret_cast<const uint32_t*>(db_);
+      a.seeds = db_ + sizeof(uint32_t) * n;
+      a.brows = reinterpret_cast<const uint64_t*>(in_place ? d_rows : db_ + rows_at);
+      a.brow_stride = in_place ? stride_polys * pw : ELL * pw;
+      a.nshards = db->nshards;
+      a.H = db->H.as<uint16_t>();
+      a.out = in_place ? const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_outp)) : c->h_out.dev<uint64_t>();
+      a.status = c->h_qstatus.dev<int32_t>();
+      CUDA_TRY(launch_nopacking(a, true, c->stream));
+      CUDA_TRY(cudaStreamSynchronize(c->stream));
+      for (uint32_t i = 0; i < n; i++)
+        if (hs[i] != 0)
+          return fail(INSPIRE_ERR_DEVICE_STATUS,
+                      "nopacking kernel status " + std::to_string(hs[i]) + " for query " + std::to_string(i));
+      if (!in_place) memcpy(out_ct, c->h_out.host<uint64_t>(), out_span);
+      return INSPIRE_OK;
+    }
+  }
   if (int rc = enqueue_nopacking(c, db, n, shard_ids, seeds, seed_stride, a_rows, b_rows, stride_polys,
                                  out_columns != nullptr))
     return rc;
@@ -1252,6 +1304,7 @@ int inspire_respond_seeded_packed_noalloc_device(inspire_ctx* c, const inspire_d
   a.seeds = d_seeds;
   a.arows = nullptr;
   a.brows = d_b_rows;
+  a.brow_stride = ELL * pw;
   a.nshards = db->nshards;
   a.H = db->H.as<uint16_t>();
   a.out = comb;

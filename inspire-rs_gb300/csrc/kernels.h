@@ -77,7 +77,8 @@ struct NoPackingArgs {
   const uint32_t* shard;
   const uint8_t* seeds;          // [nq][ELL][32] or null
   const uint64_t* arows;         // [nq][ELL][2][N] or null
-  const uint64_t* brows;         // [nq][ELL][2][N]
+  const uint64_t* brows;         // [nq] queries brow_stride words apart, each [ELL][2][N]
+  size_t brow_stride;            // ELL * 2 * N with column ciphertexts
   int nshards;
   const uint16_t* H;             // [nshards][gamma][N]
   uint64_t* out;

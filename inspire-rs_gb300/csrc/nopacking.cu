@@ -1,4 +1,4 @@
-// nopacking.cu -- NoPacking Respond: one CTA per query.
+// nopacking.cu -- NoPacking Respond.
 //
 // respond (src/pir/respond.rs:71-115) and respond_seeded (:408-415): for every
 // column c of the named shard, column_ciphertexts[c] =
@@ -8,21 +8,24 @@
 // trivial encryption is zero), so a_c = sum_t D_{c,t} * a_t and
 // b_c = sum_t D_{c,t} * b_t with D_{c,t} the base-2^20 digit t of Delta*h_c.
 //
-// Layout: 768 threads = six groups of 128; group g = 3 r + t owns CRT residue
-// r and row/digit t and keeps NTT(a_t), NTT(b_t) of its residue in registers
-// (Montgomery form with n^-1 folded) for all columns.  Per column: six digit
-// NTTs and products, then groups (r,0)/(r,1) sum the three digits and run the
-// inverse NTTs of a_c / b_c.  No global scratch.
-#include "expand.cuh"
-#include "kernels.h"
+// With column ciphertexts (nopacking_kernel): 768 threads = six groups of 128;
+// group g = 3 r + t owns CRT residue r and row/digit t and keeps NTT(a_t),
+// NTT(b_t) of its residue in registers (Montgomery form with n^-1 folded) for
+// all columns.  Per column: six digit NTTs and products, then groups
+// (r,0)/(r,1) sum the three digits and run the inverse NTTs of a_c / b_c.
+//
+// Combined ciphertexts only (nopacking_sum_kernel): the NTT is linear, so the
+// columns' digits are summed before they are transformed.
+#include "ntt_joint.cuh"
+#include "respond_draws.cuh"
 
 namespace ig {
 
 namespace {
 
-template <int MODE_UNUSED, bool SEEDED>
+template <bool SEEDED>
 __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_constant__ NoPackingArgs A) {
-  extern __shared__ __align__(16) uint32_t smem[];
+  extern __shared__ __align__(128) uint32_t smem[];
   uint32_t* SC = smem;                        // [RG][NTT_SCRATCH]
   uint32_t* PB = SC + RG * NTT_SCRATCH;       // [2 r][3 t][2 (a,b)][N] products, slot layout (swizzled)
   uint32_t* SUMB = PB + 12 * N;               // [2 r][2 (a,b)][N] running sum over columns (swizzled)
@@ -61,77 +64,6 @@ __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_const
   __syncthreads();
   // the query's status is written once, by one thread
   if (tid == 0 && cg == 0) A.status[qi] = (!SEEDED || (wsb[17] && wsb[37] && wsb[57])) ? 0 : ERR_EXPAND;
-  if (!A.out_columns) {
-    // Combined ciphertext only.  The NTT is linear mod q_r, so
-    // sum_c NTT(D_{c,t}) = NTT(sum_c D_{c,t} mod q_r): one transform of the
-    // digit sum per group gives the sum of the column products exactly.
-    const ResidueConsts& C = P.r[r];
-    uint32_t v[16], w[16];
-#pragma unroll
-    for (int j = 0; j < 16; j++) v[j] = 0;
-    for (int c = 0; c < gamma; c++) {
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        const uint64_t xv = P.delta * (uint64_t)__ldg(H + (size_t)c * N + x + 128 * j);
-        const uint32_t s = v[j] + ((uint32_t)(xv >> (ZBITS * t)) & ((1u << ZBITS) - 1));
-        v[j] = min(s, s - q);  // < q
-      }
-    }
-    ntt_fwd<false>(v, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
-#pragma unroll
-    for (int j = 0; j < 16; j++) w[j] = PB[t * 2 * N + r * N + x + 128 * j];
-    __syncthreads();  // every group holds its a row: PB (row staging) is reused for products
-    const int f = (x >> 1) & 3;
-    const uint64_t* brow = A.brows + (((size_t)qi * ELL + t) * 2 + r) * N;
-#pragma unroll 1
-    for (int ab = 0; ab < 2; ab++) {
-      if (ab == 1) {
-#pragma unroll
-        for (int j = 0; j < 16; j++) w[j] = (uint32_t)__ldg(brow + x + 128 * j);
-      }
-      ntt_fwd<false>(w, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
-      uint32_t* dst = PB + ((r * 3 + t) * 2 + ab) * N + 16 * x;
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        uint32_t pr[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int j = 4 * r4 + e;
-          const uint32_t h = mul_shoup(w[j], C.ninv_mont, C.ninv_mont_p, q);
-          pr[e] = redc_lazy((uint64_t)v[j] * h, q, qinv);
-        }
-        *reinterpret_cast<uint4*>(dst + 4 * (r4 ^ f)) = make_uint4(pr[0], pr[1], pr[2], pr[3]);
-      }
-    }
-    __syncthreads();
-    if (t < 2) {  // (r,0): a, (r,1): b
-      const uint32_t* p0 = PB + ((r * 3 + 0) * 2 + t) * N + 16 * x;
-      const uint32_t* p1 = PB + ((r * 3 + 1) * 2 + t) * N + 16 * x;
-      const uint32_t* p2 = PB + ((r * 3 + 2) * 2 + t) * N + 16 * x;
-#pragma unroll
-      for (int r4 = 0; r4 < 4; r4++) {
-        const int o = 4 * (r4 ^ f);
-        const uint4 a4 = *reinterpret_cast<const uint4*>(p0 + o);
-        const uint4 b4 = *reinterpret_cast<const uint4*>(p1 + o);
-        const uint4 c4 = *reinterpret_cast<const uint4*>(p2 + o);
-        const uint32_t aa[4] = {a4.x, a4.y, a4.z, a4.w}, bb[4] = {b4.x, b4.y, b4.z, b4.w},
-                       cc[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          uint32_t sm = aa[e] + bb[e] + cc[e];  // < 6q
-          sm = min(sm, sm - 4 * q);
-          sm = min(sm, sm - 2 * q);
-          v[4 * r4 + e] = min(sm, sm - q);
-        }
-      }
-      ntt_inv_noscale(v, SC + g * NTT_SCRATCH, inv_tw(C), q, x, 1 + g);
-      uint64_t* o = A.out + (size_t)qi * 4 * N + (size_t)t * 2 * N + (size_t)r * N;
-#pragma unroll
-      for (int j = 0; j < 16; j++) o[x + 128 * j] = canon2(v[j], q);
-    }
-    return;
-  }
-
   // group (r,t): NTT(a_t mod q_r), NTT(b_t mod q_r), kept as x * n^-1 * 2^32
   uint32_t ah[16], bh[16];
   {
@@ -157,7 +89,7 @@ __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_const
     const uint32_t zero[16] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
     store16(sumb, x, zero);
   }
-  uint64_t* outc = A.out_columns ? A.out_columns + (size_t)qi * gamma * 4 * N : nullptr;
+  uint64_t* outc = A.out_columns + (size_t)qi * gamma * 4 * N;
 
   for (int c = c0; c < c1; c++) {
     // digit t of Delta * h_c, NTT mod q_r, products with this group's row
@@ -215,12 +147,10 @@ __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_const
         }
         *sp = make_uint4(ss[0], ss[1], ss[2], ss[3]);
       }
-      if (outc) {
-        ntt_inv_noscale(v, SC + g * NTT_SCRATCH, inv_tw(P.r[r]), q, x, 1 + g);
-        uint64_t* o = outc + ((size_t)c * 2 + t) * 2 * N + (size_t)r * N;
+      ntt_inv_noscale(v, SC + g * NTT_SCRATCH, inv_tw(P.r[r]), q, x, 1 + g);
+      uint64_t* o = outc + ((size_t)c * 2 + t) * 2 * N + (size_t)r * N;
 #pragma unroll
-        for (int j = 0; j < 16; j++) o[x + 128 * j] = canon2(v[j], q);
-      }
+      for (int j = 0; j < 16; j++) o[x + 128 * j] = canon2(v[j], q);
     }
     __syncthreads();
   }
@@ -232,6 +162,199 @@ __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_const
     uint64_t* o = A.out + (size_t)qi * 4 * N + (size_t)t * 2 * N + (size_t)r * N;
 #pragma unroll
     for (int j = 0; j < 16; j++) o[x + 128 * j] = canon2(sv[j], q);
+  }
+}
+
+// The combined ciphertext of one query: sum_c NTT(D_{c,t}) = NTT(sum_c
+// D_{c,t} mod q_r), so per residue three digit sums, three a rows and three b
+// rows are transformed and two sums of products transformed back.
+//
+// 512 threads, group (r, s) of 128 owning residue r's side s, and a producer
+// warp.  The a groups (s = 0) expand the rows while the b groups sum and
+// transform the digits; then each side transforms its rows, multiplies them
+// with the digits' transforms (thread for thread in shared memory) and writes
+// its half of the response.  Rows may lie in page-locked host memory (the
+// producer copies them in small chunks) and the response may be written there.
+//
+// What bounds it: for rows and responses in host memory the link (measured 210
+// GB/s of reads and 200 GB/s of writes, 82 us for the 12.6 and 8.4 MB of 128
+// queries together: the kernel takes 93 us); the transforms and the expansion
+// alone take 36 us.  128 queries take 114 us per host call: 200 us through
+// device buffers (62 us of them a 768-thread kernel), 133 us with the rows
+// read where they are used.
+struct SumSmem {
+  static constexpr int AH = 0;                   // [ELL][2][N] rows' a, coefficients; exchange buffers in turn
+  static constexpr int XD = AH + ELL * 2 * N;    // [2 r][ELL][N] the digit sums' exchange buffers, then transforms
+  static constexpr int DIG = XD + 2 * ELL * N;   // [ELL][N] digit sums; then XB [2 r][N], the b rows' exchange buffers
+  static constexpr int ROWS = DIG + ELL * N;     // [ELL][2][N] u64, the staged b rows
+  static constexpr int WS = ROWS + 2 * ELL * 2 * N;  // expansion's workspace
+  static constexpr int SEED = WS + 32;           // [ELL * 8] staged seeds
+  static constexpr int BARS = SEED + 24;         // [ELL][ROW_CHUNKS] mbarriers
+  static constexpr int TOTAL = BARS + 2 * ELL * 8;
+};
+constexpr int ST = 2 * QT;      // threads of the two sides
+constexpr int CHUNK = 512;      // u64 words of a staged chunk (4 KiB)
+constexpr int ROW_CHUNKS = 2 * N / CHUNK;
+static_assert(ROW_CHUNKS == 8, "mbarriers of SumSmem");
+
+template <bool SEEDED>
+__global__ void __launch_bounds__(ST + 32, 1) nopacking_sum_kernel(const __grid_constant__ NoPackingArgs A) {
+  using L = SumSmem;
+  extern __shared__ __align__(128) uint32_t smem[];
+  uint32_t* AH = smem + L::AH;
+  uint32_t* DIG = smem + L::DIG;
+  uint64_t* rows = reinterpret_cast<uint64_t*>(smem + L::ROWS);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BARS);
+  int* ws = reinterpret_cast<int*>(smem + L::WS);
+  const DevParams& P = A.P;
+  const int qi = blockIdx.x;
+  const int tid = threadIdx.x, s = tid >> 8, r = (tid >> 7) & 1, x = tid & 127, gamma = P.gamma;
+  const int bar = 1 + (tid >> 7);  // this group's barrier
+  const uint32_t shard = A.shard[qi];
+  if (shard >= (uint32_t)A.nshards) {
+    if (tid == 0) A.status[qi] = ERR_INDEX;
+    return;  // uniform over the CTA
+  }
+  const uint16_t* H = A.H + (size_t)shard * gamma * N;
+  if (tid == ST)
+    for (int k = 0; k < ELL * ROW_CHUNKS; k++) mbar_init(bars + k);
+  if (tid < ELL) ws[20 + tid] = 1;
+  uint8_t* const seeds = reinterpret_cast<uint8_t*>(smem + L::SEED);
+  if (SEEDED && tid < ELL * 32) seeds[tid] = A.seeds[(size_t)qi * ELL * 32 + tid];
+  __syncthreads();
+  const ResidueConsts& C = P.r[r];
+  const uint32_t q = C.q, qinv = C.qinv;
+  const uint32_t xd = jx_addr(smem + L::XD + r * ELL * N), xb = jx_addr(smem + L::DIG + r * N);
+  uint32_t v[1][16], acc[1][16];
+#pragma unroll
+  for (int j = 0; j < 16; j++) acc[0][j] = 0;
+  // acc += v times the digit sum t's transform: |v|, |d| < 6.5 q, so products
+  // are below 42.3 q^2, reduced below 3.7 q and made positive; acc below 8 q
+  auto add_product = [&](int t) {
+    uint32_t d[1][16];
+    const uint32_t sd[1] = {xd + 4 * N * t};
+    jx_load_ru<1>(d, sd, x);
+#pragma unroll
+    for (int j = 0; j < 16; j++)
+      acc[0][j] = csub(acc[0][j] + redc_wide(smul(v[0][j], d[0][j]), q, qinv) + 3 * q, 8 * q);
+  };
+  bool arrived = true;
+  if (s == 2) {
+    // the producer: two chunks in flight.  A device read (twiddles, columns)
+    // queued behind a long host read waits for all of it: 96 KiB per SM at
+    // once from 128 SMs held the other groups up for 50 us.
+    if (tid == ST) {
+      const uint64_t* src = A.brows + (size_t)qi * A.brow_stride;
+      for (int k = 0; k < ELL * ROW_CHUNKS && arrived; k++) {
+        if (k >= 2) arrived = mbar_wait(bars + k - 2, 0, STAGE_WAIT_ITERS_DEFAULT);
+        mbar_expect_tx(bars + k, sizeof(uint64_t) * CHUNK);
+        bulk_g2s(rows + (size_t)k * CHUNK, src + (size_t)k * CHUNK, sizeof(uint64_t) * CHUNK, bars + k);
+      }
+    }
+  } else if (s == 0) {
+    if (SEEDED) {
+      expand_rows<2>(P, seeds, AH, ws);
+    } else {
+      const uint64_t* ar = A.arows + (size_t)qi * ELL * 2 * N;
+#pragma unroll 4
+      for (int j = tid; j < ELL * 2 * N; j += QT) AH[j] = (uint32_t)__ldg(ar + j);
+    }
+    named_sync(EXPAND_BAR, QT);
+    named_arrive(7, ST);  // the b groups may look at ws
+    const bool redo = SEEDED && !(ws[20] && ws[21] && ws[22]);  // uniform
+    if (redo) {
+      named_sync(8, ST);  // the b groups are done with the staged rows: room for candidates
+      bool good = true;
+#pragma unroll 1
+      for (int t = 0; t < ELL; t++)
+        if (!ws[20 + t]) good &= expand_row_general<2>(P, seeds + 32 * t, rows, AH + t * 2 * N, ws);
+      named_sync(EXPAND_BAR, QT);
+      if (!good) arrived = false;
+    }
+    named_sync(5 + r, QT);  // the digits' transforms of this residue are there
+#pragma unroll 1
+    for (int t = 0; t < ELL; t++) {
+      uint32_t* row = AH + (t * 2 + r) * N;
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[0][j] = row[x + 128 * j];
+      group_sync(bar);  // the row is read: its words become its exchange buffer
+      const uint32_t sc[1] = {jx_addr(row)};
+      jntt_fwd<1, JB_CANON>(v, sc, sfwd_tw(C), q, x, bar);
+      add_product(t);
+    }
+  } else {
+    // digit sums: below 2^24 (the transform takes any such sum: for q near
+    // 2^28 it is below q / 16, and for smaller q nothing comes near 32 bits)
+    const uint32_t* h2 = reinterpret_cast<const uint32_t*>(H) + (tid - QT);
+#pragma unroll 1
+    for (int m = 0; m < N / 2 / QT; m++) {
+      uint32_t sum[2][ELL] = {};
+#pragma unroll
+      for (int c = 0; c < MAX_GAMMA; c++) {
+        if (c >= gamma) continue;
+        const uint32_t hw = __ldg(h2 + (size_t)c * (N / 2) + QT * m);
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const uint64_t xv = P.delta * (uint64_t)((hw >> (16 * e)) & 0xFFFFu);
+          sum[e][0] += (uint32_t)xv & 0xFFFFFu;
+          sum[e][1] += (uint32_t)(xv >> 20) & 0xFFFFFu;
+          sum[e][2] += (uint32_t)(xv >> 40);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < ELL; t++)
+        *reinterpret_cast<uint2*>(DIG + t * N + 2 * (tid - QT + QT * m)) = make_uint2(sum[0][t], sum[1][t]);
+    }
+    named_sync(9, QT);
+    {
+      uint32_t d[ELL][16];
+#pragma unroll
+      for (int t = 0; t < ELL; t++)
+#pragma unroll
+        for (int j = 0; j < 16; j++) d[t][j] = DIG[t * N + x + 128 * j];
+      named_sync(9, QT);  // DIG is read: its words become the b rows' exchange buffers
+      const uint32_t sc[ELL] = {xd, xd + 4 * N, xd + 8 * N};
+      jntt_fwd<ELL, JB_CANON>(d, sc, sfwd_tw(C), q, x, bar);
+      jx_store_ru<ELL>(d, sc, x);
+      named_arrive(5 + r, QT);
+    }
+#pragma unroll 1
+    for (int t = 0; t < ELL; t++) {
+      for (int k = 0; k < ROW_CHUNKS; k++)
+        if (arrived) arrived = mbar_wait(bars + t * ROW_CHUNKS + k, 0, STAGE_WAIT_ITERS_DEFAULT);
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(rows + ((size_t)t * 2 + r) * N);
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[0][j] = row[2 * (x + 128 * j)];
+      if (t) group_sync(bar);  // the last transform's reads are done
+      const uint32_t sc[1] = {xb};
+      jntt_fwd<1, JB_CANON>(v, sc, sfwd_tw(C), q, x, bar);
+      add_product(t);
+    }
+    named_sync(7, ST);
+    if (SEEDED && !(ws[20] && ws[21] && ws[22])) named_arrive(8, ST);
+  }
+  if (s < 2) {
+    // this side's half of the response
+#pragma unroll
+    for (int j = 0; j < 16; j++) acc[0][j] = csub(acc[0][j], 4 * q);
+    {
+      const uint32_t sc[1] = {s ? xb : jx_addr(AH + ((ELL - 1) * 2 + r) * N)};
+      jntt_inv_scaled<1>(acc, sc, sfwd_tw(C), make_uint2(C.ninv_mont, C.ninv_mont_p), C.ninv_mont_w, q, x, bar);
+    }
+    uint64_t* o = A.out + (size_t)qi * 4 * N + (size_t)(2 * s + r) * N + x;
+#pragma unroll
+    for (int j = 0; j < 16; j++) o[128 * j] = acc[0][j];
+  }
+  // rows that did not arrive within the wait's bound end the query with a
+  // status, after another bounded wait for the copies still in flight
+  const int late = __syncthreads_or(s != 0 && !arrived), bad = __syncthreads_or(s == 0 && !arrived);
+  if (late) {
+    bool here = true;  // the producer issues at most the chunk after next beyond the last one that came
+    for (int k = 0; k < ELL * ROW_CHUNKS && here; k++) here = mbar_wait(bars + k, 0, STAGE_DRAIN_ITERS);
+    const int lost = __syncthreads_or(!here);
+    if (tid == 0) A.status[qi] = lost ? ERR_STAGE_LOST : ERR_STAGE;
+  } else if (tid == 0) {
+    A.status[qi] = bad ? ERR_EXPAND : 0;
   }
 }
 
@@ -259,7 +382,11 @@ size_t nopacking_smem_bytes() { return sizeof(uint32_t) * ((size_t)RG * NTT_SCRA
 
 template <bool SEEDED>
 static cudaError_t launch_np(const NoPackingArgs& a, cudaStream_t st) {
-  nopacking_kernel<0, SEEDED><<<a.nq * a.col_groups, RBLOCK, nopacking_smem_bytes(), st>>>(a);
+  if (!a.out_columns) {
+    nopacking_sum_kernel<SEEDED><<<a.nq, ST + 32, sizeof(uint32_t) * SumSmem::TOTAL, st>>>(a);
+    return cudaGetLastError();
+  }
+  nopacking_kernel<SEEDED><<<a.nq * a.col_groups, RBLOCK, nopacking_smem_bytes(), st>>>(a);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess && a.col_groups > 1) {
     const size_t words = (size_t)a.nq * 4 * N;
@@ -271,9 +398,14 @@ static cudaError_t launch_np(const NoPackingArgs& a, cudaStream_t st) {
 
 cudaError_t prepare_nopacking_kernels() {
   const int smem = (int)nopacking_smem_bytes();
-  cudaError_t e = cudaFuncSetAttribute(nopacking_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(nopacking_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(nopacking_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(nopacking_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const int sum = (int)sizeof(uint32_t) * SumSmem::TOTAL;
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(nopacking_sum_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, sum);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(nopacking_sum_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, sum);
   return e;
 }
 

@@ -59,8 +59,6 @@ namespace ig {
 
 namespace {
 
-constexpr int QT = 256;  // threads per query
-
 // Shared memory in u32 words (NR = residues of the a side).  80 KiB and a
 // little: two CTAs fit the SM's 164 KiB configuration, which leaves it 92 KiB
 // of L1 for the twiddles and the client keys.
@@ -96,88 +94,6 @@ __device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows
     } else {
       bulk_g2s(d, s + k0, CHW * 8, bar);
     }
-  }
-}
-
-// Poly::from_seed_moduli (poly.rs:251-281) of the ELL rows by the whole CTA.
-// Draws 0 .. 2047 (blocks 0-255, a thread each) go to residue 0, whose few
-// missing values (rejections: 2^28 - q of 2^28 draws) come from the start of
-// the next 256 blocks, found by warp 0; residue 1 follows there, and one warp
-// per row draws the last ~155 values.  Seven rounds of ChaCha20 for the three
-// rows together (one row after the other needs nine, three of them tails of
-// one warp).  A row whose stream rejects more than that leaves 0 in
-// ok[row]: a general pass redoes it.
-template <int NR>
-__device__ __forceinline__ void expand_rows(const DevParams& P, const uint8_t* seeds, uint32_t* AH, int* ws) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t q0 = P.r[0].q, z0 = (uint32_t)(P.r[0].zone >> 32);
-  const uint32_t q1 = P.r[1].q, z1 = (uint32_t)(P.r[1].zone >> 32);
-  int* tot = ws + 16;   // [ELL] values drawn so far: residue 0, then residue 1
-  int* ok = ws + 20;    // [ELL]
-#pragma unroll 1
-  for (int t = 0; t < ELL; t++) {
-    uint32_t key[8], w[16], val[8];
-    load_key(seeds + 32 * t, key);
-    chacha20_block(key, tid, P.one, w);
-    const unsigned mask = draw8(w, q0, z0, val);
-    int total;
-    const int p = scan_256(__popc(mask), ws + 8 * (t & 1), total, 0);
-    put_draws(AH + t * NR * N, p, mask, val);
-    if (tid == 0) tot[t] = total;
-  }
-  __syncthreads();
-  if (NR == 2) {
-#pragma unroll 1
-    for (int t = 0; t < ELL; t++) {
-      uint32_t key[8], w[16], val[8];
-      load_key(seeds + 32 * t, key);
-      chacha20_block(key, QT + tid, P.one, w);
-      uint32_t* a0 = AH + t * NR * N;
-      int start = 0;  // warp 0: draws before it belong to residue 0
-      if (warp == 0) {
-        const int have = tot[t];
-        if (have < N) {  // uniform over the warp
-          const unsigned m0 = draw8(w, q0, z0, val);
-          int all;
-          const int p = have + scan_warp(__popc(m0), all);
-          put_draws(a0, p, m0, val);
-          // the lane that holds value N - 1 knows where residue 1 starts
-          int end = 0, pp = p;
-#pragma unroll
-          for (int k = 0; k < 8; k++)
-            if ((m0 >> k) & 1u) {
-              if (pp == N - 1) end = 8 * lane + k + 1;
-              pp++;
-            }
-          start = __reduce_max_sync(0xffffffffu, end);
-          if (lane == 0) ok[t] = start != 0;
-        } else if (lane == 0) {
-          ok[t] = 1;
-        }
-      }
-      unsigned mask = draw8(w, q1, z1, val);
-      if (warp == 0) {
-        const int skip = start - 8 * lane;  // leading draws of this lane to skip
-        if (skip > 0) mask &= skip >= 8 ? 0u : ~((1u << skip) - 1u);
-      }
-      int total;
-      const int p = scan_256(__popc(mask), ws + 8 * ((t + 1) & 1), total, 0);
-      put_draws(a0 + N, p, mask, val);
-      if (tid == 0) tot[t] = total;
-    }
-    __syncthreads();
-  }
-  if (warp < ELL) {  // the tails, one warp per row
-    const int t = warp;
-    uint32_t key[8], w[16], val[8];
-    load_key(seeds + 32 * t, key);
-    chacha20_block(key, (NR == 2 ? 2 * QT : QT) + lane, P.one, w);
-    const unsigned mask = NR == 2 ? draw8(w, q1, z1, val) : draw8(w, q0, z0, val);
-    int all;
-    const int have = tot[t];
-    const int p = have + scan_warp(__popc(mask), all);
-    put_draws(AH + (t * NR + NR - 1) * N, p, mask, val);
-    if (lane == 0) ok[t] = (NR == 1 || ok[t]) && have + all >= N;
   }
 }
 
