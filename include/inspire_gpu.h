@@ -559,8 +559,8 @@ int inspire_extract_inspiring_device(inspire_ctx *ctx, const uint64_t *d_sk, con
  * d_b_rows [n][gadget_len][poly] of RGSW rows gadget_len..2*gadget_len-1,
  * as inspire_respond_seeded_batch_device takes them; d_out_a [n][poly],
  * d_out_b [n][2 polys], d_status [n]) and enqueues its work on `stream`
- * without allocating: its scratch (column ciphertexts, combined ciphertext,
- * the tree's work area; 2.0 MiB per query) is one static device array per
+ * without allocating: its scratch (the row transforms and the tree's
+ * ciphertexts; 1 MiB per query) is one static device array per
  * device, whose address is looked up with cudaGetSymbolAddress on every
  * call.  The first call on a device may load the library's device code into
  * that device's context (CUDA's lazy loading), so make it before any stream

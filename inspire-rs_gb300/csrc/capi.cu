@@ -511,12 +511,10 @@ int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32
   return finish_status(c, n, "nopacking");
 }
 
-// respond_one_packing (src/pir/respond.rs:213-268) of n queries: column
-// products on the GPU (the NoPacking kernel, columns kept on the device),
-// then pack_lwes with the CRS's Galois keys (tree.cu).  Query i's packed a
-// goes to out_a[i] (one poly) and its b to out_b[i] (room for two polys):
-// *b_words words, one poly, or two in compat mode (the crate's
-// dimension-2d b polynomial).
+// respond_one_packing (src/pir/respond.rs:213-268) of n queries (tree.cu)
+// with the CRS's Galois keys.  Query i's packed a goes to out_a[i] (one poly)
+// and its b to out_b[i] (room for two polys): *b_words words, one poly, or
+// two in compat mode (the crate's dimension-2d b polynomial).
 int run_tree(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* shard_ids, const uint8_t* seeds,
              size_t seed_stride, const uint64_t* a_rows, const uint64_t* b_rows, size_t stride_polys, uint64_t* out_a,
              uint64_t* out_b, uint32_t* b_words) {
@@ -525,24 +523,74 @@ int run_tree(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* s
   const uint32_t words = (c->mode == MODE_COMPAT && db->gamma > 1) ? (uint32_t)(2 * pw) : (uint32_t)pw;
   *b_words = words;
   if (n == 0) return INSPIRE_OK;
-  if (int rc = enqueue_nopacking(c, db, n, shard_ids, seeds, seed_stride, a_rows, b_rows, stride_polys, true))
-    return rc;
+  const bool seeded = seeds != nullptr;
+  const size_t rows_b = sizeof(uint64_t) * ELL * pw;
+  // page-locked rows and outputs are read and written in place; other rows
+  // are copied to the device, other outputs from it
+  const bool aligned = ((uintptr_t)b_rows | (uintptr_t)out_a | (uintptr_t)out_b) % sizeof(uint64_t) == 0;
+  const uint8_t* d_rows = seeded && aligned
+                              ? mapped_range(b_rows, sizeof(uint64_t) * stride_polys * pw * (n - 1) + rows_b)
+                              : nullptr;
+  const uint8_t* d_oa = d_rows ? mapped_range(out_a, sizeof(uint64_t) * pw * n) : nullptr;
+  const uint8_t* d_ob = d_oa ? mapped_range(out_b, sizeof(uint64_t) * 2 * pw * n) : nullptr;
+  const bool in_place = d_ob != nullptr;
   CUDA_TRY(c->tree_work.ensure(sizeof(uint32_t) * tree_work_words_per_query() * n));
-  CUDA_TRY(c->d_tree_out.ensure(sizeof(uint64_t) * 3 * pw * n));
+  // shards, seeds and status words in page-locked memory
+  CUDA_TRY(c->h_stage.ensure((size_t)n * (sizeof(uint32_t) + 32 * ELL)));
+  CUDA_TRY(c->h_qstatus.ensure(sizeof(int32_t) * n));
+  uint8_t* hb = c->h_stage.host<uint8_t>();
+  int32_t* hs = c->h_qstatus.host<int32_t>();
+  memcpy(hb, shard_ids, sizeof(uint32_t) * n);
+  for (uint32_t i = 0; i < n; i++) {
+    if (seeded) memcpy(hb + sizeof(uint32_t) * n + (size_t)32 * ELL * i, seeds + i * seed_stride, (size_t)32 * ELL);
+    hs[i] = -1;
+  }
   TreeArgs t{};
   t.P = c->P;
   t.nq = (int)n;
   t.ncols = db->gamma;
   t.mode = c->mode;
-  t.cols = c->d_cols.as<uint64_t>();
+  t.shard = c->h_stage.dev<uint32_t>();
+  t.seeds = seeded ? c->h_stage.dev<uint8_t>() + sizeof(uint32_t) * n : nullptr;
+  t.nshards = db->nshards;
+  t.E = db->E.as<uint32_t>();
+  t.H = db->H.as<uint16_t>();
   t.ks = c->galois.as<uint32_t>();
   t.work = c->tree_work.as<uint32_t>();
-  t.out_a = c->d_tree_out.as<uint64_t>();
-  t.out_b = t.out_a + pw * n;
-  CUDA_TRY(launch_pack_tree(t, c->stream));
-  CUDA_TRY(cudaMemcpyAsync(out_a, t.out_a, sizeof(uint64_t) * pw * n, cudaMemcpyDeviceToHost, c->stream));
-  CUDA_TRY(cudaMemcpyAsync(out_b, t.out_b, sizeof(uint64_t) * 2 * pw * n, cudaMemcpyDeviceToHost, c->stream));
-  return finish_status(c, n, "nopacking");
+  t.status = c->h_qstatus.dev<int32_t>();
+  if (in_place) {
+    t.brows = reinterpret_cast<const uint64_t*>(d_rows);
+    t.brow_stride = stride_polys * pw;
+    t.out_a = const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_oa));
+    t.out_b = const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_ob));
+  } else {
+    CUDA_TRY(c->d_brows.ensure(rows_b * n));
+    CUDA_TRY(c->d_tree_out.ensure(sizeof(uint64_t) * 3 * pw * n));
+    CUDA_TRY(cudaMemcpy2DAsync(c->d_brows.p, rows_b, b_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
+                               cudaMemcpyHostToDevice, c->stream));
+    if (!seeded) {
+      CUDA_TRY(c->d_arows.ensure(rows_b * n));
+      CUDA_TRY(cudaMemcpy2DAsync(c->d_arows.p, rows_b, a_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
+                                 cudaMemcpyHostToDevice, c->stream));
+      t.arows = c->d_arows.as<uint64_t>();
+    }
+    t.brows = c->d_brows.as<uint64_t>();
+    t.brow_stride = ELL * pw;
+    t.out_a = c->d_tree_out.as<uint64_t>();
+    t.out_b = t.out_a + pw * n;
+  }
+  CUDA_TRY(launch_tree(t, seeded, c->stream));
+  if (!in_place) {
+    CUDA_TRY(cudaMemcpyAsync(out_a, t.out_a, sizeof(uint64_t) * pw * n, cudaMemcpyDeviceToHost, c->stream));
+    CUDA_TRY(cudaMemcpy2DAsync(out_b, sizeof(uint64_t) * 2 * pw, t.out_b, sizeof(uint64_t) * 2 * pw,
+                               sizeof(uint64_t) * words, n, cudaMemcpyDeviceToHost, c->stream));
+  }
+  CUDA_TRY(cudaStreamSynchronize(c->stream));
+  for (uint32_t i = 0; i < n; i++)
+    if (hs[i] != 0)
+      return fail(INSPIRE_ERR_DEVICE_STATUS,
+                  "tree packing kernel status " + std::to_string(hs[i]) + " for query " + std::to_string(i));
+  return INSPIRE_OK;
 }
 
 // Validation order of respond_inspiring (src/pir/respond.rs:295-305, 365-370).
@@ -1010,7 +1058,7 @@ int inspire_crs_load_galois_keys(inspire_ctx* c, const uint64_t* keys, uint32_t 
   CUDA_TRY(staged.ensure(sizeof(uint64_t) * npolys * pw));
   CUDA_TRY(cudaMemcpyAsync(staged.p, keys, sizeof(uint64_t) * npolys * pw, cudaMemcpyHostToDevice, c->stream));
   CUDA_TRY(c->galois.ensure(sizeof(uint32_t) * npolys * pw));
-  CUDA_TRY(launch_galois_prep(c->P, staged.as<uint64_t>(), (int)npolys, c->galois.as<uint32_t>(), c->stream));
+  CUDA_TRY(launch_galois_prep(c->P, staged.as<uint64_t>(), (int)nkeys, c->galois.as<uint32_t>(), c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   c->has_galois = true;
   return INSPIRE_OK;
@@ -1293,36 +1341,24 @@ int inspire_respond_seeded_packed_noalloc_device(inspire_ctx* c, const inspire_d
   if (int rc = set_device(c)) return rc;
   void* scratch = nullptr;
   CUDA_TRY(tree_noalloc_scratch(c->device, &scratch));
-  // carve: columns [n][gamma][2][poly] u64, combined [n][2][poly] u64, tree work (u32)
-  uint64_t* cols = static_cast<uint64_t*>(scratch);
-  uint64_t* comb = cols + (size_t)n * db->gamma * 2 * pw;
-  uint32_t* work = reinterpret_cast<uint32_t*>(comb + (size_t)n * 2 * pw);
-  NoPackingArgs a{};
-  a.P = c->P;
-  a.nq = (int)n;
-  a.shard = d_shard_ids;
-  a.seeds = d_seeds;
-  a.arows = nullptr;
-  a.brows = d_b_rows;
-  a.brow_stride = ELL * pw;
-  a.nshards = db->nshards;
-  a.H = db->H.as<uint16_t>();
-  a.out = comb;
-  a.out_columns = cols;
-  a.status = d_status;
-  a.col_groups = column_groups(c, db, n, true);
-  CUDA_TRY(launch_nopacking(a, true, (cudaStream_t)stream));
   TreeArgs t{};
   t.P = c->P;
   t.nq = (int)n;
   t.ncols = db->gamma;
   t.mode = c->mode;
-  t.cols = cols;
+  t.shard = d_shard_ids;
+  t.seeds = d_seeds;
+  t.brows = d_b_rows;
+  t.brow_stride = ELL * pw;
+  t.nshards = db->nshards;
+  t.E = db->E.as<uint32_t>();
+  t.H = db->H.as<uint16_t>();
   t.ks = c->galois.as<uint32_t>();
-  t.work = work;
+  t.work = static_cast<uint32_t*>(scratch);
   t.out_a = d_out_a;
   t.out_b = d_out_b;
-  CUDA_TRY(launch_pack_tree(t, (cudaStream_t)stream));
+  t.status = d_status;
+  CUDA_TRY(launch_tree(t, true, (cudaStream_t)stream));
   return INSPIRE_OK;
 }
 

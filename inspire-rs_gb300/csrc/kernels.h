@@ -134,16 +134,24 @@ struct GaloisGenArgs {
   int* status;  // [nmat]
 };
 
-// Tree packing (respond_one_packing) of nq queries' column ciphertexts.
+// Tree packing (respond_one_packing) of nq queries.
 struct TreeArgs {
   DevParams P;
   int nq, ncols;
   int mode;
-  const uint64_t* cols;  // [nq][ncols][2 (a, b)][2][N] column ciphertexts
-  const uint32_t* ks;    // [log2 N][ELL][2 (a, b)][2][N] Galois keys, NTT domain x n^-1 2^32
-  uint32_t* work;        // [nq][tree_work_words_per_query()] ciphertexts of the tree
-  uint64_t* out_a;       // [nq][2][N]
-  uint64_t* out_b;       // [nq][4][N]: 2 residues x N, or 4 N words in compat mode
+  const uint32_t* shard;  // [nq]
+  const uint8_t* seeds;   // [nq][ELL][32] or null
+  const uint64_t* arows;  // [nq][ELL][2][N] or null
+  const uint64_t* brows;  // [nq] queries brow_stride words apart, each [ELL][2][N]
+  size_t brow_stride;
+  int nshards;
+  const uint32_t* E;      // [nshards][2][gamma][ELL][N] contracted database
+  const uint16_t* H;      // [nshards][gamma][N]
+  const uint32_t* ks;     // [log2 N][2 (a, b)][ELL][2][N] Galois keys, folded, quads
+  uint32_t* work;         // [nq][tree_work_words_per_query()]
+  uint64_t* out_a;        // [nq][2][N]
+  uint64_t* out_b;        // [nq][4][N]: 2 residues x N, or 4 N words in compat mode
+  int* status;            // [nq]
 };
 
 // Set the kernels' dynamic shared-memory limits on the current device (once
@@ -159,13 +167,11 @@ cudaError_t launch_query_gen(const QueryGenArgs& a, int n, cudaStream_t st);
 // Allocation-free tree packing: a static device array holds the scratch of
 // up to TREE_NOALLOC_MAX_QUERIES queries.
 constexpr int TREE_NOALLOC_MAX_QUERIES = 2;
-size_t tree_noalloc_query_bytes();
 cudaError_t tree_noalloc_scratch(int device, void** ptr);
-size_t tree_smem_bytes();
 size_t tree_work_words_per_query();
 cudaError_t prepare_tree_kernels();
-cudaError_t launch_pack_tree(const TreeArgs& a, cudaStream_t st);
-cudaError_t launch_galois_prep(const DevParams& P, const uint64_t* keys, int npolys, uint32_t* ks, cudaStream_t st);
+cudaError_t launch_tree(const TreeArgs& a, bool seeded, cudaStream_t st);
+cudaError_t launch_galois_prep(const DevParams& P, const uint64_t* keys, int nkeys, uint32_t* ks, cudaStream_t st);
 size_t galois_keys_smem_bytes();
 // Key-switching matrices 0 .. nmat-1 (nmat <= LOGN + 4): the LOGN Galois
 // matrices, k_g, k_h, packing_k_g, packing_k_h.

@@ -73,122 +73,6 @@ struct Smem {
   static constexpr int TOTAL = BAR + 8;
 };
 
-// Serving loop: the query's b rows (u64) are staged in four chunks, one after
-// the other in the exchange buffers.  Chunk m covers coefficients i in
-// [512 m, 512 m + 512) of the reversed rows, i.e. row words N - i: words
-// 512 (3 - m) .. and one pair more (for m = 0 that pair is words 0, 1).
-constexpr int CH = 512;
-constexpr int CHW = CH + 2;  // u64 words of one polynomial's chunk
-static_assert(2 * ELL * CHW * 8 <= 4 * N * 4, "a chunk fits the exchange buffers");
-
-__device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows, int m, uint64_t* bar) {
-  mbar_expect_tx(bar, 2 * ELL * CHW * 8);
-  const int k0 = N - CH * (m + 1);
-#pragma unroll 1
-  for (int p = 0; p < 2 * ELL; p++) {
-    uint64_t* d = dst + p * CHW;
-    const uint64_t* s = brows + (size_t)p * N;
-    if (m == 0) {
-      bulk_g2s(d, s + k0, CH * 8, bar);
-      bulk_g2s(d + CH, s, 16, bar);
-    } else {
-      bulk_g2s(d, s + k0, CHW * 8, bar);
-    }
-  }
-}
-
-// The b side (see the file comment): b0_c = -sum_i d_{c}[i] v[i] with v[0] =
-// q - b[0], v[i] = b[N - i].  Thread tid takes the coefficient pairs j = tid +
-// 256 m, m < 4, of every column, so each row word is read once, straight
-// from its buffer (QDB: from the staged chunks), and every column word once;
-// 32 sums (column, residue) per thread, exact in 64 bits (6144 products below
-// 2^48), are then transposed and added over the warp by shuffles, five
-// halving exchanges, and over the warps in shared memory.  Measured against
-// the separate launch it replaces: 14.3 us per 128 queries there.
-// Returns -1, or (QDB) the chunk that did not arrive.
-template <bool QDB>
-__device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __restrict__ H, const uint64_t* brows,
-                                          uint64_t* stage, uint64_t* bar, uint32_t wait_iters, uint64_t* red,
-                                          uint32_t* bpoly) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gamma = P.gamma;
-  const uint32_t* h2 = reinterpret_cast<const uint32_t*>(H) + tid;
-  uint64_t acc[32];  // [column][residue]
-#pragma unroll
-  for (int k = 0; k < 32; k++) acc[k] = 0;
-#pragma unroll 1
-  for (int m = 0; m < 4; m++) {
-    uint32_t hw[MAX_GAMMA];
-#pragma unroll
-    for (int c = 0; c < MAX_GAMMA; c++) hw[c] = c < gamma ? __ldg(h2 + (size_t)c * (N / 2) + QT * m) : 0u;
-    uint32_t bv[2][2 * ELL];
-    const int i0 = 2 * (tid + QT * m);
-    if (QDB) {
-      const bool arrived = mbar_wait(bar, m & 1, wait_iters);
-      if (__syncthreads_or(!arrived)) return m;
-      const uint32_t* s = reinterpret_cast<const uint32_t*>(stage);
-#pragma unroll
-      for (int p = 0; p < 2 * ELL; p++) {
-        bv[0][p] = s[2 * (p * CHW + CH - 2 * tid)];
-        bv[1][p] = s[2 * (p * CHW + CH - 2 * tid - 1)];
-      }
-      if (m < 3) {
-        __syncthreads();
-        if (tid == 0) {
-          // the next chunk's copies (async proxy) follow these reads
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          stage_chunk(stage, brows, m + 1, bar);
-        }
-      }
-    } else {
-      const uint32_t* s = reinterpret_cast<const uint32_t*>(brows);
-      const int k0 = i0 ? N - i0 : 0, k1 = N - i0 - 1;
-#pragma unroll
-      for (int p = 0; p < 2 * ELL; p++) {
-        bv[0][p] = __ldg(s + 2 * (p * N + k0));
-        bv[1][p] = __ldg(s + 2 * (p * N + k1));
-      }
-    }
-    if (i0 == 0) {
-#pragma unroll
-      for (int p = 0; p < 2 * ELL; p++) bv[0][p] = P.r[p & 1].q - bv[0][p];
-    }
-#pragma unroll
-    for (int c = 0; c < MAX_GAMMA; c++) {
-      if (c >= gamma) continue;
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const uint64_t xv = P.delta * (uint64_t)((hw[c] >> (16 * e)) & 0xFFFFu);
-        const uint32_t d0 = (uint32_t)xv & 0xFFFFFu, d1 = (uint32_t)(xv >> 20) & 0xFFFFFu, d2 = (uint32_t)(xv >> 40);
-        acc[2 * c] += (uint64_t)d0 * bv[e][0] + (uint64_t)d1 * bv[e][2] + (uint64_t)d2 * bv[e][4];
-        acc[2 * c + 1] += (uint64_t)d0 * bv[e][1] + (uint64_t)d1 * bv[e][3] + (uint64_t)d2 * bv[e][5];
-      }
-    }
-  }
-  // lane l ends with the warp's sum of value l
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const bool up = (lane & o) != 0;
-#pragma unroll
-    for (int k = 0; k < o; k++) {
-      const uint64_t send = up ? acc[k] : acc[k + o], keep = up ? acc[k + o] : acc[k];
-      acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  if (QDB) __syncthreads();  // the last chunk has been read
-  red[warp * 32 + lane] = acc[0];
-  __syncthreads();
-  if (tid < 32) {
-    uint64_t s = 0;
-#pragma unroll
-    for (int w = 0; w < QT / 32; w++) s += red[w * 32 + tid];
-    const uint32_t q = P.r[tid & 1].q;
-    const uint32_t v = (uint32_t)(s % q);
-    bpoly[(tid & 1) * 16 + (tid >> 1)] = v ? q - v : 0;
-  }
-  __syncthreads();
-  return -1;
-}
-
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
 template <int MODE, bool SEEDED, bool QDB>
 __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) {

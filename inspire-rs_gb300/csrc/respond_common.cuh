@@ -92,6 +92,22 @@ __host__ __device__ constexpr int h_of(int l) { return ((l & 1) << 3) | ((l & 2)
 __host__ __device__ constexpr int quad_word(int l, int x) { return (l >> 2) * 512 + 4 * x + (l & 3); }
 __host__ __device__ constexpr int row_word(int h, int x) { return h * 128 + x; }
 
+// A key triple's transforms (any representatives below 6.5 q in absolute value,
+// signed), scaled by n^-1 2^32 and with the third gadget digit folded in
+// (fold_third_digit_kernel, setup.cu), canonical.
+__device__ __forceinline__ void fold_keys(uint32_t (&v)[ELL][16], const ResidueConsts& C) {
+  const uint32_t q = C.q;
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    uint32_t k[ELL];
+#pragma unroll
+    for (int e = 0; e < ELL; e++) k[e] = mul_shoup(v[e][j] + 8 * q, C.ninv_mont, C.ninv_mont_p, q);
+    v[0][j] = sub_mod(k[0], mul_shoup(k[2], C.d2_z2, C.d2_z2_p, q), q);
+    v[1][j] = sub_mod(k[1], mul_shoup(k[2], C.d2_z1, C.d2_z1_p, q), q);
+    v[2][j] = mul_shoup(k[2], C.d2_nz2, C.d2_nz2_p, q);
+  }
+}
+
 __device__ __forceinline__ uint32_t u4e(const uint4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
 
 }  // namespace ig
