@@ -130,21 +130,24 @@ int build_key_table(inspire_ctx* c, const uint64_t* y_body, const uint64_t* y_al
     return fail(INSPIRE_ERR_OUT_OF_MEMORY, alloc_failure(c, "client key table allocation"));
   const size_t in_polys = y_all ? (size_t)(gamma - 1) * ELL : ELL;
   if (gamma > 1) {
+    // through page-locked memory, once the previous build has read it: a
+    // query's own keys are read there in place, a registration's go through an
+    // upload buffer (one DMA)
     const size_t in_bytes = in_polys * poly_words() * sizeof(uint64_t);
-    if (c->d_keys.ensure(in_bytes) != cudaSuccess)
+    if (sync && c->d_keys.ensure(in_bytes) != cudaSuccess)
       return fail(INSPIRE_ERR_OUT_OF_MEMORY, alloc_failure(c, "client key upload buffer"));
-    // through page-locked memory (one DMA), once the previous upload is out of it
-    if (!c->keys_ev) CUDA_TRY(cudaEventCreateWithFlags(&c->keys_ev, cudaEventDisableTiming));
-    CUDA_TRY(cudaEventSynchronize(c->keys_ev));
+    if (c->keys_in_flight) CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->keys_in_flight = false;
     CUDA_TRY(c->h_keys.ensure(in_bytes));
     memcpy(c->h_keys.p, y_all ? y_all : y_body, in_bytes);
-    CUDA_TRY(cudaMemcpyAsync(c->d_keys.p, c->h_keys.p, in_bytes, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(cudaEventRecord(c->keys_ev, c->stream));
-    CUDA_TRY(launch_client_keys_ntt(c->P, c->d_keys.as<uint64_t>(), (int)in_polys, y_all != nullptr, m.as<uint32_t>(),
-                                    c->stream));
-    // the Respond kernel multiplies the third key by R_{i+1} instead of NTT(d2)
-    CUDA_TRY(launch_fold_third_digit(c->P, m.as<uint32_t>(), m.as<uint32_t>(), (int)in_polys / ELL, false, c->stream));
-    if (sync) CUDA_TRY(cudaStreamSynchronize(c->stream));
+    c->keys_in_flight = true;
+    if (sync) CUDA_TRY(cudaMemcpyAsync(c->d_keys.p, c->h_keys.p, in_bytes, cudaMemcpyHostToDevice, c->stream));
+    CUDA_TRY(launch_client_keys(c->P, sync ? c->d_keys.as<uint64_t>() : c->h_keys.dev<uint64_t>(),
+                                (int)in_polys / ELL, y_all != nullptr, m.as<uint32_t>(), c->stream));
+    if (sync) {
+      CUDA_TRY(cudaStreamSynchronize(c->stream));
+      c->keys_in_flight = false;
+    }
   }
   return INSPIRE_OK;
 }
@@ -215,17 +218,18 @@ int finish_status(inspire_ctx* c, uint32_t n, const char* what);
 // Batches up to this size stage their inputs through page-locked memory.
 constexpr uint32_t STAGE_PINNED_MAX = 64;
 
-// Seeded queries whose rows and responses are in page-locked host memory
-// (device addresses d_rows, row_bytes apart, and d_out): the serving variant
-// of the kernel reads each query's rows in place and writes its response
-// straight to that memory, so nothing is staged or copied back.
+// Queries whose rows and responses are in page-locked host memory (device
+// addresses d_rows, row_bytes apart, and d_out; without seeds also d_arows,
+// [n][ELL][2][N]): the serving variant of the kernel reads each query's rows in
+// place and writes its response straight to that memory, so nothing is staged or
+// copied back.  new_keys: the launch before on this stream builds the key
+// table, which the kernel needs late.
 int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* shard_ids, const uint8_t* seeds,
-                     size_t seed_stride, const uint8_t* d_rows, size_t row_bytes, uint64_t* d_out,
-                     const int32_t* client_ids) {
+                     size_t seed_stride, const uint64_t* d_arows, const uint8_t* d_rows, size_t row_bytes,
+                     uint64_t* d_out, const int32_t* client_ids, bool new_keys) {
   const size_t pw = poly_words();
-  // descriptors and status words in page-locked memory: the descriptors go
-  // over by DMA, the kernel writes each status word in place
-  CUDA_TRY(c->d_desc.ensure(sizeof(QueryDesc) * n));
+  // descriptors and status words in page-locked memory, read and written in
+  // place
   CUDA_TRY(c->h_desc.ensure(sizeof(QueryDesc) * n));
   CUDA_TRY(c->h_qstatus.ensure(sizeof(int32_t) * n));
   QueryDesc* hd = c->h_desc.host<QueryDesc>();
@@ -233,7 +237,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   const DbView view{db->E.as<uint32_t>(), db->H.as<uint16_t>(), db->nshards, 0};
   for (uint32_t i = 0; i < n; i++) {
     QueryDesc& d = hd[i];
-    memcpy(d.seeds, seeds + i * seed_stride, sizeof(d.seeds));
+    if (seeds) memcpy(d.seeds, seeds + i * seed_stride, sizeof(d.seeds));
     d.brows = reinterpret_cast<const uint64_t*>(d_rows + i * row_bytes);
     d.out = d_out + (size_t)i * 2 * pw;
     d.status = c->h_qstatus.dev<int32_t>() + i;
@@ -242,7 +246,6 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
     d.client = client_ids[i];
     hs[i] = -1;
   }
-  CUDA_TRY(cudaMemcpyAsync(c->d_desc.p, hd, sizeof(QueryDesc) * n, cudaMemcpyHostToDevice, c->stream));
   if (int rc = sync_client_table(c)) return rc;
   RespondArgs a{};
   a.P = c->P;
@@ -250,10 +253,13 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.yhat_table = c->client_table.as<const uint32_t*>();
   a.nclients = (int)c->client_ptrs.size();
   a.what = c->what3.as<uint32_t>();
-  a.qdesc = c->d_desc.as<QueryDesc>();
+  a.qdesc = c->h_desc.dev<QueryDesc>();
+  a.arows = d_arows;
   a.stage_wait_iters = STAGE_WAIT_ITERS_DEFAULT;
-  CUDA_TRY(launch_respond(a, true, c->stream, 0, c->pair_max.load()));
+  a.after_keys = new_keys;
+  CUDA_TRY(launch_respond(a, seeds != nullptr, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
+  c->keys_in_flight = false;
   for (uint32_t i = 0; i < n; i++)
     if (hs[i] != 0)
       return fail(INSPIRE_ERR_DEVICE_STATUS,
@@ -261,8 +267,35 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   return INSPIRE_OK;
 }
 
+// At most STAGE_PINNED_MAX queries in any memory: the rows gathered into
+// page-locked memory, the responses written to page-locked memory and copied
+// out once.  Query i's a row t (without seeds) is at a_rows + i stride_polys +
+// t row_polys polys, likewise its b row.
+int run_batch_gathered(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* shard_ids,
+                       const uint8_t* seeds, size_t seed_stride, const uint64_t* a_rows, const uint64_t* b_rows,
+                       size_t stride_polys, size_t row_polys, const int32_t* client_ids, uint64_t* out_ct,
+                       bool new_keys) {
+  const size_t pw = poly_words(), poly_b = sizeof(uint64_t) * pw, rows_b = poly_b * ELL;
+  const size_t out_span = sizeof(uint64_t) * n * 2 * pw;
+  CUDA_TRY(c->h_stage.ensure(rows_b * n * (seeds ? 1 : 2)));
+  CUDA_TRY(c->h_out.ensure(out_span));
+  auto gather = [&](uint8_t* to, const uint64_t* rows) {
+    for (uint32_t i = 0; i < n; i++)
+      for (int t = 0; t < ELL; t++)
+        memcpy(to + rows_b * i + poly_b * t, rows + (i * stride_polys + t * row_polys) * pw, poly_b);
+  };
+  gather(c->h_stage.host<uint8_t>(), b_rows);
+  if (!seeds) gather(c->h_stage.host<uint8_t>() + rows_b * n, a_rows);
+  const uint8_t* d = c->h_stage.dev<uint8_t>();
+  if (int rc = run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride,
+                                seeds ? nullptr : reinterpret_cast<const uint64_t*>(d + rows_b * n), d, rows_b,
+                                c->h_out.dev<uint64_t>(), client_ids, new_keys))
+    return rc;
+  memcpy(out_ct, c->h_out.host<uint64_t>(), out_span);
+  return INSPIRE_OK;
+}
+
 // Stage n queries (rows ELL..2ELL-1 only) and run the Respond kernel.
-// seeds/b_rows/a_rows use the full 2*ELL-row host layout.
 // a_rows/b_rows point at the first needed poly of query 0 (ELL contiguous
 // polys per query, query pitch `stride_polys`); seeds at the first needed seed
 // (ELL contiguous seeds, query pitch `seed_stride` bytes).
@@ -281,24 +314,12 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
                                 : nullptr;
     const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
     if (d_rows && d_outp)
-      return run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride, d_rows, row_bytes,
-                              const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_outp)), client_ids);
-    if (n <= STAGE_PINNED_MAX) {
-      // small batches in other memory: the rows gathered into page-locked
-      // memory and read there in place, the responses written to page-locked
-      // memory and copied out once (no copies to and from the device)
-      const size_t rows_b = sizeof(uint64_t) * ELL * pw;
-      CUDA_TRY(c->h_stage.ensure(rows_b * n));
-      CUDA_TRY(c->h_out.ensure(out_span));
-      uint8_t* hb = c->h_stage.host<uint8_t>();
-      for (uint32_t i = 0; i < n; i++) memcpy(hb + rows_b * i, b_rows + i * stride_polys * pw, rows_b);
-      if (int rc = run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride, c->h_stage.dev<uint8_t>(), rows_b,
-                                    c->h_out.dev<uint64_t>(), client_ids))
-        return rc;
-      memcpy(out_ct, c->h_out.host<uint64_t>(), out_span);
-      return INSPIRE_OK;
-    }
+      return run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride, nullptr, d_rows, row_bytes,
+                              const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_outp)), client_ids, false);
   }
+  if (n <= STAGE_PINNED_MAX)
+    return run_batch_gathered(c, db, n, shard_ids, seeds, seed_stride, a_rows, b_rows, stride_polys, 1, client_ids,
+                              out_ct, false);
   CUDA_TRY(c->d_shard.ensure(sizeof(uint32_t) * n));
   CUDA_TRY(c->d_client.ensure(sizeof(int32_t) * n));
   CUDA_TRY(c->d_brows.ensure(sizeof(uint64_t) * n * ELL * pw));
@@ -308,40 +329,17 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   if (seeded) CUDA_TRY(c->d_seeds.ensure((size_t)32 * ELL * n));
   else CUDA_TRY(c->d_arows.ensure(rows_b * n));
   CUDA_TRY(c->h_qstatus.ensure(sizeof(int32_t) * n));
-  if (n <= STAGE_PINNED_MAX) {
-    // small batches: the inputs are gathered into page-locked memory on the
-    // host and go over by DMA without the driver's staging of pageable
-    // copies; the kernel writes the status words in place
-    const size_t a_b = seeded ? (size_t)32 * ELL * n : rows_b * n;
-    CUDA_TRY(c->h_stage.ensure(rows_b * n + a_b + sizeof(uint32_t) * 2 * n));
-    uint8_t* hb = c->h_stage.host<uint8_t>();
-    uint8_t* ha = hb + rows_b * n;
-    uint32_t* hsid = reinterpret_cast<uint32_t*>(ha + a_b);
-    int32_t* hcid = reinterpret_cast<int32_t*>(hsid + n);
-    for (uint32_t i = 0; i < n; i++) {
-      memcpy(hb + rows_b * i, b_rows + i * stride_polys * pw, rows_b);
-      if (seeded) memcpy(ha + (size_t)32 * ELL * i, seeds + i * seed_stride, (size_t)32 * ELL);
-      else memcpy(ha + rows_b * i, a_rows + i * stride_polys * pw, rows_b);
-      hsid[i] = shard_ids[i];
-      hcid[i] = client_ids[i];
-    }
-    CUDA_TRY(cudaMemcpyAsync(c->d_brows.p, hb, rows_b * n, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(seeded ? c->d_seeds.p : c->d_arows.p, ha, a_b, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(c->d_shard.p, hsid, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(c->d_client.p, hcid, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream));
-  } else {
-    CUDA_TRY(cudaMemcpyAsync(c->d_shard.p, shard_ids, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, c->stream));
-    CUDA_TRY(cudaMemcpyAsync(c->d_client.p, client_ids, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream));
-    // b rows ELL..2ELL-1 of each query: one strided copy
-    CUDA_TRY(cudaMemcpy2DAsync(c->d_brows.p, rows_b, b_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
+  CUDA_TRY(cudaMemcpyAsync(c->d_shard.p, shard_ids, sizeof(uint32_t) * n, cudaMemcpyHostToDevice, c->stream));
+  CUDA_TRY(cudaMemcpyAsync(c->d_client.p, client_ids, sizeof(int32_t) * n, cudaMemcpyHostToDevice, c->stream));
+  // b rows ELL..2ELL-1 of each query: one strided copy
+  CUDA_TRY(cudaMemcpy2DAsync(c->d_brows.p, rows_b, b_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
+                             cudaMemcpyHostToDevice, c->stream));
+  if (seeded)
+    CUDA_TRY(cudaMemcpy2DAsync(c->d_seeds.p, (size_t)32 * ELL, seeds, seed_stride, (size_t)32 * ELL, n,
                                cudaMemcpyHostToDevice, c->stream));
-    if (seeded)
-      CUDA_TRY(cudaMemcpy2DAsync(c->d_seeds.p, (size_t)32 * ELL, seeds, seed_stride, (size_t)32 * ELL, n,
-                                 cudaMemcpyHostToDevice, c->stream));
-    else
-      CUDA_TRY(cudaMemcpy2DAsync(c->d_arows.p, rows_b, a_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
-                                 cudaMemcpyHostToDevice, c->stream));
-  }
+  else
+    CUDA_TRY(cudaMemcpy2DAsync(c->d_arows.p, rows_b, a_rows, sizeof(uint64_t) * stride_polys * pw, rows_b, n,
+                               cudaMemcpyHostToDevice, c->stream));
   int rc = sync_client_table(c);
   if (rc) return rc;
   RespondArgs a{};
@@ -607,20 +605,12 @@ int single_query(inspire_ctx* c, const inspire_db* db, uint32_t shard_id, const 
   int32_t id = -1;
   int rc = inline_keys(c, y_body, y_all, &id);
   if (rc) return rc;
-  if (seeds) {
-    rc = run_batch(c, db, 1, &shard_id, seeds + 32 * ELL, (size_t)64 * ELL, nullptr, b_rows + (size_t)ELL * poly_words(),
-                   2 * ELL, &id, out_ct);
-  } else {
-    // rgsw_full holds 2*ELL rows of (a, b): row r's a is poly 2r, its b poly 2r+1
-    const size_t pw = poly_words();
-    std::vector<uint64_t> ar((size_t)ELL * pw), br((size_t)ELL * pw);
-    for (int t = 0; t < ELL; t++) {
-      memcpy(ar.data() + t * pw, rgsw_full + (size_t)(2 * (ELL + t)) * pw, pw * sizeof(uint64_t));
-      memcpy(br.data() + t * pw, rgsw_full + (size_t)(2 * (ELL + t) + 1) * pw, pw * sizeof(uint64_t));
-    }
-    rc = run_batch(c, db, 1, &shard_id, nullptr, 0, ar.data(), br.data(), ELL, &id, out_ct);
-  }
-  return rc;
+  const size_t pw = poly_words();
+  if (!seeds)  // 2*ELL rows of (a, b): row r's a is poly 2r, its b poly 2r+1
+    return run_batch_gathered(c, db, 1, &shard_id, nullptr, 0, rgsw_full + 2 * ELL * pw, rgsw_full + (2 * ELL + 1) * pw,
+                              4 * ELL, 2, &id, out_ct, c->gamma > 1);
+  return run_batch_gathered(c, db, 1, &shard_id, seeds + 32 * ELL, (size_t)64 * ELL, nullptr,
+                            b_rows + (size_t)ELL * pw, 2 * ELL, 1, &id, out_ct, c->gamma > 1);
 }
 
 }  // namespace
@@ -845,7 +835,7 @@ int inspire_crs_load(inspire_ctx* c, const uint8_t w_seed[32], uint32_t num_colu
   CUDA_TRY(c->what.ensure(sizeof(uint32_t) * (size_t)std::max(1, (gamma - 1) * ELL) * 2 * N));
   CUDA_TRY(launch_crs_what(c->P, c->wmask.as<uint32_t>(), c->what.as<uint32_t>(), c->stream));
   CUDA_TRY(c->what3.ensure(c->what.bytes));
-  CUDA_TRY(launch_fold_third_digit(c->P, c->what.as<uint32_t>(), c->what3.as<uint32_t>(), gamma - 1, true, c->stream));
+  CUDA_TRY(launch_fold_third_digit(c->P, c->what.as<uint32_t>(), c->what3.as<uint32_t>(), gamma - 1, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   // key tables of registered clients were built for the previous gamma
   for (size_t i = 0; i < c->clients.size(); i++) release_keys(c, (int32_t)i);
@@ -1167,8 +1157,11 @@ int inspire_respond_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, cons
     if (id < 0 || (size_t)id >= c->clients.size() || !c->clients[id])
       return fail(INSPIRE_ERR_KEYS_MISSING, "InspiRING client packing keys missing from query");
   }
-  // rows ELL..2ELL-1 of each query, split into their a and b polys
   const size_t pw = poly_words();
+  if (n && n <= STAGE_PINNED_MAX)
+    return run_batch_gathered(c, db, n, shard_ids, nullptr, 0, rgsw + 2 * ELL * pw, rgsw + (2 * ELL + 1) * pw, 4 * ELL,
+                              2, client_ids, out_ct, false);
+  // rows ELL..2ELL-1 of each query, split into their a and b polys
   std::vector<uint64_t> ar((size_t)n * ELL * pw), br((size_t)n * ELL * pw);
   for (uint32_t i = 0; i < n; i++)
     for (int t = 0; t < ELL; t++) {

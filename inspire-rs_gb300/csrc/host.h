@@ -154,23 +154,22 @@ struct inspire_ctx {
   int32_t inline_id = -1;
   // staging for host-buffer calls
   cudaStream_t stream = nullptr;
-  ighost::DevMem d_shard, d_seeds, d_arows, d_brows, d_client, d_out, d_cols, d_status, d_keys, d_desc;
+  ighost::DevMem d_shard, d_seeds, d_arows, d_brows, d_client, d_out, d_cols, d_status, d_keys;
   std::vector<int32_t> h_status;
   ighost::HostPinned h_desc;    // descriptors of page-locked batch calls
   ighost::HostPinned h_qstatus; // status words of the batch calls, written by the kernel
   ighost::HostPinned h_stage;   // small batches' inputs, gathered for one DMA each
-  ighost::HostPinned h_keys;    // client keys on their way to d_keys
+  ighost::HostPinned h_keys;    // client keys on their way to their table
   ighost::HostPinned h_out;     // responses of staged small batches, written by the kernel
-  cudaEvent_t keys_ev = nullptr;  // recorded after the copy out of h_keys
+  bool keys_in_flight = false;  // a launch on `stream` may still read h_keys
 
   inspire_ctx() {
     for (ighost::DevMem* m : {&tables, &what, &what3, &wmask, &galois, &tree_work, &d_tree_out, &client_table, &d_shard,
-                              &d_seeds, &d_arows, &d_brows, &d_client, &d_out, &d_cols, &d_status, &d_keys, &d_desc})
+                              &d_seeds, &d_arows, &d_brows, &d_client, &d_out, &d_cols, &d_status, &d_keys})
       m->ledger = ledger;
   }
   ~inspire_ctx() {
     for (ighost::DevMem* m : clients) delete m;
-    if (keys_ev) cudaEventDestroy(keys_ev);
     if (stream) cudaStreamDestroy(stream);
   }
 };

@@ -27,10 +27,10 @@ struct DbView {
   int pad;
 };
 
-// One admitted query of the serving loop.  The descriptor itself -- with the
-// query's seeds inline -- is copied to device memory per batch; the rows and
-// the response live in pinned host memory that the Respond kernel reads and
-// writes directly.
+// One query whose rows and response live in pinned host memory that the Respond
+// kernel reads and writes directly.  The descriptor itself -- with the query's
+// seeds inline -- is in pinned host memory too, or (serving loop) copied to
+// device memory per batch.
 struct QueryDesc {
   uint8_t seeds[ELL * 32];  // seeds of rows ELL..2ELL-1
   const uint64_t* brows;  // [ELL][2][N] b-polys of rows ELL..2ELL-1 (16-byte aligned)
@@ -59,13 +59,16 @@ struct RespondArgs {
   const uint32_t* what;          // [(gamma-1)][ELL][2][N] rotated w_mask (CRS), quads, third digit folded in
   uint64_t* out;                 // [nq][2][2][N] response (a_hat, b) residues
   int* status;                   // [nq]
-  // Serving loop: per-query descriptors in device memory (override shard,
+  // Per-query descriptors (override shard,
   // client, seeds, brows, E/H/nshards, out and status; rows are read from and
   // responses written to the pinned host memory they point at), or null.
   const struct QueryDesc* qdesc;
   // Serving loop: bound of the wait for a query's staged rows, in wait
   // iterations (0: give up at once)
   uint32_t stage_wait_iters;
+  // Host only: the stream's last launch builds a key table of this launch; the
+  // two-CTA kernel may be set up meanwhile
+  bool after_keys;
 };
 
 // NoPacking respond (respond.rs:71-115): per query the combined ciphertext
@@ -204,13 +207,12 @@ cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t*
 // (k0 - z^-2 k2, k1 - z^-1 k2, n z^-2 k2): the Respond kernel then multiplies
 // the third key by R_{i+1} instead of by NTT(d2).  In place, or (quads) from
 // slot order into the order that the Respond kernels read the CRS keys in.
-cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, bool quads,
-                                    cudaStream_t st);
+cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, cudaStream_t st);
 // NTT of a client's key polys [npolys][2][N] (y_body: ELL polys, whose
 // rotations the Respond kernels form; or, rotated, an explicit y_all, its
 // rows turned so that the kernels read either the same way).
-cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, bool rotated, uint32_t* yhat,
-                                   cudaStream_t st);
+cudaError_t launch_client_keys(const DevParams& P, const uint64_t* keys, int ntriples, bool rotated, uint32_t* yhat,
+                               cudaStream_t st);
 
 // kernel-level operations
 // decrypt + extract_inspiring of n responses ct[n][2][2][N] (u64) with the

@@ -144,7 +144,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     expand_rows<NR>(P, seeds, AH, ws);
   } else {
     const uint64_t* ar = A.arows + (size_t)qi * ELL * 2 * N;
-#pragma unroll 4
+#pragma unroll 16
     for (int j = tid; j < ELL * NR * N; j += QT) {
       const int t = j / (NR * N);
       AH[j] = (uint32_t)__ldg(ar + (size_t)t * 2 * N + (j - t * NR * N));

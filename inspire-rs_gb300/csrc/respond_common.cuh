@@ -92,6 +92,12 @@ __host__ __device__ constexpr int h_of(int l) { return ((l & 1) << 3) | ((l & 2)
 __host__ __device__ constexpr int quad_word(int l, int x) { return (l >> 2) * 512 + 4 * x + (l & 3); }
 __host__ __device__ constexpr int row_word(int h, int x) { return h * 128 + x; }
 
+// Programmatic dependent launch: a launch that allows it may be set up while the
+// one before it runs; it waits for that one's end (no wait otherwise) where it
+// first needs its results.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // A key triple's transforms (any representatives below 6.5 q in absolute value,
 // signed), scaled by n^-1 2^32 and with the third gadget digit folded in
 // (fold_third_digit_kernel, setup.cu), canonical.

@@ -198,6 +198,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
   // both CTAs read the same fields: every return here is uniform over the cluster
   if (shard >= (uint32_t)nshards || cid < 0 || cid >= A.nclients || A.yhat_table[cid] == nullptr) {
     if (r == 0 && tid == 0) *status_ptr() = ERR_INDEX;
+    pdl_wait();
     return;
   }
 
@@ -333,10 +334,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
     if (MODE != MODE_CRT_FIXED) cluster_wait();
   } else {
     const uint64_t* ar = A.arows + (size_t)qi * ELL * 2 * N + (size_t)sres * N;
-#pragma unroll 4
+#pragma unroll
     for (int j = tid; j < ELL * N; j += PT) AH[j] = (uint32_t)__ldg(ar + (size_t)(j >> LOGN) * 2 * N + (j & (N - 1)));
     cluster_wait();
   }
+
+  // the client's keys, read from the recursion on, may be the last launch's work
+  pdl_wait();
 
   // ---- the b side ----
   int missing = 0;
@@ -569,16 +573,21 @@ static cudaError_t set_pair_smem_attr() {
 
 template <int MODE>
 static cudaError_t launch_pair_mode(const RespondArgs& a, bool seeded, cudaStream_t st) {
-  const size_t smem = sizeof(uint32_t) * PairSmem::TOTAL;
-  const int ctas = 2 * a.nq;
-  if (a.qdesc) {
-    if (seeded) respond_pair_kernel<MODE, true, true><<<ctas, PT, smem, st>>>(a);
-    else respond_pair_kernel<MODE, false, true><<<ctas, PT, smem, st>>>(a);
-  } else {
-    if (seeded) respond_pair_kernel<MODE, true, false><<<ctas, PT, smem, st>>>(a);
-    else respond_pair_kernel<MODE, false, false><<<ctas, PT, smem, st>>>(a);
-  }
-  return cudaGetLastError();
+  void (*kernel)(RespondArgs) = a.qdesc ? (seeded ? respond_pair_kernel<MODE, true, true>
+                                                  : respond_pair_kernel<MODE, false, true>)
+                                        : (seeded ? respond_pair_kernel<MODE, true, false>
+                                                  : respond_pair_kernel<MODE, false, false>);
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(2 * a.nq);
+  cfg.blockDim = dim3(PT);
+  cfg.dynamicSmemBytes = sizeof(uint32_t) * PairSmem::TOTAL;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = a.after_keys ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
 }  // namespace

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "kernels.h"
+#include "ntt_joint.cuh"
 #include "respond_common.cuh"
 
 namespace ig {
@@ -128,27 +129,6 @@ __global__ void __launch_bounds__(BLOCK) crs_what_kernel(const DevParams P, cons
   }
 }
 
-// Client key table from y_body: the forward NTT of packing_online
-// (inspiring2.rs:1199-1213) of y_body[k], in rows [h][x] and times n^-1 2^32.
-// generate_rotations (:1309-1323) is a rotation of the rows (rot_rows), which
-// the Respond kernels apply as they read.  An explicit y_all ((gamma-1)*ELL
-// coefficient polys, step i = p / ELL; `rotated`) is stored with slot h in row
-// h + rot, where they look for it.
-__global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams P, const uint64_t* __restrict__ ya,
-                                                                bool rotated, uint32_t* __restrict__ yhat) {
-  __shared__ uint32_t SC[2][NTT_SCRATCH];
-  const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
-  const ResidueConsts& C = P.r[g];
-  uint32_t v[16];
-#pragma unroll
-  for (int rr = 0; rr < 16; rr++) v[rr] = (uint32_t)ya[((size_t)p * 2 + g) * N + x + 128 * rr];
-  ntt_fwd(v, SC[g], fwd_tw(C), C.q, x, 1 + g);
-  const uint32_t rot = rotated ? rot_rows(P.gamma, p / ELL, x) : 0;
-#pragma unroll
-  for (int rr = 0; rr < 16; rr++)
-    yhat[((size_t)p * 2 + g) * N + row_word((h_of(rr) + rot) & 15, x)] = mul_shoup(v[rr], C.ninv_mont, C.ninv_mont_p, C.q);
-}
-
 // Key tables with the third gadget digit folded in.  In the NTT domain of
 // residue r, the digits of the composite coefficient c = INTT(R) satisfy
 // NTT(d0) + z NTT(d1) + z^2 NTT(d2) = R (mod q_r), so for any key triple
@@ -156,10 +136,10 @@ __global__ void __launch_bounds__(BLOCK) client_keys_ntt_kernel(const DevParams 
 //   = (k0 - z^-2 k2) NTT(d0) + (k1 - z^-1 k2) NTT(d1) + (z^-2 k2) R.
 // With R kept as n^-1 R (the Respond kernel's R_{i+1}), the third key is
 // n z^-2 k2.  src and dst hold ngroups triples [g][k<3][2][N] (any constant
-// scaling, applied alike to the three keys).  In place, or with `quads` from
-// slot order into quads [l >> 2][x][l & 3].
+// scaling, applied alike to the three keys), src in slot order, dst in quads
+// [l >> 2][x][l & 3].
 __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams P, const uint32_t* src, uint32_t* dst,
-                                                                 int ngroups, bool quads) {
+                                                                 int ngroups) {
   const size_t per = (size_t)2 * N;
   const size_t total = (size_t)ngroups * per;
   for (size_t idx = (size_t)blockIdx.x * BLOCK + threadIdx.x; idx < total; idx += (size_t)gridDim.x * BLOCK) {
@@ -168,7 +148,7 @@ __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams
     const ResidueConsts& C = P.r[r];
     const int w = (int)(rs & (N - 1));
     const int x = (w >> 2) & 127, l = ((w >> 9) << 2) | (w & 3);
-    const uint32_t* f = src + g * 3 * per + (quads ? (size_t)r * N + 16 * x + l : rs);
+    const uint32_t* f = src + g * 3 * per + (size_t)r * N + 16 * x + l;
     uint32_t* t = dst + g * 3 * per + rs;
     const uint32_t k0 = f[0], k1 = f[per], k2 = f[2 * per];
     t[0] = sub_mod(k0, mul_shoup(k2, C.d2_z2, C.d2_z2_p, C.q), C.q);
@@ -177,14 +157,48 @@ __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams
   }
 }
 
+// Client key table from y_body: the forward NTT of packing_online
+// (inspiring2.rs:1199-1213) of the three y_body[k], times n^-1 2^32, the third
+// digit folded in as above, in rows [h][x].  generate_rotations (:1309-1323) is a
+// rotation of the rows (rot_rows), which the Respond kernels apply as they read.
+// An explicit y_all ((gamma-1) triples of coefficient polys; `rotated`) is
+// stored with slot h in row h + rot, where they look for it.  One CTA per triple
+// and residue, keys in device or page-locked host memory.  A single query's
+// Respond kernel, which needs the table only after the rows' expansion, starts
+// meanwhile.  Measured (one query with its keys, host call): 146 us -> 131 with
+// seeds and 155 -> 125 without, against an upload, a transform of single polys, a
+// fold in place and copies of the rows.
+__global__ void __launch_bounds__(NTT_GT) client_keys_kernel(const DevParams P, const uint64_t* __restrict__ keys,
+                                                             bool rotated, uint32_t* __restrict__ yhat) {
+  __shared__ __align__(128) uint32_t X[ELL][N];
+  pdl_trigger();
+  const int g = blockIdx.x, r = blockIdx.y, x = threadIdx.x;
+  const ResidueConsts& C = P.r[r];
+  const uint64_t* src = keys + ((size_t)g * ELL * 2 + r) * N + x;
+  uint32_t v[ELL][16];
+#pragma unroll
+  for (int k = 0; k < ELL; k++)
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[k][j] = (uint32_t)__ldg(src + (size_t)k * 2 * N + 128 * j);
+  const uint32_t sc[ELL] = {jx_addr(X[0]), jx_addr(X[1]), jx_addr(X[2])};
+  jntt_fwd<ELL, JB_CANON>(v, sc, sfwd_tw(C), C.q, x, 1);
+  fold_keys(v, C);
+  const uint32_t rot = rotated ? rot_rows(P.gamma, g, x) : 0;
+  uint32_t* o = yhat + ((size_t)g * ELL * 2 + r) * N;
+#pragma unroll
+  for (int k = 0; k < ELL; k++)
+#pragma unroll
+    for (int j = 0; j < 16; j++) o[(size_t)k * 2 * N + row_word((h_of(j) + rot) & 15, x)] = v[k][j];
+}
+
 }  // namespace
 
-cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups, bool quads,
+cudaError_t launch_fold_third_digit(const DevParams& P, const uint32_t* src, uint32_t* dst, int ngroups,
                                     cudaStream_t st) {
   if (ngroups <= 0) return cudaSuccess;
   const size_t total = (size_t)ngroups * 2 * N;
   const unsigned blocks = (unsigned)std::min<size_t>((total + BLOCK - 1) / BLOCK, 4096);
-  fold_third_digit_kernel<<<blocks, BLOCK, 0, st>>>(P, src, dst, ngroups, quads);
+  fold_third_digit_kernel<<<blocks, BLOCK, 0, st>>>(P, src, dst, ngroups);
   return cudaGetLastError();
 }
 
@@ -215,10 +229,10 @@ cudaError_t launch_crs_what(const DevParams& P, const uint32_t* wmask, uint32_t*
   return cudaGetLastError();
 }
 
-cudaError_t launch_client_keys_ntt(const DevParams& P, const uint64_t* polys, int npolys, bool rotated, uint32_t* yhat,
-                                   cudaStream_t st) {
-  if (npolys <= 0) return cudaSuccess;
-  client_keys_ntt_kernel<<<npolys, BLOCK, 0, st>>>(P, polys, rotated, yhat);
+cudaError_t launch_client_keys(const DevParams& P, const uint64_t* keys, int ntriples, bool rotated, uint32_t* yhat,
+                               cudaStream_t st) {
+  if (ntriples <= 0) return cudaSuccess;
+  client_keys_kernel<<<dim3(ntriples, 2), NTT_GT, 0, st>>>(P, keys, rotated, yhat);
   return cudaGetLastError();
 }
 

@@ -51,14 +51,6 @@
 namespace ig {
 namespace {
 
-// Programmatic dependent launch: the next launch may be set up while this one
-// runs; it waits for this one's end where it first needs its results.  Only the
-// front starts its successor early (the leaves' database words then arrive
-// meanwhile): tree_kernel's CTAs, started among the leaves', came to lie two on
-// an SM while others stayed empty, 179 us instead of 131 for 9 queries.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 constexpr int CT_WORDS = 4 * N;  // one ciphertext: alpha (2 residues), beta (2 residues), rows [h][x]
 
 // Work area of one query: the node (l, s) of levels 7..10 in buffer
@@ -77,6 +69,10 @@ constexpr size_t WORK_WORDS = WORK_GOOD + 16;
 
 // ---- the query's rows: expanded and transformed (rows [h][x] in the work
 //      area), one CTA per row, and the b side in a fourth ----
+// Only this launch lets its successor start early (the leaves' database words
+// then arrive meanwhile): tree_kernel's CTAs, started among the leaves', came to
+// lie two on an SM while others stayed empty, 179 us instead of 131 for 9
+// queries.
 template <bool SEEDED>
 __global__ void __launch_bounds__(QT, 2) tree_front_kernel(const __grid_constant__ TreeArgs A) {
   __shared__ __align__(128) uint32_t AH[2 * N];  // the row, coefficients
