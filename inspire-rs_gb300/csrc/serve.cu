@@ -61,7 +61,90 @@ struct Rec {
   int64_t t_arrival = 0, t_done = 0;
   int64_t t_enqueue = 0;  // when the query became pending
   int cuda_error = 0;  // nonzero: the batch failed on the host side
+  int kstatus = 0;     // the kernel's status word
   bool batch_lost = false;  // a CTA of the query's batch exited with copies in flight
+};
+
+// Threads that share the copies of finished responses out of the pool with the
+// caller that collects them.  One core copies about 15 GB/s of what the GPU has
+// just written; a burst's responses (64 KiB each) leave the GPU at 100.  With 8
+// helpers a burst of 601 queries, collected by 4 threads, takes 840 us
+// against 1420 with the callers' own copies.
+class CopyHelpers {
+ public:
+  // Below this many copies the caller is done before a helper has woken.
+  static constexpr size_t MIN_COPIES = 8;
+  struct Copy {
+    void* to;
+    const void* from;
+  };
+
+  void start(unsigned n) {
+    for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
+  }
+  ~CopyHelpers() {
+    {
+      std::lock_guard<std::mutex> lk(mu_);
+      stop_ = true;
+    }
+    cv_.notify_all();
+    for (std::thread& t : threads_) t.join();
+  }
+  // Every copy of `bytes` bytes, finished on return.
+  void run(std::vector<Copy> copies, size_t bytes) {
+    auto job = std::make_shared<Job>();
+    job->copies = std::move(copies);
+    job->bytes = bytes;
+    const bool share = !threads_.empty() && job->copies.size() >= MIN_COPIES;
+    if (share) {
+      {
+        std::lock_guard<std::mutex> lk(mu_);
+        jobs_.push_back(job);
+      }
+      cv_.notify_all();
+    }
+    job->take();
+    if (share) {
+      retire(job);
+      while (job->done.load(std::memory_order_acquire) < job->copies.size()) std::this_thread::yield();
+    }
+  }
+
+ private:
+  struct Job {
+    std::vector<Copy> copies;
+    size_t bytes = 0;
+    std::atomic<size_t> next{0}, done{0};
+    void take() {
+      for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < copies.size();) {
+        memcpy(copies[i].to, copies[i].from, bytes);
+        done.fetch_add(1, std::memory_order_release);
+      }
+    }
+  };
+  void retire(const std::shared_ptr<Job>& job) {  // every copy has been taken
+    std::lock_guard<std::mutex> lk(mu_);
+    const auto it = std::find(jobs_.begin(), jobs_.end(), job);
+    if (it != jobs_.end()) jobs_.erase(it);
+  }
+  void work() {
+    for (;;) {
+      std::shared_ptr<Job> job;
+      {
+        std::unique_lock<std::mutex> lk(mu_);
+        cv_.wait(lk, [&] { return stop_ || !jobs_.empty(); });
+        if (jobs_.empty()) return;
+        job = jobs_.front();
+      }
+      job->take();
+      retire(job);
+    }
+  }
+  std::mutex mu_;
+  std::condition_variable cv_;
+  std::deque<std::shared_ptr<Job>> jobs_;
+  std::vector<std::thread> threads_;
+  bool stop_ = false;
 };
 
 struct Slot {
@@ -91,6 +174,7 @@ struct inspire_server {
   uint64_t n_submitted = 0, n_completed = 0, n_batches = 0;
   int sm_count = 0;
   std::string worker_error;
+  CopyHelpers helpers;
 
   uint8_t* rec_ptr(int i) const { return pool + (size_t)i * REC_BYTES; }
   uint8_t* dev_rec_ptr(int i) const { return dpool + (size_t)i * REC_BYTES; }
@@ -137,6 +221,7 @@ void inspire_server::run() {
   cudaSetDevice(ctx->device);
   std::vector<Slot*> finished, to_launch;
   std::vector<cudaError_t> fin_err;
+  std::vector<std::vector<int>> status;  // of the finished batches' queries
   for (;;) {
     finished.clear();
     fin_err.clear();
@@ -146,6 +231,12 @@ void inspire_server::run() {
       if (e == cudaErrorNotReady) continue;
       finished.push_back(sp.get());
       fin_err.push_back(e);
+      // the status words, cold in this core's cache, before `mu` is taken
+      status.resize(std::max(status.size(), finished.size()));
+      std::vector<int>& st = status[finished.size() - 1];
+      st.clear();
+      for (int i : sp->recs)
+        st.push_back(e == cudaSuccess ? *reinterpret_cast<const volatile int32_t*>(rec_ptr(i) + REC_STATUS) : 0);
     }
     to_launch.clear();
     {
@@ -157,14 +248,14 @@ void inspire_server::run() {
         // one query whose staged rows were still in flight when its CTA
         // exited makes every result of the launch unreliable
         bool lost = false;
-        if (e == cudaSuccess)
-          for (int i : s.recs)
-            lost |= *reinterpret_cast<const volatile int32_t*>(rec_ptr(i) + REC_STATUS) == ERR_STAGE_LOST;
-        for (int i : s.recs) recs[i].batch_lost = lost;
-        for (int i : s.recs) {
-          recs[i].state = DONE;
-          recs[i].t_done = t;
-          recs[i].cuda_error = e == cudaSuccess ? 0 : (int)e;
+        for (int v : status[k]) lost |= v == ERR_STAGE_LOST;
+        for (size_t j = 0; j < s.recs.size(); j++) {
+          Rec& r = recs[s.recs[j]];
+          r.batch_lost = lost;
+          r.kstatus = status[k][j];
+          r.state = DONE;
+          r.t_done = t;
+          r.cuda_error = e == cudaSuccess ? 0 : (int)e;
         }
         if (e != cudaSuccess) worker_error = std::string("serving batch: ") + cudaGetErrorString(e);
         n_completed += s.recs.size();
@@ -370,6 +461,7 @@ int inspire_server_create(inspire_ctx* c, const inspire_server_config* cfg, insp
     if (sl.ddesc.ensure(sizeof(QueryDesc) * B))
       return bail(fail(INSPIRE_ERR_OUT_OF_MEMORY, alloc_failure(c, "serving slot buffers")));
   }
+  s->helpers.start(std::min({8u, std::thread::hardware_concurrency() / 2, cfg->capacity / (unsigned)CopyHelpers::MIN_COPIES}));
   s->worker = std::thread([s] { s->run(); });
   *out = s;
   return INSPIRE_OK;
@@ -540,10 +632,10 @@ int inspire_server_poll(inspire_server* s, uint64_t ticket, uint64_t* out_ct, in
   r.state = COLLECTING;  // this caller owns the record until it frees it
   const int cuda_error = r.cuda_error;
   const bool batch_lost = r.batch_lost;
+  const int kstatus = r.kstatus;
   const int64_t t_done = r.t_done;
   lk.unlock();
   const uint8_t* p = s->rec_ptr((int)idx);
-  const int32_t kstatus = *reinterpret_cast<const volatile int32_t*>(p + REC_STATUS);
   if (out_ct && !cuda_error && !kstatus && !batch_lost) memcpy(out_ct, p + REC_OUT, sizeof(uint64_t) * 4 * N);
   if (done_ns) *done_ns = t_done;
   lk.lock();
@@ -571,7 +663,36 @@ int inspire_server_poll_batch(inspire_server* s, uint32_t n, const uint64_t* tic
   if (!s || !collected || (n && !tickets)) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
   const int64_t deadline = timeout_us < 0 ? INT64_MAX : now_ns() + (int64_t)timeout_us * 1000;
   const size_t pw = poly_words();
+  std::vector<CopyHelpers::Copy> copies;
   for (uint32_t k = 0; k < n; k++) {
+    // the tickets from here on that are done and sound, all at once
+    const uint32_t k0 = k;
+    copies.clear();
+    {
+      std::lock_guard<std::mutex> lk(s->mu);
+      for (; k < n; k++) {
+        const uint64_t idx = tickets[k] & ((1ull << TICKET_IDX_BITS) - 1);
+        if (idx >= s->recs.size()) break;
+        Rec& r = s->recs[idx];
+        if (r.gen != (tickets[k] >> TICKET_IDX_BITS) || r.state != DONE || r.cuda_error || r.batch_lost || r.kstatus)
+          break;
+        r.state = COLLECTING;  // this caller owns the record until it frees it
+        if (done_ns) done_ns[k] = r.t_done;
+        if (out_ct) copies.push_back({out_ct + (size_t)k * 2 * pw, s->rec_ptr((int)idx) + REC_OUT});
+      }
+    }
+    if (k > k0) {
+      s->helpers.run(std::move(copies), sizeof(uint64_t) * 4 * N);
+      std::lock_guard<std::mutex> lk(s->mu);
+      for (uint32_t j = k0; j < k; j++) {
+        const uint64_t idx = tickets[j] & ((1ull << TICKET_IDX_BITS) - 1);
+        s->recs[idx].gen++;
+        s->recs[idx].state = FREE;
+        s->free_list.push_back((int)idx);
+      }
+      *collected = k;
+      if (k == n) break;
+    }
     int32_t left = 0;
     if (timeout_us < 0) {
       left = -1;

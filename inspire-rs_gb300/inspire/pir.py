@@ -64,7 +64,8 @@ def _u64(a, shape=None) -> np.ndarray:
 
 
 def _ptr(a: Optional[np.ndarray]):
-    return None if a is None else a.ctypes.data_as(C.c_void_p)
+    """The array's address; the caller holds the array until the call returns."""
+    return None if a is None else a.ctypes.data
 
 
 @dataclass
@@ -313,7 +314,7 @@ class EncodedDatabase:
 
 
 def _response(out: np.ndarray, plen: int) -> ServerResponse:
-    return ServerResponse(RlweCiphertext(out[:plen].copy(), out[plen:].copy()), [])
+    return ServerResponse(RlweCiphertext(out[:plen], out[plen:]), [])
 
 
 def respond_seeded_inspiring(crs: ServerCrs, encoded_db: EncodedDatabase, query: SeededClientQuery) -> ServerResponse:
@@ -325,9 +326,9 @@ def respond_seeded_inspiring(crs: ServerCrs, encoded_db: EncodedDatabase, query:
     keys = query.inspiring_packing_keys
     yb = None if keys is None or keys.y_body is None else _u64(keys.y_body)
     ya = None if keys is None or keys.y_all is None else _u64(keys.y_all)
-    q = nat.SeededQueryC(query.shard_id, seeds.ctypes.data_as(C.c_void_p), b_rows.ctypes.data_as(C.c_void_p),
+    q = nat.SeededQueryC(query.shard_id, _ptr(seeds), _ptr(b_rows),
                          1 if keys is not None else 0, _ptr(yb), _ptr(ya))
-    out = np.zeros(2 * plen, dtype=np.uint64)
+    out = np.empty(2 * plen, dtype=np.uint64)
     _check(crs.L.inspire_respond_seeded_inspiring(crs.h, encoded_db.h, C.byref(q), _ptr(out)))
     return _response(out, plen)
 
@@ -340,8 +341,8 @@ def respond_inspiring(crs: ServerCrs, encoded_db: EncodedDatabase, query: Client
     keys = query.inspiring_packing_keys
     yb = None if keys is None or keys.y_body is None else _u64(keys.y_body)
     ya = None if keys is None or keys.y_all is None else _u64(keys.y_all)
-    q = nat.QueryC(query.shard_id, rgsw.ctypes.data_as(C.c_void_p), 1 if keys is not None else 0, _ptr(yb), _ptr(ya))
-    out = np.zeros(2 * plen, dtype=np.uint64)
+    q = nat.QueryC(query.shard_id, _ptr(rgsw), 1 if keys is not None else 0, _ptr(yb), _ptr(ya))
+    out = np.empty(2 * plen, dtype=np.uint64)
     _check(crs.L.inspire_respond_inspiring(crs.h, encoded_db.h, C.byref(q), _ptr(out)))
     return _response(out, plen)
 
@@ -359,7 +360,7 @@ def respond(crs: ServerCrs, encoded_db: EncodedDatabase, query: ClientQuery,
     plen = crs.params.plen
     ell = crs.params.gadget_len
     rgsw = _u64(query.rgsw).reshape(2 * ell, 2, plen)
-    q = nat.QueryC(query.shard_id, rgsw.ctypes.data_as(C.c_void_p), 0, None, None)
+    q = nat.QueryC(query.shard_id, _ptr(rgsw), 0, None, None)
     out = np.zeros(2 * plen, dtype=np.uint64)
     cols = np.zeros((crs.inspiring_num_columns, 2, plen), dtype=np.uint64) if with_columns else None
     _check(crs.L.inspire_respond(crs.h, encoded_db.h, C.byref(q), _ptr(out), _ptr(cols)))
@@ -373,7 +374,7 @@ def respond_seeded(crs: ServerCrs, encoded_db: EncodedDatabase, query: SeededCli
     ell = crs.params.gadget_len
     seeds = np.ascontiguousarray(query.seeds, dtype=np.uint8).reshape(2 * ell, 32)
     b_rows = _u64(query.b_rows).reshape(2 * ell, plen)
-    q = nat.SeededQueryC(query.shard_id, seeds.ctypes.data_as(C.c_void_p), b_rows.ctypes.data_as(C.c_void_p),
+    q = nat.SeededQueryC(query.shard_id, _ptr(seeds), _ptr(b_rows),
                          0, None, None)
     out = np.zeros(2 * plen, dtype=np.uint64)
     cols = np.zeros((crs.inspiring_num_columns, 2, plen), dtype=np.uint64) if with_columns else None
@@ -393,7 +394,7 @@ def respond_one_packing(crs: ServerCrs, encoded_db: EncodedDatabase, query: Clie
     plen = crs.params.plen
     ell = crs.params.gadget_len
     rgsw = _u64(query.rgsw).reshape(2 * ell, 2, plen)
-    q = nat.QueryC(query.shard_id, rgsw.ctypes.data_as(C.c_void_p), 0, None, None)
+    q = nat.QueryC(query.shard_id, _ptr(rgsw), 0, None, None)
     out_a = np.zeros(plen, dtype=np.uint64)
     out_b = np.zeros(2 * plen, dtype=np.uint64)
     words = C.c_uint32(0)
@@ -409,7 +410,7 @@ def respond_seeded_packed(crs: ServerCrs, encoded_db: EncodedDatabase, query: Se
     ell = crs.params.gadget_len
     seeds = np.ascontiguousarray(query.seeds, dtype=np.uint8).reshape(2 * ell, 32)
     b_rows = _u64(query.b_rows).reshape(2 * ell, plen)
-    q = nat.SeededQueryC(query.shard_id, seeds.ctypes.data_as(C.c_void_p), b_rows.ctypes.data_as(C.c_void_p),
+    q = nat.SeededQueryC(query.shard_id, _ptr(seeds), _ptr(b_rows),
                          0, None, None)
     out_a = np.zeros(plen, dtype=np.uint64)
     out_b = np.zeros(2 * plen, dtype=np.uint64)
