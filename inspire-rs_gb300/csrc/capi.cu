@@ -257,6 +257,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.arows = d_arows;
   a.stage_wait_iters = STAGE_WAIT_ITERS_DEFAULT;
   a.after_keys = new_keys;
+  a.alone_max = c->sm_count;
   CUDA_TRY(launch_respond(a, seeds != nullptr, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   c->keys_in_flight = false;
@@ -360,6 +361,7 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   int32_t* hs = c->h_qstatus.host<int32_t>();
   for (uint32_t i = 0; i < n; i++) hs[i] = -1;
   a.status = c->h_qstatus.dev<int32_t>();
+  a.alone_max = c->sm_count;
   CUDA_TRY(launch_respond(a, seeded, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaMemcpyAsync(out_ct, c->d_out.p, sizeof(uint64_t) * n * 2 * pw, cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -1208,6 +1210,7 @@ int inspire_respond_seeded_batch_device_grid(inspire_ctx* c, const inspire_db* d
   a.what = c->what3.as<uint32_t>();
   a.out = d_out_ct;
   a.status = d_status;
+  a.alone_max = c->sm_count;
   CUDA_TRY(launch_respond(a, true, (cudaStream_t)stream, (int)max_ctas, c->pair_max.load()));
   return INSPIRE_OK;
 }

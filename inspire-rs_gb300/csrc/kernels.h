@@ -69,6 +69,10 @@ struct RespondArgs {
   // Host only: the stream's last launch builds a key table of this launch; the
   // two-CTA kernel may be set up meanwhile
   bool after_keys;
+  // Host only: seeded launches of at most this many queries (the SM count; 0:
+  // none, where other launches share the SMs) that are not for the two-CTA kernel
+  // take the form of the one-CTA kernel that has an SM to itself
+  int alone_max;
 };
 
 // NoPacking respond (respond.rs:71-115): per query the combined ciphertext

@@ -74,7 +74,9 @@ struct Smem {
 };
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
-template <int MODE, bool SEEDED, bool QDB>
+// ALONE: the SM is this CTA's, with registers for all of a step's database and
+// CRS words at once.
+template <int MODE, bool SEEDED, bool QDB, bool ALONE>
 __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) {
   constexpr int NR = MODE == MODE_COMPAT ? 1 : 2;
   using L = Smem<NR>;
@@ -269,19 +271,24 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
         v[1][j] = (uint32_t)(cc >> 20) & 0xFFFFFu;
       }
     }
-    // [C] with the first quad of the step's database and CRS words on its way
+    // [C] with the first quad (all four) of the step's database and CRS words on
+    // its way
     const uint32_t* wi = Wx + (size_t)i * ELL * 2 * N;
     const uint32_t* ei = Ex + (size_t)i * ELL * N;
-    uint4 nx[6];
+    uint4 nx[ALONE ? 4 : 1][6];
     auto fetch = [&](int a) {
+      uint4(&to)[6] = nx[ALONE ? a : 0];
 #pragma unroll
       for (int k = 0; k < 3; k++) {
-        nx[k] = ld_stream(ei + k * N + 512 * a);
-        nx[3 + k] = ld_stream(wi + 2 * k * N + 512 * a);
+        to[k] = ld_stream(ei + k * N + 512 * a);
+        to[3 + k] = ld_stream(wi + 2 * k * N + 512 * a);
       }
     };
     const uint32_t sc2[2] = {other, own};
-    jntt_fwd<2, JB_DIGIT>(v, sc2, sfwd_tw(C), q, x, 1 + r, [&]() { fetch(0); });  // signed, below 5.25 q
+    jntt_fwd<2, JB_DIGIT>(v, sc2, sfwd_tw(C), q, x, 1 + r, [&]() {  // signed, below 5.25 q
+#pragma unroll
+      for (int a = 0; a < (ALONE ? 4 : 1); a++) fetch(a);
+    });
     other = mine;
     mine = sc2[0];
     // [D] the nine products of each slot under two reductions, in signed
@@ -296,8 +303,8 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
       uint64_t T[4];
       uint4 cu[6];
 #pragma unroll
-      for (int k = 0; k < 6; k++) cu[k] = nx[k];
-      if (a < 3) fetch(a + 1);
+      for (int k = 0; k < 6; k++) cu[k] = nx[ALONE ? a : 0][k];
+      if (!ALONE && a < 3) fetch(a + 1);
       const uint32_t ro[4] = {row_off(rot9, h_of(4 * a)), row_off(rot9, h_of(4 * a + 1)),
                               row_off(rot9, h_of(4 * a + 2)), row_off(rot9, h_of(4 * a + 3))};
       query_only(cu[0], cu[1], cu[2], ro, T);
@@ -333,10 +340,20 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
   }
 }
 
-// One query per CTA.
+// One query per CTA, two CTAs per SM.
 template <int MODE, bool SEEDED, bool QDB>
 __global__ void __launch_bounds__(QT, 2) respond_kernel(const __grid_constant__ RespondArgs A) {
-  respond_one<MODE, SEEDED, QDB>(A, blockIdx.x);
+  respond_one<MODE, SEEDED, QDB, false>(A, blockIdx.x);
+}
+
+// One query per CTA and SM, for seeded batches of at most as many queries as SMs:
+// 128 queries take 116 us against 131 with 128 registers a thread (128 threads'
+// worth of them left idle, the step's words waited for quad by quad), 77 in
+// compat mode 115 against 129.  The same for 2048 queries takes 1570 us, 1356
+// with two CTAs per SM.
+template <int MODE, bool QDB>
+__global__ void __launch_bounds__(QT, 1) respond_kernel_alone(const __grid_constant__ RespondArgs A) {
+  respond_one<MODE, true, QDB, true>(A, blockIdx.x);
 }
 
 // Capped grid (device-resident rows): CTA b answers queries b, b + gridDim.x,
@@ -346,7 +363,7 @@ __global__ void __launch_bounds__(QT, 2) respond_kernel_loop(const __grid_consta
 #pragma unroll 1
   for (int qi = blockIdx.x; qi < A.nq; qi += gridDim.x) {
     if (qi != (int)blockIdx.x) __syncthreads();  // the previous query's shared memory is no longer read
-    respond_one<MODE, SEEDED, false>(A, qi);
+    respond_one<MODE, SEEDED, false, false>(A, qi);
   }
 }
 
@@ -378,8 +395,16 @@ static cudaError_t launch_one(const RespondArgs& a, int ctas, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <int MODE, bool QDB>
+static cudaError_t set_alone_smem_attr() {
+  return cudaFuncSetAttribute(respond_kernel_alone<MODE, QDB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)respond_smem_bytes(MODE));
+}
+
 cudaError_t prepare_respond_kernels() {
   const cudaError_t es[] = {
+      set_alone_smem_attr<MODE_COMPAT, false>(),     set_alone_smem_attr<MODE_COMPAT, true>(),
+      set_alone_smem_attr<MODE_CRT_FIXED, false>(),  set_alone_smem_attr<MODE_CRT_FIXED, true>(),
       set_smem_attr<MODE_COMPAT, false, false>(),    set_smem_attr<MODE_COMPAT, true, false>(),
       set_smem_attr<MODE_COMPAT, false, true>(),     set_smem_attr<MODE_COMPAT, true, true>(),
       set_smem_attr<MODE_CRT_FIXED, false, false>(), set_smem_attr<MODE_CRT_FIXED, true, false>(),
@@ -387,6 +412,13 @@ cudaError_t prepare_respond_kernels() {
   for (cudaError_t e : es)
     if (e != cudaSuccess) return e;
   return cudaSuccess;
+}
+
+template <int MODE>
+static cudaError_t launch_alone(const RespondArgs& a, cudaStream_t st) {
+  if (a.qdesc) respond_kernel_alone<MODE, true><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
+  else respond_kernel_alone<MODE, false><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
+  return cudaGetLastError();
 }
 
 template <int MODE>
@@ -398,6 +430,8 @@ static cudaError_t launch_mode(const RespondArgs& a, bool seeded, int ctas, cuda
 cudaError_t launch_respond(const RespondArgs& a, bool seeded, cudaStream_t st, int max_ctas, int pair_max) {
   if (a.nq <= 0) return cudaSuccess;
   if (max_ctas <= 0 && a.nq <= pair_max) return launch_respond_pair(a, seeded, st);
+  if (max_ctas <= 0 && seeded && a.nq <= a.alone_max)
+    return a.P.mode == MODE_COMPAT ? launch_alone<MODE_COMPAT>(a, st) : launch_alone<MODE_CRT_FIXED>(a, st);
   const int ctas = (max_ctas > 0 && max_ctas < a.nq) ? max_ctas : a.nq;
   return a.P.mode == MODE_COMPAT ? launch_mode<MODE_COMPAT>(a, seeded, ctas, st)
                                  : launch_mode<MODE_CRT_FIXED>(a, seeded, ctas, st);
