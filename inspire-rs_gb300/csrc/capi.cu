@@ -550,6 +550,7 @@ int run_tree(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* s
   t.nq = (int)n;
   t.ncols = db->gamma;
   t.mode = c->mode;
+  t.sm_count = c->sm_count;
   t.shard = c->h_stage.dev<uint32_t>();
   t.seeds = seeded ? c->h_stage.dev<uint8_t>() + sizeof(uint32_t) * n : nullptr;
   t.nshards = db->nshards;
@@ -1218,14 +1219,14 @@ int inspire_respond_seeded_batch_device_grid(inspire_ctx* c, const inspire_db* d
 int inspire_ntt_forward_device(inspire_ctx* c, uint32_t* d_polys, uint32_t npolys, void* stream) {
   if (!c || (npolys && !d_polys)) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
   if (int rc = set_device(c)) return rc;
-  CUDA_TRY(launch_ntt_ref(c->P, d_polys, (int)npolys, false, (cudaStream_t)stream));
+  CUDA_TRY(launch_ntt_ref(c->P, d_polys, (int)npolys, false, c->sm_count, (cudaStream_t)stream));
   return INSPIRE_OK;
 }
 
 int inspire_ntt_inverse_device(inspire_ctx* c, uint32_t* d_polys, uint32_t npolys, void* stream) {
   if (!c || (npolys && !d_polys)) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
   if (int rc = set_device(c)) return rc;
-  CUDA_TRY(launch_ntt_ref(c->P, d_polys, (int)npolys, true, (cudaStream_t)stream));
+  CUDA_TRY(launch_ntt_ref(c->P, d_polys, (int)npolys, true, c->sm_count, (cudaStream_t)stream));
   return INSPIRE_OK;
 }
 
@@ -1342,6 +1343,7 @@ int inspire_respond_seeded_packed_noalloc_device(inspire_ctx* c, const inspire_d
   t.nq = (int)n;
   t.ncols = db->gamma;
   t.mode = c->mode;
+  t.sm_count = c->sm_count;
   t.shard = d_shard_ids;
   t.seeds = d_seeds;
   t.brows = d_b_rows;
@@ -1409,7 +1411,7 @@ int inspire_external_product_device(inspire_ctx* c, const uint32_t* d_ct, const 
                                     uint32_t npairs, void* stream) {
   if (!c || (npairs && (!d_ct || !d_rgsw || !d_out))) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
   if (int rc = set_device(c)) return rc;
-  CUDA_TRY(launch_external_product(c->P, d_ct, d_rgsw, d_out, (int)npairs, (cudaStream_t)stream));
+  CUDA_TRY(launch_external_product(c->P, d_ct, d_rgsw, d_out, (int)npairs, c->sm_count, (cudaStream_t)stream));
   return INSPIRE_OK;
 }
 

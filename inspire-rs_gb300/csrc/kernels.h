@@ -146,6 +146,7 @@ struct TreeArgs {
   DevParams P;
   int nq, ncols;
   int mode;
+  int sm_count;           // (host)
   const uint32_t* shard;  // [nq]
   const uint8_t* seeds;   // [nq][ELL][32] or null
   const uint64_t* arows;  // [nq][ELL][2][N] or null
@@ -229,9 +230,9 @@ cudaError_t launch_mulmod_rate(const DevParams& P, int blocks, int iters, uint32
 // receives warp 0's accumulators (= iters * A B for iters <= 4096).
 cudaError_t launch_int8_mma_rate(const int8_t* A, const int8_t* B, int blocks, int iters, int32_t* out,
                                  cudaStream_t st);
-cudaError_t launch_ntt_ref(const DevParams& P, uint32_t* polys, int npolys, bool inverse,
+cudaError_t launch_ntt_ref(const DevParams& P, uint32_t* polys, int npolys, bool inverse, int sm_count,
                            cudaStream_t st);
-cudaError_t launch_external_product(const DevParams& P, const uint32_t* ct, const uint32_t* rgsw,
-                                    uint32_t* out, int npairs, cudaStream_t st);
+cudaError_t launch_external_product(const DevParams& P, const uint32_t* ct, const uint32_t* rgsw, uint32_t* out,
+                                    int npairs, int sm_count, cudaStream_t st);
 
 }  // namespace ig

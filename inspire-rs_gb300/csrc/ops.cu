@@ -22,9 +22,11 @@ namespace {
 // full sectors, 10 us of the stores alone), inverse 41 us (47 us).  Fetching
 // the next polynomials while these are transformed (persistent CTAs, in
 // registers or by cp.async) took 44-47 us: it only adds instructions.
-constexpr int NTT_REF_K = 2;
+// Up to as many polynomials as CTAs fit the chip (3 per SM), a CTA takes one:
+// 456 take 8.5 us, 10.3 two by two; 301 and fewer take 7 us either way.
+constexpr int NTT_REF_K = 2, NTT_REF_CTAS = 3;
 template <int K, bool INVERSE>
-__global__ void __launch_bounds__(BLOCK, 3) ntt_ref_kernel(const DevParams P, uint32_t* __restrict__ polys, int npolys) {
+__global__ void __launch_bounds__(BLOCK, NTT_REF_CTAS) ntt_ref_kernel(const DevParams P, uint32_t* __restrict__ polys, int npolys) {
   __shared__ __align__(128) uint32_t SC[2][K][N];
   const int tid = threadIdx.x, g = tid >> 7, x = tid & 127;
   const int p0 = blockIdx.x * K;
@@ -74,13 +76,15 @@ __global__ void __launch_bounds__(BLOCK, 3) ntt_ref_kernel(const DevParams P, ui
 // external_product(rlwe, rgsw): result = sum_i g^-1(a)_i * C[i] + g^-1(b)_i * C[ELL+i].
 // ct[p][2 (a,b)][2][N]; rgsw[p][2*ELL rows][2 (a,b)][2][N]; out[p][2][2][N].
 // One pair per CTA, one residue per group; the transforms of a digit and of
-// its row's two parts share their twiddles.  1024 products take 188 us (235 us
+// its row's two parts share their twiddles.  CTAS per SM: one, with the registers
+// of both, while there is an SM for each pair (152 products 31 us, 35 with two).  1024 products take 188 us (235 us
 // one transform after the other, four CTAs per SM); 40 transforms a product
 // are 137 us at the rate above.
 constexpr int EXT_WORDS = 2 * ELL * N + 6 * N;  // digits, three exchange buffers per group
-__global__ void __launch_bounds__(BLOCK, 2) external_product_kernel(const DevParams P, const uint32_t* __restrict__ ct,
-                                                                    const uint32_t* __restrict__ rgsw,
-                                                                    uint32_t* __restrict__ out) {
+template <int CTAS>
+__global__ void __launch_bounds__(BLOCK, CTAS)
+    external_product_kernel(const DevParams P, const uint32_t* __restrict__ ct, const uint32_t* __restrict__ rgsw,
+                            uint32_t* __restrict__ out) {
   extern __shared__ __align__(128) uint32_t smem[];
   uint32_t* dig = smem;  // [2*ELL][N]: digits of a (rows 0..ELL-1), of b (ELL..)
   const int p = blockIdx.x, tid = threadIdx.x, g = tid >> 7, x = tid & 127;
@@ -296,26 +300,36 @@ cudaError_t launch_mulmod_rate(const DevParams& P, int blocks, int iters, uint32
   return cudaGetLastError();
 }
 
-cudaError_t launch_ntt_ref(const DevParams& P, uint32_t* polys, int npolys, bool inverse, cudaStream_t st) {
-  if (npolys <= 0) return cudaSuccess;
-  constexpr int K = NTT_REF_K;
+template <int K>
+static void launch_ntt_k(const DevParams& P, uint32_t* polys, int npolys, bool inverse, cudaStream_t st) {
   const int grid = (npolys + K - 1) / K;
   if (inverse) ntt_ref_kernel<K, true><<<grid, BLOCK, 0, st>>>(P, polys, npolys);
   else ntt_ref_kernel<K, false><<<grid, BLOCK, 0, st>>>(P, polys, npolys);
+}
+
+cudaError_t launch_ntt_ref(const DevParams& P, uint32_t* polys, int npolys, bool inverse, int sm_count,
+                           cudaStream_t st) {
+  if (npolys <= 0) return cudaSuccess;
+  if (npolys <= NTT_REF_CTAS * sm_count) launch_ntt_k<1>(P, polys, npolys, inverse, st);
+  else launch_ntt_k<NTT_REF_K>(P, polys, npolys, inverse, st);
   return cudaGetLastError();
 }
 
 constexpr size_t EXT_SMEM = sizeof(uint32_t) * (size_t)EXT_WORDS;
 
 cudaError_t launch_external_product(const DevParams& P, const uint32_t* ct, const uint32_t* rgsw, uint32_t* out,
-                                    int npairs, cudaStream_t st) {
+                                    int npairs, int sm_count, cudaStream_t st) {
   if (npairs <= 0) return cudaSuccess;
-  external_product_kernel<<<npairs, BLOCK, EXT_SMEM, st>>>(P, ct, rgsw, out);
+  if (npairs <= sm_count) external_product_kernel<1><<<npairs, BLOCK, EXT_SMEM, st>>>(P, ct, rgsw, out);
+  else external_product_kernel<2><<<npairs, BLOCK, EXT_SMEM, st>>>(P, ct, rgsw, out);
   return cudaGetLastError();
 }
 
 cudaError_t prepare_ops_kernels() {
-  return cudaFuncSetAttribute(external_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXT_SMEM);
+  const cudaError_t e =
+      cudaFuncSetAttribute(external_product_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXT_SMEM);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(external_product_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXT_SMEM);
 }
 
 }  // namespace ig

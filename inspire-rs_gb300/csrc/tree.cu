@@ -298,7 +298,10 @@ __device__ __forceinline__ void key_switch(const TreeArgs& A, uint32_t base, int
 // (automorph_pack.rs:466-484): b_val_z * d added at coefficient z < ncols; one
 // LWE alone is returned unpacked (automorph_pack.rs:439-446), (a, b_val at
 // coefficient 0).
-__global__ void __launch_bounds__(QT, 2) tree_kernel(const __grid_constant__ TreeArgs A) {
+// CTAS per SM: one, with the registers of both, while every LWE has an SM (9
+// queries of 16 take 126 us, 132 with two; 33 take 282, 291 with one).
+template <int CTAS>
+__global__ void __launch_bounds__(QT, CTAS) tree_kernel(const __grid_constant__ TreeArgs A) {
   extern __shared__ __align__(128) uint32_t smem[];
   __shared__ uint32_t arrived;
   const DevParams& P = A.P;
@@ -477,7 +480,9 @@ size_t tree_work_words_per_query() { return WORK_WORDS; }
 constexpr int SWITCH_BYTES = (int)sizeof(uint32_t) * SwitchSmem::TOTAL;
 
 cudaError_t prepare_tree_kernels() {
-  return cudaFuncSetAttribute(tree_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SWITCH_BYTES);
+  const cudaError_t e = cudaFuncSetAttribute(tree_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SWITCH_BYTES);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(tree_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SWITCH_BYTES);
 }
 
 cudaError_t launch_tree(const TreeArgs& a, bool seeded, cudaStream_t st) {
@@ -506,7 +511,7 @@ cudaError_t launch_tree(const TreeArgs& a, bool seeded, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   cfg.gridDim = dim3(a.nq * a.ncols);
   cfg.dynamicSmemBytes = SWITCH_BYTES;
-  return cudaLaunchKernelEx(&cfg, tree_kernel, a);
+  return cudaLaunchKernelEx(&cfg, a.nq * a.ncols <= a.sm_count ? tree_kernel<1> : tree_kernel<2>, a);
 }
 
 cudaError_t launch_galois_prep(const DevParams& P, const uint64_t* keys, int nkeys, uint32_t* ks, cudaStream_t st) {
