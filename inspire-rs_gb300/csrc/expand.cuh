@@ -136,69 +136,4 @@ __device__ bool expand_seeded_row(const DevParams& P, const uint8_t* __restrict_
   return false;
 }
 
-// One residue of Poly::from_seed_moduli (poly.rs:251-281) by one 256-thread
-// sub-block, for the kernels that expand each residue on its own CTA: the
-// first N accepted draws of gen_range(0..q_res) among the stream's 64-bit
-// candidates from global index `first` on (candidate 8 b + k is word pair k
-// of block b).  Residue 0 starts at 0; residue 1 at the index after residue
-// 0's last accepted draw.  Returns the index after the last accepted
-// candidate, or -1 if the iteration bound was hit.
-//
-// Speculative start (spec_blk > 0): the first batch, from block spec_blk on,
-// is drawn before `first` is known; then every thread calls get_first(),
-// which returns it (at least 8 spec_blk for residue 1, whose position the
-// other CTA finds).  Candidates before `first` are skipped, and blocks wholly
-// before it are not drawn after the first batch, so the result does not
-// depend on the guess.
-template <class GetFirst>
-__device__ long long expand_residue(const DevParams& P, const uint32_t key[8], int res, uint64_t first,
-                                    uint64_t spec_blk, GetFirst&& get_first, uint64_t* cand, uint32_t* dst, int* ws,
-                                    int bar, int lt) {
-  const uint64_t q = P.r[res].q, zone = P.r[res].zone;
-  uint64_t blk = spec_blk ? spec_blk : first / 8;
-  int pos = 0;
-  for (int it = 0; it < 64; it++) {
-    const int nblk = min(SUB, ((N - pos) * 9) / 64 + 3);
-    if (lt < nblk) {
-      uint32_t w[16];
-      chacha20_block(key, blk + lt, P.one, w);
-#pragma unroll
-      for (int k = 0; k < 8; k++) cand[k * SUB + lt] = (uint64_t)w[2 * k] | ((uint64_t)w[2 * k + 1] << 32);
-    }
-    const uint64_t gbase = 8 * blk;  // global index of local candidate 0
-    blk += nblk;
-    named_sync(bar, SUB);
-    if (it == 0 && spec_blk) first = get_first();
-    uint32_t vals[8];
-    unsigned fl = 0;
-    int cnt = 0;
-    if (lt < nblk) {
-#pragma unroll
-      for (int k = 0; k < 8; k++)
-        if (gbase + 8 * lt + k >= first && uniform_accept(cand[k * SUB + lt], q, zone, vals[k])) {
-          fl |= 1u << k;
-          cnt++;
-        }
-    }
-    int total;
-    int p = pos + sub_scan_excl(cnt, ws, total, bar, lt);
-#pragma unroll
-    for (int k = 0; k < 8; k++)
-      if ((fl >> k) & 1u) {
-        if (p < N) dst[p] = vals[k];
-        if (p == N - 1) ws[16] = 8 * lt + k;
-        p++;
-      }
-    named_sync(bar, SUB);
-    if (pos + total >= N) {
-      const long long end = (long long)(gbase + (uint64_t)ws[16] + 1);
-      named_sync(bar, SUB);  // ws[16] is read before the next use of ws
-      return end;
-    }
-    pos += total;
-    if (blk < first / 8) blk = first / 8;
-  }
-  return -1;
-}
-
 }  // namespace ig

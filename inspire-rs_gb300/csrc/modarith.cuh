@@ -51,10 +51,4 @@ __device__ __forceinline__ uint32_t mont_mul(uint32_t a, uint32_t b, uint32_t q,
   return redc((uint64_t)a * b, q, qinv);
 }
 
-// Lazy accumulate: x, r in [0, 2q) -> x + r in [0, 2q)
-__device__ __forceinline__ uint32_t acc_2q(uint32_t x, uint32_t r, uint32_t q2) {
-  uint32_t s = x + r;
-  return min(s, s - q2);
-}
-
 }  // namespace ig

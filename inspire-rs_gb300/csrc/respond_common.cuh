@@ -1,7 +1,7 @@
 // respond_common.cuh -- device helpers shared by the Respond kernels
 // (respond.cu: one CTA per query; respond_pair.cu: a cluster of two CTAs
-// per query, one per CRT residue): bulk copies and mbarriers, the scatter of
-// the query-only term R_i, and the client key-table runs.
+// per query, one per CRT residue) and by the kernels that build their tables:
+// bulk copies and mbarriers, the layouts of slots, the folded keys.
 #pragma once
 #include "common.cuh"
 
@@ -32,11 +32,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 __device__ __forceinline__ void mbar_init(uint64_t* bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// Invalidate an mbarrier before its words are used for anything else.
-__device__ __forceinline__ void mbar_inval(uint64_t* bar) {
-  asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // The single arrival, announcing `bytes` of bulk copies to complete.
