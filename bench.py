@@ -807,7 +807,7 @@ def main():
             "scaling": "weak", "vs_baseline": None, "dtype": "u32 modular integer (exact)", "data": "synthetic",
             "config": {"workload": f"batched InsPIRe^2 respond: 2^{args.log2_entries} entries x 32 B resident "
                                    f"({nshards} shards), B={B} seeded queries per launch, uniform shard ids",
-                       "step": f"{L} batch calls x {B} queries (a b-side and a Respond launch each) over "
+                       "step": f"{L} batch calls x {B} queries (one Respond launch each) over "
                                f"{len(side)} streams",
                        "streams": len(side),
                        "queries": f"{QUERY_POOL} distinct real seeded queries from {N_CLIENTS} clients generated "
@@ -833,7 +833,7 @@ def main():
                                      "peak = the rate probe (independent lazy Shoup multiply chains, all SMs)"},
             "cpu_baseline": cpu,
             "clocks": clk.summary(),
-            "gpu_launches": args.steps * L * 2,  # each device-row batch call: b-side launch + Respond launch
+            "gpu_launches": args.steps * L,  # one Respond launch per device-row batch call
             "verified_responses": verified,
             "value_cuda_graph": value_graph,
             "value_capped_grid": value_grid,

@@ -215,6 +215,25 @@ void release_keys(inspire_ctx* c, int32_t id) {
 
 int finish_status(inspire_ctx* c, uint32_t n, const char* what);
 
+// Queries up to which a batch on `st` may take the Respond kernel's form that has
+// an SM to itself: the SM count, or none while the last device batch, on another
+// stream, still runs (batches that overlap do better two CTAs to an SM: 2048
+// queries take 1356 us so, 1570 one to an SM) or when captured into a graph, whose
+// launches may overlap.
+int alone_limit(inspire_ctx* c, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusNone) return 0;
+  if (!c->batch_stream_set || c->batch_stream == st) return c->sm_count;
+  // (relaxed: the query must not end another thread's capture)
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const bool running = cudaEventQuery(c->batch_ev) == cudaErrorNotReady;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (running) cudaGetLastError();
+  return running ? 0 : c->sm_count;
+}
+
 // Batches up to this size stage their inputs through page-locked memory.
 constexpr uint32_t STAGE_PINNED_MAX = 64;
 
@@ -257,7 +276,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.arows = d_arows;
   a.stage_wait_iters = STAGE_WAIT_ITERS_DEFAULT;
   a.after_keys = new_keys;
-  a.alone_max = c->sm_count;
+  a.alone_max = alone_limit(c, c->stream);
   CUDA_TRY(launch_respond(a, seeds != nullptr, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   c->keys_in_flight = false;
@@ -361,7 +380,7 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   int32_t* hs = c->h_qstatus.host<int32_t>();
   for (uint32_t i = 0; i < n; i++) hs[i] = -1;
   a.status = c->h_qstatus.dev<int32_t>();
-  a.alone_max = c->sm_count;
+  a.alone_max = alone_limit(c, c->stream);
   CUDA_TRY(launch_respond(a, seeded, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaMemcpyAsync(out_ct, c->d_out.p, sizeof(uint64_t) * n * 2 * pw, cudaMemcpyDeviceToHost, c->stream));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
@@ -677,6 +696,11 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
   if (e != cudaSuccess) {
     delete c;
     return fail(INSPIRE_ERR_CUDA, std::string("cudaStreamCreate: ") + cudaGetErrorString(e));
+  }
+  e = cudaEventCreateWithFlags(&c->batch_ev, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    delete c;
+    return fail(INSPIRE_ERR_CUDA, std::string("cudaEventCreate: ") + cudaGetErrorString(e));
   }
   if (cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       c->sm_count <= 0) {
@@ -1211,8 +1235,17 @@ int inspire_respond_seeded_batch_device_grid(inspire_ctx* c, const inspire_db* d
   a.what = c->what3.as<uint32_t>();
   a.out = d_out_ct;
   a.status = d_status;
-  a.alone_max = c->sm_count;
-  CUDA_TRY(launch_respond(a, true, (cudaStream_t)stream, (int)max_ctas, c->pair_max.load()));
+  const int pair_max = c->pair_max.load();
+  const bool large = (int)n > pair_max && (int)n <= c->sm_count && max_ctas == 0;
+  if (large) a.alone_max = alone_limit(c, (cudaStream_t)stream);
+  CUDA_TRY(launch_respond(a, true, (cudaStream_t)stream, (int)max_ctas, pair_max));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (large) CUDA_TRY(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
+  if (large && cap == cudaStreamCaptureStatusNone) {  // for the next batch's choice
+    CUDA_TRY(cudaEventRecord(c->batch_ev, (cudaStream_t)stream));
+    c->batch_stream = (cudaStream_t)stream;
+    c->batch_stream_set = true;
+  }
   return INSPIRE_OK;
 }
 

@@ -541,12 +541,12 @@ def respond_seeded_batch_device(crs: ServerCrs, encoded_db: EncodedDatabase, n: 
 
 def ntt_forward_device(crs: ServerCrs, d_polys: int, npolys: int, stream: int) -> None:
     """Batched NttContext::forward (ntt.rs:223-246) on device u32 data."""
-    _check(crs.L.inspire_ntt_forward_device(crs.h, C.c_void_p(d_polys), npolys, C.c_void_p(stream)))
+    _check(crs.L.inspire_ntt_forward_device(crs.h, d_polys, npolys, stream))
 
 
 def ntt_inverse_device(crs: ServerCrs, d_polys: int, npolys: int, stream: int) -> None:
     """Batched NttContext::inverse (ntt.rs:308-325) on device u32 data."""
-    _check(crs.L.inspire_ntt_inverse_device(crs.h, C.c_void_p(d_polys), npolys, C.c_void_p(stream)))
+    _check(crs.L.inspire_ntt_inverse_device(crs.h, d_polys, npolys, stream))
 
 
 def extract_inspiring_device(crs: ServerCrs, d_sk: int, d_ct: int, n: int, entry_size: int, d_entries: int,
@@ -639,8 +639,7 @@ def int8_mma_rate_device(crs: ServerCrs, blocks: int, iters: int, d_a: int, d_b:
 
 def external_product_device(crs: ServerCrs, d_ct: int, d_rgsw: int, d_out: int, npairs: int, stream: int) -> None:
     """Batched external_product (external_product.rs:88-150) on device u32 data."""
-    _check(crs.L.inspire_external_product_device(crs.h, C.c_void_p(d_ct), C.c_void_p(d_rgsw), C.c_void_p(d_out),
-                                                 npairs, C.c_void_p(stream)))
+    _check(crs.L.inspire_external_product_device(crs.h, d_ct, d_rgsw, d_out, npairs, stream))
 
 
 def write_crs_json(path: str, params: InspireParams, *, k_g: np.ndarray, k_h: np.ndarray, galois_keys: np.ndarray,
