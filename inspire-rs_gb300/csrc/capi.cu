@@ -843,8 +843,8 @@ int inspire_crs_load(inspire_ctx* c, const uint8_t w_seed[32], uint32_t num_colu
   c->P.gamma = gamma;
   for (int r = 0; r < 2; r++) {
     const uint64_t qm = c->params.crt_moduli[r];
-    const uint64_t r96 = (uint64_t)(((u128)1 << 96) % qm);
-    const uint64_t k = (uint64_t)((u128)((u128)inv_prime(gamma, qm) * inv_prime(N, qm) % qm) * r96 % qm);
+    const uint64_t r32 = ((uint64_t)1 << 32) % qm;
+    const uint64_t k = (uint64_t)((u128)((u128)inv_prime(gamma, qm) * inv_prime(N, qm) % qm) * r32 % qm);
     c->P.r[r].e_scale = (uint32_t)k;
     c->P.r[r].e_scale_p = shoup(k, qm);
   }

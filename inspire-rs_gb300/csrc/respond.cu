@@ -44,11 +44,11 @@
 // What bounds it: the integer multiply-add pipe (64 lane-operations per
 // cycle and SM, a high or wide product costs two) is 73 % busy, 86 % in the
 // digit transforms; the rest waits on 16 warps' latencies.  One call of 2048
-// queries takes 1430 us (1507 us with unsigned butterflies and the step's
+// queries takes 1354 us (1507 us with unsigned butterflies and the step's
 // database and CRS words loaded where they are used); the six-group kernel
 // before it (768 threads, one CTA per SM, four CTA-wide barriers a step, its
 // 24 warps in step with one another, the b side in a launch of its own) took
-// 2290 us, and 174 against 142 us for 128 queries (fewer queries than SMs).
+// 2290 us, and 174 against 117 us for 128 queries (fewer queries than SMs).
 // Two CTAs of different queries share the SM without waiting for each other,
 // and 128 registers a thread let each warp keep 16 independent butterflies in
 // flight.

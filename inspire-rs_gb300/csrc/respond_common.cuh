@@ -109,6 +109,31 @@ __device__ __forceinline__ void fold_keys(uint32_t (&v)[ELL][16], const ResidueC
   }
 }
 
+__host__ __device__ constexpr int brv_of(int v, int bits) {
+  int r = 0;
+  for (int i = 0; i < bits; i++) r |= ((v >> i) & 1) << (bits - 1 - i);
+  return r;
+}
+
+// The DFT of a slot's G values, G_m = sum_i zeta^(i m) f_i with zeta = psi^(2N/G),
+// by decimation in frequency: f[k] = G_m, m the bit reversal of k.  Values in
+// [0, 2q) both ways.
+template <int G>
+__device__ __forceinline__ void slot_dft(uint32_t (&f)[G], const ResidueConsts& C) {
+  const uint32_t q = C.q, q2 = 2 * q;
+#pragma unroll
+  for (int len = G; len > 1; len >>= 1)
+#pragma unroll
+    for (int b = 0; b < G; b += len)
+#pragma unroll
+      for (int p = 0; p < len / 2; p++) {
+        const uint32_t u = f[b + p], v = f[b + p + len / 2];
+        f[b + p] = csub(u + v, q2);
+        const uint32_t d = u - v + q2;
+        f[b + p + len / 2] = p == 0 ? csub(d, q2) : mul_shoup_lazy(d, __ldg(C.fwd + brv_of(2 * N / len * p, LOGN)), q);
+      }
+}
+
 __device__ __forceinline__ uint32_t u4e(const uint4& v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; }
 
 }  // namespace ig

@@ -23,7 +23,7 @@ inline bool launch_batch_now(size_t pending, size_t max_batch, size_t inflight_s
 // SMs per query, the lower latency) when the batch is at most pair_max
 // queries and those SMs are idle, else one CTA per query (the higher rate per
 // SM, which a loaded GPU needs: the cluster kernel alone serves at most
-// ~70 % of the one-CTA rate).  While at most half the SMs are busy a cluster
+// ~60 % of the one-CTA rate).  While at most half the SMs are busy a cluster
 // batch may exceed the idle SMs by a quarter of the SM count (an SM frees
 // about every microsecond); that slack at any load let cluster batches starve
 // a 75 %-load stream (measured: the achieved rate fell below the offered one,

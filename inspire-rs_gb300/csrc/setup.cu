@@ -34,63 +34,76 @@ __global__ void columns_from_raw_kernel(const uint8_t* __restrict__ raw, uint64_
   }
 }
 
-// E[s][r][t][k][u] = K * sum_j zeta^(k j) * omega_u^j * NTT(d_t(Delta h_j))[u]
+// Contracted database: K * sum_j zeta^(k j) * omega_u^j * NTT(d_t(Delta h_j))[u]
 // with omega_u = psi^(2brv(u)+1), zeta = psi^(2n/gamma), K = gamma^-1 n^-1
 // 2^32 (Montgomery form, n^-1 pre-applied for the unscaled inverse NTTs of
 // the Respond kernel).  Grid: (shard, residue, digit t).
-__global__ void __launch_bounds__(BLOCK) encode_E_kernel(const DevParams P, const uint16_t* __restrict__ H,
-                                                         uint32_t* __restrict__ E) {
-  extern __shared__ __align__(16) uint32_t smem[];
-  const int gamma = P.gamma;
-  uint32_t* Dh = smem;                  // [gamma][N]
-  uint32_t* SC = Dh + gamma * N;        // [2][NTT_SCRATCH]
-  uint32_t* zp = SC + 2 * NTT_SCRATCH;  // [gamma] powers of zeta
+//
+// Stored by recursion step i and, within it, by the slot s that R_i takes
+// the value at: source slot u contributes the DFT output k = (2brv(u)+1) m_i
+// mod gamma, m_i = (gamma - i) mod gamma, to s = tau_i^-1(u), i.e. (rot_rows)
+// to row h - rot of the same 16-slot run.  For odd 2brv(u)+1 the map i -> k
+// is a bijection: the table is a permutation of the outputs.  A slot's G values
+// stay its thread's until they are written, a quad at a time.
+// 2^20 entries (512 shards) come from host memory into this form in 1.0 ms, 1.7
+// with G products per output and 4-byte stores.
+constexpr int ENC_GROUPS = 4;
+template <int G>
+__global__ void __launch_bounds__(ENC_GROUPS* NTT_GT, 1)
+    encode_E_kernel(const DevParams P, const uint16_t* __restrict__ H, uint32_t* __restrict__ E) {
+  constexpr int LG = G == 16 ? 4 : G == 8 ? 3 : G == 4 ? 2 : G == 2 ? 1 : 0;
+  extern __shared__ __align__(128) uint32_t smem[];
+  uint32_t* Dh = smem;  // [G][16 rows h][128]; then the exchange buffers
   const int s = blockIdx.x, r = blockIdx.y, t = blockIdx.z;
   const int tid = threadIdx.x, g = tid >> 7, x = tid & 127;
   const ResidueConsts& C = P.r[r];
-  const uint32_t q = C.q, qinv = C.qinv;
-  if (tid < gamma) zp[tid] = C.psi_pow[((2 * N / gamma) * tid) & (2 * N - 1)];
-  for (int j = g; j < gamma; j += 2) {
-    const uint16_t* h = H + ((size_t)s * gamma + j) * N;
-    uint32_t v[16];
+  const uint32_t q = C.q;
+#pragma unroll 1
+  for (int j = g; j < G; j += ENC_GROUPS) {
+    const uint16_t* h = H + ((size_t)s * G + j) * N;
+    uint32_t v[1][16];
 #pragma unroll
     for (int rr = 0; rr < 16; rr++) {
       const uint64_t xv = P.delta * (uint64_t)h[x + 128 * rr];
-      v[rr] = (uint32_t)(xv >> (ZBITS * t)) & ((1u << ZBITS) - 1);  // digit t < 2^20 < q
+      v[0][rr] = (uint32_t)(xv >> (ZBITS * t)) & ((1u << ZBITS) - 1);  // digit t < 2^20 < q
     }
-    ntt_fwd(v, SC + g * NTT_SCRATCH, fwd_tw(C), q, x, 1 + g);
+    group_sync(1 + g);  // the last transform's reads are done
+    const uint32_t sc[1] = {jx_addr(Dh + (G + g) * N)};
+    jntt_fwd<1, JB_CANON>(v, sc, sfwd_tw(C), q, x, 1 + g);
 #pragma unroll
-    for (int rr = 0; rr < 16; rr++) v[rr] = canon16(v[rr], q);
-    uint4* dst = reinterpret_cast<uint4*>(Dh + j * N + 16 * x);
-#pragma unroll
-    for (int rr = 0; rr < 4; rr++) dst[rr] = make_uint4(v[4 * rr], v[4 * rr + 1], v[4 * rr + 2], v[4 * rr + 3]);
+    for (int rr = 0; rr < 16; rr++) Dh[j * N + row_word(h_of(rr), x)] = jcanon_fwd(v[0][rr], q);
   }
   __syncthreads();
-  // Stored by recursion step i and, within it, by the slot s that R_i takes
-  // the value at: source slot u contributes the DFT output k = (2brv(u)+1) m_i
-  // mod gamma, m_i = (gamma - i) mod gamma, to s = tau_i^-1(u), i.e. (rot_rows)
-  // to row h - rot of the same 16-slot run.  For odd 2brv(u)+1 the map i -> k
-  // is a bijection: the table is a permutation of the outputs.  A warp's 32
-  // source slots are two runs, whose words of each quad plane are 32 bytes together.
-  uint32_t* Eo = E + (((size_t)s * 2 + r) * gamma * ELL + t) * N;
-  for (int v = 0; v < N / BLOCK; v++) {
-    const int u = tid + BLOCK * v;
-    const uint32_t e = 2 * brv11(u) + 1;
-    uint32_t c[MAX_GAMMA];
+  const uint32_t c = 2u * (__brev((uint32_t)x) >> 25) + 1u;  // 2brv(u)+1 = 256 h + c
+  const uint32_t cinv = c * c * c;                           // c^4 = 1 mod 16
+#pragma unroll 1
+  for (int h = g; h < 16; h += ENC_GROUPS) {
+    uint32_t* slot = Dh + row_word(h, x);
+    uint32_t f[G];
 #pragma unroll
-    for (int j = 0; j < MAX_GAMMA; j++)
-      if (j < gamma) c[j] = mont_mul(Dh[j * N + u], __ldg(C.psi_pow + ((e * j) & (2 * N - 1))), q, qinv);
-    const int ux = u >> 4, uh = h_of(u & 15);
-    for (int i = 0; i < gamma; i++) {
-      const int k = (int)((e * ((uint32_t)(gamma - i) & (uint32_t)(gamma - 1))) & (uint32_t)(gamma - 1));
-      uint64_t T = 0;
-#pragma unroll
-      for (int j = 0; j < MAX_GAMMA; j++)
-        if (j < gamma) T += (uint64_t)zp[(k * j) & (gamma - 1)] * c[j];
-      // the two REDCs divided by 2^64; e_scale = gamma^-1 n^-1 2^96 leaves
-      // the factor 2^32 gamma^-1 n^-1
-      Eo[(size_t)i * ELL * N + quad_word(h_of((uh - (int)rot_rows(gamma, i, ux)) & 15), ux)] = mul_shoup(redc(T, q, qinv), C.e_scale, C.e_scale_p, q);
+    for (int j = 0; j < G; j++) {
+      const uint32_t ex = ((256u * (uint32_t)h + c) * (uint32_t)j) & (2 * N - 1);  // omega_u^j = psi^ex, psi^N = -1
+      f[j] = slot[j * N];
+      if (j) f[j] = mul_shoup_lazy(f[j], __ldg(C.fwd + brv11(ex & (N - 1))), q);
+      if (ex & N) f[j] = 2 * q - f[j];
+      if (j) f[j] = csub(f[j], 2 * q);
     }
+    slot_dft<G>(f, C);
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      const uint32_t i = (0u - cinv * (uint32_t)brv_of(k, LG)) & (uint32_t)(G - 1);
+      slot[i * N] = mul_shoup(f[k], C.e_scale, C.e_scale_p, q);
+    }
+  }
+  __syncthreads();
+  uint32_t* Eo = E + (((size_t)s * 2 + r) * G * ELL + t) * N;
+#pragma unroll 1
+  for (int i = 0; i < G; i++) {
+    const uint32_t rot = rot_rows(G, i, x);
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) w[j] = Dh[i * N + row_word(((uint32_t)h_of(4 * g + j) + rot) & 15u, x)];
+    *reinterpret_cast<uint4*>(Eo + (size_t)i * ELL * N + 512 * g + 4 * x) = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -210,16 +223,38 @@ cudaError_t launch_columns_from_raw(const uint8_t* raw, uint64_t n_entries, int 
   return cudaGetLastError();
 }
 
+template <int G>
+static constexpr int encode_smem_bytes() {
+  return (int)sizeof(uint32_t) * (G + ENC_GROUPS) * N;
+}
+template <int G>
+static cudaError_t set_encode_smem() {
+  return cudaFuncSetAttribute(encode_E_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, encode_smem_bytes<G>());
+}
 cudaError_t prepare_setup_kernels() {
-  const size_t smem = sizeof(uint32_t) * ((size_t)MAX_GAMMA * N + 2 * NTT_SCRATCH + MAX_GAMMA);
-  return cudaFuncSetAttribute(encode_E_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t es[] = {set_encode_smem<1>(), set_encode_smem<2>(), set_encode_smem<4>(), set_encode_smem<8>(),
+                            set_encode_smem<16>()};
+  for (cudaError_t e : es)
+    if (e != cudaSuccess) return e;
+  return cudaSuccess;
+}
+
+template <int G>
+static void launch_encode(const DevParams& P, const uint16_t* H, int nshards, uint32_t* E, cudaStream_t st) {
+  // grid.x is limited to 2^31-1 shards; y = residue, z = digit
+  encode_E_kernel<G><<<dim3(nshards, 2, ELL), ENC_GROUPS * NTT_GT, encode_smem_bytes<G>(), st>>>(P, H, E);
 }
 
 cudaError_t launch_encode_E(const DevParams& P, const uint16_t* H, int nshards, uint32_t* E, cudaStream_t st) {
   if (nshards <= 0) return cudaSuccess;
-  const size_t smem = sizeof(uint32_t) * ((size_t)P.gamma * N + 2 * NTT_SCRATCH + MAX_GAMMA);
-  // grid.x is limited to 2^31-1 shards; y = residue, z = digit
-  encode_E_kernel<<<dim3(nshards, 2, ELL), BLOCK, smem, st>>>(P, H, E);
+  switch (P.gamma) {
+    case 1: launch_encode<1>(P, H, nshards, E, st); break;
+    case 2: launch_encode<2>(P, H, nshards, E, st); break;
+    case 4: launch_encode<4>(P, H, nshards, E, st); break;
+    case 8: launch_encode<8>(P, H, nshards, E, st); break;
+    case 16: launch_encode<16>(P, H, nshards, E, st); break;
+    default: return cudaErrorInvalidValue;
+  }
   return cudaGetLastError();
 }
 

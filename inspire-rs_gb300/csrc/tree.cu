@@ -118,11 +118,6 @@ __global__ void __launch_bounds__(QT, 2) tree_front_kernel(const __grid_constant
 
 // ---- leaves: alpha_j of every LWE, from the contracted database ----
 constexpr int LEAF_RUNS = 16;  // runs x per CTA: one class x >> 4, so that c and the outputs' columns are uniform
-constexpr int brv_of(int v, int bits) {
-  int r = 0;
-  for (int i = 0; i < bits; i++) r |= ((v >> i) & 1) << (bits - 1 - i);
-  return r;
-}
 
 template <int G>
 __global__ void __launch_bounds__(256) tree_leaves_kernel(const __grid_constant__ TreeArgs A) {
@@ -170,23 +165,12 @@ __global__ void __launch_bounds__(256) tree_leaves_kernel(const __grid_constant_
     }
   }
   __syncthreads();
-  // G_m = sum_i zeta^(i m) T_i per slot (decimation in frequency, zeta =
-  // psi^(2N/G)), then alpha_j = omega_u^-j G_(c j)
+  // G_m = sum_i zeta^(i m) T_i per slot, then alpha_j = omega_u^-j G_(c j)
   const int h = tid >> 4;
   uint32_t f[G];
 #pragma unroll
   for (int i = 0; i < G; i++) f[i] = F[i][h][xl];
-#pragma unroll
-  for (int len = G; len > 1; len >>= 1)
-#pragma unroll
-    for (int b = 0; b < G; b += len)
-#pragma unroll
-      for (int p = 0; p < len / 2; p++) {
-        const uint32_t u = f[b + p], v = f[b + p + len / 2];
-        f[b + p] = csub(u + v, q2);
-        const uint32_t d = u - v + q2;
-        f[b + p + len / 2] = p == 0 ? csub(d, q2) : mul_shoup_lazy(d, __ldg(C.fwd + brv_of(2 * N / len * p, LOGN)), q);
-      }
+  slot_dft<G>(f, C);
   const uint32_t c = 2u * (__brev((uint32_t)x) >> 25) + 1u;      // 2brv(u)+1 mod 16, odd
   const uint32_t cinv = (c * c * c) & (uint32_t)(G - 1);         // c^4 = 1 mod 16
   const uint32_t eu = 256u * (uint32_t)h + c;                    // 2brv(u)+1
