@@ -50,3 +50,48 @@ def test_respond_counts(oracle_mod, which, mode, entry):
         assert np.array_equal(out.array, want[pick])
         rows.close()
         out.close()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_overlapping_batches(captured):
+    """Device batches of one query per SM on two streams at once, and captured
+    into a graph, where the kernel keeps the form that shares an SM: the same
+    responses as alone."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import inspire
+
+    n = torch.cuda.get_device_properties(0).multi_processor_count // 2 + 1
+    rng = np.random.default_rng(n)
+    crs = inspire.ServerCrs(inspire.InspireParams(p=1 << 16), bytes(32), 16)
+    q = crs.params.crt_moduli
+    polys = lambda *s: np.concatenate([rng.integers(0, m, size=(*s, N), dtype=np.uint64) for m in q], axis=-1)  # noqa: E731
+    edb = inspire.EncodedDatabase(crs, rng.integers(0, 256, size=N * 32, dtype=np.uint8), 32)
+    cid = crs.register_client(inspire.ClientPackingKeys(y_body=polys(3)))
+    d = [torch.from_numpy(a).cuda() for a in (np.zeros(n, np.int32),
+                                              rng.integers(0, 256, size=(n, 3, 32), dtype=np.uint8),
+                                              polys(n, 3).view(np.int64), np.full(n, cid, np.int32))]
+    outs = [torch.zeros((n, 2, 2 * N), dtype=torch.int64, device="cuda") for _ in range(5)]
+    status = torch.full((5, n), -1, dtype=torch.int32, device="cuda")
+
+    def batch(k, stream):
+        inspire.respond_seeded_batch_device(crs, edb, n, *[t.data_ptr() for t in d], outs[k].data_ptr(),
+                                            status[k].data_ptr(), stream.cuda_stream)
+
+    batch(0, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    if captured:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for k in range(1, 5):
+                batch(k, torch.cuda.current_stream())
+        g.replay()
+    else:
+        streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+        for k in range(1, 5):
+            batch(k, streams[k & 1])
+    torch.cuda.synchronize()
+    assert not status.cpu().numpy().any()
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
