@@ -263,16 +263,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
         put_draws(AH + k * N, p, mask, val);
         if (t == 0) tot[k] = total;
       }
+      // the next 256 draws, by warps of team 1 while team 0 has the third row (a
+      // lone warp's ChaCha20 off the path of both CTAs: 1.6 us of a launch)
+      const int k = warp - TEAM / 32;
+      const bool tail = k >= 0 && k < ELL;
+      uint32_t val[8];
+      unsigned mask = 0;
+      if (tail) {
+        uint32_t key[8], w[16];
+        load_key(seeds + 32 * k, key);
+        chacha20_block(key, 256 + lane, P.one, w);
+        mask = draw8(w, sq, sz, val);
+      }
       __syncthreads();
       if (MODE == MODE_CRT_FIXED) cluster_wait();
-      if (warp < ELL) {
-        const int k = warp, have = tot[k];
+      if (tail) {
+        const int have = tot[k];
         uint32_t end = 0;  // draws past the first 2048 that residue 0 takes
         if (have < N) {    // uniform over the warp
-          uint32_t key[8], w[16], val[8];
-          load_key(seeds + 32 * k, key);
-          chacha20_block(key, 256 + lane, P.one, w);
-          const unsigned mask = draw8(w, sq, sz, val);
           int all;
           const int p = have + scan_warp(__popc(mask), all);
           put_draws(AH + k * N, p, mask, val);
@@ -304,6 +312,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
         chacha20_block(key, 256 + t, P.one, w);
         mask[u] = draw8(w, sq, sz, val[u]);
       }
+      // the last values, one warp per row, from the blocks after these (as above)
+      const int k = warp - TEAM / 32;
+      const bool tail = k >= 0 && k < ELL;
+      uint32_t v8[8];
+      unsigned m = 0;
+      if (tail) {
+        uint32_t key[8], w[16];
+        load_key(seeds + 32 * k, key);
+        chacha20_block(key, 512 + lane, P.one, w);
+        m = draw8(w, sq, sz, v8);
+      }
       cluster_wait();
       cluster_sync_all();
 #pragma unroll
@@ -319,12 +338,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
         if (t == 0) tot[k] = total;
       }
       __syncthreads();
-      if (warp < ELL) {  // the last values, one warp per row
-        const int k = warp;
-        uint32_t key[8], w[16], v8[8];
-        load_key(seeds + 32 * k, key);
-        chacha20_block(key, 512 + lane, P.one, w);
-        const unsigned m = draw8(w, sq, sz, v8);
+      if (tail) {
         int all;
         const int p = tot[k] + scan_warp(__popc(m), all);
         put_draws(AH + k * N, p, m, v8);
