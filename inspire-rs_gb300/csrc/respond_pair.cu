@@ -24,7 +24,7 @@
 // coefficients, R_i).
 //
 // What bounds it: latency; a CTA's 312 K warp instructions issue at 1.6 per cycle
-// and SM.  A batch of 8 takes 88 us; the kernel before it (768 threads per
+// and SM.  A batch of 8 takes 86.5 us; the kernel before it (768 threads per
 // CTA, every product's exchange through shared memory, three CTA-wide and one
 // cluster barrier a step) took 111 us, and this one with 256 threads per CTA
 // and 16 values a thread 111 us too (a lone warp issues an instruction every
