@@ -289,7 +289,10 @@ int inspire_respond_seeded(inspire_ctx *ctx, const inspire_db *db, const inspire
 
 /* Batched respond_seeded (combined ciphertexts only), host buffers laid out
  * as for inspire_respond_seeded_batch: shard_ids[n], seeds[n][2*gadget_len][32],
- * b_rows[n][2*gadget_len][poly], out_ct[n][2][poly]. */
+ * b_rows[n][2*gadget_len][poly], out_ct[n][2][poly].  When both are
+ * page-locked, b_rows 16-byte and out_ct 8-byte aligned, and do not overlap,
+ * the GPU reads the rows and writes the responses in place; otherwise they are
+ * staged. */
 int inspire_respond_seeded_nopacking_batch(inspire_ctx *ctx, const inspire_db *db, uint32_t n,
                                            const uint32_t *shard_ids, const uint8_t *seeds, const uint64_t *b_rows,
                                            uint64_t *out_ct);
@@ -299,9 +302,9 @@ int inspire_respond_seeded_nopacking_batch(inspire_ctx *ctx, const inspire_db *d
  * b_rows[n][2*gadget_len][poly], client_ids[n], out_ct[n][2][poly].  Queries
  * may name different shards.  Each result is the one respond_seeded_inspiring
  * returns for that query alone.  When b_rows and out_ct are page-locked
- * (inspire_pinned_alloc, cudaHostAlloc or cudaHostRegister memory) and
- * 16-byte aligned, the GPU reads the rows and writes the responses in place
- * (no staging copies); other memory is staged through device buffers. */
+ * (inspire_pinned_alloc, cudaHostAlloc or cudaHostRegister memory), 16-byte
+ * aligned and do not overlap, the GPU reads the rows and writes the responses
+ * in place (no staging copies); otherwise they are staged. */
 int inspire_respond_seeded_batch(inspire_ctx *ctx, const inspire_db *db, uint32_t n, const uint32_t *shard_ids,
                                  const uint8_t *seeds, const uint64_t *b_rows, const int32_t *client_ids,
                                  uint64_t *out_ct);

@@ -325,11 +325,13 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   if (n == 0) return INSPIRE_OK;
   const size_t pw = poly_words();
   if (seeds) {
-    // page-locked rows and responses (16-byte aligned): read and written in place
+    // page-locked rows and responses (16-byte aligned, apart): read and written
+    // in place
     const size_t row_bytes = sizeof(uint64_t) * stride_polys * pw;
     const size_t rows_span = row_bytes * (n - 1) + sizeof(uint64_t) * ELL * pw;
     const size_t out_span = sizeof(uint64_t) * n * 2 * pw;
-    const uint8_t* d_rows = ((uintptr_t)b_rows % 16 == 0 && row_bytes % 16 == 0 && (uintptr_t)out_ct % 16 == 0)
+    const uint8_t* d_rows = rows_and_out_in_place(b_rows, rows_span, out_ct, out_span) && row_bytes % 16 == 0 &&
+                                    aligned(out_ct, 16)
                                 ? mapped_range(b_rows, rows_span)
                                 : nullptr;
     const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
@@ -471,15 +473,15 @@ int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32
   const size_t col_words = (size_t)db->gamma * 2 * pw;
   if (seeds && !out_columns) {
     // Combined ciphertexts of seeded queries whose rows and responses are
-    // page-locked: the kernel reads the rows and writes the responses in
-    // place.  Small batches in other memory are gathered into page-locked
-    // memory first (as in run_batch).  Shards, seeds and status words go
-    // through page-locked memory either way.
+    // page-locked, aligned and apart: the kernel reads the rows and writes the
+    // responses in place.  Small batches in other memory are gathered into
+    // page-locked memory first (as in run_batch).  Shards, seeds and status
+    // words go through page-locked memory either way.
     const size_t out_span = sizeof(uint64_t) * n * 2 * pw;
     const size_t rows_b = sizeof(uint64_t) * ELL * pw;
-    const uint8_t* d_rows = (uintptr_t)b_rows % 16 == 0  // (the rows are bulk-copied)
-                                ? mapped_range(b_rows, sizeof(uint64_t) * stride_polys * pw * (n - 1) + rows_b)
-                                : nullptr;
+    const size_t rows_span = sizeof(uint64_t) * stride_polys * pw * (n - 1) + rows_b;
+    const uint8_t* d_rows =
+        rows_and_out_in_place(b_rows, rows_span, out_ct, out_span) ? mapped_range(b_rows, rows_span) : nullptr;
     const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
     const bool in_place = d_rows && d_outp;
     if (in_place || n <= STAGE_PINNED_MAX) {
@@ -544,8 +546,9 @@ int run_tree(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* s
   if (n == 0) return INSPIRE_OK;
   const bool seeded = seeds != nullptr;
   const size_t rows_b = sizeof(uint64_t) * ELL * pw;
-  // page-locked rows and outputs are read and written in place; other rows
-  // are copied to the device, other outputs from it
+  // page-locked rows and outputs are read and written in place (the outputs by
+  // the last launch, when every row has been read: they may lie over the rows);
+  // other rows are copied to the device, other outputs from it
   const bool aligned = ((uintptr_t)b_rows | (uintptr_t)out_a | (uintptr_t)out_b) % sizeof(uint64_t) == 0;
   const uint8_t* d_rows = seeded && aligned
                               ? mapped_range(b_rows, sizeof(uint64_t) * stride_polys * pw * (n - 1) + rows_b)

@@ -13,6 +13,7 @@
 #include "inspire_gpu.h"
 #include "kernels.h"
 #include "ledger.h"
+#include "ranges.h"
 
 namespace ighost {
 

@@ -452,7 +452,8 @@ def respond_seeded_packed_batch(crs: ServerCrs, encoded_db: EncodedDatabase, sha
 def respond_seeded_nopacking_batch(crs: ServerCrs, encoded_db: EncodedDatabase, shard_ids: Sequence[int],
                                    seeds: np.ndarray, b_rows: np.ndarray, out: np.ndarray = None) -> np.ndarray:
     """Batched respond_seeded: (n, 2, plen) combined ciphertexts, into `out`
-    when given (page-locked arrays copy faster)."""
+    when given.  Page-locked b_rows and out that do not overlap are read and
+    written in place."""
     n = len(shard_ids)
     plen = crs.params.plen
     sid = np.ascontiguousarray(shard_ids, dtype=np.uint32)
