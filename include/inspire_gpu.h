@@ -107,6 +107,12 @@ int inspire_ctx_device_memory(inspire_ctx *ctx, uint64_t *used, uint64_t *budget
 int inspire_ctx_set_pair_threshold(inspire_ctx *ctx, uint32_t max_queries);
 uint32_t inspire_ctx_pair_threshold(const inspire_ctx *ctx);
 
+/* Bound, in wait iterations, of the waits for a query's rows in the kernels
+ * that host-buffer calls launch (default 2^20, the serving loop's
+ * stage_wait_iters; 0 gives up at once).  When it runs out the call fails with
+ * INSPIRE_ERR_DEVICE_STATUS and the context stays usable. */
+int inspire_ctx_set_row_wait_iters(inspire_ctx *ctx, uint32_t iters);
+
 /* Load the InspiRING part of ServerCrs (src/pir/setup.rs:52-87): the shared
  * seed `inspiring_w_seed` and `inspiring_num_columns` (gamma).  Builds the
  * rotated w_mask table of OfflinePackingKeys::generate

@@ -274,7 +274,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.what = c->what3.as<uint32_t>();
   a.qdesc = c->h_desc.dev<QueryDesc>();
   a.arows = d_arows;
-  a.stage_wait_iters = STAGE_WAIT_ITERS_DEFAULT;
+  a.stage_wait_iters = c->row_wait_iters;
   a.after_keys = new_keys;
   a.alone_max = alone_limit(c, c->stream);
   CUDA_TRY(launch_respond(a, seeds != nullptr, c->stream, 0, c->pair_max.load()));
@@ -436,6 +436,7 @@ int enqueue_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const ui
   a.P = c->P;
   a.nq = (int)n;
   a.col_groups = column_groups(c, db, n, columns);
+  a.row_wait_iters = c->row_wait_iters;
   a.shard = c->d_shard.as<uint32_t>();
   a.seeds = seeded ? c->d_seeds.as<uint8_t>() : nullptr;
   a.arows = seeded ? nullptr : c->d_arows.as<uint64_t>();
@@ -504,6 +505,7 @@ int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32
       a.P = c->P;
       a.nq = (int)n;
       a.col_groups = 1;
+      a.row_wait_iters = c->row_wait_iters;
       a.shard = reinterpret_cast<const uint32_t*>(db_);
       a.seeds = db_ + sizeof(uint32_t) * n;
       a.brows = reinterpret_cast<const uint64_t*>(in_place ? d_rows : db_ + rows_at);
@@ -956,6 +958,13 @@ int inspire_ctx_set_pair_threshold(inspire_ctx* c, uint32_t max_queries) {
   if (max_queries > (1u << 30)) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "max_queries out of range");
   std::lock_guard<std::mutex> lk(c->mu);
   c->pair_max.store((int)max_queries);
+  return INSPIRE_OK;
+}
+
+int inspire_ctx_set_row_wait_iters(inspire_ctx* c, uint32_t iters) {
+  if (!c) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->row_wait_iters = iters;
   return INSPIRE_OK;
 }
 

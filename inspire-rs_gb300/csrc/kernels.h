@@ -63,7 +63,7 @@ struct RespondArgs {
   // client, seeds, brows, E/H/nshards, out and status; rows are read from and
   // responses written to the pinned host memory they point at), or null.
   const struct QueryDesc* qdesc;
-  // Serving loop: bound of the wait for a query's staged rows, in wait
+  // With descriptors: bound of the wait for a query's staged rows, in wait
   // iterations (0: give up at once)
   uint32_t stage_wait_iters;
   // Host only: the stream's last launch builds a key table of this launch; the
@@ -95,6 +95,9 @@ struct NoPackingArgs {
   // (1: one CTA per query).  Above 1, out_columns is required and the
   // combined ciphertexts are summed from the columns by a second launch.
   int col_groups;
+  // Combined ciphertexts: bound of the waits for a query's staged rows, in wait
+  // iterations (0: give up at once)
+  uint32_t row_wait_iters;
 };
 
 // Seeded query generation (client side): query first_query + i asks for

@@ -187,7 +187,7 @@ struct SumSmem {
   static constexpr int XD = AH + ELL * 2 * N;    // [2 r][ELL][N] the digit sums' exchange buffers, then transforms
   static constexpr int DIG = XD + 2 * ELL * N;   // [ELL][N] digit sums; then XB [2 r][N], the b rows' exchange buffers
   static constexpr int ROWS = DIG + ELL * N;     // [ELL][2][N] u64, the staged b rows
-  static constexpr int WS = ROWS + 2 * ELL * 2 * N;  // expansion's workspace
+  static constexpr int WS = ROWS + 2 * ELL * 2 * N;  // expansion's workspace, [24] chunks issued
   static constexpr int SEED = WS + 32;           // [ELL * 8] staged seeds
   static constexpr int BARS = SEED + 24;         // [ELL][ROW_CHUNKS] mbarriers
   static constexpr int TOTAL = BARS + 2 * ELL * 8;
@@ -245,11 +245,14 @@ __global__ void __launch_bounds__(ST + 32, 1) nopacking_sum_kernel(const __grid_
     // once from 128 SMs held the other groups up for 50 us.
     if (tid == ST) {
       const uint64_t* src = A.brows + (size_t)qi * A.brow_stride;
-      for (int k = 0; k < ELL * ROW_CHUNKS && arrived; k++) {
-        if (k >= 2) arrived = mbar_wait(bars + k - 2, 0, STAGE_WAIT_ITERS_DEFAULT);
+      int k = 0;
+      for (; k < ELL * ROW_CHUNKS; k++) {
+        if (k >= 2) arrived = mbar_wait(bars + k - 2, 0, A.row_wait_iters);
+        if (!arrived) break;
         mbar_expect_tx(bars + k, sizeof(uint64_t) * CHUNK);
         bulk_g2s(rows + (size_t)k * CHUNK, src + (size_t)k * CHUNK, sizeof(uint64_t) * CHUNK, bars + k);
       }
+      ws[24] = k;
     }
   } else if (s == 0) {
     if (SEEDED) {
@@ -321,7 +324,7 @@ __global__ void __launch_bounds__(ST + 32, 1) nopacking_sum_kernel(const __grid_
 #pragma unroll 1
     for (int t = 0; t < ELL; t++) {
       for (int k = 0; k < ROW_CHUNKS; k++)
-        if (arrived) arrived = mbar_wait(bars + t * ROW_CHUNKS + k, 0, STAGE_WAIT_ITERS_DEFAULT);
+        if (arrived) arrived = mbar_wait(bars + t * ROW_CHUNKS + k, 0, A.row_wait_iters);
       const uint32_t* row = reinterpret_cast<const uint32_t*>(rows + ((size_t)t * 2 + r) * N);
 #pragma unroll
       for (int j = 0; j < 16; j++) v[0][j] = row[2 * (x + 128 * j)];
@@ -349,8 +352,8 @@ __global__ void __launch_bounds__(ST + 32, 1) nopacking_sum_kernel(const __grid_
   // status, after another bounded wait for the copies still in flight
   const int late = __syncthreads_or(s != 0 && !arrived), bad = __syncthreads_or(s == 0 && !arrived);
   if (late) {
-    bool here = true;  // the producer issues at most the chunk after next beyond the last one that came
-    for (int k = 0; k < ELL * ROW_CHUNKS && here; k++) here = mbar_wait(bars + k, 0, STAGE_DRAIN_ITERS);
+    bool here = true;  // (the chunks after those issued never come)
+    for (int k = 0; k < ws[24] && here; k++) here = mbar_wait(bars + k, 0, STAGE_DRAIN_ITERS);
     const int lost = __syncthreads_or(!here);
     if (tid == 0) A.status[qi] = lost ? ERR_STAGE_LOST : ERR_STAGE;
   } else if (tid == 0) {
