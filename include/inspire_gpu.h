@@ -112,6 +112,11 @@ uint32_t inspire_ctx_pair_threshold(const inspire_ctx *ctx);
  * stage_wait_iters; 0 gives up at once).  When it runs out the call fails with
  * INSPIRE_ERR_DEVICE_STATUS and the context stays usable. */
 int inspire_ctx_set_row_wait_iters(inspire_ctx *ctx, uint32_t iters);
+/* The same for the waits of a query's two CTAs for each other's coefficients,
+ * in every later launch of the cluster kernel: host-buffer calls and served
+ * queries fail with INSPIRE_ERR_DEVICE_STATUS, device batches report a
+ * nonzero d_status. */
+int inspire_ctx_set_peer_wait_iters(inspire_ctx *ctx, uint32_t iters);
 
 /* Load the InspiRING part of ServerCrs (src/pir/setup.rs:52-87): the shared
  * seed `inspiring_w_seed` and `inspiring_num_columns` (gamma).  Builds the

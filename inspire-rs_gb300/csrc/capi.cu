@@ -272,6 +272,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.yhat_table = c->client_table.as<const uint32_t*>();
   a.nclients = (int)c->client_ptrs.size();
   a.what = c->what3.as<uint32_t>();
+  a.peer_wait_iters = c->peer_wait_iters;
   a.qdesc = c->h_desc.dev<QueryDesc>();
   a.arows = d_arows;
   a.stage_wait_iters = c->row_wait_iters;
@@ -378,6 +379,7 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   a.E = db->E.as<uint32_t>();
   a.H = db->H.as<uint16_t>();
   a.what = c->what3.as<uint32_t>();
+  a.peer_wait_iters = c->peer_wait_iters;
   a.out = c->d_out.as<uint64_t>();
   int32_t* hs = c->h_qstatus.host<int32_t>();
   for (uint32_t i = 0; i < n; i++) hs[i] = -1;
@@ -968,6 +970,13 @@ int inspire_ctx_set_row_wait_iters(inspire_ctx* c, uint32_t iters) {
   return INSPIRE_OK;
 }
 
+int inspire_ctx_set_peer_wait_iters(inspire_ctx* c, uint32_t iters) {
+  if (!c) return fail(INSPIRE_ERR_INVALID_ARGUMENT, "null argument");
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->peer_wait_iters = iters;
+  return INSPIRE_OK;
+}
+
 uint32_t inspire_ctx_pair_threshold(const inspire_ctx* c) { return c ? (uint32_t)c->pair_max.load() : 0; }
 
 int inspire_ctx_device_memory(inspire_ctx* c, uint64_t* used, uint64_t* budget) {
@@ -1245,6 +1254,7 @@ int inspire_respond_seeded_batch_device_grid(inspire_ctx* c, const inspire_db* d
   a.E = db->E.as<uint32_t>();
   a.H = db->H.as<uint16_t>();
   a.what = c->what3.as<uint32_t>();
+  a.peer_wait_iters = c->peer_wait_iters;
   a.out = d_out_ct;
   a.status = d_status;
   const int pair_max = c->pair_max.load();

@@ -131,6 +131,7 @@ struct inspire_ctx {
   // (one SM per CRT residue; lower latency while the SMs are not all busy)
   std::atomic<int> pair_max{0};  // read by serving dispatchers without the lock
   uint32_t row_wait_iters = ig::STAGE_WAIT_ITERS_DEFAULT;  // of host-buffer calls whose kernels stage rows
+  uint32_t peer_wait_iters = ig::STAGE_WAIT_ITERS_DEFAULT;
   inspire_params params{};
   uint64_t q = 0;  // composite modulus
   ig::DevParams P{};

@@ -16,6 +16,9 @@ constexpr int ERR_STAGE = 3;   // the query's rows did not arrive in shared memo
 // the late copies in its shared memory)
 constexpr int ERR_STAGE_LOST = 4;
 constexpr int ERR_PEER = 5;    // the other CTA's coefficients did not come within the wait bound (two-CTA kernel)
+constexpr int ERR_PEER_LOST = 6;  // ... nor within the drain wait: as ERR_STAGE_LOST
+// Whether a query's status makes every result of its launch unreliable.
+inline bool launch_lost(int status) { return status == ERR_STAGE_LOST || status == ERR_PEER_LOST; }
 constexpr uint32_t STAGE_WAIT_ITERS_DEFAULT = 1u << 20;
 constexpr uint32_t STAGE_DRAIN_ITERS = 1u << 22;
 
@@ -66,6 +69,9 @@ struct RespondArgs {
   // With descriptors: bound of the wait for a query's staged rows, in wait
   // iterations (0: give up at once)
   uint32_t stage_wait_iters;
+  // Two-CTA kernel: bound of the wait for the other CTA's coefficients of a
+  // step, in wait iterations (0: give up at once)
+  uint32_t peer_wait_iters = STAGE_WAIT_ITERS_DEFAULT;
   // Host only: the stream's last launch builds a key table of this launch; the
   // two-CTA kernel may be set up meanwhile
   bool after_keys;

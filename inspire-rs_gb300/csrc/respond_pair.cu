@@ -88,6 +88,34 @@ __device__ __forceinline__ bool mbar_wait_peer(uint64_t* bar, uint32_t parity, u
   return false;
 }
 
+// Thread 0, which stopped waiting for the peer's coefficients at step `late`:
+// waits, with an iteration bound, until those of that and all later steps have
+// come.  The mbarriers' phases of steps late and late - 1 are armed; the steps
+// after them, which it has not armed, are one more phase each.  What came for
+// these before they are announced here counts towards whichever phase is
+// current, so the phases' order, not their split by step, is what is waited
+// for.  (test_wait: the bound is a bound in time, about 0.1 s.)
+__device__ __noinline__ bool drain_peer(uint64_t* cbar, int late, int gamma) {
+  for (int s = late; s >= 0 && s >= late - 1; s--) {
+    uint64_t* bar = cbar + (s & 1);
+    uint32_t phase = ((gamma - 2 - s) >> 1) & 1;
+    for (int more = s >> 1;; more = 0, phase ^= 1) {
+      uint32_t done = 0;
+      for (uint32_t it = 0; !done && it < STAGE_DRAIN_ITERS; it++)
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n "
+            "selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(smem_u32(bar)), "r"(phase)
+            : "memory");
+      if (!done) return false;
+      if (!more) break;
+      mbar_expect_tx(bar, 4 * N * more);
+    }
+  }
+  return true;
+}
+
 // Shared-memory layout in u32 words.
 struct PairSmem {
   static constexpr int AH = 0;              // [ELL][16 rows h][128] row transforms of the a-side residue (ah_word)
@@ -103,7 +131,8 @@ struct PairSmem {
   static constexpr int OK = TOT + 4;        // [4] rows complete
   static constexpr int BP = OK + 4;         // [16] the b side
   static constexpr int SEED = BP + 16;      // [ELL * 8] staged seeds (serving loop)
-  static constexpr int MISC = SEED + 24;    // [4] residue 1's stream positions, [2] flags, [2] drain results by rank
+  static constexpr int MISC = SEED + 24;    // [3] residue 1's stream positions, [1] the last step whose wait thread 0
+                                            // ended, [2] flags, [2] drain results by rank, or CTA 1's outcome in [6]
   static constexpr int BARS = MISC + 8;     // mbarriers: the staged rows', then the peer's coefficients' [2 parity]
   static constexpr int TOTAL = BARS + 8;
 };
@@ -223,6 +252,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
     for (int k = 0; k < 3; k++) mbar_init(rbar + k);
     mbar_expect_tx(cbar, 4 * N);
     mbar_expect_tx(cbar + 1, 4 * N);
+    misc[3] = gamma - 1;
+    misc[6] = 0;
     prefetch_l2(H, sizeof(uint16_t) * (size_t)gamma * N);
     // the contracted shard's blocks of the first three steps (the rest are
     // prefetched two steps ahead of their use in the recursion)
@@ -504,7 +535,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
       named_sync(4, PT);
       jt_load_ru(c, ocb, t);
     }
-    if (arrived) arrived = mbar_wait_peer(cbar + par, ((gamma - 2 - i) >> 1) & 1, STAGE_WAIT_ITERS_DEFAULT);
+    if (arrived) arrived = mbar_wait_peer(cbar + par, ((gamma - 2 - i) >> 1) & 1, A.peer_wait_iters);
     jt_load_ru(o, rc, t);
     // [B] this team's digit of the composite coefficients
     //     (gadget_decompose, rgsw/external_product.rs:16-37)
@@ -543,8 +574,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
         jt_store_ru(R, rnb, t);
         named_arrive(5, PT);
       }
-      // both teams have read the peer's coefficients: its next but one step's may come
-      if (t == 0 && i >= 2) mbar_expect_tx(cbar + par, 4 * N);
+      // both teams have read the peer's coefficients: its next but one step's may
+      // come (not announced in a phase that has not ended)
+      if (t == 0 && arrived) {
+        if (i >= 2) mbar_expect_tx(cbar + par, 4 * N);
+        misc[3] = i;
+      }
     }
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[j] = csub(acc[j] + redc_wide(smul(v[j], yv[j]), q, qinv) + q, 8 * q);
@@ -570,13 +605,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
 #pragma unroll
   for (int j = 0; j < 8; j++) out[team * 2 * N + t + TEAM * j] = f[j];
 
-  // Neither CTA exits before the other has sent all its coefficients.  If some
-  // did not come within the wait's bound, the response is wrong and says so;
-  // the last ones get another bounded wait before the CTA's memory is freed.
-  const int lost = __syncthreads_or(!arrived);
-  if (lost && tid == 0) *status_ptr() = ERR_PEER;
+  // Some of the peer's coefficients did not come within the wait's bound: the
+  // response is wrong and says so.  The CTA's memory is not freed while they may
+  // still come; if another bounded wait for them runs out too, ERR_PEER_LOST
+  // tells the host to drop every result of this launch.  (Where thread 0 saw
+  // every step arrive, nothing is in flight.)
+  int outcome = __syncthreads_or(!arrived) ? ERR_PEER : 0;
+  if (tid == 0) {
+    if (!arrived && !drain_peer(cbar, misc[3] - 1, gamma)) outcome = ERR_PEER_LOST;
+    if (r == 1 && outcome) st_peer(peer_smem(misc + 6, peer), (uint32_t)outcome);
+  }
   cluster_sync_all();
-  if (lost) mbar_wait_peer(cbar, ((gamma - 2) >> 1) & 1, STAGE_WAIT_ITERS_DEFAULT);
+  if (r == 0 && tid == 0) {
+    outcome = max(outcome, misc[6]);
+    if (outcome) *status_ptr() = outcome;
+  }
 }
 
 template <int MODE, bool SEEDED, bool QDB>

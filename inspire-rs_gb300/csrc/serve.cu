@@ -209,6 +209,7 @@ int inspire_server::launch(Slot& s, const std::vector<int>& batch) {
   a.what = ctx->what3.as<uint32_t>();
   a.qdesc = s.ddesc.as<QueryDesc>();
   a.stage_wait_iters = cfg.stage_wait_iters;
+  a.peer_wait_iters = ctx->peer_wait_iters;
   CUDA_TRY(launch_respond(a, true, s.st, 0, s.pair ? n : 0));
   CUDA_TRY(cudaEventRecord(s.ev, s.st));
   return INSPIRE_OK;
@@ -245,10 +246,10 @@ void inspire_server::run() {
       for (size_t k = 0; k < finished.size(); k++) {
         Slot& s = *finished[k];
         const cudaError_t e = fin_err[k];
-        // one query whose staged rows were still in flight when its CTA
-        // exited makes every result of the launch unreliable
+        // one query whose staged rows or coefficients were still in flight when
+        // its CTA exited makes every result of the launch unreliable
         bool lost = false;
-        for (int v : status[k]) lost |= v == ERR_STAGE_LOST;
+        for (int v : status[k]) lost |= launch_lost(v);
         for (size_t j = 0; j < s.recs.size(); j++) {
           Rec& r = recs[s.recs[j]];
           r.batch_lost = lost;
@@ -646,7 +647,7 @@ int inspire_server_poll(inspire_server* s, uint64_t ticket, uint64_t* out_ct, in
   lk.unlock();
   if (cuda_error) return fail(INSPIRE_ERR_CUDA, werr.empty() ? "serving batch failed" : werr);
   if (batch_lost)
-    return fail(INSPIRE_ERR_DEVICE_STATUS, "batch dropped: a query's rows were still being copied when its "
+    return fail(INSPIRE_ERR_DEVICE_STATUS, "batch dropped: copies of a query were still in flight when its "
                                            "Respond CTA gave up waiting (ticket " + std::to_string(ticket) + ")");
   if (kstatus == ERR_STAGE)
     return fail(INSPIRE_ERR_DEVICE_STATUS, "query rows did not reach the GPU within stage_wait_iters (ticket " +

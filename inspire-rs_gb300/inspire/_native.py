@@ -195,6 +195,7 @@ def load(path: str = LIB_PATH):
         "inspire_ctx_set_pair_threshold": (C.c_int, [vp, u32]),
         "inspire_ctx_pair_threshold": (u32, [vp]),
         "inspire_ctx_set_row_wait_iters": (C.c_int, [vp, u32]),
+        "inspire_ctx_set_peer_wait_iters": (C.c_int, [vp, u32]),
         "inspire_http_config_default": (None, [C.POINTER(HttpConfigC)]),
         "inspire_http_start": (C.c_int, [vp, vp, vp, C.POINTER(HttpConfigC), C.c_char_p, C.c_size_t,
                                          C.POINTER(vp)]),
