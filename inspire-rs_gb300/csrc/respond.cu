@@ -71,6 +71,8 @@ struct Smem {
   static constexpr int SEED = BP + 32;         // [ELL * 8] staged seeds (serving loop)
   static constexpr int BAR = SEED + 24;        // the staged rows' mbarrier
   static constexpr int TOTAL = BAR + 8;
+  // (the transforms' swizzled accesses XOR address bits 2-6)
+  static_assert(AH * 4 % 128 == 0 && XC * 4 % 128 == 0 && BAR % 2 == 0, "alignment of rows, buffers and mbarrier");
 };
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
@@ -80,7 +82,7 @@ template <int MODE, bool SEEDED, bool QDB, bool ALONE>
 __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) {
   constexpr int NR = MODE == MODE_COMPAT ? 1 : 2;
   using L = Smem<NR>;
-  extern __shared__ __align__(16) uint32_t smem[];
+  extern __shared__ __align__(128) uint32_t smem[];
   uint32_t* AH = smem + L::AH;
   uint32_t* XC = smem + L::XC;
   int* ws = reinterpret_cast<int*>(smem + L::WS);
