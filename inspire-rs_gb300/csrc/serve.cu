@@ -18,12 +18,14 @@
 #include <condition_variable>
 #include <cstring>
 #include <deque>
+#include <exception>
 #include <map>
 #include <memory>
 #include <thread>
 
 #include <cuda.h>
 
+#include "copy_helpers.h"
 #include "host.h"
 #include "serve_policy.h"
 
@@ -63,88 +65,6 @@ struct Rec {
   int cuda_error = 0;  // nonzero: the batch failed on the host side
   int kstatus = 0;     // the kernel's status word
   bool batch_lost = false;  // a CTA of the query's batch exited with copies in flight
-};
-
-// Threads that share the copies of finished responses out of the pool with the
-// caller that collects them.  One core copies about 15 GB/s of what the GPU has
-// just written; a burst's responses (64 KiB each) leave the GPU at 100.  With 8
-// helpers a burst of 601 queries, collected by 4 threads, takes 840 us
-// against 1420 with the callers' own copies.
-class CopyHelpers {
- public:
-  // Below this many copies the caller is done before a helper has woken.
-  static constexpr size_t MIN_COPIES = 8;
-  struct Copy {
-    void* to;
-    const void* from;
-  };
-
-  void start(unsigned n) {
-    for (unsigned i = 0; i < n; i++) threads_.emplace_back([this] { work(); });
-  }
-  ~CopyHelpers() {
-    {
-      std::lock_guard<std::mutex> lk(mu_);
-      stop_ = true;
-    }
-    cv_.notify_all();
-    for (std::thread& t : threads_) t.join();
-  }
-  // Every copy of `bytes` bytes, finished on return.
-  void run(std::vector<Copy> copies, size_t bytes) {
-    auto job = std::make_shared<Job>();
-    job->copies = std::move(copies);
-    job->bytes = bytes;
-    const bool share = !threads_.empty() && job->copies.size() >= MIN_COPIES;
-    if (share) {
-      {
-        std::lock_guard<std::mutex> lk(mu_);
-        jobs_.push_back(job);
-      }
-      cv_.notify_all();
-    }
-    job->take();
-    if (share) {
-      retire(job);
-      while (job->done.load(std::memory_order_acquire) < job->copies.size()) std::this_thread::yield();
-    }
-  }
-
- private:
-  struct Job {
-    std::vector<Copy> copies;
-    size_t bytes = 0;
-    std::atomic<size_t> next{0}, done{0};
-    void take() {
-      for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < copies.size();) {
-        memcpy(copies[i].to, copies[i].from, bytes);
-        done.fetch_add(1, std::memory_order_release);
-      }
-    }
-  };
-  void retire(const std::shared_ptr<Job>& job) {  // every copy has been taken
-    std::lock_guard<std::mutex> lk(mu_);
-    const auto it = std::find(jobs_.begin(), jobs_.end(), job);
-    if (it != jobs_.end()) jobs_.erase(it);
-  }
-  void work() {
-    for (;;) {
-      std::shared_ptr<Job> job;
-      {
-        std::unique_lock<std::mutex> lk(mu_);
-        cv_.wait(lk, [&] { return stop_ || !jobs_.empty(); });
-        if (jobs_.empty()) return;
-        job = jobs_.front();
-      }
-      job->take();
-      retire(job);
-    }
-  }
-  std::mutex mu_;
-  std::condition_variable cv_;
-  std::deque<std::shared_ptr<Job>> jobs_;
-  std::vector<std::thread> threads_;
-  bool stop_ = false;
 };
 
 struct Slot {
@@ -463,7 +383,11 @@ int inspire_server_create(inspire_ctx* c, const inspire_server_config* cfg, insp
       return bail(fail(INSPIRE_ERR_OUT_OF_MEMORY, alloc_failure(c, "serving slot buffers")));
   }
   s->helpers.start(std::min({8u, std::thread::hardware_concurrency() / 2, cfg->capacity / (unsigned)CopyHelpers::MIN_COPIES}));
-  s->worker = std::thread([s] { s->run(); });
+  try {
+    s->worker = std::thread([s] { s->run(); });
+  } catch (const std::exception& ex) {
+    return bail(fail(INSPIRE_ERR_OUT_OF_MEMORY, std::string("serving dispatcher thread: ") + ex.what()));
+  }
   *out = s;
   return INSPIRE_OK;
 }
@@ -665,11 +589,17 @@ int inspire_server_poll_batch(inspire_server* s, uint32_t n, const uint64_t* tic
   const int64_t deadline = timeout_us < 0 ? INT64_MAX : now_ns() + (int64_t)timeout_us * 1000;
   const size_t pw = poly_words();
   std::vector<CopyHelpers::Copy> copies;
+  bool claim = true;  // (without memory for the list: one ticket after the other)
+  try {
+    copies.reserve(std::min<size_t>(n, s->recs.size()));
+  } catch (const std::exception&) {
+    claim = false;
+  }
   for (uint32_t k = 0; k < n; k++) {
     // the tickets from here on that are done and sound, all at once
     const uint32_t k0 = k;
     copies.clear();
-    {
+    if (claim) {
       std::lock_guard<std::mutex> lk(s->mu);
       for (; k < n; k++) {
         const uint64_t idx = tickets[k] & ((1ull << TICKET_IDX_BITS) - 1);
@@ -683,7 +613,7 @@ int inspire_server_poll_batch(inspire_server* s, uint32_t n, const uint64_t* tic
       }
     }
     if (k > k0) {
-      s->helpers.run(std::move(copies), sizeof(uint64_t) * 4 * N);
+      s->helpers.run(copies, sizeof(uint64_t) * 4 * N);
       std::lock_guard<std::mutex> lk(s->mu);
       for (uint32_t j = k0; j < k; j++) {
         const uint64_t idx = tickets[j] & ((1ull << TICKET_IDX_BITS) - 1);
