@@ -215,23 +215,30 @@ void release_keys(inspire_ctx* c, int32_t id) {
 
 int finish_status(inspire_ctx* c, uint32_t n, const char* what);
 
-// Queries up to which a batch on `st` may take the Respond kernel's form that has
-// an SM to itself: the SM count, or none while the last device batch, on another
-// stream, still runs (batches that overlap do better two CTAs to an SM: 2048
-// queries take 1356 us so, 1570 one to an SM) or when captured into a graph, whose
-// launches may overlap.
-int alone_limit(inspire_ctx* c, cudaStream_t st) {
+bool capturing(cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-  if (cap != cudaStreamCaptureStatusNone) return 0;
-  if (!c->batch_stream_set || c->batch_stream == st) return c->sm_count;
-  // (relaxed: the query must not end another thread's capture)
-  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  const bool running = cudaEventQuery(c->batch_ev) == cudaErrorNotReady;
-  cudaThreadExchangeStreamCaptureMode(&mode);
-  if (running) cudaGetLastError();
-  return running ? 0 : c->sm_count;
+  return cap != cudaStreamCaptureStatusNone;
+}
+
+// Queries up to which a batch on `st` may take the Respond kernel's form that has
+// an SM to itself (batch_policy.h).
+int alone_limit(inspire_ctx* c, cudaStream_t st) {
+  unsigned long long id = 0;
+  const bool captured = capturing(st);
+  if (!captured && cudaStreamGetId(st, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return ighost::alone_limit(c->sm_count, captured, c->last_batch, id, [&] {
+    // (relaxed: the query must not end another thread's capture)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool running = cudaEventQuery(c->batch_ev) == cudaErrorNotReady;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (running) cudaGetLastError();
+    return !running;
+  });
 }
 
 // Batches up to this size stage their inputs through page-locked memory.
@@ -1261,12 +1268,11 @@ int inspire_respond_seeded_batch_device_grid(inspire_ctx* c, const inspire_db* d
   const bool large = (int)n > pair_max && (int)n <= c->sm_count && max_ctas == 0;
   if (large) a.alone_max = alone_limit(c, (cudaStream_t)stream);
   CUDA_TRY(launch_respond(a, true, (cudaStream_t)stream, (int)max_ctas, pair_max));
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (large) CUDA_TRY(cudaStreamIsCapturing((cudaStream_t)stream, &cap));
-  if (large && cap == cudaStreamCaptureStatusNone) {  // for the next batch's choice
+  if (large && !capturing((cudaStream_t)stream)) {  // for the next batch's choice
+    unsigned long long id = 0;
+    CUDA_TRY(cudaStreamGetId((cudaStream_t)stream, &id));
     CUDA_TRY(cudaEventRecord(c->batch_ev, (cudaStream_t)stream));
-    c->batch_stream = (cudaStream_t)stream;
-    c->batch_stream_set = true;
+    c->last_batch = {true, id};
   }
   return INSPIRE_OK;
 }

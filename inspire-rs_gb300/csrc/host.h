@@ -10,6 +10,7 @@
 #include <string>
 #include <vector>
 
+#include "batch_policy.h"
 #include "inspire_gpu.h"
 #include "kernels.h"
 #include "ledger.h"
@@ -165,9 +166,8 @@ struct inspire_ctx {
   ighost::HostPinned h_keys;    // client keys on their way to their table
   ighost::HostPinned h_out;     // responses of staged small batches, written by the kernel
   bool keys_in_flight = false;  // a launch on `stream` may still read h_keys
-  cudaEvent_t batch_ev = nullptr;  // after the last device batch of one query per SM, on batch_stream
-  cudaStream_t batch_stream = nullptr;
-  bool batch_stream_set = false;
+  ighost::LastBatch last_batch;
+  cudaEvent_t batch_ev = nullptr;  // after last_batch
 
   inspire_ctx() {
     for (ighost::DevMem* m : {&tables, &what, &what3, &wmask, &galois, &tree_work, &d_tree_out, &client_table, &d_shard,
