@@ -116,6 +116,17 @@ __device__ __noinline__ bool drain_peer(uint64_t* cbar, int late, int gamma) {
   return true;
 }
 
+// Some of the peer's coefficients did not come within the wait's bound (late: in
+// thread 0, the caller): the response is wrong and says so.  The CTA's memory is
+// not freed while they may still come; if another bounded wait for them runs out
+// too, ERR_PEER_LOST tells the host to drop every result of this launch.  (Where
+// thread 0 saw every step arrive, nothing is in flight.)  CTA 0 writes the status.
+__device__ __noinline__ int peer_missing(uint64_t* cbar, int* misc, int gamma, bool late) {
+  const int outcome = late && !drain_peer(cbar, misc[3] - 1, gamma) ? ERR_PEER_LOST : ERR_PEER;
+  if (cluster_rank() == 1) st_peer(peer_smem(misc + 6, 0), (uint32_t)outcome);
+  return outcome;
+}
+
 // Shared-memory layout in u32 words.
 struct PairSmem {
   static constexpr int AH = 0;              // [ELL][16 rows h][128] row transforms of the a-side residue (ah_word)
@@ -590,7 +601,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
   //      1, this residue's halves of the response ----
   uint64_t* out = (QDB ? reload_ptr(&D->out) : A.out + (size_t)qi * 4 * N) + (size_t)r * N;
   if (team == 0) jt_store_ru(acc, s1b, t);
-  __syncthreads();
+  int outcome = 0;
+  if (__syncthreads_or(!arrived) && tid == 0) outcome = peer_missing(cbar, misc, gamma, !arrived);
+  cluster_arrive();
   uint32_t f[8];
   if (team == 0) {
 #pragma unroll
@@ -605,17 +618,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
 #pragma unroll
   for (int j = 0; j < 8; j++) out[team * 2 * N + t + TEAM * j] = f[j];
 
-  // Some of the peer's coefficients did not come within the wait's bound: the
-  // response is wrong and says so.  The CTA's memory is not freed while they may
-  // still come; if another bounded wait for them runs out too, ERR_PEER_LOST
-  // tells the host to drop every result of this launch.  (Where thread 0 saw
-  // every step arrive, nothing is in flight.)
-  int outcome = __syncthreads_or(!arrived) ? ERR_PEER : 0;
-  if (tid == 0) {
-    if (!arrived && !drain_peer(cbar, misc[3] - 1, gamma)) outcome = ERR_PEER_LOST;
-    if (r == 1 && outcome) st_peer(peer_smem(misc + 6, peer), (uint32_t)outcome);
-  }
-  cluster_sync_all();
+  cluster_wait();
   if (r == 0 && tid == 0) {
     outcome = max(outcome, misc[6]);
     if (outcome) *status_ptr() = outcome;
