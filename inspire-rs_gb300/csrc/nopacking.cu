@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(ST + 32, 1) nopacking_sum_kernel(const __grid_
   uint32_t v[1][16], acc[1][16];
 #pragma unroll
   for (int j = 0; j < 16; j++) acc[0][j] = 0;
+  static_assert(JFWD_OUT * JFWD_OUT <= 3 * 16 * 64 * 64, "q < 2^28: reduced products above -3 q");
   // acc += v times the digit sum t's transform: |v|, |d| < 6.5 q, so products
   // are below 42.3 q^2, reduced below 3.7 q and made positive; acc below 8 q
   auto add_product = [&](int t) {

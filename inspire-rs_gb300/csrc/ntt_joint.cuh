@@ -140,10 +140,27 @@ __device__ __forceinline__ uint32_t jx_lin(int x, int c) {
 //      forward transform); 32-bit signed values allow 8 q = 512 units ----
 constexpr int JB_MAX = 512;
 
-__host__ __device__ constexpr int jb_max(const int (&B)[16]) {
+template <int V>
+__host__ __device__ constexpr int jb_max(const int (&B)[V]) {
   int m = 0;
-  for (int r = 0; r < 16; r++) m = B[r] > m ? B[r] : m;
+  for (int r = 0; r < V; r++) m = B[r] > m ? B[r] : m;
   return m;
+}
+// After an exchange any value may be any register's.
+template <int V>
+__host__ __device__ constexpr void jb_level(int (&B)[V]) {
+  const int m = jb_max(B);
+  for (int r = 0; r < V; r++) B[r] = m;
+}
+// A forward butterfly's bounds, a' = a + (b w mod q), b' = a - (b w mod q);
+// true if a has to be centred first.
+__host__ __device__ constexpr bool jb_fwd(int& a, int& b) {
+  const int grow = 64 + (b + 31) / 32;  // |b w mod q| <= q (1 + |b| / 2^33)
+  const bool c = a + grow > JB_MAX;
+  if (c) a = JB_MAX / 2;
+  a += grow;
+  b = a;
+  return c;
 }
 
 // Forward stage S (element r pairs with r + H, twiddle (1 << S) + first +
@@ -157,11 +174,9 @@ __device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], int (&B)[16], T
 #pragma unroll
   for (int r = 0; r < 16; r++)
     if ((r & H) == 0) {
-      const int grow = 64 + (B[r + H] + 31) / 32;  // |b w mod q| <= q (1 + |b| / 2^33)
-      if (B[r] + grow > JB_MAX) {
+      if (jb_fwd(B[r], B[r + H])) {
 #pragma unroll
         for (int k = 0; k < K; k++) v[k][r] = centre(v[k][r], 4 * q);
-        B[r] = JB_MAX / 2;
       }
       const uint2 w = run[r >> SHIFT];
 #pragma unroll
@@ -172,8 +187,6 @@ __device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], int (&B)[16], T
         v[k][r] = s - h * q;
         v[k][r + H] = twice_minus(a, v[k][r]);
       }
-      B[r] += grow;
-      B[r + H] = B[r];
     }
 }
 
@@ -187,7 +200,42 @@ __device__ __forceinline__ void jfwd_stage(uint32_t (&v)[K][16], int (&B)[16], T
 // for smaller q every bound, an absolute sum of 2^20 and multiples of q, is
 // smaller too.
 constexpr int JB_DIGIT = 1, JB_CANON = 64;
-constexpr int JFWD_OUT = 416;
+constexpr int JFWD_OUT = 416, JFWD_OUT_DIGIT = 336;  // 6.5 q, 5.25 q: what the callers' sums are bounded with
+
+// The bound that the stages below reach: V values per thread, `phases` runs of
+// stages on register bits from the highest down, by their counts of stages and
+// their highest register bits.
+struct JbPhase {
+  int stages, top;
+};
+template <int V, int NP>
+__host__ __device__ constexpr int jfwd_bound(int (&B)[V], const JbPhase (&phases)[NP], int first = 0) {
+  for (int p = 0; p < NP; p++) {
+    if (p) jb_level(B);
+    for (int s = p ? 0 : first; s < phases[p].stages; s++) {
+      const int H = phases[p].top >> s;
+      for (int r = 0; r < V; r++)
+        if ((r & H) == 0) jb_fwd(B[r], B[r + H]);
+    }
+  }
+  return jb_max(B);
+}
+// ... of inputs below b0 q / 64, by 16 values per thread (stages 0-3, 4-7, 8-10)
+__host__ __device__ constexpr int jfwd_out(int b0) {
+  const JbPhase phases[3] = {{4, 8}, {4, 8}, {3, 4}};
+  int B[16] = {};
+  for (int r = 0; r < 16; r++) B[r] = b0;
+  return jfwd_bound(B, phases);
+}
+// ... with stage 0 by multiples of both operands (jntt_fwd_scaled)
+__host__ __device__ constexpr int jfwd_out_scaled() {
+  const JbPhase phases[3] = {{4, 8}, {4, 8}, {3, 4}};
+  int B[16] = {};
+  for (int r = 0; r < 16; r++) B[r] = r < 8 ? 256 : 128;
+  return jfwd_bound(B, phases, 1);
+}
+static_assert(jfwd_out(JB_CANON) <= JFWD_OUT && jfwd_out_scaled() <= JFWD_OUT, "forward outputs of residues");
+static_assert(jfwd_out(JB_DIGIT) <= JFWD_OUT_DIGIT, "forward outputs of digits");
 struct NoHook {
   __device__ __forceinline__ void operator()() const {}
 };
@@ -201,11 +249,7 @@ __device__ __forceinline__ void jntt_fwd_from1(uint32_t (&v)[K][16], int (&B)[16
   jx_store_co<K>(v, sc, x);
   group_sync(bar);
   jx_load_tr<K>(v, sc, x);
-  {
-    const int m = jb_max(B);
-#pragma unroll
-    for (int r = 0; r < 16; r++) B[r] = m;
-  }
+  jb_level(B);
   const int b = x >> 3;
   jfwd_stage<K, 4, 4>(v, B, tw, b, q);
   jfwd_stage<K, 5, 3>(v, B, tw, b << 1, q);
@@ -215,11 +259,7 @@ __device__ __forceinline__ void jntt_fwd_from1(uint32_t (&v)[K][16], int (&B)[16
   __syncwarp();
   jx_load_ru<K>(v, sc, x);
   hook();
-  {
-    const int m = jb_max(B);
-#pragma unroll
-    for (int r = 0; r < 16; r++) B[r] = m;
-  }
+  jb_level(B);
   jfwd_stage<K, 8, 3>(v, B, tw, x << 1, q);
   jfwd_stage<K, 9, 2>(v, B, tw, x << 2, q);
   jfwd_stage<K, 10, 1>(v, B, tw, x << 3, q);
@@ -256,6 +296,7 @@ __device__ __forceinline__ void jntt_fwd_scaled(uint32_t (&v)[K][16], const uint
 }
 
 // A forward output brought to [0, q).
+static_assert(JFWD_OUT <= 8 * 64, "jcanon_fwd");
 __device__ __forceinline__ uint32_t jcanon_fwd(uint32_t x, uint32_t q) {
   x = min(x, x + 8 * q);  // negative values are large as unsigned ones
   return canon16(x, q);

@@ -86,29 +86,24 @@ __device__ __forceinline__ void jt_fwd_stage(uint32_t (&v)[8], int (&B)[8], cons
 #pragma unroll
   for (int r = 0; r < 8; r++)
     if ((r & H) == 0) {
-      const int grow = 64 + (B[r + H] + 31) / 32;
-      if (B[r] + grow > JB_MAX) {
-        v[r] = centre(v[r], 4 * q);
-        B[r] = JB_MAX / 2;
-      }
+      if (jb_fwd(B[r], B[r + H])) v[r] = centre(v[r], 4 * q);
       const uint2 w = run[r >> SH];
       const uint32_t a = v[r], b = v[r + H];
       const uint32_t h = (uint32_t)__mulhi((int)b, (int)w.y);
       const uint32_t s = b * w.x + a;
       v[r] = s - h * q;
       v[r + H] = twice_minus(a, v[r]);
-      B[r] += grow;
-      B[r + H] = B[r];
     }
 }
 
-__device__ __forceinline__ void jt_level(int (&B)[8]) {
-  int m = 0;
-#pragma unroll
-  for (int r = 0; r < 8; r++) m = B[r] > m ? B[r] : m;
-#pragma unroll
-  for (int r = 0; r < 8; r++) B[r] = m;
+// (stages 0-2, 3-5, 6-8, 9 and 10)
+__host__ __device__ constexpr int jt_fwd_out(int b0) {
+  const JbPhase phases[4] = {{3, 4}, {3, 4}, {3, 4}, {2, 2}};
+  int B[8] = {};
+  for (int r = 0; r < 8; r++) B[r] = b0;
+  return jfwd_bound(B, phases);
 }
+static_assert(jt_fwd_out(JB_CANON) <= JFWD_OUT && jt_fwd_out(JB_DIGIT) <= JFWD_OUT_DIGIT, "forward outputs");
 
 // Forward transform; inputs in [0, B0 q / 64), outputs as jntt_fwd's (signed,
 // below JFWD_OUT q / 64).  `hook` runs before the last
@@ -128,7 +123,7 @@ __device__ __forceinline__ void jt_fwd(uint32_t (&v)[8], uint32_t sc, TwiddleRef
   jt_runs(w, tw, 3, t >> 5);
   team_sync(bar);
   jt_load_hi(v, sc, t);
-  jt_level(B);
+  jb_level(B);
   jt_fwd_stage<4, 3, 1>(v, B, w.a, q);
   jt_fwd_stage<2, 2, 2>(v, B, w.b, q);
   jt_fwd_stage<1, 1, 4>(v, B, w.c, q);
@@ -136,7 +131,7 @@ __device__ __forceinline__ void jt_fwd(uint32_t (&v)[8], uint32_t sc, TwiddleRef
   jt_runs(w, tw, 6, t >> 2);
   __syncwarp();
   jt_load_mf(v, sc, t);
-  jt_level(B);
+  jb_level(B);
   jt_fwd_stage<4, 3, 1>(v, B, w.a, q);
   jt_fwd_stage<2, 2, 2>(v, B, w.b, q);
   jt_fwd_stage<1, 1, 4>(v, B, w.c, q);
@@ -146,7 +141,7 @@ __device__ __forceinline__ void jt_fwd(uint32_t (&v)[8], uint32_t sc, TwiddleRef
   __syncwarp();
   jt_load_ru(v, sc, t);
   hook();
-  jt_level(B);
+  jb_level(B);
   jt_fwd_stage<2, 2, 2>(v, B, w.b, q);
   jt_fwd_stage<1, 1, 4>(v, B, w.c, q);
 }

@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(BLOCK, CTAS)
     const uint32_t sc[3] = {xb, xb + 4 * N, xb + 8 * N};
     jntt_fwd<3, JB_CANON>(v, sc, sfwd_tw(C), q, x, 1 + g);
     // |v| < 6.5 q: products below 42.3 q^2, reduced below 3.7 q and made positive
+    static_assert(JFWD_OUT * JFWD_OUT <= 3 * 16 * 64 * 64, "q < 2^28: reduced products above -3 q");
 #pragma unroll
     for (int part = 0; part < 2; part++)
 #pragma unroll
