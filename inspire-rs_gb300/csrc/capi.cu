@@ -764,8 +764,6 @@ int inspire_ctx_create(const inspire_params* prm, int device, int mode, inspire_
     const uint64_t nm = (uint64_t)((u128)ninv * r32 % qm);
     C.ninv_mont = (uint32_t)nm;
     C.ninv_mont_p = shoup(nm, qm);
-    C.mont = (uint32_t)r32;
-    C.mont_p = shoup(r32, qm);
     const uint64_t w1 = t[2], w1i = t[2 * N + 2];  // psi^(+-brv(1))
     auto pair_of = [&](uint64_t a, uint64_t b) {
       const uint64_t w = (uint64_t)((u128)a * b % qm);

@@ -32,7 +32,6 @@ struct ResidueConsts {
   uint32_t r64, r64_p;               // 2^64 mod q: reference Montgomery factor
   uint32_t ref_inv_scale, ref_inv_scale_p;  // n^-1 * 2^-64 mod q
   uint32_t ninv_mont, ninv_mont_p;   // n^-1 * 2^32 mod q
-  uint32_t mont, mont_p;             // 2^32 mod q
   uint32_t e_scale, e_scale_p;       // gamma^-1 * n^-1 * 2^32 mod q (database contraction)
   uint32_t d2_nz2, d2_nz2_p;         // n z^-2 mod q  (third gadget digit's transform, z = 2^20)
   uint32_t d2_z2, d2_z2_p;           // z^-2 mod q

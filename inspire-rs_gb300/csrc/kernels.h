@@ -202,7 +202,8 @@ size_t nopacking_smem_bytes();
 cudaError_t launch_nopacking(const NoPackingArgs& a, bool seeded, cudaStream_t st);
 
 size_t respond_smem_bytes(int mode);
-// max_ctas > 0 caps the grid: each CTA then answers several queries in turn.
+// max_ctas > 0 caps the grid (seeded queries in device memory): each CTA then
+// answers several queries in turn.
 // Otherwise batches of at most pair_max queries run on the two-CTA cluster
 // kernel (respond_pair.cu), larger ones on the one-CTA kernel.
 cudaError_t launch_respond(const RespondArgs& a, bool seeded, cudaStream_t st, int max_ctas = 0, int pair_max = 0);

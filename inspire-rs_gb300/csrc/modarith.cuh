@@ -46,9 +46,4 @@ __device__ __forceinline__ uint32_t redc(uint64_t T, uint32_t q, uint32_t qinv) 
   return min(r, r - q);
 }
 
-// a * b * 2^-32 mod q (canonical)
-__device__ __forceinline__ uint32_t mont_mul(uint32_t a, uint32_t b, uint32_t q, uint32_t qinv) {
-  return redc((uint64_t)a * b, q, qinv);
-}
-
 }  // namespace ig

@@ -358,14 +358,14 @@ __global__ void __launch_bounds__(QT, 1) respond_kernel_alone(const __grid_const
   respond_one<MODE, true, QDB, true>(A, blockIdx.x);
 }
 
-// Capped grid (device-resident rows): CTA b answers queries b, b + gridDim.x,
-// ... in turn.
-template <int MODE, bool SEEDED>
+// Capped grid (seeded queries, device-resident rows): CTA b answers queries b,
+// b + gridDim.x, ... in turn.
+template <int MODE>
 __global__ void __launch_bounds__(QT, 2) respond_kernel_loop(const __grid_constant__ RespondArgs A) {
 #pragma unroll 1
   for (int qi = blockIdx.x; qi < A.nq; qi += gridDim.x) {
     if (qi != (int)blockIdx.x) __syncthreads();  // the previous query's shared memory is no longer read
-    respond_one<MODE, SEEDED, false, false>(A, qi);
+    respond_one<MODE, true, false, false>(A, qi);
   }
 }
 
@@ -377,23 +377,26 @@ size_t respond_smem_bytes(int mode) {
 
 template <int MODE, bool SEEDED, bool QDB>
 static cudaError_t set_smem_attr() {
-  cudaError_t e = cudaFuncSetAttribute(respond_kernel<MODE, SEEDED, QDB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)respond_smem_bytes(MODE));
-  if (e == cudaSuccess && !QDB)
-    e = cudaFuncSetAttribute(respond_kernel_loop<MODE, SEEDED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)respond_smem_bytes(MODE));
-  return e;
+  return cudaFuncSetAttribute(respond_kernel<MODE, SEEDED, QDB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)respond_smem_bytes(MODE));
+}
+template <int MODE>
+static cudaError_t set_loop_smem_attr() {
+  return cudaFuncSetAttribute(respond_kernel_loop<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)respond_smem_bytes(MODE));
 }
 
 // Launches issue no configuration call (so they can be captured in a CUDA
 // graph): the shared-memory attribute of every variant is set once per
 // device by prepare_respond_kernels.
 template <int MODE, bool SEEDED, bool QDB>
-static cudaError_t launch_one(const RespondArgs& a, int ctas, cudaStream_t st) {
-  if (!QDB && ctas < a.nq)
-    respond_kernel_loop<MODE, SEEDED><<<ctas, QT, respond_smem_bytes(MODE), st>>>(a);
-  else
-    respond_kernel<MODE, SEEDED, QDB><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
+static cudaError_t launch_one(const RespondArgs& a, cudaStream_t st) {
+  respond_kernel<MODE, SEEDED, QDB><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
+  return cudaGetLastError();
+}
+template <int MODE>
+static cudaError_t launch_loop(const RespondArgs& a, int ctas, cudaStream_t st) {
+  respond_kernel_loop<MODE><<<ctas, QT, respond_smem_bytes(MODE), st>>>(a);
   return cudaGetLastError();
 }
 
@@ -405,6 +408,7 @@ static cudaError_t set_alone_smem_attr() {
 
 cudaError_t prepare_respond_kernels() {
   const cudaError_t es[] = {
+      set_loop_smem_attr<MODE_COMPAT>(),             set_loop_smem_attr<MODE_CRT_FIXED>(),
       set_alone_smem_attr<MODE_COMPAT, false>(),     set_alone_smem_attr<MODE_COMPAT, true>(),
       set_alone_smem_attr<MODE_CRT_FIXED, false>(),  set_alone_smem_attr<MODE_CRT_FIXED, true>(),
       set_smem_attr<MODE_COMPAT, false, false>(),    set_smem_attr<MODE_COMPAT, true, false>(),
@@ -424,9 +428,9 @@ static cudaError_t launch_alone(const RespondArgs& a, cudaStream_t st) {
 }
 
 template <int MODE>
-static cudaError_t launch_mode(const RespondArgs& a, bool seeded, int ctas, cudaStream_t st) {
-  if (a.qdesc) return seeded ? launch_one<MODE, true, true>(a, ctas, st) : launch_one<MODE, false, true>(a, ctas, st);
-  return seeded ? launch_one<MODE, true, false>(a, ctas, st) : launch_one<MODE, false, false>(a, ctas, st);
+static cudaError_t launch_mode(const RespondArgs& a, bool seeded, cudaStream_t st) {
+  if (a.qdesc) return seeded ? launch_one<MODE, true, true>(a, st) : launch_one<MODE, false, true>(a, st);
+  return seeded ? launch_one<MODE, true, false>(a, st) : launch_one<MODE, false, false>(a, st);
 }
 
 cudaError_t launch_respond(const RespondArgs& a, bool seeded, cudaStream_t st, int max_ctas, int pair_max) {
@@ -434,9 +438,12 @@ cudaError_t launch_respond(const RespondArgs& a, bool seeded, cudaStream_t st, i
   if (max_ctas <= 0 && a.nq <= pair_max) return launch_respond_pair(a, seeded, st);
   if (max_ctas <= 0 && seeded && a.nq <= a.alone_max)
     return a.P.mode == MODE_COMPAT ? launch_alone<MODE_COMPAT>(a, st) : launch_alone<MODE_CRT_FIXED>(a, st);
-  const int ctas = (max_ctas > 0 && max_ctas < a.nq) ? max_ctas : a.nq;
-  return a.P.mode == MODE_COMPAT ? launch_mode<MODE_COMPAT>(a, seeded, ctas, st)
-                                 : launch_mode<MODE_CRT_FIXED>(a, seeded, ctas, st);
+  if (max_ctas > 0 && max_ctas < a.nq) {
+    if (!seeded || a.qdesc) return cudaErrorInvalidValue;
+    return a.P.mode == MODE_COMPAT ? launch_loop<MODE_COMPAT>(a, max_ctas, st)
+                                   : launch_loop<MODE_CRT_FIXED>(a, max_ctas, st);
+  }
+  return a.P.mode == MODE_COMPAT ? launch_mode<MODE_COMPAT>(a, seeded, st) : launch_mode<MODE_CRT_FIXED>(a, seeded, st);
 }
 
 }  // namespace ig
