@@ -162,7 +162,7 @@ struct inspire_ctx {
   std::vector<int32_t> h_status;
   ighost::HostPinned h_desc;    // descriptors of page-locked batch calls
   ighost::HostPinned h_qstatus; // status words of the batch calls, written by the kernel
-  ighost::HostPinned h_stage;   // small batches' inputs, gathered for one DMA each
+  ighost::HostPinned h_stage;   // small batches' rows, shards and seeds, read in place by the kernels
   ighost::HostPinned h_keys;    // client keys on their way to their table
   ighost::HostPinned h_out;     // responses of staged small batches, written by the kernel
   bool keys_in_flight = false;  // a launch on `stream` may still read h_keys

@@ -179,9 +179,8 @@ __global__ void __launch_bounds__(RBLOCK, 1) nopacking_kernel(const __grid_const
 // What bounds it: for rows and responses in host memory the link (measured 210
 // GB/s of reads and 200 GB/s of writes, 82 us for the 12.6 and 8.4 MB of 128
 // queries together: the kernel takes 93 us); the transforms and the expansion
-// alone take 36 us.  128 queries take 114 us per host call: 200 us through
-// device buffers (62 us of them a 768-thread kernel), 133 us with the rows
-// read where they are used.
+// alone take 36 us.  128 queries take 111 us per host call, 133 us with the rows
+// read where they are used, 200 us copied through device buffers.
 struct SumSmem {
   static constexpr int AH = 0;                   // [ELL][2][N] rows' a, coefficients; exchange buffers in turn
   static constexpr int XD = AH + ELL * 2 * N;    // [2 r][ELL][N] the digit sums' exchange buffers, then transforms

@@ -176,12 +176,9 @@ __device__ __forceinline__ void xpose_16(uint32_t* v, int y) {
 // Forward transform (Cooley-Tukey, decimation in time), coefficient layout in
 // ([0, 4q)), slot layout out ([0, 14q)).  `sc` is this group's scratch; `bar`
 // its barrier id.  SHFL: the second exchange by warp shuffles (xpose_16)
-// instead of shared memory and two barriers.  Measured on GB300 in one A/B
-// comparison: the batched transform 4 % faster, the Respond kernels
-// unchanged, the NoPacking and tree kernels 2-4 % slower (about their
-// run-to-run spread); those keep the shared-memory form.  The same 8-lane
-// shuffle transpose in the 256-thread inverse made the two-CTA Respond
-// kernel 15 % slower, so the inverse transforms keep shared memory.
+// instead of shared memory and two barriers, 4 % faster for transforms by
+// themselves; the kernel of the column ciphertexts (nopacking.cu), 2-4 % slower
+// with it, and the inverse transforms keep shared memory.
 template <bool SHFL = true>
 __device__ __forceinline__ void ntt_fwd(uint32_t v[16], uint32_t* sc, TwiddleRef tw, uint32_t q, int x, int bar) {
   const uint32_t q2 = 2 * q;

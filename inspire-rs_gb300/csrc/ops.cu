@@ -17,13 +17,13 @@ namespace {
 // What bounds it: the integer multiply-add pipe in the butterflies (300 M
 // transforms/s with everything in registers and shared memory) and the
 // instructions of the loads and stores beside them.  4096 polynomials forward
-// take 41 us (47 us with one polynomial per CTA, the scale as a multiply of
-// its own and each thread storing its 64 bytes of slots directly: quarter
-// full sectors, 10 us of the stores alone), inverse 41 us (47 us).  Fetching
-// the next polynomials while these are transformed (persistent CTAs, in
-// registers or by cp.async) took 44-47 us: it only adds instructions.
-// Up to as many polynomials as CTAs fit the chip (3 per SM), a CTA takes one:
-// 456 take 8.5 us, 10.3 two by two; 301 and fewer take 7 us either way.
+// take 41 us, inverse too; 47 us with one polynomial per CTA, a multiply of its
+// own for the scale and each thread's 64 bytes of slots stored directly (quarter
+// full sectors).  Fetching the next polynomials while these are transformed
+// (persistent CTAs, in registers or by cp.async) took 44-47 us: it only adds
+// instructions.  Up to as many polynomials as CTAs fit the chip (3 per SM), a
+// CTA takes one: 456 take 8.5 us, 10.3 two by two.  In a graph 301 take 4.6 us a
+// launch and one 2.75; a native loop of calls 6.2 and 4.1.
 constexpr int NTT_REF_K = 2, NTT_REF_CTAS = 3;
 template <int K, bool INVERSE>
 __global__ void __launch_bounds__(BLOCK, NTT_REF_CTAS) ntt_ref_kernel(const DevParams P, uint32_t* __restrict__ polys, int npolys) {
@@ -77,9 +77,9 @@ __global__ void __launch_bounds__(BLOCK, NTT_REF_CTAS) ntt_ref_kernel(const DevP
 // ct[p][2 (a,b)][2][N]; rgsw[p][2*ELL rows][2 (a,b)][2][N]; out[p][2][2][N].
 // One pair per CTA, one residue per group; the transforms of a digit and of
 // its row's two parts share their twiddles.  CTAS per SM: one, with the registers
-// of both, while there is an SM for each pair (152 products 31 us, 35 with two).  1024 products take 188 us (235 us
-// one transform after the other, four CTAs per SM); 40 transforms a product
-// are 137 us at the rate above.
+// of both, while there is an SM for each pair (152 products 31 us, 35 with two).
+// 1024 products take 187 us, 235 us one transform after the other with four CTAs
+// per SM; 40 transforms a product are 137 us at the rate above.
 constexpr int EXT_WORDS = 2 * ELL * N + 6 * N;  // digits, three exchange buffers per group
 template <int CTAS>
 __global__ void __launch_bounds__(BLOCK, CTAS)

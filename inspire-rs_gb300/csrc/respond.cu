@@ -43,15 +43,12 @@
 //
 // What bounds it: the integer multiply-add pipe (64 lane-operations per
 // cycle and SM, a high or wide product costs two) is 73 % busy, 86 % in the
-// digit transforms; the rest waits on 16 warps' latencies.  One call of 2048
-// queries takes 1354 us (1507 us with unsigned butterflies and the step's
-// database and CRS words loaded where they are used); the six-group kernel
-// before it (768 threads, one CTA per SM, four CTA-wide barriers a step, its
-// 24 warps in step with one another, the b side in a launch of its own) took
-// 2290 us, and 174 against 117 us for 128 queries (fewer queries than SMs).
-// Two CTAs of different queries share the SM without waiting for each other,
-// and 128 registers a thread let each warp keep 16 independent butterflies in
-// flight.
+// digit transforms; the rest waits on 16 warps' latencies.  Two CTAs of different
+// queries share the SM without waiting for each other, and 128 registers a
+// thread let each warp keep 16 independent butterflies in flight.  One call of
+// 2048 queries takes 1355 us, 1507 us with unsigned butterflies and the step's
+// database and CRS words loaded where they are used, 2290 us with one CTA of 24
+// warps in step per SM.
 #include "ntt_joint.cuh"
 #include "respond_draws.cuh"
 
@@ -349,10 +346,9 @@ __global__ void __launch_bounds__(QT, 2) respond_kernel(const __grid_constant__ 
 }
 
 // One query per CTA and SM, for seeded batches of at most as many queries as SMs:
-// 128 queries take 116 us against 131 with 128 registers a thread (128 threads'
-// worth of them left idle, the step's words waited for quad by quad), 77 in
-// compat mode 115 against 129.  The same for 2048 queries takes 1570 us, 1356
-// with two CTAs per SM.
+// 128 queries take 117 us, 131 with 128 registers a thread (half the register
+// file idle, the step's words waited for quad by quad), 77 in compat mode 115
+// and 129.  The same for 2048 queries takes 1570 us, 1355 with two CTAs per SM.
 template <int MODE, bool QDB>
 __global__ void __launch_bounds__(QT, 1) respond_kernel_alone(const __grid_constant__ RespondArgs A) {
   respond_one<MODE, true, QDB, true>(A, blockIdx.x);

@@ -208,8 +208,7 @@ __device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows
 // from its buffer (QDB: from the staged chunks), and every column word once;
 // 32 sums (column, residue) per thread, exact in 64 bits (6144 products below
 // 2^48), are then transposed and added over the warp by shuffles, five
-// halving exchanges, and over the warps in shared memory.  Measured against
-// the separate launch it replaces: 14.3 us per 128 queries there.
+// halving exchanges, and over the warps in shared memory.
 // Returns -1, or (QDB) the chunk that did not arrive.
 template <bool QDB>
 __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __restrict__ H, const uint64_t* brows,

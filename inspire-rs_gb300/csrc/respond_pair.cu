@@ -23,12 +23,10 @@
 // of all threads (team 1's sum) and two that team 1 alone waits for (the
 // coefficients, R_i).
 //
-// What bounds it: latency; a CTA's 312 K warp instructions issue at 1.6 per cycle
-// and SM.  A batch of 8 takes 86.5 us; the kernel before it (768 threads per
-// CTA, every product's exchange through shared memory, three CTA-wide and one
-// cluster barrier a step) took 111 us, and this one with 256 threads per CTA
-// and 16 values a thread 111 us too (a lone warp issues an instruction every
-// seven cycles, so halving each thread's chain pays).
+// What bounds it: latency; a CTA's 316 K warp instructions issue at 1.7 per cycle
+// and SM.  A batch of 8 takes 86.5 us, 111 us with 256 threads per CTA and 16
+// values a thread (a lone warp issues an instruction every seven cycles, so
+// halving each thread's chain pays).
 #include "ntt_team.cuh"
 #include "respond_draws.cuh"
 

@@ -178,9 +178,9 @@ __global__ void __launch_bounds__(BLOCK) fold_third_digit_kernel(const DevParams
 // stored with slot h in row h + rot, where they look for it.  One CTA per triple
 // and residue, keys in device or page-locked host memory.  A single query's
 // Respond kernel, which needs the table only after the rows' expansion, starts
-// meanwhile.  Measured (one query with its keys, host call): 146 us -> 131 with
-// seeds and 155 -> 125 without, against an upload, a transform of single polys, a
-// fold in place and copies of the rows.
+// meanwhile.  Measured (one query with its keys, host call): 131 us with seeds and
+// 125 without; 146 and 155 with an upload, a transform of single polys, a fold in
+// place and copies of the rows.
 __global__ void __launch_bounds__(NTT_GT) client_keys_kernel(const DevParams P, const uint64_t* __restrict__ keys,
                                                              bool rotated, uint32_t* __restrict__ yhat) {
   __shared__ __align__(128) uint32_t X[ELL][N];

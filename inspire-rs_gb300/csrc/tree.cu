@@ -41,10 +41,9 @@
 // takes 7.4 k cycles of it per SM (6 transforms of 704, the products, the
 // digits) and 12.4 k in all, whether one CTA runs on an SM or two.  A batch of 33
 // takes 282 us per host call, 224 of them in tree_kernel (4191 key switches in
-// 3.5 chains per SM; the fullest SM has 1.4 times the average); it took 566 us
-// with the ciphertexts in coefficients, ten transforms per key switch by 768
-// threads, 48 digit transforms per residue and query for the columns and a launch
-// per level.  At 9 queries or fewer (one chain per SM) the call takes 125-133 us.
+// 3.5 chains per SM; the fullest SM has 1.4 times the average), 299 us with a
+// launch per level from the eighth on.  At 9 queries or fewer (one chain per SM)
+// the call takes 125-133 us.
 #include "ntt_joint.cuh"
 #include "respond_draws.cuh"
 
