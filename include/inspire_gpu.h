@@ -332,7 +332,8 @@ int inspire_respond_batch(inspire_ctx *ctx, const inspire_db *db, uint32_t n, co
  * gadget_len..2*gadget_len-1 ([n][gadget_len][32]) and b_rows only those rows
  * ([n][gadget_len][poly], 16-byte aligned); d_status[n] receives 0 or a
  * nonzero kernel status (unknown shard or client id, exhausted expansion
- * bound; its d_out_ct slot then holds no response).  One launch.
+ * bound, a wait that ran out; its d_out_ct slot then holds no response).  One
+ * launch.
  * No allocation and no configuration call: the call can be captured in a
  * CUDA graph. */
 int inspire_respond_seeded_batch_device(inspire_ctx *ctx, const inspire_db *db, uint32_t n,
