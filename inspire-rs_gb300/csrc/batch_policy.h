@@ -30,4 +30,14 @@ int alone_limit(int sm_count, bool captured, const LastBatch& last, uint64_t str
   return last.any && last.stream != stream && !ended() ? 0 : sm_count;
 }
 
+// Whether a host call's batch of more queries than SMs, whose rows are read and
+// responses written over the host link, takes an SM to each query with its whole
+// rows staged while they are expanded.  With two CTAs to an SM the rows come in
+// four chunks, three of them after the expansion; of few columns the steps that
+// follow are too short to cover that, and all of a wave's reads, then all its
+// writes, meet on the link.  So / two to an SM, us: 600 queries of 1, 2, 4 columns
+// 388 / 445, 392 / 449, 398 / 454; 200 of 4 columns 187 / 185; but 200 of 8
+// columns 232 / 212, 1200 of 16 1122 / 1004.
+inline bool whole_rows(int gamma, uint32_t n, int sm_count) { return gamma <= 4 && (int64_t)n > sm_count; }
+
 }  // namespace ighost

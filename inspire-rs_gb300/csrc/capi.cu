@@ -285,6 +285,7 @@ int run_batch_mapped(inspire_ctx* c, const inspire_db* db, uint32_t n, const uin
   a.stage_wait_iters = c->row_wait_iters;
   a.after_keys = new_keys;
   a.alone_max = alone_limit(c, c->stream);
+  a.whole_rows = a.alone_max > 0 && whole_rows(c->gamma, n, c->sm_count);
   CUDA_TRY(launch_respond(a, seeds != nullptr, c->stream, 0, c->pair_max.load()));
   CUDA_TRY(cudaStreamSynchronize(c->stream));
   c->keys_in_flight = false;

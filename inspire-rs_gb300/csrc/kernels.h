@@ -79,6 +79,9 @@ struct RespondArgs {
   // none, where other launches share the SMs) that are not for the two-CTA kernel
   // take the form of the one-CTA kernel that has an SM to itself
   int alone_max;
+  // Host only: seeded queries with descriptors, too many for the two-CTA kernel,
+  // take an SM each with their whole rows staged
+  bool whole_rows;
 };
 
 // NoPacking respond (respond.rs:71-115): per query the combined ciphertext

@@ -69,13 +69,15 @@ struct Smem {
   static constexpr int BAR = SEED + 24;        // the staged rows' mbarrier
   static constexpr int TOTAL = BAR + 8;
   // (the transforms' swizzled accesses XOR address bits 2-6)
-  static_assert(AH * 4 % 128 == 0 && XC * 4 % 128 == 0 && BAR % 2 == 0, "alignment of rows, buffers and mbarrier");
+  static_assert(AH * 4 % 128 == 0 && XC * 4 % 128 == 0 && BAR % 2 == 0 && TOTAL % 4 == 0,
+                "alignment of rows, buffers, mbarrier and whole staged rows");
 };
 
 // One query (index qi) by the whole CTA; every return is uniform over the CTA.
 // ALONE: the SM is this CTA's, with registers for all of a step's database and
-// CRS words at once.
-template <int MODE, bool SEEDED, bool QDB, bool ALONE>
+// CRS words at once.  WHOLE (QDB, ALONE): and with shared memory for the whole
+// rows, from Smem::TOTAL on.
+template <int MODE, bool SEEDED, bool QDB, bool ALONE, bool WHOLE = false>
 __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) {
   constexpr int NR = MODE == MODE_COMPAT ? 1 : 2;
   using L = Smem<NR>;
@@ -118,7 +120,7 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
   const uint32_t q = C.q, qinv = C.qinv, qo = P.r[r ^ 1].q;
   const uint64_t* brows = QDB ? D->brows : A.brows + (size_t)qi * ELL * 2 * N;
   uint64_t* rbar = reinterpret_cast<uint64_t*>(smem + L::BAR);
-  uint64_t* stage = reinterpret_cast<uint64_t*>(XC);
+  uint64_t* stage = reinterpret_cast<uint64_t*>(WHOLE ? smem + L::TOTAL : XC);
 
   if (tid == 0) {
     if (QDB) mbar_init(rbar);
@@ -137,7 +139,10 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
     // the seeds, inline in the query's descriptor
     if (SEEDED && tid < ELL * 32) reinterpret_cast<uint8_t*>(smem + L::SEED)[tid] = D->seeds[tid];
     __syncthreads();  // the mbarrier is initialised, the seeds staged
-    if (tid == 0) stage_chunk(stage, brows, 0, rbar);
+    if (tid == 0) {
+      if (WHOLE) stage_rows(stage, brows, rbar);
+      else stage_chunk(stage, brows, 0, rbar);
+    }
   }
 
   // ---- rows ELL..2ELL-1, coefficients, into AH [t][NR][N] ----
@@ -153,7 +158,8 @@ __device__ __forceinline__ void respond_one(const RespondArgs& A, const int qi) 
   }
 
   // ---- the b side ----
-  const int missing = column_b0<QDB>(P, H, brows, stage, rbar, A.stage_wait_iters, reinterpret_cast<uint64_t*>(XC), bpoly);
+  constexpr RowSource SRC = WHOLE ? ROWS_WHOLE : QDB ? ROWS_CHUNKS : ROWS_DIRECT;
+  const int missing = column_b0<SRC>(P, H, brows, stage, rbar, A.stage_wait_iters, reinterpret_cast<uint64_t*>(XC), bpoly);
   if (QDB && missing >= 0) {
     // The CTA must not exit while its bulk copies can still write into its
     // shared memory (the next CTA on this SM would own it): a second bounded
@@ -354,6 +360,13 @@ __global__ void __launch_bounds__(QT, 1) respond_kernel_alone(const __grid_const
   respond_one<MODE, true, QDB, true>(A, blockIdx.x);
 }
 
+// The same with the whole rows staged while they are expanded, for large batches
+// of few columns whose rows and responses cross the host link (batch_policy.h).
+template <int MODE>
+__global__ void __launch_bounds__(QT, 1) respond_kernel_whole(const __grid_constant__ RespondArgs A) {
+  respond_one<MODE, true, true, true, true>(A, blockIdx.x);
+}
+
 // Capped grid (seeded queries, device-resident rows): CTA b answers queries b,
 // b + gridDim.x, ... in turn.
 template <int MODE>
@@ -370,6 +383,7 @@ __global__ void __launch_bounds__(QT, 2) respond_kernel_loop(const __grid_consta
 size_t respond_smem_bytes(int mode) {
   return sizeof(uint32_t) * (mode == MODE_COMPAT ? Smem<1>::TOTAL : Smem<2>::TOTAL);
 }
+static size_t whole_smem_bytes(int mode) { return respond_smem_bytes(mode) + sizeof(uint64_t) * 2 * ELL * N; }
 
 template <int MODE, bool SEEDED, bool QDB>
 static cudaError_t set_smem_attr() {
@@ -385,6 +399,11 @@ static cudaError_t set_loop_smem_attr() {
 // Launches issue no configuration call (so they can be captured in a CUDA
 // graph): the shared-memory attribute of every variant is set once per
 // device by prepare_respond_kernels.
+template <int MODE>
+static cudaError_t launch_whole(const RespondArgs& a, cudaStream_t st) {
+  respond_kernel_whole<MODE><<<a.nq, QT, whole_smem_bytes(MODE), st>>>(a);
+  return cudaGetLastError();
+}
 template <int MODE, bool SEEDED, bool QDB>
 static cudaError_t launch_one(const RespondArgs& a, cudaStream_t st) {
   respond_kernel<MODE, SEEDED, QDB><<<a.nq, QT, respond_smem_bytes(MODE), st>>>(a);
@@ -396,6 +415,11 @@ static cudaError_t launch_loop(const RespondArgs& a, int ctas, cudaStream_t st) 
   return cudaGetLastError();
 }
 
+template <int MODE>
+static cudaError_t set_whole_smem_attr() {
+  return cudaFuncSetAttribute(respond_kernel_whole<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)whole_smem_bytes(MODE));
+}
 template <int MODE, bool QDB>
 static cudaError_t set_alone_smem_attr() {
   return cudaFuncSetAttribute(respond_kernel_alone<MODE, QDB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -404,6 +428,7 @@ static cudaError_t set_alone_smem_attr() {
 
 cudaError_t prepare_respond_kernels() {
   const cudaError_t es[] = {
+      set_whole_smem_attr<MODE_COMPAT>(),            set_whole_smem_attr<MODE_CRT_FIXED>(),
       set_loop_smem_attr<MODE_COMPAT>(),             set_loop_smem_attr<MODE_CRT_FIXED>(),
       set_alone_smem_attr<MODE_COMPAT, false>(),     set_alone_smem_attr<MODE_COMPAT, true>(),
       set_alone_smem_attr<MODE_CRT_FIXED, false>(),  set_alone_smem_attr<MODE_CRT_FIXED, true>(),
@@ -432,6 +457,8 @@ static cudaError_t launch_mode(const RespondArgs& a, bool seeded, cudaStream_t s
 cudaError_t launch_respond(const RespondArgs& a, bool seeded, cudaStream_t st, int max_ctas, int pair_max) {
   if (a.nq <= 0) return cudaSuccess;
   if (max_ctas <= 0 && a.nq <= pair_max) return launch_respond_pair(a, seeded, st);
+  if (a.whole_rows && max_ctas <= 0 && seeded && a.qdesc)
+    return a.P.mode == MODE_COMPAT ? launch_whole<MODE_COMPAT>(a, st) : launch_whole<MODE_CRT_FIXED>(a, st);
   if (max_ctas <= 0 && seeded && a.nq <= a.alone_max)
     return a.P.mode == MODE_COMPAT ? launch_alone<MODE_COMPAT>(a, st) : launch_alone<MODE_CRT_FIXED>(a, st);
   if (max_ctas > 0 && max_ctas < a.nq) {

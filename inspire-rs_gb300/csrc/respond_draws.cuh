@@ -200,17 +200,28 @@ __device__ __forceinline__ void stage_chunk(uint64_t* dst, const uint64_t* brows
   }
 }
 
+// Where a query's b rows come from: device (or mapped) memory, read where used;
+// staged chunks; or staged as a whole.
+enum RowSource { ROWS_DIRECT, ROWS_CHUNKS, ROWS_WHOLE };
+
+// The whole rows (96 KiB) on one mbarrier.
+__device__ __forceinline__ void stage_rows(uint64_t* dst, const uint64_t* brows, uint64_t* bar) {
+  mbar_expect_tx(bar, 2 * ELL * N * 8);
+#pragma unroll 1
+  for (int p = 0; p < 2 * ELL; p++) bulk_g2s(dst + p * N, brows + (size_t)p * N, N * 8, bar);
+}
+
 // The b side of the column products, coefficient 0 only (rlwe/enc.rs:195-208;
-// see respond.cu) by 256 threads (whole warps, barrier `named`; QDB: the whole
-// CTA): b0_c = -sum_i d_{c}[i] v[i] with v[0] = q - b[0], v[i] = b[N - i].
+// see respond.cu) by 256 threads (whole warps, barrier `named`; staged rows: the
+// whole CTA): b0_c = -sum_i d_{c}[i] v[i] with v[0] = q - b[0], v[i] = b[N - i].
 // Thread tid takes the coefficient pairs j = tid +
 // 256 m, m < 4, of every column, so each row word is read once, straight
-// from its buffer (QDB: from the staged chunks), and every column word once;
+// from its buffer (or where it is staged), and every column word once;
 // 32 sums (column, residue) per thread, exact in 64 bits (6144 products below
 // 2^48), are then transposed and added over the warp by shuffles, five
 // halving exchanges, and over the warps in shared memory.
-// Returns -1, or (QDB) the chunk that did not arrive.
-template <bool QDB>
+// Returns -1, or the chunk (0: the rows) that did not arrive.
+template <RowSource SRC>
 __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __restrict__ H, const uint64_t* brows,
                                           uint64_t* stage, uint64_t* bar, uint32_t wait_iters, uint64_t* red,
                                           uint32_t* bpoly, int named = 0) {
@@ -219,6 +230,10 @@ __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __r
   uint64_t acc[32];  // [column][residue]
 #pragma unroll
   for (int k = 0; k < 32; k++) acc[k] = 0;
+  if (SRC == ROWS_WHOLE) {
+    const bool arrived = mbar_wait(bar, 0, wait_iters);
+    if (__syncthreads_or(!arrived)) return 0;
+  }
 #pragma unroll 1
   for (int m = 0; m < 4; m++) {
     uint32_t hw[MAX_GAMMA];
@@ -226,7 +241,7 @@ __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __r
     for (int c = 0; c < MAX_GAMMA; c++) hw[c] = c < gamma ? __ldg(h2 + (size_t)c * (N / 2) + QT * m) : 0u;
     uint32_t bv[2][2 * ELL];
     const int i0 = 2 * (tid + QT * m);
-    if (QDB) {
+    if (SRC == ROWS_CHUNKS) {
       const bool arrived = mbar_wait(bar, m & 1, wait_iters);
       if (__syncthreads_or(!arrived)) return m;
       const uint32_t* s = reinterpret_cast<const uint32_t*>(stage);
@@ -244,12 +259,12 @@ __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __r
         }
       }
     } else {
-      const uint32_t* s = reinterpret_cast<const uint32_t*>(brows);
+      const uint32_t* s = reinterpret_cast<const uint32_t*>(SRC == ROWS_WHOLE ? stage : brows);
       const int k0 = i0 ? N - i0 : 0, k1 = N - i0 - 1;
 #pragma unroll
       for (int p = 0; p < 2 * ELL; p++) {
-        bv[0][p] = __ldg(s + 2 * (p * N + k0));
-        bv[1][p] = __ldg(s + 2 * (p * N + k1));
+        bv[0][p] = SRC == ROWS_WHOLE ? s[2 * (p * N + k0)] : __ldg(s + 2 * (p * N + k0));
+        bv[1][p] = SRC == ROWS_WHOLE ? s[2 * (p * N + k1)] : __ldg(s + 2 * (p * N + k1));
       }
     }
     if (i0 == 0) {
@@ -278,7 +293,7 @@ __device__ __forceinline__ int column_b0(const DevParams& P, const uint16_t* __r
       acc[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
     }
   }
-  if (QDB) named_sync(named, QT);  // the last chunk has been read
+  if (SRC == ROWS_CHUNKS) named_sync(named, QT);  // the last chunk has been read
   red[warp * 32 + lane] = acc[0];
   named_sync(named, QT);
   if (tid < 32) {

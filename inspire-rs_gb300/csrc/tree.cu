@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(QT, 2) tree_front_kernel(const __grid_constant
   if (shard >= (uint32_t)A.nshards) return;  // uniform over the CTA; tree_kernel reports it
   if (t == ELL) {
     if (tid < 16) W[WORK_ARRIVED + tid] = 0;
-    column_b0<false>(P, A.H + (size_t)shard * P.gamma * N, A.brows + (size_t)qi * A.brow_stride, nullptr, nullptr, 0,
+    column_b0<ROWS_DIRECT>(P, A.H + (size_t)shard * P.gamma * N, A.brows + (size_t)qi * A.brow_stride, nullptr, nullptr, 0,
                      reinterpret_cast<uint64_t*>(X), bp);
     if (tid < 32) W[WORK_BVALS + tid] = bp[tid];
     return;

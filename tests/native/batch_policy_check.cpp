@@ -28,6 +28,10 @@ int main() {
   CHECK(alone_limit(152, true, LastBatch{}, 7, ended) == 0 && asked == 2);
   CHECK(alone_limit(152, false, LastBatch{true, 0}, 8, runs) == 0);                // id 0 is an id like any other
 
+  // whole rows: few columns, more queries than SMs
+  CHECK(whole_rows(1, 153, 152) && whole_rows(4, 153, 152) && whole_rows(2, 0xFFFFFFFFu, 152));
+  CHECK(!whole_rows(1, 152, 152) && !whole_rows(8, 153, 152) && !whole_rows(16, 5000, 152));
+
   if (fails) return 1;
   std::printf("ok\n");
   return 0;
