@@ -476,6 +476,12 @@ int finish_status(inspire_ctx* c, uint32_t n, const char* what) {
   return INSPIRE_OK;
 }
 
+// NoPacking batches of at most this many queries in ordinary memory are gathered
+// into page-locked memory by the caller's thread; larger ones are copied to and
+// from the device, at several times one thread's rate.  Gathered / copied, us: 1
+// query 54 / 80, 4 76 / 91, 5 84 / 90, 6 92 / 91, 16 180 / 102, 64 611 / 146.
+constexpr uint32_t NOPACKING_GATHER_MAX = 5;
+
 int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* shard_ids, const uint8_t* seeds,
                   size_t seed_stride, const uint64_t* a_rows, const uint64_t* b_rows, size_t stride_polys,
                   uint64_t* out_ct, uint64_t* out_columns) {
@@ -495,7 +501,7 @@ int run_nopacking(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32
         rows_and_out_in_place(b_rows, rows_span, out_ct, out_span) ? mapped_range(b_rows, rows_span) : nullptr;
     const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
     const bool in_place = d_rows && d_outp;
-    if (in_place || n <= STAGE_PINNED_MAX) {
+    if (in_place || n <= NOPACKING_GATHER_MAX) {
       const size_t head = (size_t)n * (sizeof(uint32_t) + 32 * ELL);
       const size_t rows_at = (head + 255) & ~(size_t)255;
       CUDA_TRY(c->h_stage.ensure(rows_at + (in_place ? 0 : rows_b * n)));

@@ -13,7 +13,7 @@ ENTRY = 4
 DEFAULT = 1 << 20
 
 
-@pytest.mark.parametrize("n", [1, 64, 65, 160])  # from ordinary memory: gathered up to 64, staged on the device above
+@pytest.mark.parametrize("n", [1, 64, 65, 160])  # (in ordinary memory gathered or copied to the device)
 @pytest.mark.parametrize("kind", ["nopacking", "respond"])
 def test_row_wait_running_out(oracle_mod, kind, n):
     torch = pytest.importorskip("torch")
