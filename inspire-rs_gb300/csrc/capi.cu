@@ -244,6 +244,16 @@ int alone_limit(inspire_ctx* c, cudaStream_t st) {
 // Batches up to this size stage their inputs through page-locked memory.
 constexpr uint32_t STAGE_PINNED_MAX = 64;
 
+// Device addresses of page-locked rows and responses that the Respond kernels may
+// read and write in place (16-byte aligned, apart), or null.
+const uint8_t* map_in_place(const uint64_t* rows, size_t rows_bytes, uint64_t* out, size_t out_bytes, uint64_t** d_out) {
+  if (!rows_and_out_in_place(rows, rows_bytes, out, out_bytes) || !aligned(out, 16)) return nullptr;
+  const uint8_t* d_rows = mapped_range(rows, rows_bytes);
+  const uint8_t* o = d_rows ? mapped_range(out, out_bytes) : nullptr;
+  *d_out = const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(o));
+  return o ? d_rows : nullptr;
+}
+
 // Queries whose rows and responses are in page-locked host memory (device
 // addresses d_rows, row_bytes apart, and d_out; without seeds also d_arows,
 // [n][ELL][2][N]): the serving variant of the kernel reads each query's rows in
@@ -334,19 +344,14 @@ int run_batch(inspire_ctx* c, const inspire_db* db, uint32_t n, const uint32_t* 
   if (n == 0) return INSPIRE_OK;
   const size_t pw = poly_words();
   if (seeds) {
-    // page-locked rows and responses (16-byte aligned, apart): read and written
-    // in place
+    // page-locked rows and responses: read and written in place
     const size_t row_bytes = sizeof(uint64_t) * stride_polys * pw;
     const size_t rows_span = row_bytes * (n - 1) + sizeof(uint64_t) * ELL * pw;
-    const size_t out_span = sizeof(uint64_t) * n * 2 * pw;
-    const uint8_t* d_rows = rows_and_out_in_place(b_rows, rows_span, out_ct, out_span) && row_bytes % 16 == 0 &&
-                                    aligned(out_ct, 16)
-                                ? mapped_range(b_rows, rows_span)
-                                : nullptr;
-    const uint8_t* d_outp = d_rows ? mapped_range(out_ct, out_span) : nullptr;
-    if (d_rows && d_outp)
-      return run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride, nullptr, d_rows, row_bytes,
-                              const_cast<uint64_t*>(reinterpret_cast<const uint64_t*>(d_outp)), client_ids, false);
+    uint64_t* d_out = nullptr;
+    const uint8_t* d_rows = map_in_place(b_rows, rows_span, out_ct, sizeof(uint64_t) * n * 2 * pw, &d_out);
+    if (d_rows)
+      return run_batch_mapped(c, db, n, shard_ids, seeds, seed_stride, nullptr, d_rows, row_bytes, d_out, client_ids,
+                              false);
   }
   if (n <= STAGE_PINNED_MAX)
     return run_batch_gathered(c, db, n, shard_ids, seeds, seed_stride, a_rows, b_rows, stride_polys, 1, client_ids,
@@ -652,8 +657,13 @@ int single_query(inspire_ctx* c, const inspire_db* db, uint32_t shard_id, const 
   if (!seeds)  // 2*ELL rows of (a, b): row r's a is poly 2r, its b poly 2r+1
     return run_batch_gathered(c, db, 1, &shard_id, nullptr, 0, rgsw_full + 2 * ELL * pw, rgsw_full + (2 * ELL + 1) * pw,
                               4 * ELL, 2, &id, out_ct, c->gamma > 1);
-  return run_batch_gathered(c, db, 1, &shard_id, seeds + 32 * ELL, (size_t)64 * ELL, nullptr,
-                            b_rows + (size_t)ELL * pw, 2 * ELL, 1, &id, out_ct, c->gamma > 1);
+  const uint64_t* rows = b_rows + (size_t)ELL * pw;
+  uint64_t* d_out = nullptr;
+  const uint8_t* d_rows = map_in_place(rows, sizeof(uint64_t) * ELL * pw, out_ct, sizeof(uint64_t) * 2 * pw, &d_out);
+  if (d_rows)
+    return run_batch_mapped(c, db, 1, &shard_id, seeds + 32 * ELL, 0, nullptr, d_rows, 0, d_out, &id, c->gamma > 1);
+  return run_batch_gathered(c, db, 1, &shard_id, seeds + 32 * ELL, (size_t)64 * ELL, nullptr, rows, 2 * ELL, 1, &id,
+                            out_ct, c->gamma > 1);
 }
 
 }  // namespace
