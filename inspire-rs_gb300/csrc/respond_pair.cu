@@ -92,21 +92,13 @@ __device__ __forceinline__ bool mbar_wait_peer(uint64_t* bar, uint32_t parity, u
 // after them, which it has not armed, are one more phase each.  What came for
 // these before they are announced here counts towards whichever phase is
 // current, so the phases' order, not their split by step, is what is waited
-// for.  (test_wait: the bound is a bound in time, about 0.1 s.)
+// for.
 __device__ __noinline__ bool drain_peer(uint64_t* cbar, int late, int gamma) {
   for (int s = late; s >= 0 && s >= late - 1; s--) {
     uint64_t* bar = cbar + (s & 1);
     uint32_t phase = ((gamma - 2 - s) >> 1) & 1;
     for (int more = s >> 1;; more = 0, phase ^= 1) {
-      uint32_t done = 0;
-      for (uint32_t it = 0; !done && it < STAGE_DRAIN_ITERS; it++)
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n "
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(phase)
-            : "memory");
-      if (!done) return false;
+      if (!mbar_wait_peer(bar, phase, STAGE_WAIT_ITERS_DEFAULT)) return false;
       if (!more) break;
       mbar_expect_tx(bar, 4 * N * more);
     }
@@ -616,7 +608,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PT, 1)
 #pragma unroll
   for (int j = 0; j < 8; j++) out[team * 2 * N + t + TEAM * j] = f[j];
 
-  cluster_wait();
+  cluster_wait();  // (the peer sent its last coefficients most of a step before it arrived)
   if (r == 0 && tid == 0) {
     outcome = max(outcome, misc[6]);
     if (outcome) *status_ptr() = outcome;
